@@ -399,7 +399,7 @@ struct oxgb_md {
 	std::vector<float> dh2;               // bound of the Debye-Hueckel rows: (dh_rc + 2 skin + 1e-3)^2 on backbone sites
 	std::vector<int> nside, cell0;        // cells per side, first cell (cell0[n_systems] = all cells)
 	std::vector<int> chunk_sys, chunk_first, sys_chunk0;  // Bussi / energy chunks of <= 256 nucleotides
-	int n_chunks = 0, tab_span = 1;
+	int n_chunks = 0;
 
 	std::vector<int> h_n3, h_n5, h_btype, h_type;
 	bool have_topology = false, have_state = false;
@@ -581,8 +581,7 @@ static ForceArgs force_args(oxgb_md *h, int step_offset = 0, bool engine_step = 
 	a.forces = energy_buffers ? h->Fe : h->F;
 	a.torques = energy_buffers ? h->Te : h->T;
 	a.table = h->d_tab;
-	a.sys = h->d_sys;
-	a.tab_span = h->tab_span;
+	a.sys = h->n_systems > 1 ? h->d_sys : nullptr;
 	a.status = h->status;
 	a.esplit = h->esplit;
 	a.shape = h->shape;
@@ -833,8 +832,10 @@ extern "C" int oxgb_md_create(int n_systems, const int *offsets, const double *b
 	}
 	h->n_chunks = (int) h->chunk_sys.size();
 	h->sys_chunk0[n_systems] = h->n_chunks;
-	for(int b = 0; b < N; b += 128) h->tab_span = std::max(h->tab_span, sys[std::min(N, b + 128) - 1] - sys[b] + 1);
-	if(set_forces_smem(h->dbl, tab * h->tab_span)) return bail(fail(OXGB_E_INVALID, "systems too small: one block would need the tables of " + std::to_string(h->tab_span) + " systems"));
+	int tab_span = 1;
+	for(int b = 0; b < N; b += 128) tab_span = std::max(tab_span, sys[std::min(N, b + 128) - 1] - sys[b] + 1);
+	// the double engine takes at most 78 systems in 128 consecutive nucleotides
+	if(h->dbl && tab_span > 78) return bail(fail(OXGB_E_INVALID, "systems too small: one block would need the tables of " + std::to_string(tab_span) + " systems"));
 	std::vector<unsigned long long> seeds(n_systems);
 	for(int k = 0; k < n_systems; k++) seeds[k] = h->md.seed + (unsigned long long) k;
 

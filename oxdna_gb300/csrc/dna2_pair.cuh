@@ -17,27 +17,99 @@
 
 namespace oxgb {
 
-// per-system parameter tables, filled on the host from the settings
+// What the settings decide, per system, filled on the host.  The model's own constants are not in
+// it: they are compile-time constants below, so that they reach the arithmetic as immediates.  (As
+// members of a table copied into shared memory by every block, they cost a shared-memory load each on
+// the critical path of a term, and a block its start-up copy and barrier: MD step of one 24-nt duplex
+// 37.6 -> 35.1 us, of 40,000 nt 79.0 -> 75.7 us, of 250,000 nt 130.3 -> 124.1 us.)
 template <typename R>
 struct DNA2Table {
 	R f1_eps[2][5][5], f1_shift[2][5][5];
-	R f1_a[2], f1_r0[2], f1_blow[2], f1_bhigh[2], f1_rlow[2], f1_rhigh[2], f1_rclow[2], f1_rchigh[2];
-	R f2_k[2], f2_r0[2], f2_rc[2], f2_blow[2], f2_bhigh[2], f2_rlow[2], f2_rhigh[2], f2_rclow[2], f2_rchigh[2];
-	R f4_a[13], f4_b[13], f4_t0[13], f4_ts[13], f4_tc[13];
-	R f4_sa, f4_sb;
-	// support of f4 type i in cos(theta), slightly widened: outside (f4_clo, f4_chi) the factor
-	// and its derivative are exactly zero, which a pair can be told from without an acos
-	R f4_clo[13], f4_chi[13];
-	R f5_a[4], f5_b[4], f5_xc[4], f5_xs[4];
 	R hb_multiplier;
 	R dh_prefactor, dh_rhigh, dh_rc, dh_b, dh_minus_kappa;
 	R mbf_fmax, mbf_finf, mbf_xmax, mbf_fene_xmax, mbf_long_xmax;
-	R fene_r0, rcut2;
+	R rcut2;
 	R box_hi, box_lo;  // box side as an unevaluated sum hi + lo (exact FP64 value)
 	R inv_box;         // about 1 / box_hi: picks the periodic image (an integer; see LoadMixed::sep)
-	R pos_base_over_stack;
 	int dh_half_charged_ends, use_mbf, pad0, pad1;
 };
+
+// The model's constants as functions of a set's index, which is a literal wherever they are used.
+// They are the float literals of dna2_model.h, exact in both arithmetic types.
+#define OXGB_MODEL_TABLE(name, n, values)        \
+	template <typename R>                        \
+	OXGB_HD R name(int i) {                      \
+		constexpr float t[n] = values;           \
+		return R(t[i]);                          \
+	}
+OXGB_MODEL_TABLE(f1_a, 2, OXM_F1_TABLE_A)
+OXGB_MODEL_TABLE(f1_r0, 2, OXM_F1_TABLE_R0)
+OXGB_MODEL_TABLE(f1_blow, 2, OXM_F1_TABLE_BLOW)
+OXGB_MODEL_TABLE(f1_bhigh, 2, OXM_F1_TABLE_BHIGH)
+OXGB_MODEL_TABLE(f1_rlow, 2, OXM_F1_TABLE_RLOW)
+OXGB_MODEL_TABLE(f1_rhigh, 2, OXM_F1_TABLE_RHIGH)
+OXGB_MODEL_TABLE(f1_rclow, 2, OXM_F1_TABLE_RCLOW)
+OXGB_MODEL_TABLE(f1_rchigh, 2, OXM_F1_TABLE_RCHIGH)
+OXGB_MODEL_TABLE(f2_k, 2, OXM_F2_TABLE_K)
+OXGB_MODEL_TABLE(f2_r0, 2, OXM_F2_TABLE_R0)
+OXGB_MODEL_TABLE(f2_rc, 2, OXM_F2_TABLE_RC)
+OXGB_MODEL_TABLE(f2_blow, 2, OXM_F2_TABLE_BLOW)
+OXGB_MODEL_TABLE(f2_bhigh, 2, OXM_F2_TABLE_BHIGH)
+OXGB_MODEL_TABLE(f2_rlow, 2, OXM_F2_TABLE_RLOW)
+OXGB_MODEL_TABLE(f2_rhigh, 2, OXM_F2_TABLE_RHIGH)
+OXGB_MODEL_TABLE(f2_rclow, 2, OXM_F2_TABLE_RCLOW)
+OXGB_MODEL_TABLE(f2_rchigh, 2, OXM_F2_TABLE_RCHIGH)
+OXGB_MODEL_TABLE(f4_a, OXM_N_F4, OXM_F4_TABLE_A)
+OXGB_MODEL_TABLE(f4_b, OXM_N_F4, OXM_F4_TABLE_B)
+OXGB_MODEL_TABLE(f4_t0, OXM_N_F4, OXM_F4_TABLE_T0)
+OXGB_MODEL_TABLE(f4_ts, OXM_N_F4, OXM_F4_TABLE_TS)
+OXGB_MODEL_TABLE(f4_tc, OXM_N_F4, OXM_F4_TABLE_TC)
+OXGB_MODEL_TABLE(f5_a, 4, OXM_F5_TABLE_A)
+OXGB_MODEL_TABLE(f5_b, 4, OXM_F5_TABLE_B)
+OXGB_MODEL_TABLE(f5_xc, 4, OXM_F5_TABLE_XC)
+OXGB_MODEL_TABLE(f5_xs, 4, OXM_F5_TABLE_XS)
+#undef OXGB_MODEL_TABLE
+
+// cos(x) for |x| <= 4 as its Taylor series, at compile time (terms to x^40 / 40!, below 1e-22)
+OXGB_HD constexpr double const_cos(double x) {
+	double sum = 1.0, term = 1.0;
+	for(int k = 1; k <= 20; k++) {
+		term *= -x * x / double((2 * k - 1) * (2 * k));
+		sum += term;
+	}
+	return sum;
+}
+
+// The support of f4 set i in cos(theta): |theta - t0| < tc, widened by 1e-5 in the cosine (far more
+// than the FP32 error of an angle), open on a side that reaches 0 or pi.  Outside (f4_clo, f4_chi)
+// the factor and its derivative are exactly zero, which a pair can be told from without an angle.
+// Set 10's pure-harmonic coaxial theta1 term adds for theta >= sb, up to pi.
+struct F4Support {
+	double lo[OXM_N_F4], hi[OXM_N_F4];
+};
+OXGB_HD constexpr F4Support f4_support() {
+	constexpr float t0[OXM_N_F4] = OXM_F4_TABLE_T0, tc[OXM_N_F4] = OXM_F4_TABLE_TC;
+	F4Support s{};
+	for(int i = 0; i < OXM_N_F4; i++) {
+		const double a = (double) t0[i] - (double) tc[i], b = (double) t0[i] + (double) tc[i];
+		s.hi[i] = a <= 0.0 ? 2.0 : const_cos(a) + 1e-5;
+		s.lo[i] = b >= 3.141592653589793 ? -2.0 : const_cos(b) - 1e-5;
+	}
+	const double sb = const_cos((double) OXM_CXST_THETA1_SB) + 1e-5;
+	s.lo[OXM_F4_CX_T1] = -2.0;
+	if(s.hi[OXM_F4_CX_T1] < sb) s.hi[OXM_F4_CX_T1] = sb;
+	return s;
+}
+template <typename R>
+OXGB_HD R f4_clo(int i) {
+	constexpr F4Support s = f4_support();
+	return R(s.lo[i]);
+}
+template <typename R>
+OXGB_HD R f4_chi(int i) {
+	constexpr F4Support s = f4_support();
+	return R(s.hi[i]);
+}
 
 // one nucleotide: lab-frame axes and interaction-site offsets from its centre
 template <typename R>
@@ -51,10 +123,10 @@ struct Nuc {
 // stack * (POS_BASE / POS_STACK); the FP64 path keeps that, the FP32 path uses a1 * POS_BASE
 // (the same value with one rounding instead of two).
 template <typename R>
-OXGB_HD void make_sites(const DNA2Table<R> &P, Nuc<R> &n) {
+OXGB_HD void make_sites(Nuc<R> &n) {
 	n.back = n.a1 * R(OXM_POS_MM_BACK1) + n.a2 * R(OXM_POS_MM_BACK2);
 	n.stack = n.a1 * R(OXM_POS_STACK);
-	n.base = (sizeof(R) == 4) ? n.a1 * R(OXM_POS_BASE) : n.stack * P.pos_base_over_stack;
+	n.base = (sizeof(R) == 4) ? n.a1 * R(OXM_POS_BASE) : n.stack * R((double) OXM_POS_BASE / (double) OXM_POS_STACK);
 }
 
 // centre-centre separation of a pair as an unevaluated sum hi + lo: the FP32 path carries the
@@ -143,49 +215,49 @@ template <typename R>
 OXGB_HD void f1_both(const DNA2Table<R> &P, R r, int t, int i, int j, R &f, R &fd, R rl = R(0)) {
 	f = R(0);
 	fd = R(0);
-	if(r < P.f1_rchigh[t]) {
+	if(r < f1_rchigh<R>(t)) {
 		const R eps = P.f1_eps[t][i][j];
-		if(r > P.f1_rhigh[t]) {
-			const R d = rdiff(r, P.f1_rchigh[t], rl);
-			f = eps * P.f1_bhigh[t] * d * d;
-			fd = eps * (R(2) * P.f1_bhigh[t] * d);
+		if(r > f1_rhigh<R>(t)) {
+			const R d = rdiff(r, f1_rchigh<R>(t), rl);
+			f = eps * f1_bhigh<R>(t) * d * d;
+			fd = eps * (R(2) * f1_bhigh<R>(t) * d);
 		}
-		else if(r > P.f1_rlow[t]) {
+		else if(r > f1_rlow<R>(t)) {
 			// FP32: 1 - exp(-y) through expm1, exact near the well bottom where it cancels
-			const R y = -rdiff(r, P.f1_r0[t], rl) * P.f1_a[t];
+			const R y = -rdiff(r, f1_r0<R>(t), rl) * f1_a<R>(t);
 			const R x = m_exp(y);
 			const R tmp = (sizeof(R) == 4) ? -m_expm1(y) : R(1) - x;
 			f = eps * tmp * tmp - P.f1_shift[t][i][j];
-			fd = eps * (R(2) * tmp * x * P.f1_a[t]);
+			fd = eps * (R(2) * tmp * x * f1_a<R>(t));
 		}
-		else if(r > P.f1_rclow[t]) {
-			const R d = rdiff(r, P.f1_rclow[t], rl);
-			f = eps * P.f1_blow[t] * d * d;
-			fd = eps * (R(2) * P.f1_blow[t] * d);
+		else if(r > f1_rclow<R>(t)) {
+			const R d = rdiff(r, f1_rclow<R>(t), rl);
+			f = eps * f1_blow<R>(t) * d * d;
+			fd = eps * (R(2) * f1_blow<R>(t) * d);
 		}
 	}
 }
 
 // harmonic f2 and its derivative (DNAInteraction.cpp:1278-1310); rl: see rdiff
 template <typename R>
-OXGB_HD void f2_both(const DNA2Table<R> &P, R r, int t, R &f, R &fd, R rl = R(0)) {
+OXGB_HD void f2_both(R r, int t, R &f, R &fd, R rl = R(0)) {
 	f = R(0);
 	fd = R(0);
-	if(r < P.f2_rchigh[t]) {
-		if(r > P.f2_rhigh[t]) {
-			const R d = rdiff(r, P.f2_rchigh[t], rl);
-			f = P.f2_k[t] * P.f2_bhigh[t] * d * d;
-			fd = R(2) * P.f2_k[t] * P.f2_bhigh[t] * d;
+	if(r < f2_rchigh<R>(t)) {
+		if(r > f2_rhigh<R>(t)) {
+			const R d = rdiff(r, f2_rchigh<R>(t), rl);
+			f = f2_k<R>(t) * f2_bhigh<R>(t) * d * d;
+			fd = R(2) * f2_k<R>(t) * f2_bhigh<R>(t) * d;
 		}
-		else if(r > P.f2_rlow[t]) {
-			const R d = rdiff(r, P.f2_r0[t], rl);
-			f = (P.f2_k[t] / R(2)) * (d * d - (P.f2_rc[t] - P.f2_r0[t]) * (P.f2_rc[t] - P.f2_r0[t]));
-			fd = P.f2_k[t] * d;
+		else if(r > f2_rlow<R>(t)) {
+			const R d = rdiff(r, f2_r0<R>(t), rl);
+			f = (f2_k<R>(t) / R(2)) * (d * d - (f2_rc<R>(t) - f2_r0<R>(t)) * (f2_rc<R>(t) - f2_r0<R>(t)));
+			fd = f2_k<R>(t) * d;
 		}
-		else if(r > P.f2_rclow[t]) {
-			const R d = rdiff(r, P.f2_rclow[t], rl);
-			f = P.f2_k[t] * P.f2_blow[t] * d * d;
-			fd = R(2) * P.f2_k[t] * P.f2_blow[t] * d;
+		else if(r > f2_rclow<R>(t)) {
+			const R d = rdiff(r, f2_rclow<R>(t), rl);
+			f = f2_k<R>(t) * f2_blow<R>(t) * d * d;
+			fd = R(2) * f2_k<R>(t) * f2_blow<R>(t) * d;
 		}
 	}
 }
@@ -207,7 +279,7 @@ OXGB_HD R sin_between(const v3<R> &a, const v3<R> &b) {
 // theta = 0.1, where several modulations peak (theta0 = 0), which alone made force errors of
 // 1e-5; atan2 of the cross product's norm is well conditioned at every angle.
 template <typename R>
-OXGB_HD void f4_both(const DNA2Table<R> &P, R c, R sn, int i, R &f, R &fd) {
+OXGB_HD void f4_both(R c, R sn, int i, R &f, R &fd) {
 	R t, s2, sint;
 	if(sizeof(R) == 4) {
 		t = m_atan2(sn, c);
@@ -222,27 +294,27 @@ OXGB_HD void f4_both(const DNA2Table<R> &P, R c, R sn, int i, R &f, R &fd) {
 	}
 	f = R(0);
 	R dsin = R(0);
-	R tt0 = t - P.f4_t0[i];
+	R tt0 = t - f4_t0<R>(i);
 	R m = R(1);
 	if(tt0 < R(0)) {
 		tt0 = -tt0;
 		m = R(-1);
 	}
-	if(tt0 < P.f4_tc[i]) {
-		if(tt0 > P.f4_ts[i]) {
-			f = P.f4_b[i] * (P.f4_tc[i] - tt0) * (P.f4_tc[i] - tt0);
-			dsin = m * R(2) * P.f4_b[i] * (tt0 - P.f4_tc[i]) / sint;
+	if(tt0 < f4_tc<R>(i)) {
+		if(tt0 > f4_ts<R>(i)) {
+			f = f4_b<R>(i) * (f4_tc<R>(i) - tt0) * (f4_tc<R>(i) - tt0);
+			dsin = m * R(2) * f4_b<R>(i) * (tt0 - f4_tc<R>(i)) / sint;
 		}
 		else {
-			f = R(1) - P.f4_a[i] * tt0 * tt0;
-			dsin = (s2 > R(1e-8)) ? -m * R(2) * P.f4_a[i] * tt0 / sint : -m * R(2) * P.f4_a[i];
+			f = R(1) - f4_a<R>(i) * tt0 * tt0;
+			dsin = (s2 > R(1e-8)) ? -m * R(2) * f4_a<R>(i) * tt0 / sint : -m * R(2) * f4_a<R>(i);
 		}
 	}
 	if(i == OXM_F4_CX_T1) {
-		const R h = t - P.f4_sb;
+		const R h = t - R(OXM_CXST_THETA1_SB);
 		if(h >= R(0)) {
-			f += P.f4_sa * h * h;
-			dsin += (s2 > R(1e-8)) ? R(2) * P.f4_sa * h / sint : R(2) * P.f4_sa;
+			f += R(OXM_CXST_THETA1_SA) * h * h;
+			dsin += (s2 > R(1e-8)) ? R(2) * R(OXM_CXST_THETA1_SA) * h / sint : R(2) * R(OXM_CXST_THETA1_SA);
 		}
 	}
 	fd = -dsin;
@@ -250,23 +322,23 @@ OXGB_HD void f4_both(const DNA2Table<R> &P, R c, R sn, int i, R &f, R &fd) {
 
 // f4 of type i can be non-zero at cos(theta) = c
 template <typename R>
-OXGB_HD bool f4_may(const DNA2Table<R> &P, R c, int i) {
-	return c > P.f4_clo[i] && c < P.f4_chi[i];
+OXGB_HD bool f4_may(R c, int i) {
+	return c > f4_clo<R>(i) && c < f4_chi<R>(i);
 }
 
 // f5 of cos(phi) and its derivative (DNAInteraction.cpp:1418-1450)
 template <typename R>
-OXGB_HD void f5_both(const DNA2Table<R> &P, R x, int t, R &f, R &fd) {
+OXGB_HD void f5_both(R x, int t, R &f, R &fd) {
 	f = R(0);
 	fd = R(0);
-	if(x > P.f5_xc[t]) {
-		if(x < P.f5_xs[t]) {
-			f = P.f5_b[t] * (P.f5_xc[t] - x) * (P.f5_xc[t] - x);
-			fd = R(2) * P.f5_b[t] * (x - P.f5_xc[t]);
+	if(x > f5_xc<R>(t)) {
+		if(x < f5_xs<R>(t)) {
+			f = f5_b<R>(t) * (f5_xc<R>(t) - x) * (f5_xc<R>(t) - x);
+			fd = R(2) * f5_b<R>(t) * (x - f5_xc<R>(t));
 		}
 		else if(x < R(0)) {
-			f = R(1) - P.f5_a[t] * x * x;
-			fd = R(-2) * P.f5_a[t] * x;
+			f = R(1) - f5_a<R>(t) * x * x;
+			fd = R(-2) * f5_a<R>(t) * x;
 		}
 		else f = R(1);
 	}
@@ -524,7 +596,7 @@ struct BaseGeo {
 };
 
 template <typename R>
-OXGB_HD BaseGeo<R> base_geo(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R> &q, const Sep<R> &sep) {
+OXGB_HD BaseGeo<R> base_geo(const Nuc<R> &p, const Nuc<R> &q, const Sep<R> &sep) {
 	BaseGeo<R> g;
 	g.hb = g.crst = false;
 	const v3<R> rhydro = site_vec(sep, q.base, p.base);
@@ -537,15 +609,15 @@ OXGB_HD BaseGeo<R> base_geo(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R>
 	g.rd = rhydro * (R(1) / g.rmod);
 	const v3<R> a1 = p.a1, a3 = p.a3, b1 = q.a1, b3 = q.a3;
 	g.c1 = -dot(a1, b1), g.c2 = -dot(b1, g.rd), g.c3 = dot(a1, g.rd), g.c4 = dot(a3, b3), g.c7 = -dot(b3, g.rd), g.c8 = dot(a3, g.rd);
-	g.hb = hb_range && R(OXM_HYDR_RCLOW) < g.rmod && g.rmod < R(OXM_HYDR_RCHIGH) && f4_may(P, g.c1, OXM_F4_HB_T1) &&
-			f4_may(P, g.c2, OXM_F4_HB_T2) && f4_may(P, g.c3, OXM_F4_HB_T2) && f4_may(P, g.c4, OXM_F4_HB_T4) &&
-			f4_may(P, g.c7, OXM_F4_HB_T7) && f4_may(P, g.c8, OXM_F4_HB_T7);
+	g.hb = hb_range && R(OXM_HYDR_RCLOW) < g.rmod && g.rmod < R(OXM_HYDR_RCHIGH) && f4_may(g.c1, OXM_F4_HB_T1) &&
+			f4_may(g.c2, OXM_F4_HB_T2) && f4_may(g.c3, OXM_F4_HB_T2) && f4_may(g.c4, OXM_F4_HB_T4) &&
+			f4_may(g.c7, OXM_F4_HB_T7) && f4_may(g.c8, OXM_F4_HB_T7);
 	// theta4, theta7, theta8 of cross stacking enter through f4(theta) + f4(pi - theta)
-	g.crst = cr_range && R(OXM_CRST_RCLOW) < g.rmod && g.rmod < R(OXM_CRST_RCHIGH) && f4_may(P, g.c1, OXM_F4_CR_T1) &&
-			f4_may(P, g.c2, OXM_F4_CR_T2) && f4_may(P, g.c3, OXM_F4_CR_T2) &&
-			(f4_may(P, g.c4, OXM_F4_CR_T4) || f4_may(P, -g.c4, OXM_F4_CR_T4)) &&
-			(f4_may(P, g.c7, OXM_F4_CR_T7) || f4_may(P, -g.c7, OXM_F4_CR_T7)) &&
-			(f4_may(P, g.c8, OXM_F4_CR_T7) || f4_may(P, -g.c8, OXM_F4_CR_T7));
+	g.crst = cr_range && R(OXM_CRST_RCLOW) < g.rmod && g.rmod < R(OXM_CRST_RCHIGH) && f4_may(g.c1, OXM_F4_CR_T1) &&
+			f4_may(g.c2, OXM_F4_CR_T2) && f4_may(g.c3, OXM_F4_CR_T2) &&
+			(f4_may(g.c4, OXM_F4_CR_T4) || f4_may(-g.c4, OXM_F4_CR_T4)) &&
+			(f4_may(g.c7, OXM_F4_CR_T7) || f4_may(-g.c7, OXM_F4_CR_T7)) &&
+			(f4_may(g.c8, OXM_F4_CR_T7) || f4_may(-g.c8, OXM_F4_CR_T7));
 	return g;
 }
 
@@ -562,12 +634,12 @@ OXGB_HD void hb_term(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R> &q, co
 	F1D *= hbm;
 	const R s1 = sin_between(a1, b1), s2 = sin_between(b1, rd), s3 = sin_between(a1, rd), s4 = sin_between(a3, b3),
 			s7 = sin_between(b3, rd), s8 = sin_between(a3, rd);
-	f4_both(P, g.c1, s1, OXM_F4_HB_T1, g1, d1);
-	f4_both(P, c2, s2, OXM_F4_HB_T2, g2, d2);
-	f4_both(P, c3, s3, OXM_F4_HB_T2, g3, d3);
-	f4_both(P, g.c4, s4, OXM_F4_HB_T4, g4, d4);
-	f4_both(P, c7, s7, OXM_F4_HB_T7, g7, d7);
-	f4_both(P, c8, s8, OXM_F4_HB_T7, g8, d8);
+	f4_both(g.c1, s1, OXM_F4_HB_T1, g1, d1);
+	f4_both(c2, s2, OXM_F4_HB_T2, g2, d2);
+	f4_both(c3, s3, OXM_F4_HB_T2, g3, d3);
+	f4_both(g.c4, s4, OXM_F4_HB_T4, g4, d4);
+	f4_both(c7, s7, OXM_F4_HB_T7, g7, d7);
+	f4_both(c8, s8, OXM_F4_HB_T7, g8, d8);
 	d3 = -d3;
 	d4 = -d4;
 	d8 = -d8;
@@ -591,23 +663,23 @@ OXGB_HD void hb_term(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R> &q, co
 
 // cross stacking of a pair whose geometry admits it (g.crst)
 template <typename R, bool SPLIT>
-OXGB_HD void crst_term(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R> &q, const BaseGeo<R> &g, PairOut<R> &o,
+OXGB_HD void crst_term(const Nuc<R> &p, const Nuc<R> &q, const BaseGeo<R> &g, PairOut<R> &o,
 		R rl = R(0)) {
 	const v3<R> a1 = p.a1, a3 = p.a3, b1 = q.a1, b3 = q.a3, rd = g.rd;
 	const R rmod = g.rmod, c2 = g.c2, c3 = g.c3, c4 = g.c4, c7 = g.c7, c8 = g.c8;
 	R F2, F2D, g1, d1, g2, d2, g3, d3, g4a, d4a, g4b, d4b, g7a, d7a, g7b, d7b, g8a, d8a, g8b, d8b;
-	f2_both(P, rmod, OXM_F2_CRST, F2, F2D, rl);
+	f2_both(rmod, OXM_F2_CRST, F2, F2D, rl);
 	const R s1 = sin_between(a1, b1), s2 = sin_between(b1, rd), s3 = sin_between(a1, rd), s4 = sin_between(a3, b3),
 			s7 = sin_between(b3, rd), s8 = sin_between(a3, rd);
-	f4_both(P, g.c1, s1, OXM_F4_CR_T1, g1, d1);
-	f4_both(P, c2, s2, OXM_F4_CR_T2, g2, d2);
-	f4_both(P, c3, s3, OXM_F4_CR_T2, g3, d3);
-	f4_both(P, c4, s4, OXM_F4_CR_T4, g4a, d4a);
-	f4_both(P, -c4, s4, OXM_F4_CR_T4, g4b, d4b);
-	f4_both(P, c7, s7, OXM_F4_CR_T7, g7a, d7a);
-	f4_both(P, -c7, s7, OXM_F4_CR_T7, g7b, d7b);
-	f4_both(P, c8, s8, OXM_F4_CR_T7, g8a, d8a);
-	f4_both(P, -c8, s8, OXM_F4_CR_T7, g8b, d8b);
+	f4_both(g.c1, s1, OXM_F4_CR_T1, g1, d1);
+	f4_both(c2, s2, OXM_F4_CR_T2, g2, d2);
+	f4_both(c3, s3, OXM_F4_CR_T2, g3, d3);
+	f4_both(c4, s4, OXM_F4_CR_T4, g4a, d4a);
+	f4_both(-c4, s4, OXM_F4_CR_T4, g4b, d4b);
+	f4_both(c7, s7, OXM_F4_CR_T7, g7a, d7a);
+	f4_both(-c7, s7, OXM_F4_CR_T7, g7b, d7b);
+	f4_both(c8, s8, OXM_F4_CR_T7, g8a, d8a);
+	f4_both(-c8, s8, OXM_F4_CR_T7, g8b, d8b);
 	const R g4 = g4a + g4b, g7 = g7a + g7b, g8 = g8a + g8b;
 	d3 = -d3;
 	const R d4 = -d4a + d4b, d7 = d7a - d7b, d8 = -d8a + d8b;
@@ -640,9 +712,9 @@ OXGB_HD float site_dist_remainder(const Sep<float> &sep, const Nuc<float> &p, co
 // hydrogen bonding and cross stacking, both on the base-base vector (DNAInteraction.cpp:779-1021)
 template <typename R, bool SPLIT>
 OXGB_HD void pair_base(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R> &q, const Sep<R> &sep, PairOut<R> &o) {
-	const BaseGeo<R> g = base_geo(P, p, q, sep);
+	const BaseGeo<R> g = base_geo(p, q, sep);
 	if(g.hb) hb_term<R, SPLIT>(P, p, q, g, o);
-	if(g.crst) crst_term<R, SPLIT>(P, p, q, g, o);
+	if(g.crst) crst_term<R, SPLIT>(p, q, g, o);
 }
 
 // The stacking-site vector of a pair and its cosines, with whether coaxial stacking can be
@@ -655,7 +727,7 @@ struct StackGeo {
 };
 
 template <typename R>
-OXGB_HD StackGeo<R> stack_geo(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R> &q, const Sep<R> &sep) {
+OXGB_HD StackGeo<R> stack_geo(const Nuc<R> &p, const Nuc<R> &q, const Sep<R> &sep) {
 	StackGeo<R> g;
 	g.cxst = false;
 	const v3<R> rstack = site_vec(sep, q.stack, p.stack);
@@ -665,29 +737,29 @@ OXGB_HD StackGeo<R> stack_geo(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<
 	if(!(R(OXM_CXST_RCLOW) < g.rmod && g.rmod < R(OXM_CXST_RCHIGH))) return g;
 	g.rd = rstack * (R(1) / g.rmod);
 	g.c1 = -dot(p.a1, q.a1), g.c4 = dot(p.a3, q.a3), g.c5 = dot(p.a3, g.rd), g.c6 = -dot(q.a3, g.rd);
-	g.cxst = f4_may(P, g.c1, OXM_F4_CX_T1) && f4_may(P, g.c4, OXM_F4_CX_T4) &&
-			(f4_may(P, g.c5, OXM_F4_CX_T5) || f4_may(P, -g.c5, OXM_F4_CX_T5)) &&
-			(f4_may(P, g.c6, OXM_F4_CX_T5) || f4_may(P, -g.c6, OXM_F4_CX_T5));
+	g.cxst = f4_may(g.c1, OXM_F4_CX_T1) && f4_may(g.c4, OXM_F4_CX_T4) &&
+			(f4_may(g.c5, OXM_F4_CX_T5) || f4_may(-g.c5, OXM_F4_CX_T5)) &&
+			(f4_may(g.c6, OXM_F4_CX_T5) || f4_may(-g.c6, OXM_F4_CX_T5));
 	return g;
 }
 
 // coaxial stacking, oxDNA2 form: no phi3 factor, pure-harmonic theta1 term
 // (DNA2Interaction.cpp:214-306), of a pair whose geometry admits it (g.cxst)
 template <typename R, bool SPLIT>
-OXGB_HD void cxst_term(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R> &q, const StackGeo<R> &g, PairOut<R> &o,
+OXGB_HD void cxst_term(const Nuc<R> &p, const Nuc<R> &q, const StackGeo<R> &g, PairOut<R> &o,
 		R rl = R(0)) {
 	const v3<R> a1 = p.a1, a3 = p.a3, b1 = q.a1, b3 = q.a3, rd = g.rd;
 	const R rmod = g.rmod, c5 = g.c5, c6 = g.c6;
 	R F2, F2D, g1, d1, g4, d4, g5a, d5a, g5b, d5b, g6a, d6a, g6b, d6b;
-	f2_both(P, rmod, OXM_F2_CXST, F2, F2D, rl);
+	f2_both(rmod, OXM_F2_CXST, F2, F2D, rl);
 	const R s1 = sin_between(p.a1, q.a1), s4 = sin_between(p.a3, q.a3), s5 = sin_between(p.a3, g.rd),
 			s6 = sin_between(q.a3, g.rd);
-	f4_both(P, g.c1, s1, OXM_F4_CX_T1, g1, d1);
-	f4_both(P, g.c4, s4, OXM_F4_CX_T4, g4, d4);
-	f4_both(P, c5, s5, OXM_F4_CX_T5, g5a, d5a);
-	f4_both(P, -c5, s5, OXM_F4_CX_T5, g5b, d5b);
-	f4_both(P, c6, s6, OXM_F4_CX_T5, g6a, d6a);
-	f4_both(P, -c6, s6, OXM_F4_CX_T5, g6b, d6b);
+	f4_both(g.c1, s1, OXM_F4_CX_T1, g1, d1);
+	f4_both(g.c4, s4, OXM_F4_CX_T4, g4, d4);
+	f4_both(c5, s5, OXM_F4_CX_T5, g5a, d5a);
+	f4_both(-c5, s5, OXM_F4_CX_T5, g5b, d5b);
+	f4_both(c6, s6, OXM_F4_CX_T5, g6a, d6a);
+	f4_both(-c6, s6, OXM_F4_CX_T5, g6b, d6b);
 	const R g5 = g5a + g5b, g6 = g6a + g6b;
 	d4 = -d4;
 	const R d5 = -d5a + d5b, d6 = d6a - d6b;
@@ -709,9 +781,9 @@ OXGB_HD void cxst_term(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R> &q, 
 
 // coaxial stacking of a pair
 template <typename R, bool SPLIT>
-OXGB_HD void pair_stack(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R> &q, const Sep<R> &sep, PairOut<R> &o) {
-	const StackGeo<R> g = stack_geo(P, p, q, sep);
-	if(g.cxst) cxst_term<R, SPLIT>(P, p, q, g, o);
+OXGB_HD void pair_stack(const Nuc<R> &p, const Nuc<R> &q, const Sep<R> &sep, PairOut<R> &o) {
+	const StackGeo<R> g = stack_geo(p, q, sep);
+	if(g.cxst) cxst_term<R, SPLIT>(p, q, g, o);
 }
 
 // Debye-Hueckel between backbone sites rback = back site of q - back site of p, halved charges at
@@ -761,7 +833,7 @@ OXGB_HD void nonbonded_p(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R> &q
 	if(dot(r, r) >= P.rcut2) return;
 	pair_ev<R, SPLIT>(p, q, sep, o);
 	pair_base<R, SPLIT>(P, p, q, sep, o);
-	pair_stack<R, SPLIT>(P, p, q, sep, o);
+	pair_stack<R, SPLIT>(p, q, sep, o);
 	pair_dh<R, SPLIT>(P, p, q, r, o);
 }
 
@@ -799,7 +871,7 @@ OXGB_HD bool bonded_both(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R> &q
 		const R rmod = m_sqrt(dot(rback, rback));
 		R rl = R(0);
 		if constexpr(X::on && sizeof(R) == 4) rl = dist_remainder(site_vec_lo(sep, q.back, lq.back, p.back, lp.back), rmod);
-		const R x = rdiff(rmod, P.fene_r0, rl);
+		const R x = rdiff(rmod, R(OXM_FENE_R0_OXDNA2), rl);
 		v3<R> force;
 		R e;
 		if(P.use_mbf && m_fabs(x) > P.mbf_xmax) {
@@ -861,11 +933,11 @@ OXGB_HD bool bonded_both(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R> &q
 		R F1, F1D, g4, d4, g5, d5, g6, d6, h1, h1d, h2, h2d;
 		f1_both(P, rsm, OXM_F1_ST, q.type, p.type, F1, F1D, rl);
 		const R s4 = sin_between(a3, b3), s5 = sin_between(a3, rd), s6 = sin_between(b3, rd);
-		f4_both(P, c4, s4, OXM_F4_ST_T4, g4, d4);
-		f4_both(P, -c5, s5, OXM_F4_ST_T5, g5, d5);
-		f4_both(P, c6, s6, OXM_F4_ST_T5, g6, d6);
-		f5_both(P, cp1, OXM_F5_PHI1, h1, h1d);
-		f5_both(P, cp2, OXM_F5_PHI2, h2, h2d);
+		f4_both(c4, s4, OXM_F4_ST_T4, g4, d4);
+		f4_both(-c5, s5, OXM_F4_ST_T5, g5, d5);
+		f4_both(c6, s6, OXM_F4_ST_T5, g6, d6);
+		f5_both(cp1, OXM_F5_PHI1, h1, h1d);
+		f5_both(cp2, OXM_F5_PHI2, h2, h2d);
 		d4 = -d4;
 		d5 = -d5;
 		d6 = -d6;

@@ -55,11 +55,11 @@ inline CF m_max(CF a, CF b) { return CF(std::fmax(a.v, b.v)); }
 
 using namespace oxgb;
 
-static void frame_of(const double *a1, const double *a3, int i, Nuc<CF> &n, const DNA2Table<CF> &P) {
+static void frame_of(const double *a1, const double *a3, int i, Nuc<CF> &n) {
 	n.a1 = v3<CF>{CF(a1[3 * i]), CF(a1[3 * i + 1]), CF(a1[3 * i + 2])};
 	n.a3 = v3<CF>{CF(a3[3 * i]), CF(a3[3 * i + 1]), CF(a3[3 * i + 2])};
 	n.a2 = cross(n.a3, n.a1);
-	make_sites(P, n);
+	make_sites(n);
 }
 
 extern "C" int oxgb_count_flops(int N, const double *pos, const double *a1, const double *a3, const int *n3, const int *n5,
@@ -91,7 +91,7 @@ extern "C" int oxgb_count_flops(int N, const double *pos, const double *a1, cons
 	};
 	double pairs = 0, in_range = 0;
 	auto load = [&](int j, Nuc<CF> &q) {
-		frame_of(a1, a3, j, q, P);
+		frame_of(a1, a3, j, q);
 		q.type = type[j];
 		q.btype = btype[j];
 		q.is_end = n3[j] < 0 || n5[j] < 0;
@@ -148,7 +148,7 @@ extern "C" int oxgb_count_flops(int N, const double *pos, const double *a1, cons
 					ss += (d[c] + 0.34 * da) * (d[c] + 0.34 * da);
 				}
 				if(bb < tr.base2) pair_base<CF, false>(P, p, q, sp, o);
-				if(ss < tr.stk2) pair_stack<CF, false>(P, p, q, sp, o);
+				if(ss < tr.stk2) pair_stack<CF, false>(p, q, sp, o);
 			}
 			if(r2 < tr.ev2) g_flops += 12;  // the partner's torque (rigid-rotation balance)
 			pairs += 1;

@@ -58,31 +58,12 @@ __device__ __forceinline__ int ref_type_of_btype(int bt) {
 	return (bt > 0) ? (bt & 3) : 3 - ((3 - bt) & 3);
 }
 
+// the settings table of system sy (read through L1: a handful of values per thread, the same for all
+// threads of a system)
 template <typename R>
-__device__ __forceinline__ void load_table(const DNA2Table<R> *g, DNA2Table<R> *s) {
-	const int n = sizeof(DNA2Table<R>) / sizeof(int);
-	const int *src = reinterpret_cast<const int *>(g);
-	int *dst = reinterpret_cast<int *>(s);
-	for(int k = threadIdx.x; k < n; k += blockDim.x) dst[k] = src[k];
-	__syncthreads();
+__device__ __forceinline__ const DNA2Table<R> &table_of(const ForceArgs &a, int sy) {
+	return reinterpret_cast<const DNA2Table<R> *>(a.table)[sy];
 }
-
-// The tables of the systems the nucleotides first .. last of this block belong to, copied into
-// dynamic shared memory (a plain run has one system); returns the first of those systems.
-// The host sizes the shared memory for the largest span of any block (ForceArgs::tab_span).
-template <typename R>
-__device__ __forceinline__ int load_table_span(const ForceArgs &a, int first, int last, DNA2Table<R> *s) {
-	const int s0 = a.sys ? a.sys[first] : 0;
-	const int s1 = a.sys ? a.sys[last] : 0;
-	const int n = (s1 - s0 + 1) * (int) (sizeof(DNA2Table<R>) / sizeof(int));
-	const int *src = reinterpret_cast<const int *>(reinterpret_cast<const DNA2Table<R> *>(a.table) + s0);
-	int *dst = reinterpret_cast<int *>(s);
-	for(int k = threadIdx.x; k < n; k += blockDim.x) dst[k] = src[k];
-	__syncthreads();
-	return s0;
-}
-
-extern __shared__ __align__(16) unsigned char g_tables_smem[];
 
 // ---------------------------------------------------------------- particle loaders
 
@@ -96,7 +77,7 @@ struct LoadMixed {
 		n.a1 = v3<float>{x1.x, x1.y, x1.z};
 		n.a3 = v3<float>{x3.x, x3.y, x3.z};
 		n.a2 = cross(n.a3, n.a1);
-		make_sites(P, n);
+		make_sites(n);
 		n.btype = __float_as_int(hi.w) >> 22;
 		n.type = __float_as_int(lo.w) & 7;
 		n.is_end = (b.x < 0 || b.y < 0);
@@ -161,7 +142,7 @@ struct LoadDouble {
 		ps = pos[i];
 		const double4_32a q = quat[i];
 		quat_frame(q.x, q.y, q.z, q.w, n.a1, n.a2, n.a3);
-		make_sites(P, n);
+		make_sites(n);
 		n.btype = __float_as_int(meta[i].w) >> 22;
 		n.type = __float_as_int(meta_lo[i].w) & 7;
 		n.is_end = (b.x < 0 || b.y < 0);
@@ -187,7 +168,7 @@ struct LoadRef {
 		lo = make_float4(0.f, 0.f, 0.f, 0.f);
 		const float4 q = quat[i];
 		quat_frame(q.x, q.y, q.z, q.w, n.a1, n.a2, n.a3);
-		make_sites(P, n);
+		make_sites(n);
 		n.btype = __float_as_int(hi.w) >> 22;
 		n.type = ref_type_of_btype(n.btype);
 		n.is_end = (b.x < 0 || b.y < 0);
@@ -220,8 +201,7 @@ struct Vec4Of<double> {
 template <typename R, class Loader, bool SPLIT, bool ACCUMULATE>
 __global__ void __launch_bounds__(128) k_forces(ForceArgs a, Loader ld) {
 	using V4 = typename Vec4Of<R>::T;
-	__shared__ DNA2Table<R> P;
-	load_table(reinterpret_cast<const DNA2Table<R> *>(a.table), &P);
+	const DNA2Table<R> &P = table_of<R>(a, 0);
 
 	const int lane = threadIdx.x & 31;
 	const int warps_per_block = blockDim.x >> 5;
@@ -358,8 +338,7 @@ cudaError_t launch_forces_reference_layout(const ForceArgs &a, cudaStream_t s) {
 template <int MODE>
 __global__ void k_order_params(const float4 *poss, const float4 *quat, const int *op1, const int *op2, int n,
 		const DNA2Table<float> *table, float *val, bool *flag) {
-	__shared__ DNA2Table<float> P;
-	load_table(table, &P);
+	const DNA2Table<float> &P = *table;
 	const int k = blockIdx.x * blockDim.x + threadIdx.x;
 	if(k >= n) return;
 	const LoadRef ld{poss, quat};
@@ -381,12 +360,12 @@ __global__ void k_order_params(const float4 *poss, const float4 *quat, const int
 		const v3<float> rd = rb * (1.f / rmod);
 		float f1, f1d, g[6], gd;
 		f1_both(P, rmod, OXM_F1_HB, p.type, q.type, f1, f1d);
-		f4_both(P, -dot(p.a1, q.a1), sin_between(p.a1, q.a1), OXM_F4_HB_T1, g[0], gd);
-		f4_both(P, -dot(q.a1, rd), sin_between(q.a1, rd), OXM_F4_HB_T2, g[1], gd);
-		f4_both(P, dot(p.a1, rd), sin_between(p.a1, rd), OXM_F4_HB_T2, g[2], gd);
-		f4_both(P, dot(p.a3, q.a3), sin_between(p.a3, q.a3), OXM_F4_HB_T4, g[3], gd);
-		f4_both(P, -dot(rd, q.a3), sin_between(q.a3, rd), OXM_F4_HB_T7, g[4], gd);
-		f4_both(P, dot(rd, p.a3), sin_between(p.a3, rd), OXM_F4_HB_T7, g[5], gd);
+		f4_both(-dot(p.a1, q.a1), sin_between(p.a1, q.a1), OXM_F4_HB_T1, g[0], gd);
+		f4_both(-dot(q.a1, rd), sin_between(q.a1, rd), OXM_F4_HB_T2, g[1], gd);
+		f4_both(dot(p.a1, rd), sin_between(p.a1, rd), OXM_F4_HB_T2, g[2], gd);
+		f4_both(dot(p.a3, q.a3), sin_between(p.a3, q.a3), OXM_F4_HB_T4, g[3], gd);
+		f4_both(-dot(rd, q.a3), sin_between(q.a3, rd), OXM_F4_HB_T7, g[4], gd);
+		f4_both(dot(rd, p.a3), sin_between(p.a3, rd), OXM_F4_HB_T7, g[5], gd);
 		e = f1;
 		int on = f1 < 0.f;
 #pragma unroll
@@ -560,8 +539,6 @@ template <typename R, class Loader, bool SPLIT, bool ENERGY>
 __device__ __forceinline__ void bonded_block(const ForceArgs &a, const Loader &ld, int b) {
 	using V4 = typename Vec4Of<R>::T;
 	const int first = b * blockDim.x;
-	DNA2Table<R> *Ps = reinterpret_cast<DNA2Table<R> *>(g_tables_smem);
-	const int s0 = load_table_span<R>(a, first, min(first + (int) blockDim.x, a.N) - 1, Ps);
 	// an MD step: from here on its second half kick is pending (the first step has read the mark)
 	if(a.th.open_step && b == 0 && threadIdx.x == 0) *a.th.open_step = *a.th.step_base + a.th.step_offset;
 	const int p = first + threadIdx.x;
@@ -569,7 +546,7 @@ __device__ __forceinline__ void bonded_block(const ForceArgs &a, const Loader &l
 		const int q = a.bonds[p].x;
 		if(q < 0) return;
 		const int sy = a.sys ? a.sys[p] : 0;
-		const DNA2Table<R> &P = Ps[sy - s0];
+		const DNA2Table<R> &P = table_of<R>(a, sy);
 		Nuc<R> np, nq;
 		V4 ph, pl, qh, ql;
 		load_full<Loader, R>(ld, p, P, np, ph, pl);
@@ -687,8 +664,7 @@ __device__ __forceinline__ void atomic_add_v4(double4_32a *p, const double4_32a 
 // its batch is evaluated (inlined copies may contract products into FMAs differently); the term
 // is evaluated only if this copy's own screening admits it.
 template <typename R, class Loader, bool SPLIT, bool ENERGY>
-__device__ __noinline__ void eval_terms(const ForceArgs &a, const Loader &ld, const DNA2Table<R> *Ps, int s0,
-		const int4 *t, int n, int term) {
+__device__ __noinline__ void eval_terms(const ForceArgs &a, const Loader &ld, const int4 *t, int n, int term) {
 	using V4 = typename Vec4Of<R>::T;
 	const int lane = threadIdx.x & 31;
 	if(lane >= n) return;
@@ -696,7 +672,7 @@ __device__ __noinline__ void eval_terms(const ForceArgs &a, const Loader &ld, co
 	const int i = it.x, j = it.y, k = it.z, m = it.w;
 	const long long N = a.N;
 	const int sy = a.sys ? a.sys[i] : 0;
-	const DNA2Table<R> &P = Ps[sy - s0];
+	const DNA2Table<R> &P = table_of<R>(a, sy);
 	Nuc<R> p, qn;
 	V4 ph, pl, qh, ql;
 	load_full<Loader, R>(ld, i, P, p, ph, pl);
@@ -706,21 +682,21 @@ __device__ __noinline__ void eval_terms(const ForceArgs &a, const Loader &ld, co
 	// FP32 engine path: the remainder of the site distance (the stiff radial factors, see rdiff)
 	const auto x = ld.refine(i, j);
 	if(term == 2) {
-		const StackGeo<R> g = stack_geo(P, p, qn, d);
+		const StackGeo<R> g = stack_geo(p, qn, d);
 		R rl = R(0);
 		if constexpr(decltype(x)::on) {
 			if(g.cxst) rl = site_dist_remainder(d, p, x.lo(0), qn, x.lo(1), true, g.rmod);
 		}
-		if(g.cxst) cxst_term<R, SPLIT>(P, p, qn, g, o, rl);
+		if(g.cxst) cxst_term<R, SPLIT>(p, qn, g, o, rl);
 	}
 	else {
-		const BaseGeo<R> g = base_geo(P, p, qn, d);
+		const BaseGeo<R> g = base_geo(p, qn, d);
 		R rl = R(0);
 		if constexpr(decltype(x)::on) {
 			if((term == 0 && g.hb) || (term == 1 && g.crst)) rl = site_dist_remainder(d, p, x.lo(0), qn, x.lo(1), false, g.rmod);
 		}
 		if(term == 0 && g.hb) hb_term<R, SPLIT>(P, p, qn, g, o, rl);
-		if(term == 1 && g.crst) crst_term<R, SPLIT>(P, p, qn, g, o, rl);
+		if(term == 1 && g.crst) crst_term<R, SPLIT>(p, qn, g, o, rl);
 	}
 	// the potential is invariant under rigid rotations, so the torques balance:
 	// T_j = -T_i + (r_j - r_i) x F_i, the cross product with error-free products
@@ -757,8 +733,6 @@ __device__ __forceinline__ void pair_block(const ForceArgs &a, const Loader &ld,
 	const bool is_base = b < base_blocks;
 	const int per_block = (blockDim.x / 32) * NPW;
 	const int first = (is_base ? b : b - base_blocks) * per_block;
-	DNA2Table<R> *Ps = reinterpret_cast<DNA2Table<R> *>(g_tables_smem);
-	const int s0 = load_table_span<R>(a, first, min(first + per_block, a.N) - 1, Ps);
 	const long long N = a.N;
 	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 	const int wbase = first + w * NPW;
@@ -814,19 +788,19 @@ __device__ __forceinline__ void pair_block(const ForceArgs &a, const Loader &ld,
 			const int j = nb[(long long) k * N + i];
 			const int m = (is_base ? a.base_pos : a.stk_pos)[(long long) k * N + i];
 			const int sy = a.sys ? a.sys[i] : 0;
-			const DNA2Table<R> &P = Ps[sy - s0];
+			const DNA2Table<R> &P = table_of<R>(a, sy);
 			Nuc<R> p, qn;
 			V4 ph, pl, qh, ql;
 			load_full<Loader, R>(ld, i, P, p, ph, pl);
 			load_full<Loader, R>(ld, j, P, qn, qh, ql);
 			const Sep<R> d = ld.sep(ph, pl, qh, ql, P);
 			if(is_base) {
-				const BaseGeo<R> g = base_geo(P, p, qn, d);
+				const BaseGeo<R> g = base_geo(p, qn, d);
 				live0 = g.hb;
 				live1 = g.crst;
 			}
 			else {
-				live0 = stack_geo(P, p, qn, d).cxst;
+				live0 = stack_geo(p, qn, d).cxst;
 			}
 			// both slots start from zero; the live terms add into them
 			V4 z;
@@ -847,17 +821,17 @@ __device__ __forceinline__ void pair_block(const ForceArgs &a, const Loader &ld,
 		__syncwarp();  // the queued items and the zeroed slots are visible to the whole warp
 		if(n0 >= 32) {
 			n0 -= 32;
-			eval_terms<R, Loader, SPLIT, ENERGY>(a, ld, Ps, s0, tq[w][0] + n0, 32, term0);
+			eval_terms<R, Loader, SPLIT, ENERGY>(a, ld, tq[w][0] + n0, 32, term0);
 			__syncwarp();
 		}
 		if(n1 >= 32) {
 			n1 -= 32;
-			eval_terms<R, Loader, SPLIT, ENERGY>(a, ld, Ps, s0, tq[w][1] + n1, 32, 1);
+			eval_terms<R, Loader, SPLIT, ENERGY>(a, ld, tq[w][1] + n1, 32, 1);
 			__syncwarp();
 		}
 	}
-	if(n0 > 0) eval_terms<R, Loader, SPLIT, ENERGY>(a, ld, Ps, s0, tq[w][0], n0, term0);
-	if(n1 > 0) eval_terms<R, Loader, SPLIT, ENERGY>(a, ld, Ps, s0, tq[w][1], n1, 1);
+	if(n0 > 0) eval_terms<R, Loader, SPLIT, ENERGY>(a, ld, tq[w][0], n0, term0);
+	if(n1 > 0) eval_terms<R, Loader, SPLIT, ENERGY>(a, ld, tq[w][1], n1, 1);
 }
 
 // minimum resident blocks per SM asked of the register allocator for the bonded/pair kernel
@@ -900,13 +874,11 @@ __device__ __forceinline__ void edge_block(const ForceArgs &a, const Loader &ld,
 	const int sub = threadIdx.x % K;
 	const int per_block = blockDim.x / K;
 	const int first = b * per_block;
-	DNA2Table<R> *Ps = reinterpret_cast<DNA2Table<R> *>(g_tables_smem);
-	const int s0 = load_table_span<R>(a, first, min(first + per_block, a.N) - 1, Ps);
 	const int i_raw = first + (int) threadIdx.x / K;
 	const bool live = i_raw < a.N;
 	const int i = live ? i_raw : a.N - 1;
 	const int sy = a.sys ? a.sys[i] : 0;
-	const DNA2Table<R> &P = Ps[sy - s0];
+	const DNA2Table<R> &P = table_of<R>(a, sy);
 	Nuc<R> p;
 	V4 ph, pl;
 	load_full<Loader, R>(ld, i, P, p, ph, pl);
@@ -1003,14 +975,11 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? MINB : 1) k_nonbonded_sp
 	// one nucleotide per group of K lanes: the grid covers every nucleotide (nonbonded_blocks);
 	// the lanes of a group past the last nucleotide still take part in the shuffles
 	const int i_raw = (blockIdx.x * blockDim.x + threadIdx.x) / K;
-	const int first = blockIdx.x * (blockDim.x / K);
-	DNA2Table<R> *Ps = reinterpret_cast<DNA2Table<R> *>(g_tables_smem);
-	const int s0 = load_table_span<R>(a, first, min(first + (int) (blockDim.x / K), a.N) - 1, Ps);
 	{
 		const bool live = i_raw < a.N;
 		const int i = live ? i_raw : a.N - 1;
 		const int sy = a.sys ? a.sys[i] : 0;
-		const DNA2Table<R> &P = Ps[sy - s0];
+		const DNA2Table<R> &P = table_of<R>(a, sy);
 		Nuc<R> p;
 		V4 ph, pl;
 		load_full<Loader, R>(ld, i, P, p, ph, pl);
@@ -1465,30 +1434,18 @@ template <typename R, class Loader, bool SPLIT, bool ENERGY, int NPW = OXGB_PAIR
 static void launch_split_t(const ForceArgs &a, Loader ld, cudaStream_t s, cudaEvent_t wait) {
 	const int tpb = 128;
 	const int blocks = a.N > 0 ? (a.N + tpb - 1) / tpb : 1;
-	const size_t smem = sizeof(DNA2Table<R>) * (size_t) (a.tab_span > 0 ? a.tab_span : 1);
 	// pair blocks of 4 warps x NPW nucleotides per term, then one bonded block per 128
 	// nucleotides, then (use_edge) one edge block per 128 / K nucleotides
 	const int pair_blocks = (a.N + 4 * NPW - 1) / (4 * NPW);
 	const int edge_blocks = EDGE ? nonbonded_blocks(a.N, K) : 0;
-	k_bonded_pairs<R, Loader, SPLIT, ENERGY, NPW, EDGE, K><<<2 * pair_blocks + blocks + edge_blocks, tpb, smem, s>>>(a, ld, pair_blocks);
+	k_bonded_pairs<R, Loader, SPLIT, ENERGY, NPW, EDGE, K><<<2 * pair_blocks + blocks + edge_blocks, tpb, 0, s>>>(a, ld, pair_blocks);
 	// the non-bonded kernel starts its Debye-Hueckel and excluded-volume work while the tail of
 	// the bonded and pair blocks runs; the external forces follow it the same way
 	if(wait) cudaStreamWaitEvent(s, wait, 0);
-	if(wait) k_nonbonded_split<R, Loader, SPLIT, ENERGY, K, NBMINB, EDGE><<<nonbonded_blocks(a.N, K), tpb, smem, s>>>(a, ld);
-	else launch_after(k_nonbonded_split<R, Loader, SPLIT, ENERGY, K, NBMINB, EDGE>, dim3(nonbonded_blocks(a.N, K)), dim3(tpb), smem,
+	if(wait) k_nonbonded_split<R, Loader, SPLIT, ENERGY, K, NBMINB, EDGE><<<nonbonded_blocks(a.N, K), tpb, 0, s>>>(a, ld);
+	else launch_after(k_nonbonded_split<R, Loader, SPLIT, ENERGY, K, NBMINB, EDGE>, dim3(nonbonded_blocks(a.N, K)), dim3(tpb), 0,
 			s, a, ld);
 	if(a.ext_n > 0) launch_after(k_external<typename Vec4Of<R>::T>, dim3((a.ext_n + tpb - 1) / tpb), dim3(tpb), 0, s, a);
-}
-
-template <typename R, class Loader, bool SPLIT, bool ENERGY, int NPW = OXGB_PAIR_NPW, int K = OXGB_NB_LANES,
-		int NBMINB = OXGB_NB_MINB, bool EDGE = false>
-static cudaError_t allow_smem_t(int bytes) {
-	cudaError_t e = cudaFuncSetAttribute(k_bonded_pairs<R, Loader, SPLIT, ENERGY, NPW, EDGE, K>,
-			cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-	if(e == cudaSuccess)
-		e = cudaFuncSetAttribute(k_nonbonded_split<R, Loader, SPLIT, ENERGY, K, NBMINB, EDGE>,
-				cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-	return e;
 }
 
 // the MD step's kernels (mixed / float engine) in shape k of FORCE_SHAPES
@@ -1496,36 +1453,6 @@ template <int k>
 static void launch_md_shape(const ForceArgs &a, const SplitMixed &ld, cudaStream_t s, cudaEvent_t wait) {
 	constexpr ForceShapeDef d = FORCE_SHAPES[k];
 	launch_split_t<float, SplitMixed, false, false, d.npw, d.lanes, d.minb>(a, ld, s, wait);
-}
-
-template <int k>
-static cudaError_t allow_smem_shape(int bytes) {
-	constexpr ForceShapeDef d = FORCE_SHAPES[k];
-	return allow_smem_t<float, SplitMixed, false, false, d.npw, d.lanes, d.minb>(bytes);
-}
-
-template <typename R, class Loader>
-static cudaError_t allow_smem(int bytes) {
-	cudaError_t e = allow_smem_t<R, Loader, true, true>(bytes);
-	if(e == cudaSuccess) e = allow_smem_t<R, Loader, false, true>(bytes);
-	if(e == cudaSuccess) e = allow_smem_t<R, Loader, false, false>(bytes);
-	if(e == cudaSuccess) e = allow_smem_t<R, Loader, true, true, OXGB_PAIR_NPW, OXGB_NB_LANES, OXGB_NB_MINB, true>(bytes);
-	if(e == cudaSuccess) e = allow_smem_t<R, Loader, false, true, OXGB_PAIR_NPW, OXGB_NB_LANES, OXGB_NB_MINB, true>(bytes);
-	if(e == cudaSuccess) e = allow_smem_t<R, Loader, false, false, OXGB_PAIR_NPW, OXGB_NB_LANES, OXGB_NB_MINB, true>(bytes);
-	if constexpr(sizeof(R) == 4) {
-		if(e == cudaSuccess) e = allow_smem_shape<1>(bytes);
-		if(e == cudaSuccess) e = allow_smem_shape<2>(bytes);
-		if(e == cudaSuccess) e = allow_smem_shape<3>(bytes);
-		if(e == cudaSuccess) e = allow_smem_shape<4>(bytes);
-		if(e == cudaSuccess) e = allow_smem_shape<5>(bytes);
-	}
-	return e;
-}
-
-int set_forces_smem(bool dbl, size_t bytes) {
-	if(bytes <= 48 * 1024) return 0;
-	if(bytes > 160 * 1024) return 1;
-	return (dbl ? allow_smem<double, SplitDouble>((int) bytes) : allow_smem<float, SplitMixed>((int) bytes)) != cudaSuccess;
 }
 
 // use_edge: the default shape with the edge blocks

@@ -100,7 +100,6 @@ struct ForceArgs {
 	void *forces, *torques;               // float4 or double4_32a per particle
 	const void *table;                    // DNA2Table<float> or DNA2Table<double>, one per system
 	const int *sys;                       // [N] system of each nucleotide (null: one system)
-	int tab_span;                         // most systems one block of the split kernels touches
 	int *status;
 	double *esplit;                       // [8 * n_systems] energies (split kernels only)
 	// split path (engine layout): backbone-site offsets (w = strand-end flag), term lists
@@ -157,9 +156,6 @@ int nonbonded_blocks(int N, int lanes);
 // shape k's nucleotides per pair-block warp queue, non-bonded lanes per nucleotide and register cap
 int force_shape_count();
 void force_shape_of(int k, int *npw, int *lanes, int *minb);
-// lets the split kernels use `bytes` of dynamic shared memory (per-block system tables);
-// nonzero if that is more than they may have
-int set_forces_smem(bool dbl, size_t bytes);
 
 struct ListArgs {
 	int N;

@@ -31,64 +31,9 @@ inline void default_settings(oxgb_dna2_settings *s, double T, double salt) {
 
 // returns 0, or -1 for invalid settings
 inline int build_table(const oxgb_dna2_settings &s, double box, DNA2Table<double> &P, double &rcut) {
-	static const float f1a[2] = OXM_F1_TABLE_A, f1rc[2] = OXM_F1_TABLE_RC, f1r0[2] = OXM_F1_TABLE_R0,
-			f1bl[2] = OXM_F1_TABLE_BLOW, f1bh[2] = OXM_F1_TABLE_BHIGH, f1rl[2] = OXM_F1_TABLE_RLOW,
-			f1rh[2] = OXM_F1_TABLE_RHIGH, f1rcl[2] = OXM_F1_TABLE_RCLOW, f1rch[2] = OXM_F1_TABLE_RCHIGH;
-	static const float f2k[2] = OXM_F2_TABLE_K, f2rc[2] = OXM_F2_TABLE_RC, f2r0[2] = OXM_F2_TABLE_R0,
-			f2bl[2] = OXM_F2_TABLE_BLOW, f2rl[2] = OXM_F2_TABLE_RLOW, f2rcl[2] = OXM_F2_TABLE_RCLOW,
-			f2bh[2] = OXM_F2_TABLE_BHIGH, f2rh[2] = OXM_F2_TABLE_RHIGH, f2rch[2] = OXM_F2_TABLE_RCHIGH;
-	static const float f4a[13] = OXM_F4_TABLE_A, f4b[13] = OXM_F4_TABLE_B, f4t0[13] = OXM_F4_TABLE_T0,
-			f4ts[13] = OXM_F4_TABLE_TS, f4tc[13] = OXM_F4_TABLE_TC;
-	static const float f5a[4] = OXM_F5_TABLE_A, f5b[4] = OXM_F5_TABLE_B, f5xc[4] = OXM_F5_TABLE_XC,
-			f5xs[4] = OXM_F5_TABLE_XS;
+	static const float f1a[2] = OXM_F1_TABLE_A, f1rc[2] = OXM_F1_TABLE_RC, f1r0[2] = OXM_F1_TABLE_R0;
 	if(!(s.T > 0) || !(s.salt > 0) || !(box > 0)) return -1;
 	std::memset(&P, 0, sizeof(P));
-	for(int t = 0; t < 2; t++) {
-		P.f1_a[t] = f1a[t];
-		P.f1_r0[t] = f1r0[t];
-		P.f1_blow[t] = f1bl[t];
-		P.f1_bhigh[t] = f1bh[t];
-		P.f1_rlow[t] = f1rl[t];
-		P.f1_rhigh[t] = f1rh[t];
-		P.f1_rclow[t] = f1rcl[t];
-		P.f1_rchigh[t] = f1rch[t];
-		P.f2_k[t] = f2k[t];
-		P.f2_r0[t] = f2r0[t];
-		P.f2_rc[t] = f2rc[t];
-		P.f2_blow[t] = f2bl[t];
-		P.f2_bhigh[t] = f2bh[t];
-		P.f2_rlow[t] = f2rl[t];
-		P.f2_rhigh[t] = f2rh[t];
-		P.f2_rclow[t] = f2rcl[t];
-		P.f2_rchigh[t] = f2rch[t];
-	}
-	for(int i = 0; i < OXM_N_F4; i++) {
-		P.f4_a[i] = f4a[i];
-		P.f4_b[i] = f4b[i];
-		P.f4_t0[i] = f4t0[i];
-		P.f4_ts[i] = f4ts[i];
-		P.f4_tc[i] = f4tc[i];
-	}
-	P.f4_sa = OXM_CXST_THETA1_SA;
-	P.f4_sb = OXM_CXST_THETA1_SB;
-	// support of each f4 in cos(theta): |theta - t0| < tc, widened by 1e-5 in the cosine (far
-	// more than the FP32 error of an acos); open on a side that reaches 0 or pi
-	const double pi = 3.141592653589793;
-	for(int i = 0; i < OXM_N_F4; i++) {
-		const double lo_t = (double) f4t0[i] - (double) f4tc[i], hi_t = (double) f4t0[i] + (double) f4tc[i];
-		P.f4_chi[i] = lo_t <= 0.0 ? 2.0 : std::cos(lo_t) + 1e-5;
-		P.f4_clo[i] = hi_t >= pi ? -2.0 : std::cos(hi_t) - 1e-5;
-	}
-	// the oxDNA2 pure-harmonic coaxial theta1 term adds for theta >= sb
-	P.f4_clo[OXM_F4_CX_T1] = -2.0;
-	P.f4_chi[OXM_F4_CX_T1] = std::fmax((double) P.f4_chi[OXM_F4_CX_T1], std::cos((double) OXM_CXST_THETA1_SB) + 1e-5);
-	for(int i = 0; i < 4; i++) {
-		P.f5_a[i] = f5a[i];
-		P.f5_b[i] = f5b[i];
-		P.f5_xc[i] = f5xc[i];
-		P.f5_xs[i] = f5xs[i];
-	}
-
 	const double T = s.T;
 	// exponent in float arithmetic on the float constants, exp in double
 	const double st_x = 1 - std::exp((double) (-(f1rc[1] - f1r0[1]) * f1a[1]));
@@ -126,7 +71,6 @@ inline int build_table(const oxgb_dna2_settings &s, double box, DNA2Table<double
 		}
 	}
 	P.hb_multiplier = s.hb_multiplier;
-	P.fene_r0 = OXM_FENE_R0_OXDNA2;
 
 	P.use_mbf = s.use_mbf ? 1 : 0;
 	if(s.use_mbf) {
@@ -159,7 +103,6 @@ inline int build_table(const oxgb_dna2_settings &s, double box, DNA2Table<double
 	P.box_hi = box;
 	P.box_lo = 0.0;
 	P.inv_box = 1.0 / box;
-	P.pos_base_over_stack = (double) OXM_POS_BASE / (double) OXM_POS_STACK;
 	return 0;
 }
 
