@@ -247,35 +247,32 @@ struct ListBuffers {
 
 // term lists of the engine's split force path (column-major, element k of i at [k * N + i])
 struct TermLists {
-	int N = 0, ev_cap = 0, base_cap = 0, stk_cap = 0;
-	int *ev_nb = nullptr, *ev_n = nullptr, *base_nb = nullptr, *base_n = nullptr, *stk_nb = nullptr, *stk_n = nullptr;
-	void *base_res = nullptr, *stk_res = nullptr;  // per-slot pair results, two 4-vectors of v4 bytes each
-	int *base_pos = nullptr, *stk_pos = nullptr;   // owned entries: the position in the partner's list
+	int N = 0, ev_cap = 0, pt_cap = 0;
+	int *ev_nb = nullptr, *ev_n = nullptr, *pt_nb = nullptr, *pt_n = nullptr, *own_n = nullptr;
+	int2 *own = nullptr;                  // owned pair-term entries (ForceArgs::own)
+	void *pt_res = nullptr;               // per-slot pair results, two 4-vectors of v4 bytes each
+	unsigned long long *pt_live = nullptr; // slots written since the last gather (zero between force launches)
 
-	int alloc(int N_, int ev, int base, int stk, size_t v4) {
+	int alloc(int N_, int ev, int pt, size_t v4, cudaStream_t s) {
 		free_all();
 		N = std::max(N_, 1);
 		ev_cap = ev;
-		base_cap = base;
-		stk_cap = stk;
+		pt_cap = pt;
+		const size_t words = (size_t) (pt_cap + 63) / 64;
 		CK(cudaMalloc(&ev_nb, sizeof(int) * (size_t) N * ev_cap));
-		CK(cudaMalloc(&base_nb, sizeof(int) * (size_t) N * base_cap));
-		CK(cudaMalloc(&stk_nb, sizeof(int) * (size_t) N * stk_cap));
+		CK(cudaMalloc(&pt_nb, sizeof(int) * (size_t) N * pt_cap));
+		CK(cudaMalloc(&own, sizeof(int2) * (size_t) (N + PAIR_GROUP) * pt_cap));
 		CK(cudaMalloc(&ev_n, sizeof(int) * N));
-		CK(cudaMalloc(&base_n, sizeof(int) * N));
-		CK(cudaMalloc(&stk_n, sizeof(int) * N));
-		CK(cudaMalloc(&base_res, 2 * v4 * (size_t) N * base_cap));
-		CK(cudaMalloc(&stk_res, 2 * v4 * (size_t) N * stk_cap));
-		CK(cudaMalloc(&base_pos, sizeof(int) * (size_t) N * base_cap));
-		CK(cudaMalloc(&stk_pos, sizeof(int) * (size_t) N * stk_cap));
+		CK(cudaMalloc(&pt_n, sizeof(int) * N));
+		CK(cudaMalloc(&own_n, sizeof(int) * N));
+		CK(cudaMalloc(&pt_res, 2 * v4 * (size_t) N * pt_cap));
+		CK(cudaMalloc(&pt_live, sizeof(unsigned long long) * words * N));
+		CK(cudaMemsetAsync(pt_live, 0, sizeof(unsigned long long) * words * N, s));
 		return OXGB_OK;
 	}
 	void free_all() {
-		for(int **p : {&ev_nb, &ev_n, &base_nb, &base_n, &stk_nb, &stk_n, &base_pos, &stk_pos}) {
-			if(*p) cudaFree(*p);
-			*p = nullptr;
-		}
-		for(void **p : {&base_res, &stk_res}) {
+		for(void **p : {(void **) &ev_nb, (void **) &ev_n, (void **) &pt_nb, (void **) &pt_n, (void **) &own_n, (void **) &own, &pt_res,
+					(void **) &pt_live}) {
 			if(*p) cudaFree(*p);
 			*p = nullptr;
 		}
@@ -592,21 +589,17 @@ static ForceArgs force_args(oxgb_md *h, int step_offset = 0, bool engine_step = 
 	a.fbacklo = h->fbacklo;
 	a.ev_nb = h->tl.ev_nb;
 	a.ev_n = h->tl.ev_n;
-	a.base_nb = h->tl.base_nb;
-	a.base_n = h->tl.base_n;
-	a.stk_nb = h->tl.stk_nb;
-	a.stk_n = h->tl.stk_n;
+	a.pt_nb = h->tl.pt_nb;
+	a.pt_n = h->tl.pt_n;
+	a.own = h->tl.own;
+	a.own_n = h->tl.own_n;
 	a.ev_cap = h->tl.ev_cap;
-	a.base_cap = h->tl.base_cap;
-	a.stk_cap = h->tl.stk_cap;
+	a.pt_cap = h->tl.pt_cap;
 	a.bond_f = h->bond_f;
 	a.bond_tp = h->bond_tp;
 	a.bond_tq = h->bond_tq;
-	a.base_res = h->tl.base_res;
-	a.stk_res = h->tl.stk_res;
-	a.base_pos = h->tl.base_pos;
-	a.stk_pos = h->tl.stk_pos;
-	a.term_max = h->term_max;
+	a.pt_res = h->tl.pt_res;
+	a.pt_live = h->tl.pt_live;
 	a.ext_rec = h->ext_rec;
 	a.ext_nuc = h->ext_nuc;
 	a.ext_off = h->ext_off;
@@ -941,7 +934,7 @@ extern "C" int oxgb_md_create(int n_systems, const int *offsets, const double *b
 	rc = h->lb.alloc(N, h->nside[0], cap, h->cell0[n_systems]);
 	if(rc) return bail(rc);
 	h->radii = term_radii(h->md.verlet_skin);
-	rc = h->tl.alloc(N, std::min(std::max(N - 1, 1), 128), std::min(std::max(N - 1, 1), 64), std::min(std::max(N - 1, 1), 64), v4);
+	rc = h->tl.alloc(N, std::min(std::max(N - 1, 1), 128), std::min(std::max(N - 1, 1), 128), v4, h->stream);
 	if(rc) return bail(rc);
 	for(int k = 0; k < n_systems; k++)
 		if((rc = reset_bussi(h, k))) return bail(rc);
@@ -1037,13 +1030,12 @@ static ListArgs md_list_args(oxgb_md *h, int check_flag) {
 	a.fback = h->fback;
 	a.ev_nb = h->tl.ev_nb;
 	a.ev_n = h->tl.ev_n;
-	a.base_nb = h->tl.base_nb;
-	a.base_n = h->tl.base_n;
-	a.stk_nb = h->tl.stk_nb;
-	a.stk_n = h->tl.stk_n;
+	a.pt_nb = h->tl.pt_nb;
+	a.pt_n = h->tl.pt_n;
+	a.own = h->tl.own;
+	a.own_n = h->tl.own_n;
 	a.ev_cap = h->tl.ev_cap;
-	a.base_cap = h->tl.base_cap;
-	a.stk_cap = h->tl.stk_cap;
+	a.pt_cap = h->tl.pt_cap;
 	a.ev_r2 = h->radii.ev2;
 	for(int k = 0; k < 3; k++) a.evs_r2[k] = h->radii.evs2[k];
 	a.base_r2 = h->radii.base2;
@@ -1051,8 +1043,6 @@ static ListArgs md_list_args(oxgb_md *h, int check_flag) {
 	a.list_a1 = h->list_a1;
 	a.list_back = h->list_back;
 	a.term_max = h->term_max;
-	a.base_pos = h->tl.base_pos;
-	a.stk_pos = h->tl.stk_pos;
 	a.list_kind = h->list_kind;
 	if(h->sorting()) {
 		a.sort_every = h->md.sort_every;
@@ -1256,15 +1246,15 @@ static int size_and_build_list(oxgb_md *h) {
 	const int mx = tm[3];
 	int want = ((std::max(64, mx + mx / 2 + 32) + 31) / 32) * 32;
 	auto cap_of = [](int m) { return ((std::max(16, m + m / 2 + 8) + 7) / 8) * 8; };
-	// base / stack rows at most 64 long (the pair kernel keeps a row's owned entries in a 64-bit
-	// mask; physically a nucleotide has a handful)
-	const int we = cap_of(tm[0]), wb = std::min(64, cap_of(tm[1])), ws = std::min(64, cap_of(tm[2]));
-	if(we != h->tl.ev_cap || wb != h->tl.base_cap || ws != h->tl.stk_cap) {
+	// pair-term rows at most 128 long (a slot number has 8 bits, 255 meaning none; physically a
+	// nucleotide has a handful)
+	const int we = cap_of(tm[0]), wp = std::min(128, cap_of(tm[1]));
+	if(we != h->tl.ev_cap || wp != h->tl.pt_cap) {
 		if(h->gexec) {
 			cudaGraphExecDestroy(h->gexec);
 			h->gexec = nullptr;
 		}
-		rc = h->tl.alloc(h->N, we, wb, ws, h->dbl ? sizeof(double4_32a) : sizeof(float4));
+		rc = h->tl.alloc(h->N, we, wp, h->dbl ? sizeof(double4_32a) : sizeof(float4), h->stream);
 		if(rc) return rc;
 		want = want > 0 ? want : h->lb.max_nb;
 		rc = h->lb.alloc(h->N, h->lb.n_side, want, h->cell0[h->n_systems]);

@@ -469,6 +469,17 @@ struct SplitMixed {
 		n.type = __float_as_int(l.w) & 7;
 		n.is_end = bk.w != 0.f;
 	}
+	// position, axes a1 and a3, base site and types: what the pair terms read
+	__device__ __forceinline__ void axes(int j, Nuc<float> &n, float4 &h, float4 &l) const {
+		h = __ldg(hi + j);
+		l = __ldg(lo + j);
+		const float4 x1 = __ldg(fa1 + j), x3 = __ldg(fa3 + j);
+		n.a1 = v3<float>{x1.x, x1.y, x1.z};
+		n.a3 = v3<float>{x3.x, x3.y, x3.z};
+		n.base = n.a1 * float(OXM_POS_BASE);
+		n.btype = __float_as_int(h.w) >> 22;
+		n.type = __float_as_int(l.w) & 7;
+	}
 	__device__ __forceinline__ void dh(int j, Nuc<float> &n, float4 &h, float4 &l) const {
 		h = __ldg(hi + j);
 		l = __ldg(lo + j);
@@ -533,38 +544,67 @@ __device__ __forceinline__ void load_dh<SplitMixed, float>(const SplitMixed &ld,
 	ld.dh(j, n, h, l);
 }
 
-// bonded block b: one bond (owner p, partner q = n3[p]) per thread; the bonded blocks cover
-// every nucleotide
+template <class Loader, typename R>
+__device__ __forceinline__ void load_axes(const Loader &ld, int j, const DNA2Table<R> &P, Nuc<R> &n, typename Vec4Of<R>::T &h,
+		typename Vec4Of<R>::T &l) {
+	load_full<Loader, R>(ld, j, P, n, h, l);
+}
+template <>
+__device__ __forceinline__ void load_axes<SplitMixed, float>(const SplitMixed &ld, int j, const DNA2Table<float> &, Nuc<float> &n,
+		float4 &h, float4 &l) {
+	ld.axes(j, n, h, l);
+}
+
+// Bonded block b: 64 bonds (owner p, partner q = n3[p]), a pair of threads each, in different warps:
+// the first half of the block evaluates the stacking, the second half FENE and the bonded excluded
+// volume, joined through shared memory.  One thread for all of a bond is a dependent chain twice as
+// long, and as long as that chain is what a launch lasts where the chip is not full.
+constexpr int BONDS_PER_BLOCK = 64;
+
 template <typename R, class Loader, bool SPLIT, bool ENERGY>
 __device__ __forceinline__ void bonded_block(const ForceArgs &a, const Loader &ld, int b) {
 	using V4 = typename Vec4Of<R>::T;
-	const int first = b * blockDim.x;
+	__shared__ R part[BONDS_PER_BLOCK][11];  // force, torques, energy of the backbone part (an odd number of words)
+	const int t = threadIdx.x & (BONDS_PER_BLOCK - 1);
+	const bool backbone = threadIdx.x >= BONDS_PER_BLOCK;  // warp-uniform
 	// an MD step: from here on its second half kick is pending (the first step has read the mark)
 	if(a.th.open_step && b == 0 && threadIdx.x == 0) *a.th.open_step = *a.th.step_base + a.th.step_offset;
-	const int p = first + threadIdx.x;
-	if(p < a.N) {
-		const int q = a.bonds[p].x;
-		if(q < 0) return;
+	const int p = b * BONDS_PER_BLOCK + t;
+	const int q = p < a.N ? a.bonds[p].x : -1;
+	BondOut<R> o;
+	o.f = o.tp = o.tq = v3<R>{R(0), R(0), R(0)};
+	if(q >= 0) {
 		const int sy = a.sys ? a.sys[p] : 0;
 		const DNA2Table<R> &P = table_of<R>(a, sy);
 		Nuc<R> np, nq;
 		V4 ph, pl, qh, ql;
 		load_full<Loader, R>(ld, p, P, np, ph, pl);
 		load_full<Loader, R>(ld, q, P, nq, qh, ql);
-		BondOut<R> b;
-		if(!bonded_both(P, np, nq, ld.diff(ph, pl, qh, ql), b, ld.refine(p, q))) atomicOr(a.status, OXGB_ERR_FENE);
+		if(backbone) {
+			if(!bonded_backbone(P, np, nq, ld.diff(ph, pl, qh, ql), o, ld.refine(p, q))) atomicOr(a.status, OXGB_ERR_FENE);
+			const R v[10] = {o.f.x, o.f.y, o.f.z, o.tp.x, o.tp.y, o.tp.z, o.tq.x, o.tq.y, o.tq.z, o.split[0] + o.split[1]};
+#pragma unroll
+			for(int k = 0; k < (ENERGY ? 10 : 9); k++) part[t][k] = v[k];
+			if(SPLIT) {
+				atomicAdd(a.esplit + 8 * sy + T_FENE, (double) o.split[0]);
+				atomicAdd(a.esplit + 8 * sy + T_BEXC, (double) o.split[1]);
+			}
+		}
+		else {
+			bonded_stacking(P, np, nq, ld.diff(ph, pl, qh, ql), o, ld.refine(p, q));
+			if(SPLIT) atomicAdd(a.esplit + 8 * sy + T_STCK, (double) o.split[2]);
+		}
+	}
+	__syncthreads();
+	if(q >= 0 && !backbone) {
+		const R *v = part[t];
 		V4 f, tp, tq;
-		f.x = b.f.x, f.y = b.f.y, f.z = b.f.z, f.w = ENERGY ? b.E : R(0);
-		tp.x = b.tp.x, tp.y = b.tp.y, tp.z = b.tp.z, tp.w = R(0);
-		tq.x = b.tq.x, tq.y = b.tq.y, tq.z = b.tq.z, tq.w = R(0);
+		f.x = v[0] + o.f.x, f.y = v[1] + o.f.y, f.z = v[2] + o.f.z, f.w = ENERGY ? v[9] + o.split[2] : R(0);
+		tp.x = v[3] + o.tp.x, tp.y = v[4] + o.tp.y, tp.z = v[5] + o.tp.z, tp.w = R(0);
+		tq.x = v[6] + o.tq.x, tq.y = v[7] + o.tq.y, tq.z = v[8] + o.tq.z, tq.w = R(0);
 		reinterpret_cast<V4 *>(a.bond_f)[p] = f;
 		reinterpret_cast<V4 *>(a.bond_tp)[p] = tp;
 		reinterpret_cast<V4 *>(a.bond_tq)[p] = tq;
-		if(SPLIT) {
-			atomicAdd(a.esplit + 8 * sy + T_FENE, (double) b.split[0]);
-			atomicAdd(a.esplit + 8 * sy + T_BEXC, (double) b.split[1]);
-			atomicAdd(a.esplit + 8 * sy + T_STCK, (double) b.split[2]);
-		}
 	}
 }
 
@@ -619,34 +659,7 @@ struct SplitAcc {
 			for(int k = 0; k < N_TERMS; k++) split[k] += o.split[k];
 		}
 	}
-	// entry k of nucleotide i's list: its result, written by the pair blocks of k_bonded_pairs
-	template <typename V4>
-	__device__ __forceinline__ void add_slot(const V4 *res, long long N, int i, int k) {
-		const long long s = (long long) k * N + i;
-		const V4 f = res[2 * s], t = res[2 * s + 1];
-		F.add(v3<R>{f.x, f.y, f.z});
-		T.add(v3<R>{t.x, t.y, t.z});
-		if(ENERGY) {
-			KahanV<R>::kadd(E, Ec, f.w);
-			KahanV<R>::kadd(Eh, Ehc, t.w);
-		}
-	}
 };
-
-// Base-base pairs (hydrogen bonding + cross stacking; blocks 0 .. base_blocks - 1) and
-// stack-stack pairs (coaxial stacking; the other blocks), each evaluated once, by its lower
-// nucleotide i (partner j above i by caller's index, at position k of i's list and m of j's): slot k of i gets
-// (force on i, E), (torque on i, E_hb) and slot m of j gets (-force, E), (torque on j, E_hb), at
-// [2 (k N + i) + 0..1] of base_res / stk_res.  Every slot of every list is written by its pair
-// alone.  These are the costliest terms and their lists are short, so the owned slots of a
-// warp's nucleotides are queued (a warp prefix sum over the per-lane counts) and dealt 32 at a
-// time: every lane works on a pair in every round but the last.
-// nucleotides per warp in a pair block: a full warp (32) fills each queue round with the most
-// pairs; measured against 16 it is faster by 1.0 us per force launch at 40k and 12.5 us on
-// the 250k melt (8 is slower still)
-#ifndef OXGB_PAIR_NPW
-#define OXGB_PAIR_NPW 32
-#endif
 
 __device__ __forceinline__ void atomic_add_v4(float4 *p, const float4 &v) { atomicAdd(p, v); }
 __device__ __forceinline__ void atomic_add_v4(double4_32a *p, const double4_32a &v) {
@@ -656,182 +669,351 @@ __device__ __forceinline__ void atomic_add_v4(double4_32a *p, const double4_32a 
 	atomicAdd(&p->w, v.w);
 }
 
-// one term (0 hydrogen bonding, 1 cross stacking, 2 coaxial stacking; warp-uniform) of the
-// queued pairs t[0 .. n - 1], lane l taking t[l]: the pair's result is added to its two slots
-// (zeroed when the pair was screened).  A slot receives at most two terms (hydrogen bonding and
-// cross stacking of one pair), whose sum does not depend on their order.  Not inlined: it is
-// called from several places, and one compiled copy gives a pair the same rounding wherever
-// its batch is evaluated (inlined copies may contract products into FMAs differently); the term
-// is evaluated only if this copy's own screening admits it.
-template <typename R, class Loader, bool SPLIT, bool ENERGY>
-__device__ __noinline__ void eval_terms(const ForceArgs &a, const Loader &ld, const int4 *t, int n, int term) {
-	using V4 = typename Vec4Of<R>::T;
-	const int lane = threadIdx.x & 31;
-	if(lane >= n) return;
-	const int4 it = t[lane];
-	const int i = it.x, j = it.y, k = it.z, m = it.w;
-	const long long N = a.N;
-	const int sy = a.sys ? a.sys[i] : 0;
-	const DNA2Table<R> &P = table_of<R>(a, sy);
-	Nuc<R> p, qn;
-	V4 ph, pl, qh, ql;
-	load_full<Loader, R>(ld, i, P, p, ph, pl);
-	load_full<Loader, R>(ld, j, P, qn, qh, ql);
-	const Sep<R> d = ld.sep(ph, pl, qh, ql, P);
-	PairOut<R> o{};
-	// FP32 engine path: the remainder of the site distance (the stiff radial factors, see rdiff)
-	const auto x = ld.refine(i, j);
-	if(term == 2) {
-		const StackGeo<R> g = stack_geo(p, qn, d);
-		R rl = R(0);
-		if constexpr(decltype(x)::on) {
-			if(g.cxst) rl = site_dist_remainder(d, p, x.lo(0), qn, x.lo(1), true, g.rmod);
+// ---------------------------------------------------------------- pair terms
+//
+// Hydrogen bonding, cross and coaxial stacking are products of a radial factor F(r) and up to six
+// angular factors g_k(cos theta_k).  The six angles are the same for all three terms (only the
+// sites differ: base sites, or stacking sites for coaxial stacking), each between a unit vector u
+// and a unit vector v:
+//     lane   u   v   cos      factors of HB, CRST, CXST
+//      0     a1  b1  -u.v     theta1
+//      1     b1  rd  -u.v     theta2, theta2, none
+//      2     a1  rd  +u.v     theta3, theta3, none
+//      3     a3  b3  +u.v     theta4
+//      4     b3  rd  -u.v     theta7, theta7, theta6
+//      5     a3  rd  +u.v     theta8, theta8, theta5
+// (a: axes of p, b: axes of q, rd: unit vector from p's site to q's).  With s the sign of the cosine,
+// X = u x v and e_k = F prod_(j != k) g_j dg_k/dcos, the factor's torque on p is -s e_k X (none where
+// u is q's and v = rd) and its force on q's site -s e_k (u - (u.v) v) / r (only where v = rd).  So a
+// term's angular factors are evaluated by eight lanes, one factor each by the same instructions, with
+// the product of the others' factors and the six sums by butterflies of shuffles.
+//
+// A block takes its pairs through four stages, each dealt to as many threads as it has work for, with
+// what they pass on in shared memory:
+//   1  screening: a thread per owned entry; pairs with live terms are queued, an item per term;
+//   2  a thread per item: separation, site distance, radial factor;
+//   3  eight lanes per item: the angular factors (lane 6 adds the radial force);
+//   4  a thread per pair: forces and torques of both nucleotides into the pair's two slots.
+// Why: one lane per pair was a chain of some 1,500 dependent instructions (nine angles one after the
+// other), and since a chip full of such warps has nothing else to issue, the launch lasted as long as
+// that chain.
+template <typename R>
+struct __align__(16) Angular {
+	R a, b, t0, ts, tc;  // f4 (see f4_both); a = b = 0 with a support that covers every angle: 1
+	R both;              // 1: f4(theta) + f4(pi - theta)
+	R harm;              // strength of the coaxial theta1 harmonic beyond sb
+	R pi_t0;             // pi - t0 (from the exact pi): theta - t0 of an obtuse theta is this less pi - theta
+};
+template <typename R>
+struct AngularTable {
+	Angular<R> t[3][8];  // [term: 0 HB, 1 CRST, 2 CXST][lane]
+};
+template <typename R>
+constexpr AngularTable<R> angular_table() {
+	constexpr float A[OXM_N_F4] = OXM_F4_TABLE_A, B[OXM_N_F4] = OXM_F4_TABLE_B, T0[OXM_N_F4] = OXM_F4_TABLE_T0,
+			TS[OXM_N_F4] = OXM_F4_TABLE_TS, TC[OXM_N_F4] = OXM_F4_TABLE_TC;
+	// the f4 set of every factor (-1: none) and whether it enters as f4(theta) + f4(pi - theta)
+	const int set[3][6] = {{OXM_F4_HB_T1, OXM_F4_HB_T2, OXM_F4_HB_T2, OXM_F4_HB_T4, OXM_F4_HB_T7, OXM_F4_HB_T7},
+			{OXM_F4_CR_T1, OXM_F4_CR_T2, OXM_F4_CR_T2, OXM_F4_CR_T4, OXM_F4_CR_T7, OXM_F4_CR_T7},
+			{OXM_F4_CX_T1, -1, -1, OXM_F4_CX_T4, OXM_F4_CX_T5, OXM_F4_CX_T5}};
+	const int both[3][6] = {{0, 0, 0, 0, 0, 0}, {0, 0, 0, 1, 1, 1}, {0, 0, 0, 0, 1, 1}};
+	const double pi = 3.14159265358979323846;
+	AngularTable<R> r{};
+	for(int m = 0; m < 3; m++)
+		for(int l = 0; l < 8; l++) {
+			const int i = l < 6 ? set[m][l] : -1;
+			if(i < 0) r.t[m][l] = Angular<R>{R(0), R(0), R(0), R(16), R(32), R(0), R(0), R(pi)};
+			else
+				r.t[m][l] = Angular<R>{R(A[i]), R(B[i]), R(T0[i]), R(TS[i]), R(TC[i]), R(both[m][l]),
+						i == OXM_F4_CX_T1 ? R(OXM_CXST_THETA1_SA) : R(0), R(pi - (double) T0[i])};
 		}
-		if(g.cxst) cxst_term<R, SPLIT>(p, qn, g, o, rl);
-	}
-	else {
-		const BaseGeo<R> g = base_geo(p, qn, d);
-		R rl = R(0);
-		if constexpr(decltype(x)::on) {
-			if((term == 0 && g.hb) || (term == 1 && g.crst)) rl = site_dist_remainder(d, p, x.lo(0), qn, x.lo(1), false, g.rmod);
-		}
-		if(term == 0 && g.hb) hb_term<R, SPLIT>(P, p, qn, g, o, rl);
-		if(term == 1 && g.crst) crst_term<R, SPLIT>(p, qn, g, o, rl);
-	}
-	// the potential is invariant under rigid rotations, so the torques balance:
-	// T_j = -T_i + (r_j - r_i) x F_i, the cross product with error-free products
-	const v3<R> c = cross_accurate(d, o.F);
-	V4 fi, ti, fj, tj;
-	fi.x = o.F.x, fi.y = o.F.y, fi.z = o.F.z, fi.w = ENERGY ? o.E : R(0);
-	ti.x = o.T.x, ti.y = o.T.y, ti.z = o.T.z, ti.w = ENERGY ? o.Ehb : R(0);
-	fj.x = -o.F.x, fj.y = -o.F.y, fj.z = -o.F.z, fj.w = fi.w;
-	tj.x = c.x - o.T.x, tj.y = c.y - o.T.y, tj.z = c.z - o.T.z, tj.w = ti.w;
-	V4 *res = reinterpret_cast<V4 *>(term == 2 ? a.stk_res : a.base_res);
-	atomic_add_v4(res + 2 * ((long long) k * N + i), fi);
-	atomic_add_v4(res + 2 * ((long long) k * N + i) + 1, ti);
-	if(m >= 0) {  // (a missing position is flagged by the list build)
-		atomic_add_v4(res + 2 * ((long long) m * N + j), fj);
-		atomic_add_v4(res + 2 * ((long long) m * N + j) + 1, tj);
-	}
-	if(SPLIT) {
-#pragma unroll
-		for(int u = 0; u < N_TERMS; u++)
-			if(o.split[u] != R(0)) atomicAdd(a.esplit + 8 * sy + u, (double) o.split[u]);
-	}
+	return r;
+}
+__device__ const AngularTable<float> g_angular_f = angular_table<float>();
+__device__ const AngularTable<double> g_angular_d = angular_table<double>();
+__device__ __forceinline__ const Angular<float> &angular_of(int term, int lane, float) { return g_angular_f.t[term][lane]; }
+__device__ __forceinline__ const Angular<double> &angular_of(int term, int lane, double) { return g_angular_d.t[term][lane]; }
+
+// one f4 factor at the angle theta = t0 + d: its value, and df/dtheta / sin(theta) (inv = 1 / sin;
+// flat: the angle is within 1e-4 of 0 or pi, where d / sin counts as +-1, as in f4_both)
+template <typename R>
+__device__ __forceinline__ void angular_factor(const Angular<R> &c, R d, R inv, bool flat, R &f, R &slope) {
+	const R ad = m_fabs(d), far = c.tc - ad;
+	const bool inner = ad <= c.ts, in = ad < c.tc;
+	f = inner ? R(1) - c.a * ad * ad : c.b * far * far;
+	slope = inner ? R(-2) * c.a * (flat ? m_copysign(R(1), d) : d * inv) : -m_copysign(R(2) * c.b * far, d) * inv;
+	if(!in) f = slope = R(0);
 }
 
-// Pair block b: base-base pairs (hydrogen bonding + cross stacking; blocks 0 .. base_blocks -
-// 1) or stack-stack pairs (coaxial stacking; the other blocks).  Each warp deals the owned pairs
-// of its nucleotides 32 at a time (as above) and screens them (base_geo / stack_geo: distance
-// windows and angular supports); only about a third of the pairs has a non-zero term, so the
-// live terms go to per-warp queues in shared memory and are evaluated 32 at a time, every lane
-// on the same term, instead of on the few lanes of each round whose pair happens to be live.
-template <typename R, class Loader, bool SPLIT, bool ENERGY, int NPW>
-__device__ __forceinline__ void pair_block(const ForceArgs &a, const Loader &ld, int b, int base_blocks) {
+template <typename R>
+__device__ __forceinline__ R shfl8(R v, int off) {
+	return __shfl_xor_sync(0xffffffffu, v, off, 8);
+}
+template <typename R>
+__device__ __forceinline__ R sum8(R v) {
+	v += shfl8(v, 1);
+	v += shfl8(v, 2);
+	return v + shfl8(v, 4);
+}
+
+// Which terms of pair (p, q) can be non-zero: 1 hydrogen bonding, 2 cross stacking, 4 coaxial stacking.
+// Distance windows (a little wider than the terms' own, for the plain FP32 separation) and the support
+// of every angular factor in its cosine; the terms themselves are zero outside them.
+template <typename R>
+__device__ __forceinline__ int live_terms(const Nuc<R> &p, const Nuc<R> &q, const v3<R> &r) {
+	constexpr R lo = R(0.9999), hi = R(1.0001);
+	const v3<R> da = q.a1 - p.a1;
+	const v3<R> rb = r + da * R(OXM_POS_BASE), rk = r + da * R(OXM_POS_STACK);
+	const R b2 = dot(rb, rb), k2 = dot(rk, rk);
+	const bool hb = p.btype + q.btype == 3 && b2 > lo * R(OXM_HYDR_RCLOW * OXM_HYDR_RCLOW) && b2 < hi * R(OXM_HYDR_RCHIGH * OXM_HYDR_RCHIGH);
+	const bool cr = b2 > lo * R(OXM_CRST_RCLOW * OXM_CRST_RCLOW) && b2 < hi * R(OXM_CRST_RCHIGH * OXM_CRST_RCHIGH);
+	const bool cx = k2 > lo * R(OXM_CXST_RCLOW * OXM_CXST_RCLOW) && k2 < hi * R(OXM_CXST_RCHIGH * OXM_CXST_RCHIGH);
+	if(!(hb || cr || cx)) return 0;
+	const R c1 = -dot(p.a1, q.a1), c4 = dot(p.a3, q.a3);
+	int m = 0;
+	if(hb || cr) {
+		const v3<R> rd = rb * (R(1) / m_sqrt(b2));
+		const R c2 = -dot(q.a1, rd), c3 = dot(p.a1, rd), c7 = -dot(q.a3, rd), c8 = dot(p.a3, rd);
+		if(hb && f4_may(c1, OXM_F4_HB_T1) && f4_may(c2, OXM_F4_HB_T2) && f4_may(c3, OXM_F4_HB_T2) && f4_may(c4, OXM_F4_HB_T4) &&
+				f4_may(c7, OXM_F4_HB_T7) && f4_may(c8, OXM_F4_HB_T7))
+			m |= 1;
+		// theta4, theta7, theta8 of cross stacking enter through f4(theta) + f4(pi - theta)
+		if(cr && f4_may(c1, OXM_F4_CR_T1) && f4_may(c2, OXM_F4_CR_T2) && f4_may(c3, OXM_F4_CR_T2) &&
+				(f4_may(c4, OXM_F4_CR_T4) || f4_may(-c4, OXM_F4_CR_T4)) && (f4_may(c7, OXM_F4_CR_T7) || f4_may(-c7, OXM_F4_CR_T7)) &&
+				(f4_may(c8, OXM_F4_CR_T7) || f4_may(-c8, OXM_F4_CR_T7)))
+			m |= 2;
+	}
+	if(cx && f4_may(c1, OXM_F4_CX_T1) && f4_may(c4, OXM_F4_CX_T4)) {
+		const v3<R> rd = rk * (R(1) / m_sqrt(k2));
+		const R c5 = dot(p.a3, rd), c6 = -dot(q.a3, rd);
+		if((f4_may(c5, OXM_F4_CX_T5) || f4_may(-c5, OXM_F4_CX_T5)) && (f4_may(c6, OXM_F4_CX_T5) || f4_may(-c6, OXM_F4_CX_T5))) m |= 4;
+	}
+	return m;
+}
+
+constexpr int PAIR_CHUNK = 64;             // items taken through stages 2 to 4 at a time
+constexpr int PAIR_QUEUE = 512 + 3 * 128;  // items waiting (a round of screening adds at most 3 x 128)
+
+// one item between the stages (an odd number of words apart: no bank conflicts)
+template <typename R>
+struct PairItem {
+	R axes[12];            // a1, a3 of p; a1, a3 of q
+	R rd[3], ir, F, FD;    // site direction, 1 / site distance, radial factor and its derivative
+	R d[6];                // centre separation, hi and lo
+	R out[7];              // force on q's site, torque on p without its lever arm, energy
+};
+static_assert(sizeof(PairItem<float>) == 31 * 4, "an odd number of words");
+
+// stage 2 of item m of pair (i, j), term 0 hydrogen bonding, 1 cross stacking, 2 coaxial stacking
+template <typename R, class Loader>
+__device__ __forceinline__ void pair_radial(const ForceArgs &a, const Loader &ld, int i, int j, int term, PairItem<R> &m) {
 	using V4 = typename Vec4Of<R>::T;
-	__shared__ int4 tq[4][2][64];  // per warp: live hydrogen-bonding (or coaxial) and cross-stacking terms
-	const bool is_base = b < base_blocks;
-	const int per_block = (blockDim.x / 32) * NPW;
-	const int first = (is_base ? b : b - base_blocks) * per_block;
+	const DNA2Table<R> &P = table_of<R>(a, a.sys ? a.sys[i] : 0);
+	Nuc<R> p, q;
+	V4 ph, pl, qh, ql;
+	load_axes<Loader, R>(ld, i, P, p, ph, pl);
+	load_axes<Loader, R>(ld, j, P, q, qh, ql);
+	const Sep<R> d = ld.sep(ph, pl, qh, ql, P);
+	const bool stack = term == 2;
+	p.stack = p.a1 * R(OXM_POS_STACK), q.stack = q.a1 * R(OXM_POS_STACK);
+	const v3<R> rs = stack ? site_vec(d, q.stack, p.stack) : site_vec(d, q.base, p.base);
+	const R r = m_sqrt(dot(rs, rs)), ir = m_rcp(r);
+	const v3<R> rd = rs * ir;
+	R rl = R(0);
+	const auto x = ld.refine(i, j);
+	if constexpr(decltype(x)::on) rl = site_dist_remainder(d, p, x.lo(0), q, x.lo(1), stack, r);
+	R F, FD;
+	if(term == 0) {
+		const R hbm = (abs(q.btype) >= 300 && abs(p.btype) >= 300) ? P.hb_multiplier : R(1);
+		f1_both(P, r, OXM_F1_HB, q.type, p.type, F, FD, rl);
+		F *= hbm;
+		FD *= hbm;
+	}
+	else if(term == 1) f2_both(r, OXM_F2_CRST, F, FD, rl);
+	else f2_both(r, OXM_F2_CXST, F, FD, rl);
+	const v3<R> ax[4] = {p.a1, p.a3, q.a1, q.a3};
+#pragma unroll
+	for(int k = 0; k < 4; k++) m.axes[3 * k] = ax[k].x, m.axes[3 * k + 1] = ax[k].y, m.axes[3 * k + 2] = ax[k].z;
+	m.rd[0] = rd.x, m.rd[1] = rd.y, m.rd[2] = rd.z;
+	m.ir = ir, m.F = F, m.FD = FD;
+	m.d[0] = d.hi.x, m.d[1] = d.hi.y, m.d[2] = d.hi.z, m.d[3] = d.lo.x, m.d[4] = d.lo.y, m.d[5] = d.lo.z;
+}
+
+// stage 3: eight lanes, this one the factor of its lane; the whole warp takes part
+template <typename R>
+__device__ __forceinline__ void pair_angles(int term, PairItem<R> &m) {
+	const int sub = threadIdx.x & 7;
+	const bool u_q = sub == 1 || sub == 4;              // u is an axis of q
+	const bool v_rd = sub != 0 && sub != 3 && sub < 6;  // v is the site direction
+	const R s = (u_q || sub == 0) ? R(-1) : R(1);
+	const Angular<R> c = angular_of(term, sub, R(0));
+	// u: a1 b1 a1 a3 b3 a3; v: b1 rd rd b3 rd rd (word offsets into the item)
+	const R *pu = m.axes + (sub == 1 ? 6 : sub == 4 ? 9 : (sub == 3 || sub == 5) ? 3 : 0);
+	const R *pv = v_rd ? m.rd : m.axes + (sub == 3 ? 9 : 6);
+	const v3<R> u{pu[0], pu[1], pu[2]}, v{pv[0], pv[1], pv[2]};
+	const v3<R> X = cross(u, v);
+	const R uv = dot(u, v), s2 = dot(X, X), sn = m_sqrt(s2);
+	const bool flat = !(s2 > R(1e-8));
+	const R inv = R(1) / (flat ? R(1) : sn);
+	// From the angle to the nearer of +v and -v: theta or pi - theta, and their distances from t0
+	// without rounding an angle near pi (an ulp of 3 is 2.4e-7, which the factors' slopes carry on)
+	const R acute = m_atan2(sn, m_fabs(uv));
+	const R near = acute - c.t0, far = c.pi_t0 - acute;
+	const bool neg = s * uv < R(0);  // theta is the obtuse one
+	R g, sl, g2, sl2;
+	angular_factor(c, neg ? far : near, inv, flat, g, sl);
+	angular_factor(c, neg ? near : far, inv, flat, g2, sl2);
+	g += c.both * g2;
+	sl -= c.both * sl2;
+	const R h = m_max(neg ? R(3.14159265358979323846 - (double) OXM_CXST_THETA1_SB) - acute : acute - R(OXM_CXST_THETA1_SB), R(0));
+	g += c.harm * h * h;
+	sl += R(2) * c.harm * (flat ? (h > R(0) ? R(1) : R(0)) : h * inv);
+	// the product of the other lanes' factors
+	R all = g, others = R(1);
+#pragma unroll
+	for(int off = 1; off < 8; off <<= 1) {
+		const R z = shfl8(all, off);
+		others *= z;
+		all *= z;
+	}
+	const R F = m.F;
+	const R ek = F * others * -sl;  // F prod_(j != k) g_j dg_k/dcos
+	const R ft = v_rd ? -s * ek * m.ir : R(0), tt = (u_q || sub > 5) ? R(0) : -s * ek;
+	v3<R> f = (u - v * uv) * ft, tq = X * tt;
+	if(sub == 6) f = v3<R>{m.rd[0], m.rd[1], m.rd[2]} * (-(m.FD * all));
+	f.x = sum8(f.x), f.y = sum8(f.y), f.z = sum8(f.z);
+	tq.x = sum8(tq.x), tq.y = sum8(tq.y), tq.z = sum8(tq.z);
+	const R e = F * all;
+	const R out = sub == 0 ? f.x : sub == 1 ? f.y : sub == 2 ? f.z : sub == 3 ? tq.x : sub == 4 ? tq.y : sub == 5 ? tq.z : e;
+	if(sub < 7) m.out[sub] = out;
+}
+
+// Pair block b (128 threads): the entries owned by G groups of 32 nucleotides, in the four stages above
+template <typename R, class Loader, bool SPLIT, bool ENERGY, int G>
+__device__ __forceinline__ void pair_block(const ForceArgs &a, const Loader &ld, int b) {
+	using V4 = typename Vec4Of<R>::T;
+	__shared__ int2 queue[PAIR_QUEUE];  // partner; k | m << 8 | term << 16 | further term of the pair << 18 | i - first << 19
+	__shared__ PairItem<R> item[PAIR_CHUNK];
+	__shared__ int wcount[4];
 	const long long N = a.N;
-	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-	const int wbase = first + w * NPW;
-	if(wbase >= a.N) return;  // warp-uniform
-	const int cap = is_base ? a.base_cap : a.stk_cap;
-	const int *nb = is_base ? a.base_nb : a.stk_nb;
-	V4 *res = reinterpret_cast<V4 *>(is_base ? a.base_res : a.stk_res);
-	// this lane's nucleotide (lanes below NPW): which of its entries it owns (partner above
-	// it by caller's index), as a bit mask
-	const int il = wbase + lane;
-	unsigned lo = 0u, hi = 0u;
-	if(lane < NPW && il < a.N) {
-		const int n = min(min(is_base ? a.base_n[il] : a.stk_n[il], cap), 64);
-		const int key = a.id ? a.id[il] : il;
-		for(int k = 0; k < n; k++) {
-			const int j = nb[(long long) k * N + il];
-			if((a.id ? a.id[j] : j) > key) {
-				if(k < 32) lo |= 1u << k;
-				else hi |= 1u << (k - 32);
-			}
-		}
-	}
-	const int own = __popc(lo) + __popc(hi);
-	int incl = own;
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const int g0 = b * G, first = g0 * PAIR_GROUP, groups = (a.N + PAIR_GROUP - 1) / PAIR_GROUP;
+	int start[G + 1];  // the groups' entries, one after the other
+	start[0] = 0;
 #pragma unroll
-	for(int off = 1; off < 32; off <<= 1) {
-		const int u = __shfl_up_sync(0xffffffffu, incl, off);
-		if(lane >= off) incl += u;
-	}
-	const int total = __shfl_sync(0xffffffffu, incl, 31);
-	const int excl = incl - own;
-	const unsigned below = (1u << lane) - 1u;
-	int n0 = 0, n1 = 0;  // queued terms (warp-uniform)
-	const int term0 = is_base ? 0 : 2;
-	for(int q0 = 0; q0 < total; q0 += 32) {
-		const int q = q0 + lane;
-		// the lane that owns queue entry q: the first whose inclusive count exceeds q
-		int l = 0;
+	for(int g = 0; g < G; g++) start[g + 1] = start[g] + (g0 + g < groups ? a.own_n[g0 + g] : 0);
+	V4 *res = reinterpret_cast<V4 *>(a.pt_res);
+	int n = 0;  // queued items (block-uniform)
+	bool more = start[G] > 0;
+	for(int r0 = 0; more; r0 += 128) {
+		// stage 1
+		int mask = 0, i0 = 0;
+		int2 it = make_int2(0, 0);
+		const int r = r0 + (int) threadIdx.x;
+		if(r < start[G]) {
+			int g = 0;
 #pragma unroll
-		for(int step = 16; step > 0; step >>= 1) {
-			const int v = __shfl_sync(0xffffffffu, incl, l + step - 1);
-			if(v <= q) l += step;
-		}
-		const int ex_l = __shfl_sync(0xffffffffu, excl, l & 31);
-		const unsigned lo_l = __shfl_sync(0xffffffffu, lo, l & 31), hi_l = __shfl_sync(0xffffffffu, hi, l & 31);
-		bool live0 = false, live1 = false;
-		int4 item = make_int4(0, 0, 0, -1);
-		if(q < total) {
-			// the r-th owned entry of nucleotide i
-			const int r = q - ex_l, nlo = __popc(lo_l);
-			const int k = r < nlo ? (int) __fns(lo_l, 0u, r + 1) : 32 + (int) __fns(hi_l, 0u, r - nlo + 1);
-			const int i = wbase + l;
-			const int j = nb[(long long) k * N + i];
-			const int m = (is_base ? a.base_pos : a.stk_pos)[(long long) k * N + i];
-			const int sy = a.sys ? a.sys[i] : 0;
-			const DNA2Table<R> &P = table_of<R>(a, sy);
-			Nuc<R> p, qn;
+			for(int u = 1; u < G; u++) g += r >= start[u];
+			int base = 0;
+#pragma unroll
+			for(int u = 1; u < G; u++)
+				if(g == u) base = start[u];
+			it = a.own[(long long) (g0 + g) * PAIR_GROUP * a.pt_cap + (r - base)];
+			i0 = first + g * PAIR_GROUP + (it.y >> 16);
+			it.y &= 0xffff;
+			Nuc<R> p, q;
 			V4 ph, pl, qh, ql;
-			load_full<Loader, R>(ld, i, P, p, ph, pl);
-			load_full<Loader, R>(ld, j, P, qn, qh, ql);
-			const Sep<R> d = ld.sep(ph, pl, qh, ql, P);
-			if(is_base) {
-				const BaseGeo<R> g = base_geo(p, qn, d);
-				live0 = g.hb;
-				live1 = g.crst;
-			}
-			else {
-				live0 = stack_geo(p, qn, d).cxst;
-			}
-			// both slots start from zero; the live terms add into them
-			V4 z;
-			z.x = z.y = z.z = z.w = R(0);
-			res[2 * ((long long) k * N + i)] = z;
-			res[2 * ((long long) k * N + i) + 1] = z;
-			if(m >= 0) {
-				res[2 * ((long long) m * N + j)] = z;
-				res[2 * ((long long) m * N + j) + 1] = z;
-			}
-			item = make_int4(i, j, k, m);
+			const DNA2Table<R> &P = table_of<R>(a, a.sys ? a.sys[i0] : 0);
+			load_axes<Loader, R>(ld, i0, P, p, ph, pl);
+			load_axes<Loader, R>(ld, it.x, P, q, qh, ql);
+			mask = live_terms(p, q, ld.sep(ph, pl, qh, ql, P).plain());
 		}
-		const unsigned b0 = __ballot_sync(0xffffffffu, live0), b1 = __ballot_sync(0xffffffffu, live1);
-		if(live0) tq[w][0][n0 + __popc(b0 & below)] = item;
-		if(live1) tq[w][1][n1 + __popc(b1 & below)] = item;
-		n0 += __popc(b0);
-		n1 += __popc(b1);
-		__syncwarp();  // the queued items and the zeroed slots are visible to the whole warp
-		if(n0 >= 32) {
-			n0 -= 32;
-			eval_terms<R, Loader, SPLIT, ENERGY>(a, ld, tq[w][0] + n0, 32, term0);
-			__syncwarp();
+		int incl = __popc(mask);
+#pragma unroll
+		for(int off = 1; off < 32; off <<= 1) {
+			const int u = __shfl_up_sync(0xffffffffu, incl, off);
+			if(lane >= off) incl += u;
 		}
-		if(n1 >= 32) {
-			n1 -= 32;
-			eval_terms<R, Loader, SPLIT, ENERGY>(a, ld, tq[w][1] + n1, 32, 1);
-			__syncwarp();
+		if(lane == 31) wcount[warp] = incl;
+		__syncthreads();
+		more = r0 + 128 < start[G];
+		int at = n + incl - __popc(mask);
+#pragma unroll
+		for(int w = 0; w < 4; w++) {
+			if(w < warp) at += wcount[w];
+			n += wcount[w];
 		}
+		for(int left = mask, k = 0; left; left &= left - 1, k++)
+			queue[at + k] = make_int2(it.x, it.y | (__ffs(left) - 1) << 16 | (k > 0 ? 1 << 18 : 0) | (i0 - first) << 19);
+		__syncthreads();
+		if(more && n <= PAIR_QUEUE - 3 * 128) continue;
+		for(int c0 = 0; c0 < n;) {
+			// the next chunk ends with a whole pair
+			int c1 = min(n, c0 + PAIR_CHUNK);
+			while(c1 < n && (queue[c1].y & (1 << 18))) c1--;
+			for(int m = threadIdx.x; m < c1 - c0; m += 128) {
+				const int2 w = queue[c0 + m];
+				pair_radial<R, Loader>(a, ld, first + (w.y >> 19), w.x, (w.y >> 16) & 3, item[m]);
+			}
+			__syncthreads();
+			for(int m0 = warp * 4; m0 < c1 - c0; m0 += 16) {  // warp-uniform: four items at a time
+				// (lanes without an item repeat the last one: the same values, written again)
+				const int m = min(m0 + lane / 8, c1 - c0 - 1);
+				pair_angles<R>((queue[c0 + m].y >> 16) & 3, item[m]);
+			}
+			__syncthreads();
+			for(int m = threadIdx.x; m < c1 - c0; m += 128) {
+				const int2 w = queue[c0 + m];
+				if(w.y & (1 << 18)) continue;  // taken with the pair's first item
+				const int i = first + (w.y >> 19), j = w.x, k = w.y & 255, mj = (w.y >> 8) & 255;
+				PairOut<R> o{};
+				for(int v = m;;) {
+					const PairItem<R> &it4 = item[v];
+					const int term = (queue[c0 + v].y >> 16) & 3;
+					const R e = it4.out[6];
+					if(e != R(0)) {
+						const v3<R> f{it4.out[0], it4.out[1], it4.out[2]};
+						const v3<R> a1{it4.axes[0], it4.axes[1], it4.axes[2]};
+						// the lever arm as the loaders form it
+						const v3<R> arm = term == 2 ? a1 * R(OXM_POS_STACK) : sizeof(R) == 4 ? a1 * R(OXM_POS_BASE) :
+								a1 * R(OXM_POS_STACK) * R((double) OXM_POS_BASE / (double) OXM_POS_STACK);
+						o.F -= f;
+						o.T += v3<R>{it4.out[3], it4.out[4], it4.out[5]} - cross(arm, f);
+						add_e<R, SPLIT>(o, term == 0 ? T_HB : term == 1 ? T_CRST : T_CXST, e);
+						if(term == 0) o.Ehb += e;
+					}
+					if(++v >= c1 - c0 || !(queue[c0 + v].y & (1 << 18))) break;
+				}
+				if(o.F.x == R(0) && o.F.y == R(0) && o.F.z == R(0) && o.T.x == R(0) && o.T.y == R(0) && o.T.z == R(0) && o.E == R(0)) continue;
+				// the potential is invariant under rigid rotations, so the torques balance:
+				// T_j = -T_i + (r_j - r_i) x F_i, the cross product with error-free products
+				const R *dd = item[m].d;
+				const v3<R> c = cross_accurate(Sep<R>{v3<R>{dd[0], dd[1], dd[2]}, v3<R>{dd[3], dd[4], dd[5]}}, o.F);
+				V4 fi, ti, fj, tj;
+				fi.x = o.F.x, fi.y = o.F.y, fi.z = o.F.z, fi.w = ENERGY ? o.E : R(0);
+				ti.x = o.T.x, ti.y = o.T.y, ti.z = o.T.z, ti.w = ENERGY ? o.Ehb : R(0);
+				fj.x = -o.F.x, fj.y = -o.F.y, fj.z = -o.F.z, fj.w = fi.w;
+				tj.x = c.x - o.T.x, tj.y = c.y - o.T.y, tj.z = c.z - o.T.z, tj.w = ti.w;
+				res[2 * ((long long) k * N + i)] = fi;
+				res[2 * ((long long) k * N + i) + 1] = ti;
+				atomicOr(a.pt_live + (long long) (k >> 6) * N + i, 1ull << (k & 63));
+				if(mj < 255) {  // (a missing position is flagged by the list build)
+					res[2 * ((long long) mj * N + j)] = fj;
+					res[2 * ((long long) mj * N + j) + 1] = tj;
+					atomicOr(a.pt_live + (long long) (mj >> 6) * N + j, 1ull << (mj & 63));
+				}
+				if(SPLIT) {
+					const int sy = a.sys ? a.sys[i] : 0;
+#pragma unroll
+					for(int u = 0; u < N_TERMS; u++)
+						if(o.split[u] != R(0)) atomicAdd(a.esplit + 8 * sy + u, (double) o.split[u]);
+				}
+			}
+			__syncthreads();
+			c0 = c1;
+		}
+		n = 0;
 	}
-	if(n0 > 0) eval_terms<R, Loader, SPLIT, ENERGY>(a, ld, tq[w][0], n0, term0);
-	if(n1 > 0) eval_terms<R, Loader, SPLIT, ENERGY>(a, ld, tq[w][1], n1, 1);
 }
 
 // minimum resident blocks per SM asked of the register allocator for the bonded/pair kernel
@@ -946,18 +1128,18 @@ __device__ __forceinline__ void edge_block(const ForceArgs &a, const Loader &ld,
 	if(sub == 0 && live) partner(i, v3<R>{fx, fy, fz}, v3<R>{tx, ty, tz}, e);
 }
 
-// The bonded and the base/stack pair work are independent (both read the mirrors, each writes
-// its own result buffers), so they share one launch: blocks 0 .. 2 pair_blocks - 1 are pair
-// blocks (the costliest, dispatched first), then the bonded blocks, which fill the tail, and
-// with use_edge the edge blocks.
-template <typename R, class Loader, bool SPLIT, bool ENERGY, int NPW = OXGB_PAIR_NPW, bool EDGE = false, int K = 4>
+// The bonded and the pair-term work are independent (both read the mirrors, each writes its own
+// result buffers), so they share one launch: blocks 0 .. pair_blocks - 1 are pair blocks (the
+// costliest, dispatched first), then the bonded blocks, which fill the tail, and with use_edge the
+// edge blocks.  G: groups of 32 nucleotides per pair block.
+template <typename R, class Loader, bool SPLIT, bool ENERGY, int G, bool EDGE = false, int K = 4>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? OXGB_PAIR_MINB : 1) k_bonded_pairs(ForceArgs a, Loader ld, int pair_blocks) {
 	pdl_trigger();  // the non-bonded kernel may start (it waits before reading these results)
 	const int b = blockIdx.x;
-	const int bonded_blocks = (a.N + (int) blockDim.x - 1) / (int) blockDim.x;
-	if(b < 2 * pair_blocks) pair_block<R, Loader, SPLIT, ENERGY, NPW>(a, ld, b, pair_blocks);
-	else if(!EDGE || b < 2 * pair_blocks + bonded_blocks) bonded_block<R, Loader, SPLIT, ENERGY>(a, ld, b - 2 * pair_blocks);
-	else if constexpr(EDGE) edge_block<R, Loader, SPLIT, ENERGY, K>(a, ld, b - 2 * pair_blocks - bonded_blocks);
+	const int bonded_blocks = (a.N + BONDS_PER_BLOCK - 1) / BONDS_PER_BLOCK;
+	if(b < pair_blocks) pair_block<R, Loader, SPLIT, ENERGY, G>(a, ld, b);
+	else if(!EDGE || b < pair_blocks + bonded_blocks) bonded_block<R, Loader, SPLIT, ENERGY>(a, ld, b - pair_blocks);
+	else if constexpr(EDGE) edge_block<R, Loader, SPLIT, ENERGY, K>(a, ld, b - pair_blocks - bonded_blocks);
 }
 
 // K lanes per nucleotide: lane l of a group takes entries l, l + K, ... of every term list, so a
@@ -1070,33 +1252,37 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? MINB : 1) k_nonbonded_sp
 				acc.add_short(o);
 			}
 		}
-		// hydrogen bonding + cross stacking and coaxial stacking: evaluated per list slot by
-		// the pair blocks of k_bonded_pairs, gathered here (the terms above read only the
-		// mirrors and lists, complete before k_bonded_pairs started)
+		// hydrogen bonding, cross and coaxial stacking: evaluated by the pair blocks of
+		// k_bonded_pairs, the slots they wrote gathered here (the terms above read only the mirrors
+		// and lists, complete before k_bonded_pairs started)
 		pdl_wait();
 		pdl_trigger();
-		// the base slots then the stack slots as one sequence, the next slot loaded before the
-		// current one is added
-		const int nb_ = live ? min(a.base_n[i], a.base_cap) : 0;
-		const int ns = live ? min(a.stk_n[i], a.stk_cap) : 0;
-		{
-			const int nt = nb_ + ns;
-			const V4 *rb = reinterpret_cast<const V4 *>(a.base_res), *rs = reinterpret_cast<const V4 *>(a.stk_res);
-			auto slot = [&](int k) { return k < nb_ ? rb + 2 * ((long long) k * N + i) : rs + 2 * ((long long) (k - nb_) * N + i); };
+		for(int w = 0; w < (a.pt_cap + 63) / 64; w++) {
+			unsigned long long m = 0ull;
+			if(sub == 0 && live) {
+				unsigned long long *at = a.pt_live + (long long) w * N + i;
+				m = *at;
+				if(m) *at = 0ull;  // for the next evaluation
+			}
+			m = __shfl_sync(0xffffffffu, m, 0, K);
+			// lane l takes the live slots l, l + K, ..., the next one loaded before the current one
+			// is added
+			for(int u = 0; u < sub; u++) m &= m - 1ull;
+			const V4 *base = reinterpret_cast<const V4 *>(a.pt_res) + 2 * ((long long) w * 64 * N + i);
 			V4 f, t;
-			int k = sub;
-			if(k < nt) {
-				const V4 *q = slot(k);
+			auto next = [&]() {
+				const V4 *q = base + 2 * (long long) (__ffsll((long long) m) - 1) * N;
 				f = q[0];
 				t = q[1];
-			}
-			for(; k < nt; k += K) {
+#pragma unroll
+				for(int u = 0; u < K; u++) m &= m - 1ull;
+			};
+			bool have = m != 0ull;
+			if(have) next();
+			while(have) {
 				const V4 cf = f, ct = t;
-				if(k + K < nt) {
-					const V4 *q = slot(k + K);
-					f = q[0];
-					t = q[1];
-				}
+				have = m != 0ull;
+				if(have) next();
 				acc.F.add(v3<R>{cf.x, cf.y, cf.z});
 				acc.T.add(v3<R>{ct.x, ct.y, ct.z});
 				if(ENERGY) {
@@ -1429,16 +1615,16 @@ __global__ void k_external(ForceArgs a) {
 	F[i] = f;
 }
 
-template <typename R, class Loader, bool SPLIT, bool ENERGY, int NPW = OXGB_PAIR_NPW, int K = OXGB_NB_LANES,
-		int NBMINB = OXGB_NB_MINB, bool EDGE = false>
+template <typename R, class Loader, bool SPLIT, bool ENERGY, int G = 1, int K = OXGB_NB_LANES, int NBMINB = OXGB_NB_MINB,
+		bool EDGE = false>
 static void launch_split_t(const ForceArgs &a, Loader ld, cudaStream_t s, cudaEvent_t wait) {
 	const int tpb = 128;
-	const int blocks = a.N > 0 ? (a.N + tpb - 1) / tpb : 1;
-	// pair blocks of 4 warps x NPW nucleotides per term, then one bonded block per 128
-	// nucleotides, then (use_edge) one edge block per 128 / K nucleotides
-	const int pair_blocks = (a.N + 4 * NPW - 1) / (4 * NPW);
+	const int blocks = a.N > 0 ? (a.N + BONDS_PER_BLOCK - 1) / BONDS_PER_BLOCK : 1;
+	// pair blocks of G groups of 32 nucleotides, then one bonded block per 64 nucleotides, then
+	// (use_edge) one edge block per 128 / K nucleotides
+	const int pair_blocks = (a.N + PAIR_GROUP * G - 1) / (PAIR_GROUP * G);
 	const int edge_blocks = EDGE ? nonbonded_blocks(a.N, K) : 0;
-	k_bonded_pairs<R, Loader, SPLIT, ENERGY, NPW, EDGE, K><<<2 * pair_blocks + blocks + edge_blocks, tpb, 0, s>>>(a, ld, pair_blocks);
+	k_bonded_pairs<R, Loader, SPLIT, ENERGY, G, EDGE, K><<<pair_blocks + blocks + edge_blocks, tpb, 0, s>>>(a, ld, pair_blocks);
 	// the non-bonded kernel starts its Debye-Hueckel and excluded-volume work while the tail of
 	// the bonded and pair blocks runs; the external forces follow it the same way
 	if(wait) cudaStreamWaitEvent(s, wait, 0);
@@ -1448,20 +1634,24 @@ static void launch_split_t(const ForceArgs &a, Loader ld, cudaStream_t s, cudaEv
 	if(a.ext_n > 0) launch_after(k_external<typename Vec4Of<R>::T>, dim3((a.ext_n + tpb - 1) / tpb), dim3(tpb), 0, s, a);
 }
 
+#ifndef OXGB_PAIR_WIDE_N
+#define OXGB_PAIR_WIDE_N 100000
+#endif
 // the MD step's kernels (mixed / float engine) in shape k of FORCE_SHAPES
 template <int k>
 static void launch_md_shape(const ForceArgs &a, const SplitMixed &ld, cudaStream_t s, cudaEvent_t wait) {
 	constexpr ForceShapeDef d = FORCE_SHAPES[k];
-	launch_split_t<float, SplitMixed, false, false, d.npw, d.lanes, d.minb>(a, ld, s, wait);
+	if(a.N < OXGB_PAIR_WIDE_N) launch_split_t<float, SplitMixed, false, false, 1, d.lanes, d.minb>(a, ld, s, wait);
+	else launch_split_t<float, SplitMixed, false, false, d.npw / 8, d.lanes, d.minb>(a, ld, s, wait);
 }
 
 // use_edge: the default shape with the edge blocks
 template <typename R, class Loader>
 static void launch_edge(const ForceArgs &a, Loader ld, bool split, bool energy, cudaStream_t s, cudaEvent_t wait) {
-	constexpr int NPW = OXGB_PAIR_NPW, K = OXGB_NB_LANES, MB = OXGB_NB_MINB;
-	if(split) launch_split_t<R, Loader, true, true, NPW, K, MB, true>(a, ld, s, wait);
-	else if(energy) launch_split_t<R, Loader, false, true, NPW, K, MB, true>(a, ld, s, wait);
-	else launch_split_t<R, Loader, false, false, NPW, K, MB, true>(a, ld, s, wait);
+	constexpr int G = 1, K = OXGB_NB_LANES, MB = OXGB_NB_MINB;
+	if(split) launch_split_t<R, Loader, true, true, G, K, MB, true>(a, ld, s, wait);
+	else if(energy) launch_split_t<R, Loader, false, true, G, K, MB, true>(a, ld, s, wait);
+	else launch_split_t<R, Loader, false, false, G, K, MB, true>(a, ld, s, wait);
 }
 
 cudaError_t launch_forces_split(const ForceArgs &a, bool dbl, bool split, bool energy, cudaStream_t s, cudaEvent_t wait) {

@@ -106,14 +106,19 @@ struct ForceArgs {
 	// (column-major: element k of nucleotide i at [k * N + i]) and the per-bond buffers
 	const float4 *fback;
 	const float4 *fa1lo, *fbacklo;            // remainders of fa1 / fback (null: the FP32 sites unrefined)
-	const int *ev_nb, *ev_n, *base_nb, *base_n, *stk_nb, *stk_n;
-	int ev_cap, base_cap, stk_cap;            // capacities (an overflowed list is read up to them)
+	const int *ev_nb, *ev_n, *pt_nb, *pt_n;
+	int ev_cap, pt_cap;                       // capacities (an overflowed list is read up to them)
 	void *bond_f, *bond_tp, *bond_tq;         // per bond owner p (q = n3[p]): f on q with w = energy, torques
-	// base / stack pairs are evaluated once, by their lower nucleotide i (by caller's index), which writes slot k of i
-	// and slot pos[k N + i] of its partner j: (force, E), (torque, E_hb) as two V4 per slot
-	void *base_res, *stk_res;
-	const int *base_pos, *stk_pos;            // see ListArgs
-	const int *term_max;                      // [4] longest EV / base / stack list (slots past it are empty), full row
+	// pair-term pairs are evaluated once, from their lower nucleotide i (by caller's index): the
+	// entries owned by the PAIR_GROUP nucleotides from PAIR_GROUP g are own[g PAIR_GROUP pt_cap + r],
+	// r < own_n[g]: (partner j, k | m << 8 | (i - PAIR_GROUP g) << 16).  A pair's results go to
+	// slot k of i and slot m of j (255: none), (force, E), (torque, E_hb) as two V4 per slot at
+	// pt_res[2 (slot N + i)].  Only pairs with a non-zero term are written; bit `slot` of pt_live
+	// ([slot / 64 N + i]) says so, set by the pair blocks, read and cleared by the non-bonded kernel
+	void *pt_res;
+	const int2 *own;
+	const int *own_n;
+	unsigned long long *pt_live;
 	// MD-step bookkeeping (engine layout): the bonded kernel marks the step's half kick pending
 	ThermoArgs th;
 	// external forces (oxgb_ext_force records grouped by nucleotide): ext_n nucleotides
@@ -138,6 +143,9 @@ struct ForceArgs {
 	int edge;
 	void *edge_acc;
 };
+
+// nucleotides whose owned pair-term entries are kept together (ForceArgs::own)
+constexpr int PAIR_GROUP = 32;
 
 cudaError_t launch_forces_reference_layout(const ForceArgs &a, cudaStream_t s);
 // FFS order parameters of listed pairs on the reference layout (mode 0 hydrogen-bonding energy,
@@ -179,14 +187,15 @@ struct ListArgs {
 	int check_flag;         // 1: every kernel exits at once unless *flag is set
 	unsigned long long *rebuilds;  // counts builds (may be null)
 	// term lists (null: full rows only).  A pair enters the excluded-volume list when its centres
-	// are closer than ev_r, the base list when its base sites are closer than base_r, the stack
-	// list when its stacking sites are closer than stk_r (all thresholds include twice the skin)
+	// are closer than ev_r, the pair-term list (hydrogen bonding, cross and coaxial stacking) when its
+	// base sites are closer than base_r or its stacking sites closer than stk_r (all thresholds
+	// include twice the skin)
 	const float4 *fa1, *fback;
-	int *ev_nb, *ev_n, *base_nb, *base_n, *stk_nb, *stk_n;
-	// for every base / stack entry (k, i) whose partner j is higher (i owns the pair): the
-	// position of i in j's list, where the pair evaluation also writes j's result; -1 otherwise
-	int *base_pos, *stk_pos;
-	int ev_cap, base_cap, stk_cap;
+	int *ev_nb, *ev_n, *pt_nb, *pt_n;
+	// the pair-term entries whose partner is higher (i owns the pair), see ForceArgs::own
+	int2 *own;
+	int *own_n;
+	int ev_cap, pt_cap;
 	float ev_r2, base_r2, stk_r2;
 	// the excluded-volume list keeps only pairs with a site pair within its cutoff plus twice the
 	// skin (squared: backbone-backbone, base-base, backbone-base)
@@ -198,7 +207,7 @@ struct ListArgs {
 	float dh_r2;
 	const float *sys_dh2;
 	float4 *list_a1, *list_back;   // body axis a1 and backbone offset at this build
-	int *term_max;          // [4] longest EV / base / stack list and full row of any build so far (may be null)
+	int *term_max;          // [4] longest EV / pair-term list, -, and full row of any build so far (may be null)
 	int col_major;          // full rows column-major ([k * N + i]) instead of row-major
 	// batch of systems (sys null: one system with the scalar geometry above).  System s has
 	// its own box, cutoff and cell grid (sys_nside^3 cells from sys_cell0); only systems with

@@ -299,6 +299,16 @@ __global__ void k_sort_scatter(ListArgs a) {
 	a.cell_of[k] = si[N + k];
 }
 
+// A listed pair can have hydrogen bonding or cross stacking before the next rebuild only if its base
+// sites (0.4 a1 from the centres), coaxial stacking only if its stacking sites (0.34 a1), are within
+// their bounds.  Exactly symmetric in the two nucleotides, so the pair-term lists are symmetric.
+__device__ __forceinline__ bool pair_sites_near(const ListArgs &a, float3 d, float4 a1i, float4 a1j) {
+	const float bx = d.x + 0.4f * (a1j.x - a1i.x), by = d.y + 0.4f * (a1j.y - a1i.y), bz = d.z + 0.4f * (a1j.z - a1i.z);
+	if(bx * bx + by * by + bz * bz < a.base_r2) return true;
+	const float sx = d.x + 0.34f * (a1j.x - a1i.x), sy = d.y + 0.34f * (a1j.y - a1i.y), sz = d.z + 0.34f * (a1j.z - a1i.z);
+	return sx * sx + sy * sy + sz * sz < a.stk_r2;
+}
+
 // the minimum-image separation vector of a listed pair (the reference's FP32 geometry, explicit
 // fused multiply-adds), the image picked as in sqr_min_image_inv: the same integer as the IEEE
 // quotient's rint for any pair closer than the Verlet radius, so the same vector
@@ -382,7 +392,7 @@ __global__ void __launch_bounds__(256) k_neighbours(ListArgs a) {
 		bki = a.fback[i];
 	}
 	const unsigned below = (1u << lane) - 1u;
-	int cnt = 0, nev = 0, nbase = 0, nstk = 0, ndh = 0;
+	int cnt = 0, nev = 0, npt = 0, ndh = 0;
 	for(int t0 = 0; t0 < total; t0 += 32) {
 		const int t = t0 + lane;
 		// the cell holding candidate t: the first lane whose inclusive count exceeds t
@@ -393,7 +403,7 @@ __global__ void __launch_bounds__(256) k_neighbours(ListArgs a) {
 			if(v <= t) l += step;
 		}
 		const int cs_l = __shfl_sync(0xffffffffu, cs, l & 31), ex_l = __shfl_sync(0xffffffffu, excl, l & 31);
-		bool hit = false, hev = false, hbase = false, hstk = false, hdh = false;
+		bool hit = false, hev = false, hpt = false, hdh = false;
 		int j = -1;
 		if(t < total) {
 			j = a.cell_list[cs_l + (t - ex_l)];
@@ -408,13 +418,7 @@ __global__ void __launch_bounds__(256) k_neighbours(ListArgs a) {
 					if(terms && d2 < a.ev_r2) {
 						const float4 a1j = a.fa1[j];
 						hev = ev_sites_near(a, d, a1i, bki, a1j, bkj);
-						// base sites at 0.4 a1, stacking sites at 0.34 a1 from the centres
-						const float bx = d.x + 0.4f * (a1j.x - a1i.x), by = d.y + 0.4f * (a1j.y - a1i.y),
-								bz = d.z + 0.4f * (a1j.z - a1i.z);
-						hbase = bx * bx + by * by + bz * bz < a.base_r2;
-						const float sx = d.x + 0.34f * (a1j.x - a1i.x), sy = d.y + 0.34f * (a1j.y - a1i.y),
-								sz = d.z + 0.34f * (a1j.z - a1i.z);
-						hstk = sx * sx + sy * sy + sz * sz < a.stk_r2;
+						hpt = pair_sites_near(a, d, a1i, a1j);
 					}
 				}
 			}
@@ -434,23 +438,17 @@ __global__ void __launch_bounds__(256) k_neighbours(ListArgs a) {
 			ndh += __popc(md);
 		}
 		if(terms) {
-			const unsigned me = __ballot_sync(0xffffffffu, hev), mb = __ballot_sync(0xffffffffu, hbase),
-					ms = __ballot_sync(0xffffffffu, hstk);
+			const unsigned me = __ballot_sync(0xffffffffu, hev), mp = __ballot_sync(0xffffffffu, hpt);
 			if(hev) {
 				const int k = nev + __popc(me & below);
 				if(k < a.ev_cap) a.ev_nb[(long long) k * N + i] = j;
 			}
-			if(hbase) {
-				const int k = nbase + __popc(mb & below);
-				if(k < a.base_cap) a.base_nb[(long long) k * N + i] = j;
-			}
-			if(hstk) {
-				const int k = nstk + __popc(ms & below);
-				if(k < a.stk_cap) a.stk_nb[(long long) k * N + i] = j;
+			if(hpt) {
+				const int k = npt + __popc(mp & below);
+				if(k < a.pt_cap) a.pt_nb[(long long) k * N + i] = j;
 			}
 			nev += __popc(me);
-			nbase += __popc(mb);
-			nstk += __popc(ms);
+			npt += __popc(mp);
 		}
 	}
 	if(lane != 0) return;
@@ -460,15 +458,13 @@ __global__ void __launch_bounds__(256) k_neighbours(ListArgs a) {
 	if(dhl) a.dh_n[i] = ndh;
 	a.list_pos[i] = r;
 	if(terms) {
-		if(nev > a.ev_cap || nbase > a.base_cap || nstk > a.stk_cap) atomicOr(a.status, OXGB_ERR_NEIGH_OVERFLOW);
+		if(nev > a.ev_cap || npt > a.pt_cap) atomicOr(a.status, OXGB_ERR_NEIGH_OVERFLOW);
 		if(a.term_max) {  // read first: the maxima rarely grow, so few atomics reach them
 			if(nev > a.term_max[0]) atomicMax(a.term_max, nev);
-			if(nbase > a.term_max[1]) atomicMax(a.term_max + 1, nbase);
-			if(nstk > a.term_max[2]) atomicMax(a.term_max + 2, nstk);
+			if(npt > a.term_max[1]) atomicMax(a.term_max + 1, npt);
 		}
 		a.ev_n[i] = nev;
-		a.base_n[i] = nbase;
-		a.stk_n[i] = nstk;
+		a.pt_n[i] = npt;
 		a.list_a1[i] = a1i;
 		a.list_back[i] = bki;
 	}
@@ -501,7 +497,7 @@ __global__ void __launch_bounds__(128) k_neighbours_thread(ListArgs a) {
 		a1i = a.fa1[i];
 		bki = a.fback[i];
 	}
-	int cnt = 0, nev = 0, nbase = 0, nstk = 0, ndh = 0;
+	int cnt = 0, nev = 0, npt = 0, ndh = 0;
 	const float inv_box = __frcp_rn(g.box);
 	// the 27 cells in the serial order (dz, dy, dx from -1 to 1), wrapped without integer division.
 	// The cells x = cx - 1, cx, cx + 1 of a (z, y) row are consecutive cells, so their segments
@@ -541,18 +537,9 @@ __global__ void __launch_bounds__(128) k_neighbours_thread(ListArgs a) {
 					if(nev < a.ev_cap) a.ev_nb[(long long) nev * N + i] = j;
 					nev++;
 				}
-				// base sites at 0.4 a1, stacking sites at 0.34 a1 from the centres
-				const float bx = d.x + 0.4f * (a1j.x - a1i.x), by = d.y + 0.4f * (a1j.y - a1i.y),
-						bz = d.z + 0.4f * (a1j.z - a1i.z);
-				if(bx * bx + by * by + bz * bz < a.base_r2) {
-					if(nbase < a.base_cap) a.base_nb[(long long) nbase * N + i] = j;
-					nbase++;
-				}
-				const float sx = d.x + 0.34f * (a1j.x - a1i.x), sy2 = d.y + 0.34f * (a1j.y - a1i.y),
-						sz = d.z + 0.34f * (a1j.z - a1i.z);
-				if(sx * sx + sy2 * sy2 + sz * sz < a.stk_r2) {
-					if(nstk < a.stk_cap) a.stk_nb[(long long) nstk * N + i] = j;
-					nstk++;
+				if(pair_sites_near(a, d, a1i, a1j)) {
+					if(npt < a.pt_cap) a.pt_nb[(long long) npt * N + i] = j;
+					npt++;
 				}
 			}
 		}
@@ -563,15 +550,13 @@ __global__ void __launch_bounds__(128) k_neighbours_thread(ListArgs a) {
 	if(dhl) a.dh_n[i] = ndh;
 	a.list_pos[i] = r;
 	if(terms) {
-		if(nev > a.ev_cap || nbase > a.base_cap || nstk > a.stk_cap) atomicOr(a.status, OXGB_ERR_NEIGH_OVERFLOW);
+		if(nev > a.ev_cap || npt > a.pt_cap) atomicOr(a.status, OXGB_ERR_NEIGH_OVERFLOW);
 		if(a.term_max) {
 			if(nev > a.term_max[0]) atomicMax(a.term_max, nev);
-			if(nbase > a.term_max[1]) atomicMax(a.term_max + 1, nbase);
-			if(nstk > a.term_max[2]) atomicMax(a.term_max + 2, nstk);
+			if(npt > a.term_max[1]) atomicMax(a.term_max + 1, npt);
 		}
 		a.ev_n[i] = nev;
-		a.base_n[i] = nbase;
-		a.stk_n[i] = nstk;
+		a.pt_n[i] = npt;
 		a.list_a1[i] = a1i;
 		a.list_back[i] = bki;
 	}
@@ -653,10 +638,10 @@ __global__ void __launch_bounds__(128) k_neighbours_group(ListArgs a) {
 		bki = a.fback[i];
 	}
 	const unsigned below = ((1u << lane) - 1u) & gmask;
-	int cnt = 0, nev = 0, nbase = 0, nstk = 0, ndh = 0;
+	int cnt = 0, nev = 0, npt = 0, ndh = 0;
 	for(int t0 = 0; t0 < total; t0 += K) {
 		const int t = t0 + sub;
-		bool hit = false, hev = false, hbase = false, hstk = false, hdh = false;
+		bool hit = false, hev = false, hpt = false, hdh = false;
 		int j = -1;
 		if(t < total) {
 			// the cell holding candidate t: the last one whose first candidate is at most t
@@ -676,13 +661,7 @@ __global__ void __launch_bounds__(128) k_neighbours_group(ListArgs a) {
 					if(terms && d2 < a.ev_r2) {
 						const float4 a1j = a.fa1[j];
 						hev = ev_sites_near(a, d, a1i, bki, a1j, bkj);
-						// base sites at 0.4 a1, stacking sites at 0.34 a1 from the centres
-						const float bx = d.x + 0.4f * (a1j.x - a1i.x), by = d.y + 0.4f * (a1j.y - a1i.y),
-								bz = d.z + 0.4f * (a1j.z - a1i.z);
-						hbase = bx * bx + by * by + bz * bz < a.base_r2;
-						const float sx = d.x + 0.34f * (a1j.x - a1i.x), sy2 = d.y + 0.34f * (a1j.y - a1i.y),
-								sz = d.z + 0.34f * (a1j.z - a1i.z);
-						hstk = sx * sx + sy2 * sy2 + sz * sz < a.stk_r2;
+						hpt = pair_sites_near(a, d, a1i, a1j);
 					}
 				}
 			}
@@ -702,23 +681,17 @@ __global__ void __launch_bounds__(128) k_neighbours_group(ListArgs a) {
 			ndh += __popc(md);
 		}
 		if(terms) {
-			const unsigned me = __ballot_sync(gmask, hev) & gmask, mb = __ballot_sync(gmask, hbase) & gmask,
-					ms = __ballot_sync(gmask, hstk) & gmask;
+			const unsigned me = __ballot_sync(gmask, hev) & gmask, mp = __ballot_sync(gmask, hpt) & gmask;
 			if(hev) {
 				const int k = nev + __popc(me & below);
 				if(k < a.ev_cap) a.ev_nb[(long long) k * N + i] = j;
 			}
-			if(hbase) {
-				const int k = nbase + __popc(mb & below);
-				if(k < a.base_cap) a.base_nb[(long long) k * N + i] = j;
-			}
-			if(hstk) {
-				const int k = nstk + __popc(ms & below);
-				if(k < a.stk_cap) a.stk_nb[(long long) k * N + i] = j;
+			if(hpt) {
+				const int k = npt + __popc(mp & below);
+				if(k < a.pt_cap) a.pt_nb[(long long) k * N + i] = j;
 			}
 			nev += __popc(me);
-			nbase += __popc(mb);
-			nstk += __popc(ms);
+			npt += __popc(mp);
 		}
 	}
 	if(sub != 0) return;
@@ -728,48 +701,54 @@ __global__ void __launch_bounds__(128) k_neighbours_group(ListArgs a) {
 	if(dhl) a.dh_n[i] = ndh;
 	a.list_pos[i] = r;
 	if(terms) {
-		if(nev > a.ev_cap || nbase > a.base_cap || nstk > a.stk_cap) atomicOr(a.status, OXGB_ERR_NEIGH_OVERFLOW);
+		if(nev > a.ev_cap || npt > a.pt_cap) atomicOr(a.status, OXGB_ERR_NEIGH_OVERFLOW);
 		if(a.term_max) {
 			if(nev > a.term_max[0]) atomicMax(a.term_max, nev);
-			if(nbase > a.term_max[1]) atomicMax(a.term_max + 1, nbase);
-			if(nstk > a.term_max[2]) atomicMax(a.term_max + 2, nstk);
+			if(npt > a.term_max[1]) atomicMax(a.term_max + 1, npt);
 		}
 		a.ev_n[i] = nev;
-		a.base_n[i] = nbase;
-		a.stk_n[i] = nstk;
+		a.pt_n[i] = npt;
 		a.list_a1[i] = a1i;
 		a.list_back[i] = bki;
 	}
 }
 
-// For every base / stack list entry (k, i) with partner j above i by caller's index (i owns the
-// pair, as in an unsorted run): where i sits in
-// j's list (the lists are symmetric: the pair criteria are exactly symmetric in FP32).  One
-// thread per nucleotide and term (blocks 0 .. base_blocks - 1: base lists).
-__global__ void k_term_pos(ListArgs a, int base_blocks) {
+// The pair-term entries owned by a group of 32 nucleotides, together (ForceArgs::own): of every pair
+// the nucleotide i with the lower caller's index keeps the entry, with the pair's position k in its
+// list and m in the partner's (the lists are symmetric).  A block per group, four lanes per nucleotide
+// over its entries; the search of the partner's list reads four entries at a time (a serial walk is a
+// chain of dependent loads).  Their order within the group does not matter to the results.  A group
+// that straddles systems is rebuilt if one of them is: the other lists are as they were.
+__global__ void __launch_bounds__(4 * PAIR_GROUP) k_pair_own(ListArgs a) {
 	SKIP_IF_FRESH(a);
-	const bool is_base = (int) blockIdx.x < base_blocks;
-	const int i = (is_base ? blockIdx.x : blockIdx.x - base_blocks) * blockDim.x + threadIdx.x;
-	if(i >= a.N || !rebuilt(a, sys_of(a, i))) return;
+	__shared__ int count;
+	if(threadIdx.x == 0) count = 0;
+	const int g = blockIdx.x, i = g * PAIR_GROUP + (int) threadIdx.x / 4;
+	if(!__syncthreads_or(i < a.N && rebuilt(a, sys_of(a, i)))) return;
 	const long long N = a.N;
-	const int cap = is_base ? a.base_cap : a.stk_cap;
-	const int *nb = is_base ? a.base_nb : a.stk_nb;
-	int *pos = is_base ? a.base_pos : a.stk_pos;
-	const int n = min(is_base ? a.base_n[i] : a.stk_n[i], cap);
-	for(int k = 0; k < n; k++) {
-		const int j = nb[(long long) k * N + i];
-		int r = -1;
-		if(id_of(a, j) > id_of(a, i)) {
-			const int nj = min(is_base ? a.base_n[j] : a.stk_n[j], cap);
-			for(int m = 0; m < nj; m++)
-				if(nb[(long long) m * N + j] == i) {
-					r = m;
-					break;
-				}
-			if(r < 0) atomicOr(a.status, OXGB_ERR_NEIGH_OVERFLOW);  // an asymmetric (overflowed) list
+	int2 *own = a.own + (long long) g * PAIR_GROUP * a.pt_cap;
+	if(i < a.N) {
+		const int n = min(a.pt_n[i], a.pt_cap);
+		const int key = id_of(a, i);
+		for(int k = threadIdx.x & 3; k < n; k += 4) {
+			const int j = a.pt_nb[(long long) k * N + i];
+			if(id_of(a, j) < key) continue;
+			int m = 255;
+			const int nj = min(a.pt_n[j], a.pt_cap);
+			for(int u = 0; u < nj && m == 255; u += 4) {
+				int e[4];
+#pragma unroll
+				for(int v = 0; v < 4; v++) e[v] = u + v < nj ? a.pt_nb[(long long) (u + v) * N + j] : -1;
+#pragma unroll
+				for(int v = 0; v < 4; v++)
+					if(e[v] == i) m = u + v;
+			}
+			if(m == 255) atomicOr(a.status, OXGB_ERR_NEIGH_OVERFLOW);  // an asymmetric (overflowed) list
+			own[atomicAdd(&count, 1)] = make_int2(j, k | (m << 8) | ((int) threadIdx.x / 4) << 16);
 		}
-		pos[(long long) k * N + i] = r;
 	}
+	__syncthreads();
+	if(threadIdx.x == 0) a.own_n[g] = count;
 }
 
 // runs after every other list kernel: counts the build and clears the requests
@@ -828,7 +807,7 @@ cudaError_t launch_list_build(const ListArgs &a, cudaStream_t s) {
 		k_neighbours<<<(int) ((warps + tpb - 1) / tpb), tpb, 0, s>>>(a);
 	}
 	}
-	if(a.base_pos && a.stk_pos) k_term_pos<<<2 * gp, tpb, 0, s>>>(a, gp);
+	if(a.own) k_pair_own<<<(a.N + PAIR_GROUP - 1) / PAIR_GROUP, 4 * PAIR_GROUP, 0, s>>>(a);
 	k_list_done<<<1, 256, 0, s>>>(a);
 	return cudaGetLastError();
 }
