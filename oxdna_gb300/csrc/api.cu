@@ -404,6 +404,7 @@ struct oxgb_md {
 	double4_32a *posd = nullptr, *veld = nullptr, *Ld = nullptr, *quatd = nullptr;
 	float4 *pos_hi = nullptr, *pos_lo = nullptr, *fa1 = nullptr, *fa3 = nullptr, *fback = nullptr, *list_pos = nullptr;
 	float4 *fa1lo = nullptr, *fbacklo = nullptr;  // remainders of fa1 / fback (FP32 engines)
+	int4 *site_back = nullptr, *site_base = nullptr;  // fixed-point sites (FP32 engines)
 	float4 *list_a1 = nullptr, *list_back = nullptr;
 	int2 *bonds = nullptr;
 	void *F = nullptr, *T = nullptr, *bond_f = nullptr, *bond_tp = nullptr, *bond_tq = nullptr;
@@ -469,7 +470,7 @@ struct oxgb_md {
 		if(gexec) cudaGraphExecDestroy(gexec);
 		free_layout();
 		for(void *p : {(void *) posd, (void *) veld, (void *) Ld, (void *) quatd, (void *) pos_hi, (void *) pos_lo, (void *) fa1, (void *) fa3,
-					(void *) fback, (void *) fa1lo, (void *) fbacklo, (void *) list_pos, (void *) list_a1, (void *) list_back, (void *) bonds, F, T, Fe, Te, bond_f,
+					(void *) fback, (void *) fa1lo, (void *) fbacklo, (void *) site_back, (void *) site_base, (void *) list_pos, (void *) list_a1, (void *) list_back, (void *) bonds, F, T, Fe, Te, bond_f,
 					bond_tp, bond_tq, edge_acc, d_tab, (void *) d_sys, (void *) d_sys_off, (void *) d_sys_stale, (void *) d_chunk_sys,
 					(void *) d_chunk_first, (void *) d_sys_chunk0, (void *) d_sys_par, (void *) d_sys_seed, (void *) status,
 					(void *) flag, (void *) step, (void *) esplit, (void *) sums, (void *) bussi_partials, (void *) bussi_state,
@@ -544,6 +545,9 @@ static StepArgs step_args(oxgb_md *h, int step_offset = 0) {
 	a.fback = h->fback;
 	a.fa1lo = h->fa1lo;
 	a.fbacklo = h->fbacklo;
+	a.site_back = h->site_back;
+	a.site_base = h->site_base;
+	a.table = h->d_tab;
 	a.bonds = h->bonds;
 	a.list_a1 = h->list_a1;
 	a.list_back = h->list_back;
@@ -587,6 +591,8 @@ static ForceArgs force_args(oxgb_md *h, int step_offset = 0, bool engine_step = 
 	a.fback = h->fback;
 	a.fa1lo = h->fa1lo;
 	a.fbacklo = h->fbacklo;
+	a.site_back = h->site_back;
+	a.site_base = h->site_base;
 	a.ev_nb = h->tl.ev_nb;
 	a.ev_n = h->tl.ev_n;
 	a.pt_nb = h->tl.pt_nb;
@@ -853,6 +859,8 @@ extern "C" int oxgb_md_create(int n_systems, const int *offsets, const double *b
 	if(!h->dbl) {
 		ok &= cudaMalloc(&h->fa1lo, sizeof(float4) * N) == cudaSuccess;
 		ok &= cudaMalloc(&h->fbacklo, sizeof(float4) * N) == cudaSuccess;
+		ok &= cudaMalloc(&h->site_back, sizeof(int4) * N) == cudaSuccess;
+		ok &= cudaMalloc(&h->site_base, sizeof(int4) * N) == cudaSuccess;
 	}
 	ok &= cudaMalloc(&h->list_a1, sizeof(float4) * N) == cudaSuccess;
 	ok &= cudaMalloc(&h->list_back, sizeof(float4) * N) == cudaSuccess;
@@ -1053,6 +1061,7 @@ static ListArgs md_list_args(oxgb_md *h, int check_flag) {
 		a.st[0] = h->posd, a.st[1] = h->veld, a.st[2] = h->Ld, a.st[3] = h->quatd;
 		a.mir[0] = h->pos_hi, a.mir[1] = h->pos_lo, a.mir[2] = h->fa1, a.mir[3] = h->fa3, a.mir[4] = h->fback;
 		a.mir[5] = h->fa1lo, a.mir[6] = h->fbacklo;
+		a.mir[7] = reinterpret_cast<float4 *>(h->site_back), a.mir[8] = reinterpret_cast<float4 *>(h->site_base);
 		a.bonds_rw = h->bonds;
 		a.scratch = h->sort_scratch;
 		a.cell_hil = h->d_cell_hil;

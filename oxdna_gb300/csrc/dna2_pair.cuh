@@ -31,6 +31,8 @@ struct DNA2Table {
 	R rcut2;
 	R box_hi, box_lo;  // box side as an unevaluated sum hi + lo (exact FP64 value)
 	R inv_box;         // about 1 / box_hi: picks the periodic image (an integer; see LoadMixed::sep)
+	R fix_hi, fix_lo;  // 2^31 / box side as hi + lo, and
+	R fix_unit;        // box side / 2^32: the units of the fixed-point sites (fixed_site)
 	int dh_half_charged_ends, use_mbf, pad0, pad1;
 };
 
@@ -919,70 +921,79 @@ OXGB_HD bool bonded_backbone(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R
 	return ok;
 }
 
-// f4 factor i of the angle between unit vectors u and v (s = 1) or u and -v (s = -1): its value g, its
-// derivative D with respect to the cosine s u.v, and X = u x v.  theta - t0 is formed from the angle to
-// the nearer of +v and -v, so that an angle near pi is never rounded to an ulp of 3.
-template <typename R>
-OXGB_HD void f4_between(const v3<R> &u, const v3<R> &v, R s, int i, R &g, R &D, v3<R> &X) {
-	X = cross(u, v);
-	const R uv = dot(u, v), s2 = dot(X, X), sn = m_sqrt(s2);
-	const R acute = m_atan2(sn, m_fabs(uv));
-	const R d = s * uv < R(0) ? R(3.14159265358979323846 - (double) f4_t0<float>(i)) - acute : acute - f4_t0<R>(i);
-	const R ad = m_fabs(d), far = f4_tc<R>(i) - ad;
-	const bool flat = !(s2 > R(1e-8));
-	const R inv = R(1) / (flat ? R(1) : sn);
-	g = D = R(0);
-	if(ad < f4_tc<R>(i)) {
-		if(ad > f4_ts<R>(i)) {
-			g = f4_b<R>(i) * far * far;
-			D = m_copysign(R(2) * f4_b<R>(i) * far, d) * inv;
-		}
-		else {
-			g = R(1) - f4_a<R>(i) * ad * ad;
-			D = R(2) * f4_a<R>(i) * (flat ? m_copysign(R(1), d) : d * inv);
-		}
-	}
-}
-
-// Stacking, added to b.  E = F1(r) f4(theta4) f4(theta5) f4(theta6) f5(cos phi1) f5(cos phi2), r between
-// the stacking sites.  Each factor's derivative acts where its argument lives: theta5, theta6 and the
-// radial part on the stacking sites; phi1 and phi2, the angles of a2 and b2 to the vector w between the
-// unmodified backbone sites (POS_BACK along a1), on those sites; and each on the axis it turns.  (The
-// reference writes the phi terms out in the stacking-site vector, DNAInteraction.cpp:600-690: the same
-// forces in some 150 more operations.)
+// stacking, added to b
 template <typename R, class X = NoRefine>
 OXGB_HD void bonded_stacking(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R> &q, const Sep<R> &sep, BondOut<R> &b,
 		const X &xr = X{}) {
 	const v3<R> r = sep.plain();
-	const v3<R> w = r + (q.a1 - p.a1) * R(OXM_POS_BACK);
-	const R iw = m_rcp(m_sqrt(dot(w, w)));
-	const v3<R> wd = w * iw;
+	b.split[2] = R(0);
+	const v3<R> a1 = p.a1, a2 = p.a2, a3 = p.a3, b1 = q.a1, b2 = q.a2, b3 = q.a3;
+	const v3<R> rbackref = r + b1 * R(OXM_POS_BACK) - a1 * R(OXM_POS_BACK);
+	const R rbr = m_sqrt(dot(rbackref, rbackref));
 	const v3<R> rstack = site_vec(sep, q.stack, p.stack);
-	const R rs = m_sqrt(dot(rstack, rstack)), ir = m_rcp(rs);
+	const R rsm = m_sqrt(dot(rstack, rstack));
 	R rl = R(0);
-	if constexpr(X::on && sizeof(R) == 4) rl = site_dist_remainder(sep, p, xr.lo(0), q, xr.lo(1), true, rs);
-	const v3<R> rd = rstack * ir;
-	const R cp1 = dot(p.a2, wd), cp2 = dot(q.a2, wd);
-	R F, FD, g4, d4, g5, d5, g6, d6, h1, h1d, h2, h2d;
-	v3<R> x4, x5, x6;
-	f1_both(P, rs, OXM_F1_ST, q.type, p.type, F, FD, rl);
-	f4_between(p.a3, q.a3, R(1), OXM_F4_ST_T4, g4, d4, x4);
-	f4_between(p.a3, rd, R(-1), OXM_F4_ST_T5, g5, d5, x5);
-	f4_between(q.a3, rd, R(-1), OXM_F4_ST_T5, g6, d6, x6);
+	if constexpr(X::on && sizeof(R) == 4) rl = site_dist_remainder(sep, p, xr.lo(0), q, xr.lo(1), true, rsm);
+	const v3<R> rd = rstack * (R(1) / rsm);
+	const R c4 = dot(a3, b3), c5 = dot(a3, rd), c6 = -dot(b3, rd);
+	const R cp1 = dot(a2, rbackref) / rbr, cp2 = dot(b2, rbackref) / rbr;
+	R F1, F1D, g4, d4, g5, d5, g6, d6, h1, h1d, h2, h2d;
+	f1_both(P, rsm, OXM_F1_ST, q.type, p.type, F1, F1D, rl);
+	const R s4 = sin_between(a3, b3), s5 = sin_between(a3, rd), s6 = sin_between(b3, rd);
+	f4_both(c4, s4, OXM_F4_ST_T4, g4, d4);
+	f4_both(-c5, s5, OXM_F4_ST_T5, g5, d5);
+	f4_both(c6, s6, OXM_F4_ST_T5, g6, d6);
 	f5_both(cp1, OXM_F5_PHI1, h1, h1d);
 	f5_both(cp2, OXM_F5_PHI2, h2, h2d);
-	const R g = g4 * g5 * g6, h = h1 * h2, e = F * g * h;
+	d4 = -d4;
+	d5 = -d5;
+	d6 = -d6;
+	const R e = F1 * g4 * g5 * g6 * h1 * h2;
 	b.split[2] = e;
 	if(e != R(0)) {
-		const R Fh = F * h, Fg = F * g;
-		const R e4 = Fh * d4 * g5 * g6, e5 = Fh * g4 * d5 * g6, e6 = Fh * g4 * g5 * d6;
-		const R k1 = Fg * h1d * h2, k2 = Fg * h1 * h2d;
-		// on q's stacking site, and on q's unmodified backbone site
-		const v3<R> fs = (p.a3 - rd * dot(p.a3, rd)) * (e5 * ir) + (q.a3 - rd * dot(q.a3, rd)) * (e6 * ir) - rd * (FD * g * h);
-		const v3<R> fw = (wd * cp1 - p.a2) * (k1 * iw) + (wd * cp2 - q.a2) * (k2 * iw);
-		b.f += fs + fw;
-		b.tp += x5 * e5 - x4 * e4 - cross(p.a2, wd) * k1 - cross(p.stack, fs) - cross(p.a1, fw) * R(OXM_POS_BACK);
-		b.tq += x6 * e6 + x4 * e4 - cross(q.a2, wd) * k2 + cross(q.stack, fs) + cross(q.a1, fw) * R(OXM_POS_BACK);
+		const R gam = R(OXM_POS_STACK) - R(OXM_POS_BACK);
+		const R rbr3 = rbr * rbr * rbr;
+		v3<R> force = rd * (-(F1D * g4 * g5 * g6 * h1 * h2));
+		force -= (a3 - rd * c5) * (F1 * g4 * d5 * g6 * h1 * h2 / rsm);
+		force -= (b3 + rd * c6) * (F1 * g4 * g5 * d6 * h1 * h2 / rsm);
+
+		const R ra2 = dot(rd, a2), ra1 = dot(rd, a1), rb1 = dot(rd, b1), a2b1 = dot(a2, b1);
+		const R par1 = rsm * ra2 - a2b1 * gam;
+		const R dc1dr = (rsm * rsm * ra2 - ra2 * rbr * rbr - rsm * (a2b1 + ra2 * (-ra1 + rb1)) * gam + a2b1 * (-ra1 + rb1) * gam * gam) / rbr3;
+		const R dc1dra1 = rsm * gam * par1 / rbr3;
+		const R dc1dra2 = -rsm / rbr;
+		const R dc1drb1 = -rsm * gam * par1 / rbr3;
+		const R dc1da1b1 = -gam * gam * par1 / rbr3;
+		const R dc1da2b1 = gam / rbr;
+		const R fp1 = -F1 * g4 * g5 * g6 * h1d * h2;
+		force -= (rd * dc1dr + ((a2 - rd * ra2) * dc1dra2 + (a1 - rd * ra1) * dc1dra1 + (b1 - rd * rb1) * dc1drb1) * (R(1) / rsm)) * fp1;
+
+		const R sb2 = dot(rd, b2), sb1 = dot(rd, b1), sa1 = dot(rd, a1), b2a1 = dot(b2, a1);
+		const R par2 = rsm * sb2 + b2a1 * gam;
+		const R dc2dr = (par2 * (rsm + (sa1 - sb1) * gam) - sb2 * rbr * rbr) / rbr3;
+		const R dc2dra1 = -rsm * gam * (rsm * sb2 + b2a1 * gam) / rbr3;
+		const R dc2dra2 = -rsm / rbr;
+		const R dc2drb1 = rsm * gam * par2 / rbr3;
+		const R dc2da1b1 = -gam * gam * par2 / rbr3;
+		const R dc2da2b1 = -gam / rbr;
+		const R fp2 = -F1 * g4 * g5 * g6 * h1 * h2d;
+		force -= (rd * dc2dr + ((b2 - rd * sb2) * dc2dra2 + (b1 - rd * sb1) * dc2dra1 + (a1 - rd * sa1) * dc2drb1) * (R(1) / rsm)) * fp2;
+
+		b.f += force;
+		const v3<R> t4dir = cross(b3, a3);
+		const R tm4 = F1 * d4 * g5 * g6 * h1 * h2;
+		const v3<R> pure1 = cross(a2, b1) * (fp1 * dc1da2b1) + cross(a1, b1) * (fp1 * dc1da1b1);
+		const v3<R> pure2 = cross(a1, b2) * (fp2 * dc2da2b1) + cross(a1, b1) * (fp2 * dc2da1b1);
+		v3<R> tq = cross(q.stack, force) + t4dir * tm4;
+		tq += cross(rd, b3) * (F1 * g4 * g5 * d6 * h1 * h2);
+		tq += cross(rd, b1) * (fp1 * dc1drb1) + pure1;
+		tq += cross(rd, b2) * (fp2 * dc2dra2) + cross(rd, b1) * (fp2 * dc2dra1) + pure2;
+		b.tq += tq;
+		v3<R> tp = -cross(p.stack, force) - t4dir * tm4;
+		tp -= cross(rd, a3) * (-(F1 * g4 * d5 * g6 * h1 * h2));
+		tp += cross(rd, a2) * (fp1 * dc1dra2) + cross(rd, a1) * (fp1 * dc1dra1) - pure1;
+		tp += cross(rd, a1) * (fp2 * dc2drb1) - pure2;
+		b.tp += tp;
 	}
 }
 

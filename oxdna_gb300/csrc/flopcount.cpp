@@ -37,7 +37,6 @@ inline bool operator==(CF a, CF b) { return a.v == b.v; }
 
 namespace oxgb {
 inline CF m_sqrt(CF x) { g_sfu += 1; return CF(std::sqrt(x.v)); }
-inline CF m_rcp(CF x) { return CF(1.f) / x; }
 inline CF m_exp(CF x) { g_sfu += 1; return CF(std::exp(x.v)); }
 inline CF m_expm1(CF x) { g_sfu += 1; return CF(std::expm1(x.v)); }
 inline CF m_log(CF x) { g_sfu += 1; return CF(std::log(x.v)); }

@@ -611,42 +611,11 @@ __device__ __forceinline__ void bonded_block(const ForceArgs &a, const Loader &l
 // per-lane compensated sums of a nucleotide's pair terms; ENERGY = false leaves the energies out
 // (an MD step needs only forces and torques: the energy arithmetic of the pair functions is then
 // dead code)
-// Terms of bounded size (Debye-Hueckel, excluded volume) go to a plain per-lane sum when
-// OXGB_NB_PLAIN_SHORT is set: a lane adds only a few of them, whose rounding is far below the
-// compensated sums of the large bonded and pair terms; they join the compensated sum before the
-// group reduction.
-#ifndef OXGB_NB_PLAIN_SHORT
-#define OXGB_NB_PLAIN_SHORT 0
-#endif
-
 template <typename R, bool SPLIT, bool ENERGY = true>
 struct SplitAcc {
 	KahanV<R> F, T;
-	v3<R> Fp, Tp;
 	R E, Ec, Eh, Ehc;
 	R split[N_TERMS];
-	__device__ __forceinline__ void add_short(const PairOut<R> &o) {
-		if(!OXGB_NB_PLAIN_SHORT) {
-			add(o);
-			return;
-		}
-		Fp = Fp + o.F;
-		Tp = Tp + o.T;
-		if(ENERGY) {
-			KahanV<R>::kadd(E, Ec, o.E);
-			KahanV<R>::kadd(Eh, Ehc, o.Ehb);
-		}
-		if(SPLIT) {
-#pragma unroll
-			for(int k = 0; k < N_TERMS; k++) split[k] += o.split[k];
-		}
-	}
-	__device__ __forceinline__ void fold_short() {
-		if(OXGB_NB_PLAIN_SHORT) {
-			F.add(Fp);
-			T.add(Tp);
-		}
-	}
 	__device__ __forceinline__ void add(const PairOut<R> &o) {
 		F.add(o.F);
 		T.add(o.T);
@@ -682,18 +651,18 @@ __device__ __forceinline__ void atomic_add_v4(double4_32a *p, const double4_32a 
 //      3     a3  b3  +u.v     theta4
 //      4     b3  rd  -u.v     theta7, theta7, theta6
 //      5     a3  rd  +u.v     theta8, theta8, theta5
-// (a: axes of p, b: axes of q, rd: unit vector from p's site to q's).  With s the sign of the cosine,
-// X = u x v and e_k = F prod_(j != k) g_j dg_k/dcos, the factor's torque on p is -s e_k X (none where
-// u is q's and v = rd) and its force on q's site -s e_k (u - (u.v) v) / r (only where v = rd).  So a
-// term's angular factors are evaluated by eight lanes, one factor each by the same instructions, with
-// the product of the others' factors and the six sums by butterflies of shuffles.
+// (a: axes of p, b: axes of q, rd: unit vector from p's site to q's; coaxial stacking has theta5 on
+// lane 4 and theta6 on lane 5).  With D = dg/dcos, a factor's share of the forces is F D prod g, the
+// product over the other factors, along a vector of its own: on p's axis it turns, X = u x v; between
+// the sites, u less its part along rd, over r.  So a term's angular factors are evaluated by eight
+// lanes, one factor each by the same instructions, which hand each other their g.
 //
 // A block takes its pairs through four stages, each dealt to as many threads as it has work for, with
 // what they pass on in shared memory:
 //   1  screening: a thread per owned entry; pairs with live terms are queued, an item per term;
 //   2  a thread per item: separation, site distance, radial factor;
-//   3  eight lanes per item: the angular factors (lane 6 adds the radial force);
-//   4  a thread per pair: forces and torques of both nucleotides into the pair's two slots.
+//   3  eight lanes per item: the angular factors, each lane's vectors and their coefficients;
+//   4  a thread per pair: the sums, forces and torques of both nucleotides into the pair's two slots.
 // Why: one lane per pair was a chain of some 1,500 dependent instructions (nine angles one after the
 // other), and since a chip full of such warps has nothing else to issue, the launch lasted as long as
 // that chain.
@@ -702,7 +671,7 @@ struct __align__(16) Angular {
 	R a, b, t0, ts, tc;  // f4 (see f4_both); a = b = 0 with a support that covers every angle: 1
 	R both;              // 1: f4(theta) + f4(pi - theta)
 	R harm;              // strength of the coaxial theta1 harmonic beyond sb
-	R pi_t0;             // pi - t0 (from the exact pi): theta - t0 of an obtuse theta is this less pi - theta
+	R pad;
 };
 template <typename R>
 struct AngularTable {
@@ -717,15 +686,14 @@ constexpr AngularTable<R> angular_table() {
 			{OXM_F4_CR_T1, OXM_F4_CR_T2, OXM_F4_CR_T2, OXM_F4_CR_T4, OXM_F4_CR_T7, OXM_F4_CR_T7},
 			{OXM_F4_CX_T1, -1, -1, OXM_F4_CX_T4, OXM_F4_CX_T5, OXM_F4_CX_T5}};
 	const int both[3][6] = {{0, 0, 0, 0, 0, 0}, {0, 0, 0, 1, 1, 1}, {0, 0, 0, 0, 1, 1}};
-	const double pi = 3.14159265358979323846;
 	AngularTable<R> r{};
 	for(int m = 0; m < 3; m++)
 		for(int l = 0; l < 8; l++) {
 			const int i = l < 6 ? set[m][l] : -1;
-			if(i < 0) r.t[m][l] = Angular<R>{R(0), R(0), R(0), R(16), R(32), R(0), R(0), R(pi)};
+			if(i < 0) r.t[m][l] = Angular<R>{R(0), R(0), R(0), R(16), R(32), R(0), R(0), R(0)};
 			else
 				r.t[m][l] = Angular<R>{R(A[i]), R(B[i]), R(T0[i]), R(TS[i]), R(TC[i]), R(both[m][l]),
-						i == OXM_F4_CX_T1 ? R(OXM_CXST_THETA1_SA) : R(0), R(pi - (double) T0[i])};
+						i == OXM_F4_CX_T1 ? R(OXM_CXST_THETA1_SA) : R(0), R(0)};
 		}
 	return r;
 }
@@ -734,26 +702,31 @@ __device__ const AngularTable<double> g_angular_d = angular_table<double>();
 __device__ __forceinline__ const Angular<float> &angular_of(int term, int lane, float) { return g_angular_f.t[term][lane]; }
 __device__ __forceinline__ const Angular<double> &angular_of(int term, int lane, double) { return g_angular_d.t[term][lane]; }
 
-// one f4 factor at the angle theta = t0 + d: its value, and df/dtheta / sin(theta) (inv = 1 / sin;
-// flat: the angle is within 1e-4 of 0 or pi, where d / sin counts as +-1, as in f4_both)
+// f4_both (its FP32 form, theta = atan2(sin, cos)) with the factor's constants as values
 template <typename R>
-__device__ __forceinline__ void angular_factor(const Angular<R> &c, R d, R inv, bool flat, R &f, R &slope) {
-	const R ad = m_fabs(d), far = c.tc - ad;
-	const bool inner = ad <= c.ts, in = ad < c.tc;
-	f = inner ? R(1) - c.a * ad * ad : c.b * far * far;
-	slope = inner ? R(-2) * c.a * (flat ? m_copysign(R(1), d) : d * inv) : -m_copysign(R(2) * c.b * far, d) * inv;
-	if(!in) f = slope = R(0);
-}
-
-template <typename R>
-__device__ __forceinline__ R shfl8(R v, int off) {
-	return __shfl_xor_sync(0xffffffffu, v, off, 8);
-}
-template <typename R>
-__device__ __forceinline__ R sum8(R v) {
-	v += shfl8(v, 1);
-	v += shfl8(v, 2);
-	return v + shfl8(v, 4);
+__device__ __forceinline__ void angular_factor(const Angular<R> &k, R c, R sn, R &f, R &fd) {
+	const R t = m_atan2(sn, c), s2 = sn * sn;
+	R tt0 = t - k.t0;
+	const R m = tt0 < R(0) ? R(-1) : R(1);
+	tt0 = m_fabs(tt0);
+	R dsin;
+	if(tt0 > k.ts) {
+		f = k.b * (k.tc - tt0) * (k.tc - tt0);
+		dsin = m * (R(2) * k.b) * (tt0 - k.tc) / sn;
+	}
+	else {
+		f = R(1) - k.a * tt0 * tt0;
+		dsin = s2 > R(1e-8) ? -m * (R(2) * k.a) * tt0 / sn : -m * (R(2) * k.a);
+	}
+	if(!(tt0 < k.tc)) f = dsin = R(0);
+	if(k.harm != R(0)) {
+		const R h = t - R(OXM_CXST_THETA1_SB);
+		if(h >= R(0)) {
+			f += k.harm * h * h;
+			dsin += s2 > R(1e-8) ? R(2) * k.harm * h / sn : R(2) * k.harm;
+		}
+	}
+	fd = -dsin;
 }
 
 // Which terms of pair (p, q) can be non-zero: 1 hydrogen bonding, 2 cross stacking, 4 coaxial stacking.
@@ -798,11 +771,15 @@ constexpr int PAIR_QUEUE = 512 + 3 * 128;  // items waiting (a round of screenin
 template <typename R>
 struct PairItem {
 	R axes[12];            // a1, a3 of p; a1, a3 of q
-	R rd[3], ir, F, FD;    // site direction, 1 / site distance, radial factor and its derivative
+	R rd[3], r, F, FD;     // site direction and distance, radial factor and its derivative
 	R d[6];                // centre separation, hi and lo
-	R out[7];              // force on q's site, torque on p without its lever arm, energy
+	R g[6];                // the angular factors
+	// a vector and its coefficient: the torque axes X of lanes 0 and 3, the force directions of lanes
+	// 1, 2, 4, 5, and the torque axes rd x u of the two of them that turn p
+	R turn[2][4], push[4][4], twist[2][4];
+	R pad;
 };
-static_assert(sizeof(PairItem<float>) == 31 * 4, "an odd number of words");
+static_assert(sizeof(PairItem<float>) == 63 * 4, "an odd number of words");
 
 // stage 2 of item m of pair (i, j), term 0 hydrogen bonding, 1 cross stacking, 2 coaxial stacking
 template <typename R, class Loader>
@@ -817,8 +794,8 @@ __device__ __forceinline__ void pair_radial(const ForceArgs &a, const Loader &ld
 	const bool stack = term == 2;
 	p.stack = p.a1 * R(OXM_POS_STACK), q.stack = q.a1 * R(OXM_POS_STACK);
 	const v3<R> rs = stack ? site_vec(d, q.stack, p.stack) : site_vec(d, q.base, p.base);
-	const R r = m_sqrt(dot(rs, rs)), ir = m_rcp(r);
-	const v3<R> rd = rs * ir;
+	const R r = m_sqrt(dot(rs, rs));
+	const v3<R> rd = rs * (R(1) / r);
 	R rl = R(0);
 	const auto x = ld.refine(i, j);
 	if constexpr(decltype(x)::on) rl = site_dist_remainder(d, p, x.lo(0), q, x.lo(1), stack, r);
@@ -835,57 +812,79 @@ __device__ __forceinline__ void pair_radial(const ForceArgs &a, const Loader &ld
 #pragma unroll
 	for(int k = 0; k < 4; k++) m.axes[3 * k] = ax[k].x, m.axes[3 * k + 1] = ax[k].y, m.axes[3 * k + 2] = ax[k].z;
 	m.rd[0] = rd.x, m.rd[1] = rd.y, m.rd[2] = rd.z;
-	m.ir = ir, m.F = F, m.FD = FD;
+	m.r = r, m.F = F, m.FD = FD;
 	m.d[0] = d.hi.x, m.d[1] = d.hi.y, m.d[2] = d.hi.z, m.d[3] = d.lo.x, m.d[4] = d.lo.y, m.d[5] = d.lo.z;
 }
 
-// stage 3: eight lanes, this one the factor of its lane; the whole warp takes part
+// stage 3: eight lanes (the last two idle), this one the factor of its lane; the whole warp takes part
 template <typename R>
 __device__ __forceinline__ void pair_angles(int term, PairItem<R> &m) {
 	const int sub = threadIdx.x & 7;
-	const bool u_q = sub == 1 || sub == 4;              // u is an axis of q
-	const bool v_rd = sub != 0 && sub != 3 && sub < 6;  // v is the site direction
+	const bool v_rd = sub != 0 && sub != 3;                                  // v is the site direction
+	const bool u_q = sub == 1 || sub == (term == 2 ? 5 : 4);                 // u is an axis of q
 	const R s = (u_q || sub == 0) ? R(-1) : R(1);
 	const Angular<R> c = angular_of(term, sub, R(0));
-	// u: a1 b1 a1 a3 b3 a3; v: b1 rd rd b3 rd rd (word offsets into the item)
-	const R *pu = m.axes + (sub == 1 ? 6 : sub == 4 ? 9 : (sub == 3 || sub == 5) ? 3 : 0);
+	// u: a1 b1 a1 a3 b3 a3 (coaxial stacking: a3 b3 at the end); v: b1 rd rd b3 rd rd
+	const R *pu = m.axes + (sub < 3 ? 0 : 3) + (u_q ? 6 : 0);
 	const R *pv = v_rd ? m.rd : m.axes + (sub == 3 ? 9 : 6);
 	const v3<R> u{pu[0], pu[1], pu[2]}, v{pv[0], pv[1], pv[2]};
 	const v3<R> X = cross(u, v);
-	const R uv = dot(u, v), s2 = dot(X, X), sn = m_sqrt(s2);
-	const bool flat = !(s2 > R(1e-8));
-	const R inv = R(1) / (flat ? R(1) : sn);
-	// From the angle to the nearer of +v and -v: theta or pi - theta, and their distances from t0
-	// without rounding an angle near pi (an ulp of 3 is 2.4e-7, which the factors' slopes carry on)
-	const R acute = m_atan2(sn, m_fabs(uv));
-	const R near = acute - c.t0, far = c.pi_t0 - acute;
-	const bool neg = s * uv < R(0);  // theta is the obtuse one
-	R g, sl, g2, sl2;
-	angular_factor(c, neg ? far : near, inv, flat, g, sl);
-	angular_factor(c, neg ? near : far, inv, flat, g2, sl2);
-	g += c.both * g2;
-	sl -= c.both * sl2;
-	const R h = m_max(neg ? R(3.14159265358979323846 - (double) OXM_CXST_THETA1_SB) - acute : acute - R(OXM_CXST_THETA1_SB), R(0));
-	g += c.harm * h * h;
-	sl += R(2) * c.harm * (flat ? (h > R(0) ? R(1) : R(0)) : h * inv);
-	// the product of the other lanes' factors
-	R all = g, others = R(1);
-#pragma unroll
-	for(int off = 1; off < 8; off <<= 1) {
-		const R z = shfl8(all, off);
-		others *= z;
-		all *= z;
+	const R cs = s * dot(u, v), sn = m_sqrt(dot(X, X));
+	R g, D;
+	angular_factor(c, cs, sn, g, D);
+	if(c.both != R(0)) {
+		R g2, D2;
+		angular_factor(c, -cs, sn, g2, D2);
+		g += g2;
+		D -= D2;
 	}
-	const R F = m.F;
-	const R ek = F * others * -sl;  // F prod_(j != k) g_j dg_k/dcos
-	const R ft = v_rd ? -s * ek * m.ir : R(0), tt = (u_q || sub > 5) ? R(0) : -s * ek;
-	v3<R> f = (u - v * uv) * ft, tq = X * tt;
-	if(sub == 6) f = v3<R>{m.rd[0], m.rd[1], m.rd[2]} * (-(m.FD * all));
-	f.x = sum8(f.x), f.y = sum8(f.y), f.z = sum8(f.z);
-	tq.x = sum8(tq.x), tq.y = sum8(tq.y), tq.z = sum8(tq.z);
-	const R e = F * all;
-	const R out = sub == 0 ? f.x : sub == 1 ? f.y : sub == 2 ? f.z : sub == 3 ? tq.x : sub == 4 ? tq.y : sub == 5 ? tq.z : e;
-	if(sub < 7) m.out[sub] = out;
+	// F g0 .. g5 with this lane's D in the place of its g, a product from the left
+	R z = m.F;
+#pragma unroll
+	for(int l = 0; l < 6; l++) {
+		const R gl = __shfl_sync(0xffffffffu, g, l, 8);
+		z *= l == sub ? D : gl;
+	}
+	if(sub >= 6) return;
+	m.g[sub] = g;
+	if(!v_rd) {
+		R *o = m.turn[sub == 0 ? 0 : 1];
+		o[0] = X.x, o[1] = X.y, o[2] = X.z, o[3] = sub == 0 ? z : -z;
+		return;
+	}
+	const v3<R> w = u_q ? u + v * cs : u - v * cs;
+	R *o = m.push[sub < 3 ? sub - 1 : sub - 2];
+	o[0] = w.x, o[1] = w.y, o[2] = w.z, o[3] = (u_q ? z : -z) / m.r;
+	if(!u_q) {
+		const v3<R> y = cross(v, u);
+		R *t = m.twist[sub < 3 ? 0 : 1];
+		t[0] = y.x, t[1] = y.y, t[2] = y.z, t[3] = z;
+	}
+}
+
+// The force on q's site and the torque on p (without its lever arm) of an evaluated item, and its
+// energy: the sums in the order of hb_term, crst_term and cxst_term
+template <typename R>
+__device__ __forceinline__ R pair_sums(int term, const PairItem<R> &m, v3<R> &f, v3<R> &t) {
+	R e = m.F, ed = m.FD;
+#pragma unroll
+	for(int l = 0; l < 6; l++) e *= m.g[l], ed *= m.g[l];
+	auto vec = [](const R *o) { return v3<R>{o[0], o[1], o[2]}; };
+	f = v3<R>{m.rd[0], m.rd[1], m.rd[2]} * -ed;
+	// hydrogen bonding sums the torque of a3, b3 first, the others that of a1, b1
+	const R *t0 = m.turn[term == 0 ? 1 : 0], *t1 = m.turn[term == 0 ? 0 : 1];
+	t = vec(t0) * t0[3];
+	if(term != 1) t += vec(t1) * t1[3];
+	if(term != 2) {
+#pragma unroll
+		for(int k = 0; k < 2; k++) f += vec(m.push[k]) * m.push[k][3];
+		t += vec(m.twist[0]) * m.twist[0][3];
+	}
+	if(term == 1) t += vec(t1) * t1[3];
+#pragma unroll
+	for(int k = 2; k < 4; k++) f += vec(m.push[k]) * m.push[k][3];
+	t += vec(m.twist[1]) * m.twist[1][3];
+	return e;
 }
 
 // Pair block b (128 threads): the entries owned by G groups of 32 nucleotides, in the four stages above
@@ -966,34 +965,39 @@ __device__ __forceinline__ void pair_block(const ForceArgs &a, const Loader &ld,
 				const int2 w = queue[c0 + m];
 				if(w.y & (1 << 18)) continue;  // taken with the pair's first item
 				const int i = first + (w.y >> 19), j = w.x, k = w.y & 255, mj = (w.y >> 8) & 255;
-				PairOut<R> o{};
+				V4 fi, ti, fj, tj;
+				fi.x = fi.y = fi.z = fi.w = ti.x = ti.y = ti.z = ti.w = R(0);
+				fj = tj = fi;
+				bool any = false;
 				for(int v = m;;) {
-					const PairItem<R> &it4 = item[v];
+					const PairItem<R> &x = item[v];
 					const int term = (queue[c0 + v].y >> 16) & 3;
-					const R e = it4.out[6];
+					v3<R> f, t;
+					const R e = pair_sums<R>(term, x, f, t);
 					if(e != R(0)) {
-						const v3<R> f{it4.out[0], it4.out[1], it4.out[2]};
-						const v3<R> a1{it4.axes[0], it4.axes[1], it4.axes[2]};
+						any = true;
+						const v3<R> a1{x.axes[0], x.axes[1], x.axes[2]};
 						// the lever arm as the loaders form it
 						const v3<R> arm = term == 2 ? a1 * R(OXM_POS_STACK) : sizeof(R) == 4 ? a1 * R(OXM_POS_BASE) :
 								a1 * R(OXM_POS_STACK) * R((double) OXM_POS_BASE / (double) OXM_POS_STACK);
-						o.F -= f;
-						o.T += v3<R>{it4.out[3], it4.out[4], it4.out[5]} - cross(arm, f);
-						add_e<R, SPLIT>(o, term == 0 ? T_HB : term == 1 ? T_CRST : T_CXST, e);
-						if(term == 0) o.Ehb += e;
+						const v3<R> T = t - cross(arm, f);
+						// the potential is invariant under rigid rotations, so the torques balance:
+						// T_j = -T_i + (r_j - r_i) x F_i, the cross product with error-free products
+						const v3<R> c = cross_accurate(Sep<R>{v3<R>{x.d[0], x.d[1], x.d[2]}, v3<R>{x.d[3], x.d[4], x.d[5]}}, -f);
+						fi.x -= f.x, fi.y -= f.y, fi.z -= f.z;
+						fj.x += f.x, fj.y += f.y, fj.z += f.z;
+						ti.x += T.x, ti.y += T.y, ti.z += T.z;
+						tj.x += c.x - T.x, tj.y += c.y - T.y, tj.z += c.z - T.z;
+						if(ENERGY) {
+							fi.w += e;
+							if(term == 0) ti.w += e;
+						}
+						if(SPLIT) atomicAdd(a.esplit + 8 * (a.sys ? a.sys[i] : 0) + (term == 0 ? T_HB : term == 1 ? T_CRST : T_CXST), (double) e);
 					}
 					if(++v >= c1 - c0 || !(queue[c0 + v].y & (1 << 18))) break;
 				}
-				if(o.F.x == R(0) && o.F.y == R(0) && o.F.z == R(0) && o.T.x == R(0) && o.T.y == R(0) && o.T.z == R(0) && o.E == R(0)) continue;
-				// the potential is invariant under rigid rotations, so the torques balance:
-				// T_j = -T_i + (r_j - r_i) x F_i, the cross product with error-free products
-				const R *dd = item[m].d;
-				const v3<R> c = cross_accurate(Sep<R>{v3<R>{dd[0], dd[1], dd[2]}, v3<R>{dd[3], dd[4], dd[5]}}, o.F);
-				V4 fi, ti, fj, tj;
-				fi.x = o.F.x, fi.y = o.F.y, fi.z = o.F.z, fi.w = ENERGY ? o.E : R(0);
-				ti.x = o.T.x, ti.y = o.T.y, ti.z = o.T.z, ti.w = ENERGY ? o.Ehb : R(0);
-				fj.x = -o.F.x, fj.y = -o.F.y, fj.z = -o.F.z, fj.w = fi.w;
-				tj.x = c.x - o.T.x, tj.y = c.y - o.T.y, tj.z = c.z - o.T.z, tj.w = ti.w;
+				if(!any) continue;
+				fj.w = fi.w, tj.w = ti.w;
 				res[2 * ((long long) k * N + i)] = fi;
 				res[2 * ((long long) k * N + i) + 1] = ti;
 				atomicOr(a.pt_live + (long long) (k >> 6) * N + i, 1ull << (k & 63));
@@ -1001,12 +1005,6 @@ __device__ __forceinline__ void pair_block(const ForceArgs &a, const Loader &ld,
 					res[2 * ((long long) mj * N + j)] = fj;
 					res[2 * ((long long) mj * N + j) + 1] = tj;
 					atomicOr(a.pt_live + (long long) (mj >> 6) * N + j, 1ull << (mj & 63));
-				}
-				if(SPLIT) {
-					const int sy = a.sys ? a.sys[i] : 0;
-#pragma unroll
-					for(int u = 0; u < N_TERMS; u++)
-						if(o.split[u] != R(0)) atomicAdd(a.esplit + 8 * sy + u, (double) o.split[u]);
 				}
 			}
 			__syncthreads();
@@ -1142,6 +1140,73 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? OXGB_PAIR_MINB : 1) k_bo
 	else if constexpr(EDGE) edge_block<R, Loader, SPLIT, ENERGY, K>(a, ld, b - pair_blocks - bonded_blocks);
 }
 
+// What the bonded and pair blocks (and with use_edge the edge blocks) left for nucleotide i, added to
+// acc by the K lanes of its group: the live pair slots dealt to the lanes, the 3' bond to lane 0 and the
+// 5' bond to the next one.  (One group per nucleotide; the whole warp calls.)
+template <typename R, bool ENERGY, int K, bool EDGE, class Acc>
+__device__ __forceinline__ void gather_results(const ForceArgs &a, int i, int sub, bool live, int2 bonds, Acc &acc) {
+	using V4 = typename Vec4Of<R>::T;
+	const long long N = a.N;
+	V4 bf, bt;
+	const int lane5 = K > 1 ? 1 : 0;
+	const bool three = sub == 0 && live && bonds.x >= 0, five = sub == lane5 && live && bonds.y >= 0;
+	const V4 *bond_f = reinterpret_cast<const V4 *>(a.bond_f);
+	auto add = [&](const V4 &f, const V4 &t, R s) {
+		acc.F.add(v3<R>{s * f.x, s * f.y, s * f.z});
+		acc.T.add(v3<R>{t.x, t.y, t.z});
+		if(ENERGY) KahanV<R>::kadd(acc.E, acc.Ec, f.w);
+	};
+	// (issued before the mask is waited for)
+	if(three) bf = bond_f[i], bt = reinterpret_cast<const V4 *>(a.bond_tp)[i];
+	else if(five) bf = bond_f[bonds.y], bt = reinterpret_cast<const V4 *>(a.bond_tq)[bonds.y];
+	for(int w = 0; w < (a.pt_cap + 63) / 64; w++) {
+		unsigned long long m = 0ull;
+		if(sub == 0 && live) {
+			unsigned long long *at = a.pt_live + (long long) w * N + i;
+			m = *at;
+			if(m) *at = 0ull;  // for the next evaluation
+		}
+		m = __shfl_sync(0xffffffffu, m, 0, K);
+		// lane l takes the live slots l, l + K, ..., the next one loaded before the current one
+		// is added
+		for(int u = 0; u < sub; u++) m &= m - 1ull;
+		const V4 *base = reinterpret_cast<const V4 *>(a.pt_res) + 2 * ((long long) w * 64 * N + i);
+		V4 f, t;
+		auto next = [&]() {
+			const V4 *q = base + 2 * (long long) (__ffsll((long long) m) - 1) * N;
+			f = q[0];
+			t = q[1];
+#pragma unroll
+			for(int u = 0; u < K; u++) m &= m - 1ull;
+		};
+		bool have = m != 0ull;
+		if(have) next();
+		while(have) {
+			const V4 cf = f, ct = t;
+			have = m != 0ull;
+			if(have) next();
+			add(cf, ct, R(1));
+			if(ENERGY) KahanV<R>::kadd(acc.Eh, acc.Ehc, ct.w);
+		}
+	}
+	if(three) add(bf, bt, R(-1));
+	if(five) {
+		if(lane5 == 0 && three) bf = bond_f[bonds.y], bt = reinterpret_cast<const V4 *>(a.bond_tq)[bonds.y];
+		add(bf, bt, R(1));
+	}
+	if constexpr(EDGE) {
+		// the Debye-Hueckel and excluded-volume sums, cleared for the next evaluation
+		if(sub == 0 && live) {
+			V4 *ea = reinterpret_cast<V4 *>(a.edge_acc) + 2 * (long long) i;
+			add(ea[0], ea[1], R(1));
+			V4 z;
+			z.x = z.y = z.z = z.w = R(0);
+			ea[0] = z;
+			ea[1] = z;
+		}
+	}
+}
+
 // K lanes per nucleotide: lane l of a group takes entries l, l + K, ... of every term list, so a
 // warp holds 32 / K nucleotides and all its lanes run the same term loop
 // minimum resident blocks per SM asked of the register allocator for the non-bonded kernel
@@ -1149,8 +1214,8 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? OXGB_PAIR_MINB : 1) k_bo
 #define OXGB_NB_MINB 8
 #endif
 
-template <typename R, class Loader, bool SPLIT, bool ENERGY, int K, int MINB = OXGB_NB_MINB, bool EDGE = false>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? MINB : 1) k_nonbonded_split(ForceArgs a, Loader ld) {
+template <typename R, class Loader, bool SPLIT, bool ENERGY, int K, bool EDGE = false>
+__global__ void __launch_bounds__(128, 1) k_nonbonded_split(ForceArgs a, Loader ld) {
 	using V4 = typename Vec4Of<R>::T;
 	const long long N = a.N;
 	const int sub = threadIdx.x % K;
@@ -1204,131 +1269,27 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? MINB : 1) k_nonbonded_sp
 		}
 		// excluded volume over centre-close pairs (use_edge: the edge blocks did it)
 		const int nev = (live && !EDGE) ? min(a.ev_n[i], a.ev_cap) : 0;
-		if constexpr(decltype(ld.refine(0, 0))::on) {
-			// FP32: each window of 64 of the lane's entries is screened (a site pair inside its
-			// cutoff: a few in a thousand entries); the pairs found are evaluated refined after the
-			// window, outside the screening loop, and the others contribute nothing
-			for(int w0 = 0; w0 < nev; w0 += 64 * K) {
-				const int wend = min(nev, w0 + 64 * K);
-				unsigned long long stiff = 0ull;
-				int m = 0;
-				for(int k = w0 + sub; k < wend; k += K, m++) {
-					const int j = a.ev_nb[(long long) k * N + i];
-					Nuc<R> q;
-					V4 qh, ql;
-					load_full<Loader, R>(ld, j, P, q, qh, ql);
-					if(ev_contact(p, q, ld.sep_soft(ph, pl, qh, ql, P).plain())) stiff |= 1ull << m;
-				}
-				while(stiff) {
-					const int mm = __ffsll((long long) stiff) - 1;
-					stiff &= stiff - 1ull;
-					const int j = a.ev_nb[(long long) (w0 + sub + mm * K) * N + i];
-					Nuc<R> q;
-					V4 qh, ql;
-					load_full<Loader, R>(ld, j, P, q, qh, ql);
-					PairOut<R> o{};
-					const Sep<R> sp = ld.sep(ph, pl, qh, ql, P);
-					float3 t;
-					const float4 fe = ev_pair_refined_call(
-							ld.a1lo, ld.backlo, i, j, make_float4(sp.hi.x, sp.hi.y, sp.hi.z, 0.f), make_float4(sp.lo.x, sp.lo.y, sp.lo.z, 0.f),
-							make_float4(p.back.x, p.back.y, p.back.z, 0.f), make_float4(p.base.x, p.base.y, p.base.z, 0.f),
-							make_float4(p.a1.x, p.a1.y, p.a1.z, 0.f), make_float4(q.back.x, q.back.y, q.back.z, 0.f),
-							make_float4(q.base.x, q.base.y, q.base.z, 0.f), make_float4(q.a1.x, q.a1.y, q.a1.z, 0.f), &t);
-					o.F = v3<R>{fe.x, fe.y, fe.z};
-					o.T = v3<R>{t.x, t.y, t.z};
-					add_e<R, SPLIT>(o, T_NEXC, fe.w);
-					acc.add_short(o);
-				}
-			}
-		}
-		else {
-			for(int k = sub; k < nev; k += K) {
-				const int j = a.ev_nb[(long long) k * N + i];
-				Nuc<R> q;
-				V4 qh, ql;
-				load_full<Loader, R>(ld, j, P, q, qh, ql);
-				PairOut<R> o{};
-				pair_ev<R, SPLIT>(p, q, ld.sep(ph, pl, qh, ql, P), o);
-				acc.add_short(o);
-			}
+		for(int k = sub; k < nev; k += K) {
+			const int j = a.ev_nb[(long long) k * N + i];
+			Nuc<R> q;
+			V4 qh, ql;
+			load_full<Loader, R>(ld, j, P, q, qh, ql);
+			PairOut<R> o{};
+			pair_ev<R, SPLIT>(p, q, ld.sep(ph, pl, qh, ql, P), o);
+			acc.add(o);
 		}
 		// hydrogen bonding, cross and coaxial stacking: evaluated by the pair blocks of
 		// k_bonded_pairs, the slots they wrote gathered here (the terms above read only the mirrors
 		// and lists, complete before k_bonded_pairs started)
 		pdl_wait();
 		pdl_trigger();
-		for(int w = 0; w < (a.pt_cap + 63) / 64; w++) {
-			unsigned long long m = 0ull;
-			if(sub == 0 && live) {
-				unsigned long long *at = a.pt_live + (long long) w * N + i;
-				m = *at;
-				if(m) *at = 0ull;  // for the next evaluation
-			}
-			m = __shfl_sync(0xffffffffu, m, 0, K);
-			// lane l takes the live slots l, l + K, ..., the next one loaded before the current one
-			// is added
-			for(int u = 0; u < sub; u++) m &= m - 1ull;
-			const V4 *base = reinterpret_cast<const V4 *>(a.pt_res) + 2 * ((long long) w * 64 * N + i);
-			V4 f, t;
-			auto next = [&]() {
-				const V4 *q = base + 2 * (long long) (__ffsll((long long) m) - 1) * N;
-				f = q[0];
-				t = q[1];
-#pragma unroll
-				for(int u = 0; u < K; u++) m &= m - 1ull;
-			};
-			bool have = m != 0ull;
-			if(have) next();
-			while(have) {
-				const V4 cf = f, ct = t;
-				have = m != 0ull;
-				if(have) next();
-				acc.F.add(v3<R>{cf.x, cf.y, cf.z});
-				acc.T.add(v3<R>{ct.x, ct.y, ct.z});
-				if(ENERGY) {
-					KahanV<R>::kadd(acc.E, acc.Ec, cf.w);
-					KahanV<R>::kadd(acc.Eh, acc.Ehc, ct.w);
-				}
-			}
-		}
+		gather_results<R, ENERGY, K, EDGE>(a, i, sub, live, a.bonds[i], acc);
 		if(SPLIT && live) {
 #pragma unroll
 			for(int k = 0; k < N_TERMS; k++)
 				if(acc.split[k] != R(0)) atomicAdd(a.esplit + 8 * sy + k, 0.5 * (double) acc.split[k]);
 		}
 
-		// bonded pairs of this nucleotide, evaluated by the bonded blocks of k_bonded_pairs (first
-		// lane of the group); with use_edge also its Debye-Hueckel and excluded-volume sums, which
-		// are cleared for the next evaluation
-		if(sub == 0 && live) {
-			if constexpr(EDGE) {
-				V4 *ea = reinterpret_cast<V4 *>(a.edge_acc) + 2 * (long long) i;
-				const V4 f = ea[0], t = ea[1];
-				acc.F.add(v3<R>{f.x, f.y, f.z});
-				acc.T.add(v3<R>{t.x, t.y, t.z});
-				if(ENERGY) KahanV<R>::kadd(acc.E, acc.Ec, f.w);
-				V4 z;
-				z.x = z.y = z.z = z.w = R(0);
-				ea[0] = z;
-				ea[1] = z;
-			}
-			const int2 bi = a.bonds[i];
-			const V4 *bf = reinterpret_cast<const V4 *>(a.bond_f);
-			if(bi.x >= 0) {
-				const V4 f = bf[i], t = reinterpret_cast<const V4 *>(a.bond_tp)[i];
-				acc.F.add(v3<R>{-f.x, -f.y, -f.z});
-				acc.T.add(v3<R>{t.x, t.y, t.z});
-				if(ENERGY) KahanV<R>::kadd(acc.E, acc.Ec, f.w);
-			}
-			if(bi.y >= 0) {
-				const V4 f = bf[bi.y], t = reinterpret_cast<const V4 *>(a.bond_tq)[bi.y];
-				acc.F.add(v3<R>{f.x, f.y, f.z});
-				acc.T.add(v3<R>{t.x, t.y, t.z});
-				if(ENERGY) KahanV<R>::kadd(acc.E, acc.Ec, f.w);
-			}
-		}
-
-		acc.fold_short();
 		const R fx = group_sum_comp<R, K>(acc.F.s.x, acc.F.c.x), fy = group_sum_comp<R, K>(acc.F.s.y, acc.F.c.y),
 				fz = group_sum_comp<R, K>(acc.F.s.z, acc.F.c.z);
 		const v3<R> tl{group_sum_comp<R, K>(acc.T.s.x, acc.T.c.x), group_sum_comp<R, K>(acc.T.s.y, acc.T.c.y),
@@ -1348,6 +1309,139 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? MINB : 1) k_nonbonded_sp
 			reinterpret_cast<V4 *>(a.forces)[i] = fo;
 			reinterpret_cast<V4 *>(a.torques)[i] = to;
 		}
+	}
+}
+
+// The FP32 engine's non-bonded kernel, K lanes per nucleotide as above.  Debye-Hueckel and the
+// excluded-volume screen read the fixed-point sites: one 16-byte gather per Debye-Hueckel partner where
+// the position pair and the backbone offset took three, two per excluded-volume entry instead of five,
+// and an integer subtraction in the place of a compensated difference and its periodic image.  The
+// separation is good to one unit, box / 2^32 (5e-8 in a box of 230, where the FP32 difference of the
+// hi parts is off by up to 3.8e-6): Debye-Hueckel's force slope is below 0.1, and the screen's margin
+// is 1e-4.  Contacts are evaluated from the mirrors, refined, as everywhere.
+template <bool SPLIT, bool ENERGY, int K, int MINB = OXGB_NB_MINB, bool EDGE = false>
+__global__ void __launch_bounds__(128, MINB) k_nonbonded_mixed(ForceArgs a, SplitMixed ld) {
+	const long long N = a.N;
+	const int sub = threadIdx.x % K;
+	const int i_raw = (blockIdx.x * blockDim.x + threadIdx.x) / K;
+	const bool live = i_raw < a.N;  // (the lanes past the last nucleotide still take part in the shuffles)
+	const int i = live ? i_raw : a.N - 1;
+	const int sy = a.sys ? a.sys[i] : 0;
+	const DNA2Table<float> &P = table_of<float>(a, sy);
+	SplitAcc<float, SPLIT, ENERGY> acc{};
+	const int2 bi = a.bonds[i];
+	const float4 back = __ldg(ld.fback + i);
+	if(!EDGE) {
+		const float unit = P.fix_unit, u2 = unit * unit;
+		const int4 pk = __ldg(a.site_back + i);
+		// Debye-Hueckel (dh_sites) over its rows: the next partner's site is loaded before this
+		// partner's arithmetic, and the index after it one iteration earlier still.  The lever arm of
+		// every pair's torque on i is i's backbone offset, so the forces are summed (compensated) and
+		// the torque is taken once from the sum.
+		const int ndh = live ? min(a.dh_n[i], a.max_nb) : 0;
+		{
+			const float rc = P.dh_rc, rc2 = rc * rc, rh = P.dh_rhigh, mk = P.dh_minus_kappa, pre = P.dh_prefactor, b = P.dh_b;
+			const float half = P.dh_half_charged_ends ? 0.5f : 1.f;
+			const float pcut = back.w != 0.f ? half : 1.f;
+			KahanV<float> f{};
+			int4 qn = pk;
+			int k = sub;
+			if(k < ndh) qn = __ldg(a.site_back + a.dh_nb[(long long) k * N + i]);
+			int jn = k + K < ndh ? a.dh_nb[(long long) (k + K) * N + i] : 0;
+			for(; k < ndh; k += K) {
+				const int4 q = qn;
+				if(k + K < ndh) qn = __ldg(a.site_back + jn);
+				if(k + 2 * K < ndh) jn = a.dh_nb[(long long) (k + 2 * K) * N + i];
+				const float x = (float) (q.x - pk.x), y = (float) (q.y - pk.y), z = (float) (q.z - pk.z);
+				const float r2 = (x * x + y * y + z * z) * u2;
+				if(r2 < rc2) {
+					// 1 / r with a Newton step on the approximate reciprocal square root
+					float v = rsqrtf(r2);
+					v = v * fmaf(-0.5f * r2 * v, v, 1.5f);
+					const float r = r2 * v, cut = pcut * (q.w ? half : 1.f);
+					const float ex = pre * m_exp(mk * r), g = b * (r - rc);
+					const bool in = r < rh;
+					// -dE/dr / r, on p along its distance from q
+					const float fm = in ? ex * (v - mk) * v : -2.f * g;
+					const float s = -(fm * cut) * (v * unit);
+					f.add(v3<float>{x * s, y * s, z * s});
+					if(ENERGY) {
+						const float e = cut * (in ? ex * v : g * (r - rc));
+						KahanV<float>::kadd(acc.E, acc.Ec, e);
+						if(SPLIT) acc.split[T_DH] += e;
+					}
+				}
+			}
+			const v3<float> fs{f.s.x - f.c.x, f.s.y - f.c.y, f.s.z - f.c.z};
+			acc.F.add(fs);
+			acc.T.add(cross(v3<float>{back.x, back.y, back.z}, fs));
+		}
+		// Excluded volume over its list: each window of 64 of the lane's entries is screened (a site
+		// pair inside its cutoff, ev_contact: a few in a thousand entries); the pairs found are
+		// evaluated refined after the window, and the others contribute nothing
+		const int nev = live ? min(a.ev_n[i], a.ev_cap) : 0;
+		const int4 pb = __ldg(a.site_base + i);
+		constexpr float m = 1.0001f;
+		const float iu2 = 1.f / u2;
+		const float t1 = float(EVc<1>::RC * EVc<1>::RC) * m * iu2, t2 = float(EVc<2>::RC * EVc<2>::RC) * m * iu2,
+					t3 = float(EVc<3>::RC * EVc<3>::RC) * m * iu2;
+		static_assert(EVc<3>::RC == EVc<4>::RC, "one threshold for backbone-base");
+		auto sq = [](const int4 &p, const int4 &q) {
+			const float x = (float) (q.x - p.x), y = (float) (q.y - p.y), z = (float) (q.z - p.z);
+			return x * x + y * y + z * z;
+		};
+		for(int w0 = 0; w0 < nev; w0 += 64 * K) {
+			const int wend = min(nev, w0 + 64 * K);
+			unsigned long long stiff = 0ull;
+			int n = 0;
+			for(int k = w0 + sub; k < wend; k += K, n++) {
+				const int j = a.ev_nb[(long long) k * N + i];
+				const int4 qk = __ldg(a.site_back + j), qb = __ldg(a.site_base + j);
+				if(sq(pb, qb) < t2 || sq(pk, qb) < t3 || sq(pb, qk) < t3 || sq(pk, qk) < t1) stiff |= 1ull << n;
+			}
+			while(stiff) {
+				const int nn = __ffsll((long long) stiff) - 1;
+				stiff &= stiff - 1ull;
+				const int j = a.ev_nb[(long long) (w0 + sub + nn * K) * N + i];
+				Nuc<float> p, q;
+				float4 ph, pl, qh, ql;
+				ld.full(i, p, ph, pl);
+				ld.full(j, q, qh, ql);
+				PairOut<float> o{};
+				const Sep<float> sp = ld.sep(ph, pl, qh, ql, P);
+				float3 t;
+				const float4 fe = ev_pair_refined_call(
+						ld.a1lo, ld.backlo, i, j, make_float4(sp.hi.x, sp.hi.y, sp.hi.z, 0.f), make_float4(sp.lo.x, sp.lo.y, sp.lo.z, 0.f),
+						make_float4(p.back.x, p.back.y, p.back.z, 0.f), make_float4(p.base.x, p.base.y, p.base.z, 0.f),
+						make_float4(p.a1.x, p.a1.y, p.a1.z, 0.f), make_float4(q.back.x, q.back.y, q.back.z, 0.f),
+						make_float4(q.base.x, q.base.y, q.base.z, 0.f), make_float4(q.a1.x, q.a1.y, q.a1.z, 0.f), &t);
+				o.F = v3<float>{fe.x, fe.y, fe.z};
+				o.T = v3<float>{t.x, t.y, t.z};
+				add_e<float, SPLIT>(o, T_NEXC, fe.w);
+				acc.add(o);
+			}
+		}
+		if(SPLIT && live) {
+#pragma unroll
+			for(int k = 0; k < N_TERMS; k++)
+				if(acc.split[k] != 0.f) atomicAdd(a.esplit + 8 * sy + k, 0.5 * (double) acc.split[k]);
+		}
+	}
+	// the axes of the body frame, before the wait for the pair and bond results
+	const float4 x1 = __ldg(ld.fa1 + i), x3 = __ldg(ld.fa3 + i);
+	pdl_wait();
+	pdl_trigger();
+	gather_results<float, ENERGY, K, EDGE>(a, i, sub, live, bi, acc);
+	const float fx = group_sum_comp<float, K>(acc.F.s.x, acc.F.c.x), fy = group_sum_comp<float, K>(acc.F.s.y, acc.F.c.y),
+			fz = group_sum_comp<float, K>(acc.F.s.z, acc.F.c.z);
+	const v3<float> tl{group_sum_comp<float, K>(acc.T.s.x, acc.T.c.x), group_sum_comp<float, K>(acc.T.s.y, acc.T.c.y),
+			group_sum_comp<float, K>(acc.T.s.z, acc.T.c.z)};
+	const float e = ENERGY ? group_sum_comp<float, K>(acc.E, acc.Ec) : 0.f;
+	const float eh = ENERGY ? group_sum_comp<float, K>(acc.Eh, acc.Ehc) : 0.f;
+	if(sub == 0 && live) {
+		const v3<float> a1{x1.x, x1.y, x1.z}, a3{x3.x, x3.y, x3.z};
+		reinterpret_cast<float4 *>(a.forces)[i] = make_float4(fx, fy, fz, e);
+		reinterpret_cast<float4 *>(a.torques)[i] = make_float4(dot(a1, tl), dot(cross(a3, a1), tl), dot(a3, tl), eh);
 	}
 }
 
@@ -1628,9 +1722,12 @@ static void launch_split_t(const ForceArgs &a, Loader ld, cudaStream_t s, cudaEv
 	// the non-bonded kernel starts its Debye-Hueckel and excluded-volume work while the tail of
 	// the bonded and pair blocks runs; the external forces follow it the same way
 	if(wait) cudaStreamWaitEvent(s, wait, 0);
-	if(wait) k_nonbonded_split<R, Loader, SPLIT, ENERGY, K, NBMINB, EDGE><<<nonbonded_blocks(a.N, K), tpb, 0, s>>>(a, ld);
-	else launch_after(k_nonbonded_split<R, Loader, SPLIT, ENERGY, K, NBMINB, EDGE>, dim3(nonbonded_blocks(a.N, K)), dim3(tpb), 0,
-			s, a, ld);
+	auto nonbonded = [] {
+		if constexpr(sizeof(R) == 4) return &k_nonbonded_mixed<SPLIT, ENERGY, K, NBMINB, EDGE>;
+		else return &k_nonbonded_split<R, Loader, SPLIT, ENERGY, K, EDGE>;
+	}();
+	if(wait) nonbonded<<<nonbonded_blocks(a.N, K), tpb, 0, s>>>(a, ld);
+	else launch_after(nonbonded, dim3(nonbonded_blocks(a.N, K)), dim3(tpb), 0, s, a, ld);
 	if(a.ext_n > 0) launch_after(k_external<typename Vec4Of<R>::T>, dim3((a.ext_n + tpb - 1) / tpb), dim3(tpb), 0, s, a);
 }
 

@@ -25,20 +25,47 @@ namespace oxgb {
 // axes a1, a3 and the grooved backbone offset (src/Particles/DNANucleotide.cpp:79), each
 // rounded once (to within an ulp) from exact values; conversions and products on the FP32 and
 // integer pipes (split.cuh).  Each part returns what the staleness test needs.
-__device__ __forceinline__ float3 mirror_position(const StepArgs &a, int i, const double4_32a &r) {
+__device__ __forceinline__ void mirror_position(const StepArgs &a, int i, const double4_32a &r, float3 &rh, float3 &rl) {
 	float4 hi = a.pos_hi[i], lo = a.pos_lo[i];
 	split_rn(r.x, hi.x, lo.x);
 	split_rn(r.y, hi.y, lo.y);
 	split_rn(r.z, hi.z, lo.z);
 	a.pos_hi[i] = hi;
 	a.pos_lo[i] = lo;
-	return make_float3(hi.x, hi.y, hi.z);
+	rh = make_float3(hi.x, hi.y, hi.z);
+	rl = make_float3(lo.x, lo.y, lo.z);
 }
 
-// returns a1 and the backbone offset; with a.fa1lo also the remainders of a1 and the backbone
+// what the fixed-point sites need of a system's table
+struct FixedBox {
+	float box_hi, box_lo, inv_box, s_hi, s_lo;
+};
+
+__device__ __forceinline__ FixedBox fixed_box(const StepArgs &a, int sy) {
+	const DNA2Table<float> &P = reinterpret_cast<const DNA2Table<float> *>(a.table)[sy];
+	return FixedBox{P.box_hi, P.box_lo, P.inv_box, P.fix_hi, P.fix_lo};
+}
+
+// a position (hi + lo) in fixed point
+__device__ __forceinline__ int3 fixed_centre(const FixedBox &b, float3 hi, float3 lo) {
+	return make_int3((int) fixed_coord(hi.x, lo.x, b.box_hi, b.box_lo, b.inv_box, b.s_hi, b.s_lo),
+			(int) fixed_coord(hi.y, lo.y, b.box_hi, b.box_lo, b.inv_box, b.s_hi, b.s_lo),
+			(int) fixed_coord(hi.z, lo.z, b.box_hi, b.box_lo, b.inv_box, b.s_hi, b.s_lo));
+}
+
+// the fixed-point backbone and base sites of nucleotide i, from its position, its FP32 backbone offset
+// and a1 (base site at 0.4 a1)
+__device__ __forceinline__ void mirror_sites(const StepArgs &a, int i, const FixedBox &b, int3 c, float3 a1, float4 back) {
+	const float s2 = 2.f * b.s_hi, sb = 0.4f * s2;
+	a.site_back[i] = make_int4(c.x + fixed_round(back.x * s2), c.y + fixed_round(back.y * s2), c.z + fixed_round(back.z * s2),
+			back.w != 0.f);
+	a.site_base[i] = make_int4(c.x + fixed_round(a1.x * sb), c.y + fixed_round(a1.y * sb), c.z + fixed_round(a1.z * sb), 0);
+}
+
+// returns a1 and the backbone offset (w: the strand-end flag); with a.fa1lo also the remainders of a1 and the backbone
 // offset (exact value = mirror + remainder to ~2^-46), which the force kernels use for the stiff
 // radial factors and excluded-volume contacts
-__device__ __forceinline__ void mirror_frame(const StepArgs &a, int i, const double4_32a &q, float3 &a1o, float3 &backo) {
+__device__ __forceinline__ void mirror_frame(const StepArgs &a, int i, const double4_32a &q, float3 &a1o, float4 &backo) {
 	float qh[4], ql[4], a1[3], a3[3], bk[3], a1l[3], bkl[3];
 	split_rn(q.x, qh[0], ql[0]);
 	split_rn(q.y, qh[1], ql[1]);
@@ -53,19 +80,17 @@ __device__ __forceinline__ void mirror_frame(const StepArgs &a, int i, const dou
 	a.fa1[i] = make_float4(a1[0], a1[1], a1[2], 0.f);
 	a.fa3[i] = make_float4(a3[0], a3[1], a3[2], 0.f);
 	// the strand-end flag rides in w
-	if(a.fback) {
-		const int2 bd = a.bonds[i];
-		a.fback[i] = make_float4(bk[0], bk[1], bk[2], (bd.x < 0 || bd.y < 0) ? 1.f : 0.f);
-	}
+	const int2 bd = a.bonds[i];
+	backo = make_float4(bk[0], bk[1], bk[2], (bd.x < 0 || bd.y < 0) ? 1.f : 0.f);
+	a.fback[i] = backo;
 	a1o = make_float3(a1[0], a1[1], a1[2]);
-	backo = make_float3(bk[0], bk[1], bk[2]);
 }
 
 // true if the centre or any interaction site moved more than the skin since the last list build
 // (lp, la1, lbk: centre, a1 and backbone offset at the last build; r: the new centre in FP32,
 // a1 and back: the new axis and backbone offset)
 __device__ __forceinline__ bool list_stale(const StepArgs &a, const float4 &lp, const float4 &la1, const float4 &lbk, float3 r,
-		float3 a1, float3 bk) {
+		float3 a1, float4 bk) {
 	const float dx = r.x - lp.x, dy = r.y - lp.y, dz = r.z - lp.z;
 	if(dx * dx + dy * dy + dz * dz > a.skin2) return true;
 	if(!a.list_a1) return false;
@@ -81,9 +106,14 @@ __device__ __forceinline__ bool list_stale(const StepArgs &a, const float4 &lp, 
 __global__ void k_make_mirrors(StepArgs a) {
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
 	if(i >= a.N) return;
-	float3 a1, bk;
-	(void) mirror_position(a, i, a.pos[i]);
+	float3 a1, hi, lo;
+	float4 bk;
+	mirror_position(a, i, a.pos[i], hi, lo);
 	mirror_frame(a, i, a.quat[i], a1, bk);
+	if(a.site_back) {
+		const FixedBox b = fixed_box(a, a.th.sys[i]);
+		mirror_sites(a, i, b, fixed_centre(b, hi, lo), a1, bk);
+	}
 }
 
 // ---------------------------------------------------------------- first half step
@@ -179,26 +209,33 @@ __device__ __forceinline__ double4_32a round4(const double4_32a &v) {
 // half kick and thermostat of step s - 1, half kick, drift, position mirror), warp 1 the
 // rotation (the same for the angular momentum, rotation, frame mirror).  The chains of FP64
 // operations are half as long and twice as many warps hide them; a warp never diverges on the
-// kind of motion.
+// kind of motion.  What needs both, the sites and the staleness test, is done by the translation warp,
+// whose own chain is the shorter one.
 // (capped at 64 registers, 16 blocks per SM: measured in alternating runs, the 250k MD step
 // 138.7 -> 136.9 us and the 256-system batch 263.4 -> 261.3 us against the uncapped 80)
 template <typename V4, bool F32 = false>
 __global__ void __launch_bounds__(64, 16) k_first_step(StepArgs a) {
-	__shared__ float3 s_r32[32];
+	__shared__ float3 s_a1[32];
+	__shared__ float4 s_back[32];
 	const int lane = threadIdx.x & 31;
 	const bool rot = threadIdx.x >= 32;
 	const int i = blockIdx.x * 32 + lane;
 	const bool live = i < a.N;
-	float3 r32 = make_float3(0.f, 0.f, 0.f), fa1 = r32, fbk = r32;
+	float3 r32 = make_float3(0.f, 0.f, 0.f), r32l = r32, fa1 = r32;
+	float4 fbk = make_float4(0.f, 0.f, 0.f, 0.f);
 	int sy = 0;
 	double4_32a x, y;  // (v, r) on the translation warp, (L, q) on the rotation warp
 	float4 lp, la1, lbk;
+	constexpr bool SITES = sizeof(V4) == sizeof(float4);  // (the double engine has no fixed-point sites)
+	FixedBox fb{};
+	int3 centre = make_int3(0, 0, 0);
 	auto load_state = [&]() {
 		if(live) {
 			sy = a.th.sys[i];
 			x = rot ? a.angmom[i] : a.vel[i];
 			y = rot ? a.quat[i] : a.pos[i];
-			if(rot) {
+			if(!rot) {
+				if(SITES) fb = fixed_box(a, sy);
 				lp = a.list_pos[i];
 				if(a.list_a1) la1 = a.list_a1[i], lbk = a.list_back[i];
 			}
@@ -251,7 +288,7 @@ __global__ void __launch_bounds__(64, 16) k_first_step(StepArgs a) {
 			const double4_32a rd = widen4(r.x, r.y, r.z, 0.f);
 			a.vel[i] = x;
 			a.pos[i] = rd;
-			r32 = mirror_position(a, i, rd);
+			mirror_position(a, i, rd, r32, r32l);
 		}
 		else {
 			float4 q = make_float4(narrow(y.x), narrow(y.y), narrow(y.z), narrow(y.w));
@@ -291,7 +328,7 @@ __global__ void __launch_bounds__(64, 16) k_first_step(StepArgs a) {
 			r.z += x.z * a.dt;
 			a.vel[i] = x;
 			a.pos[i] = r;
-			r32 = mirror_position(a, i, r);
+			mirror_position(a, i, r, r32, r32l);
 		}
 		else {
 			double4_32a q = y;
@@ -303,16 +340,23 @@ __global__ void __launch_bounds__(64, 16) k_first_step(StepArgs a) {
 			mirror_frame(a, i, q, fa1, fbk);
 		}
 	}
-	// Verlet list staleness (CUDA_mixed.cuh:68, extended to the interaction sites for the term
-	// lists), per system, on the rotation warp (the slower one) with the translation warp's FP32
-	// position: the translation warp posts it and leaves (named barrier 1: arrive, no wait)
-	if(!rot) {
-		s_r32[lane] = r32;
+	// (ahead of the wait for the frame)
+	if(SITES && live && !rot) centre = fixed_centre(fb, r32, r32l);
+	// the rotation warp posts its frame and leaves (named barrier 1: arrive, no wait)
+	if(rot) {
+		s_a1[lane] = fa1;
+		s_back[lane] = fbk;
 		asm volatile("bar.arrive 1, 64;" ::: "memory");
 		return;
 	}
 	asm volatile("bar.sync 1, 64;" ::: "memory");
-	if(live && list_stale(a, lp, la1, lbk, s_r32[lane], fa1, fbk)) {
+	if(!live) return;
+	fa1 = s_a1[lane];
+	fbk = s_back[lane];
+	if(SITES) mirror_sites(a, i, fb, centre, fa1, fbk);
+	// Verlet list staleness (CUDA_mixed.cuh:68, extended to the interaction sites for the term
+	// lists), per system
+	if(list_stale(a, lp, la1, lbk, r32, fa1, fbk)) {
 		a.sys_stale[sy] = 1;
 		atomicOr(a.flag, 1);
 	}

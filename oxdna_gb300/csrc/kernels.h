@@ -106,6 +106,7 @@ struct ForceArgs {
 	// (column-major: element k of nucleotide i at [k * N + i]) and the per-bond buffers
 	const float4 *fback;
 	const float4 *fa1lo, *fbacklo;            // remainders of fa1 / fback (null: the FP32 sites unrefined)
+	const int4 *site_back, *site_base;        // fixed-point backbone (w: strand end) and base sites (FP32 engines)
 	const int *ev_nb, *ev_n, *pt_nb, *pt_n;
 	int ev_cap, pt_cap;                       // capacities (an overflowed list is read up to them)
 	void *bond_f, *bond_tp, *bond_tq;         // per bond owner p (q = n3[p]): f on q with w = energy, torques
@@ -226,7 +227,8 @@ struct ListArgs {
 	int *id, *slot;         // [N] caller's index of each slot, and its inverse
 	int *perm, *inv;        // [N] scratch: old slot of new slot k, new slot of old slot
 	double4_32a *st[4];     // FP64 state: positions, velocities, angular momenta, quaternions
-	float4 *mir[7];         // mirrors: pos_hi, pos_lo, fa1, fa3, fback, fa1lo, fbacklo (any may be null)
+	float4 *mir[9];         // mirrors: pos_hi, pos_lo, fa1, fa3, fback, fa1lo, fbacklo, site_back, site_base
+	                        // (any may be null)
 	int2 *bonds_rw;         // the bonds the rows exclude (the array of `bonds`)
 	unsigned char *scratch; // [N * SORT_BYTES]
 	// Hilbert order of the cells (null: row-major cell order): cell c of the global numbering is
@@ -239,9 +241,9 @@ struct ListArgs {
 	int list_kind;          // neighbour-row kernel: OXGB_LIST_WARP, _THREAD or _GROUP4/8/16
 };
 
-// bytes per nucleotide of the sort's staging buffer: 4 FP64 vectors, 7 FP32 vectors, bonds,
+// bytes per nucleotide of the sort's staging buffer: 4 FP64 vectors, 9 vectors of 32 bits, bonds,
 // id and cell
-#define SORT_MIRRORS 7
+#define SORT_MIRRORS 9
 #define SORT_BYTES (4 * 32 + SORT_MIRRORS * 16 + 8 + 4 + 4)
 
 // full rebuild: cells (counting sort, deterministic order) then neighbour rows
@@ -259,6 +261,8 @@ struct StepArgs {
 	const float4 *list_pos;
 	float4 *fback;                         // backbone offset (w: strand-end flag), written with the mirrors
 	float4 *fa1lo, *fbacklo;               // remainders of fa1 and fback (mixed / float engine; null: none)
+	int4 *site_back, *site_base;           // fixed-point sites (mixed / float engine; null: none), in the units of
+	const void *table;                     // the systems' tables (DNA2Table<float>)
 	const int2 *bonds;
 	const float4 *list_a1, *list_back;     // site data of the last list build (null: centres only)
 	float skin2;

@@ -67,13 +67,6 @@ OXGB_HD v3<R> cross(v3<R> a, v3<R> b) {
 // force kernels are not compiled with fast-math), the double ones the double functions
 OXGB_HD float m_sqrt(float x) { return sqrtf(x); }
 OXGB_HD double m_sqrt(double x) { return sqrt(x); }
-// 1 / x correctly rounded (the force kernels' divisions are the fast ones)
-#ifdef __CUDA_ARCH__
-OXGB_HD float m_rcp(float x) { return __frcp_rn(x); }
-#else
-OXGB_HD float m_rcp(float x) { return 1.f / x; }
-#endif
-OXGB_HD double m_rcp(double x) { return 1.0 / x; }
 OXGB_HD float m_exp(float x) { return expf(x); }
 OXGB_HD double m_exp(double x) { return exp(x); }
 OXGB_HD float m_expm1(float x) { return expm1f(x); }

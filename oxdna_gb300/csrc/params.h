@@ -103,6 +103,9 @@ inline int build_table(const oxgb_dna2_settings &s, double box, DNA2Table<double
 	P.box_hi = box;
 	P.box_lo = 0.0;
 	P.inv_box = 1.0 / box;
+	P.fix_hi = 2147483648.0 / box;
+	P.fix_lo = 0.0;
+	P.fix_unit = box / 4294967296.0;
 	return 0;
 }
 
@@ -118,6 +121,7 @@ inline void to_float(const DNA2Table<double> &d, double box, DNA2Table<float> &f
 	f.box_hi = (float) box;
 	f.box_lo = (float) (box - (double) f.box_hi);
 	f.inv_box = (float) (1.0 / (double) f.box_hi);
+	f.fix_lo = (float) (2147483648.0 / box - (double) f.fix_hi);
 }
 
 // pair-distance bounds of the force kernel's term lists: a term can only act within these

@@ -289,6 +289,29 @@ OXGB_HD F2 split2(double x) {
 	return r;
 }
 
+// ---------------------------------------------------------------- fixed-point sites
+//
+// A coordinate in units of box / 2^32, modulo the box: the difference of two of them as 32-bit integers
+// is the minimum image by itself, to one unit (5e-8 in a box of 230).  c = hi + lo is a coordinate
+// (unwrapped), box_hi + box_lo the box side, s_hi + s_lo = 2^31 / box.  hi less its whole boxes is exact
+// in FP32 (the fused product), the scaling an FP32 pair.
+OXGB_HD int fixed_round(float x) {
+#ifdef __CUDA_ARCH__
+	return __float2int_rn(x);
+#else
+	return (int) std::nearbyint(x);
+#endif
+}
+
+OXGB_HD unsigned fixed_coord(float hi, float lo, float box_hi, float box_lo, float inv_box, float s_hi, float s_lo) {
+	const float m = OXGB_FSUB(OXGB_FMAF(hi, inv_box, 12582912.f), 12582912.f);
+	const float d = OXGB_FMAF(-m, box_hi, hi), l = OXGB_FMAF(-m, box_lo, lo);
+	const float p = OXGB_FMUL(d, s_hi);
+	const float e = OXGB_FADD(OXGB_FMAF(d, s_hi, -p), OXGB_FMAF(d, s_lo, OXGB_FMUL(l, s_hi)));
+	const int i = fixed_round(p);  // |p| <= 2^30 or so
+	return 2u * (unsigned) i + (unsigned) fixed_round(2.f * OXGB_FADD(OXGB_FSUB(p, (float) i), e));
+}
+
 // The rotation of the unit quaternion q = (x, y, z, w) by the angle dt |L| about the body-frame
 // angular momentum L (hd = dt / 2): q <- q (x) (sin(t/2) L^, cos(t/2)), t = dt |L|, written
 // as q + c with the small correction c = q (x) (delta, eps), delta = k L, eps = cos(t/2) - 1,
