@@ -642,8 +642,8 @@ static int derive_system(oxgb_md *h, int k, DNA2Table<double> &t64) {
 	double *p = &h->par[(size_t) k * SP_STRIDE];
 	p[SP_T] = T;
 	p[SP_SQRTT] = std::sqrt(T);
-	p[SP_PT] = pt;
-	p[SP_PR] = (2 * T * n * dtf) / (T * n * dtf + 2 * 3 * D);
+	p[SP_PT] = draw_threshold(pt);
+	p[SP_PR] = draw_threshold((2 * T * n * dtf) / (T * n * dtf + 2 * 3 * D));
 	p[SP_1MC] = 1.0 - c;
 	p[SP_A] = (1.0 - c) * T * 0.5;
 	p[SP_B] = std::sqrt(2.0 * T * (1.0 - c) * c);

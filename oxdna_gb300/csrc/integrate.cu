@@ -271,7 +271,8 @@ __global__ void __launch_bounds__(64, 16) k_first_step(StepArgs a) {
 			u.z += gz * hdt;
 			if(brownian || bussi) {
 				x = widen4(u.x, u.y, u.z, 0.f);
-				if(brownian) x = brownian_redraw_part(a.th, sy, (a.th.id ? a.th.id[i] : i) - a.th.sys_off[sy], sp, rot ? 1 : 0, x);
+				if(brownian) x = brownian_redraw_warp(a.th, sy, (a.th.id ? a.th.id[i] : i) - a.th.sys_off[sy], sp, rot ? 1 : 0,
+						min(a.N - (int) blockIdx.x * 32, 32), x);
 				else bussi_rescale_part(a.th, sy, rot ? 1 : 0, x);
 				u = make_float3(narrow(x.x), narrow(x.y), narrow(x.z));
 			}
@@ -315,7 +316,8 @@ __global__ void __launch_bounds__(64, 16) k_first_step(StepArgs a) {
 			x.x = fma(gx, hdt, x.x);
 			x.y = fma(gy, hdt, x.y);
 			x.z = fma(gz, hdt, x.z);
-			if(brownian) x = brownian_redraw_part(a.th, sy, (a.th.id ? a.th.id[i] : i) - a.th.sys_off[sy], sp, rot ? 1 : 0, x);
+			if(brownian) x = brownian_redraw_warp(a.th, sy, (a.th.id ? a.th.id[i] : i) - a.th.sys_off[sy], sp, rot ? 1 : 0,
+						min(a.N - (int) blockIdx.x * 32, 32), x);
 			else if(bussi) bussi_rescale_part(a.th, sy, rot ? 1 : 0, x);
 		}
 		x.x = fma(gx, hdt, x.x);

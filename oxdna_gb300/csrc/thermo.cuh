@@ -36,12 +36,17 @@ static __device__ __forceinline__ void philox(unsigned k0, unsigned k1, unsigned
 
 static __device__ __forceinline__ double u01(unsigned x) { return ((double) x + 1.0) * (1.0 / 4294967296.0); }
 
-static __device__ __forceinline__ void box_muller(unsigned ua, unsigned ub, double &g0, double &g1) {
+// (one compiled copy, so that a redraw has the same bits wherever it is made)
+static __device__ __noinline__ double2 box_muller(unsigned ua, unsigned ub) {
 	const double r = sqrt(-2.0 * log(u01(ua)));
 	double s, c;
-	sincos(6.283185307179586 * u01(ub), &s, &c);
-	g0 = r * c;
-	g1 = r * s;
+	sincospi(2.0 * u01(ub), &s, &c);
+	return make_double2(r * c, r * s);
+}
+
+// u01(x) < p for a probability given as its threshold (draw_threshold): the same test on integers
+static __device__ __forceinline__ bool drawn(unsigned x, double threshold) {
+	return (unsigned long long) x < (unsigned long long) __double_as_longlong(threshold);
 }
 
 #define RNG_BROWNIAN 0x42524f57u
@@ -141,40 +146,64 @@ static __device__ __noinline__ void brownian_redraw(const ThermoArgs &t, int sy,
 	const unsigned s0 = (unsigned) s, s1 = (unsigned) ((unsigned long long) s >> 32);
 	philox(k0, k1, s0, s1, RNG_BROWNIAN, (unsigned) (2 * i_local), o0);
 	philox(k0, k1, s0, s1, RNG_BROWNIAN, (unsigned) (2 * i_local + 1), o1);
-	double g[6];
-	box_muller(o0[2], o0[3], g[0], g[1]);
-	box_muller(o1[0], o1[1], g[2], g[3]);
-	box_muller(o1[2], o1[3], g[4], g[5]);
 	const double sT = par[SP_SQRTT];
-	if(u01(o0[0]) < par[SP_PT]) v = make_double4_32a(g[0] * sT, g[1] * sT, g[2] * sT, 0.0);
-	if(u01(o0[1]) < par[SP_PR]) L = make_double4_32a(g[3] * sT, g[4] * sT, g[5] * sT, 0.0);
+	const bool dv = drawn(o0[0], par[SP_PT]), dL = drawn(o0[1], par[SP_PR]);
+	if(!(dv || dL)) return;
+	const double2 b = box_muller(o1[0], o1[1]);
+	if(dv) {
+		const double2 c = box_muller(o0[2], o0[3]);
+		v = make_double4_32a(c.x * sT, c.y * sT, b.x * sT, 0.0);
+	}
+	if(dL) {
+		const double2 c = box_muller(o1[2], o1[3]);
+		L = make_double4_32a(b.y * sT, c.x * sT, c.y * sT, 0.0);
+	}
 }
 
-// one kind of motion of brownian_redraw (which = 0: the velocity, 1: the angular momentum), with
-// the same draws; returns x, redrawn or not (by value: no stack frame for the caller)
-static __device__ __noinline__ double4_32a brownian_redraw_part(const ThermoArgs &t, int sy, int i_local, long long s,
-		int which, double4_32a x) {
+// One kind of motion of brownian_redraw (which = 0: the velocity, 1: the angular momentum) for a warp
+// whose lanes 0 .. n - 1 call it, with the same draws; returns x, redrawn or not.  A redraw takes two
+// pairs of normal deviates, each a logarithm, a square root, a sine and a cosine on the slow FP64 pipe,
+// which takes as long for one lane as for all: so the pairs of the lanes that redraw (a tenth of them at
+// most, commonly a hundredth) are dealt to the warp's lanes and made in one pass, and a warp without a
+// redraw makes none.  (Each lane made its own two pairs, one of them drawn or not: a first step that
+// redraws a tenth of 32,000 nucleotides took 28 us.)
+static __device__ __noinline__ double4_32a brownian_redraw_warp(const ThermoArgs &t, int sy, int i_local, long long s, int which,
+		int n, double4_32a x) {
 	const double *par = t.sys_par + sy * SP_STRIDE;
 	const unsigned long long seed = t.sys_seed[sy];
+	const unsigned lanes = n == 32 ? 0xffffffffu : (1u << n) - 1u, lane = threadIdx.x & 31;
 	unsigned o0[4], o1[4];
 	const unsigned k0 = (unsigned) seed, k1 = (unsigned) (seed >> 32);
 	const unsigned s0 = (unsigned) s, s1 = (unsigned) ((unsigned long long) s >> 32);
 	philox(k0, k1, s0, s1, RNG_BROWNIAN, (unsigned) (2 * i_local), o0);
+	const bool redraw = which == 0 ? drawn(o0[0], par[SP_PT]) : drawn(o0[1], par[SP_PR]);
+	const unsigned who = __ballot_sync(lanes, redraw);
+	if(who == 0u) return x;
 	philox(k0, k1, s0, s1, RNG_BROWNIAN, (unsigned) (2 * i_local + 1), o1);
-	const double sT = par[SP_SQRTT];
-	double g0, g1, g2, g3;
-	box_muller(o1[0], o1[1], g2, g3);
-	if(which == 0) {
-		if(u01(o0[0]) < par[SP_PT]) {
-			box_muller(o0[2], o0[3], g0, g1);
-			x = make_double4_32a(g0 * sT, g1 * sT, g2 * sT, 0.0);
+	// the two pairs of a nucleotide: velocity g0 g1 | g2 -, angular momentum - g3 | g4 g5
+	const unsigned a0 = which == 0 ? o0[2] : o1[0], b0 = which == 0 ? o0[3] : o1[1];
+	const unsigned a1 = which == 0 ? o1[0] : o1[2], b1 = which == 0 ? o1[1] : o1[3];
+	const int pairs = 2 * __popc(who), mine = 2 * __popc(who & ((1u << lane) - 1u));
+	double2 p0 = make_double2(0.0, 0.0), p1 = p0;
+	for(int q0 = 0; q0 < pairs; q0 += n) {
+		const int q = q0 + (int) lane;
+		const int src = q < pairs ? (int) __fns(who, 0u, q / 2 + 1) : 0;
+		const unsigned u0 = __shfl_sync(lanes, a0, src), v0 = __shfl_sync(lanes, b0, src);
+		const unsigned u1 = __shfl_sync(lanes, a1, src), v1 = __shfl_sync(lanes, b1, src);
+		double2 g = make_double2(0.0, 0.0);
+		if(q < pairs) g = box_muller(q & 1 ? u1 : u0, q & 1 ? v1 : v0);
+#pragma unroll
+		for(int h = 0; h < 2; h++) {
+			const int at = mine + h - q0;  // the lane that made this lane's pair h
+			const bool here = redraw && at >= 0 && at < n;
+			const double gx = __shfl_sync(lanes, g.x, here ? at : 0), gy = __shfl_sync(lanes, g.y, here ? at : 0);
+			if(here) (h == 0 ? p0 : p1) = make_double2(gx, gy);
 		}
 	}
-	else if(u01(o0[1]) < par[SP_PR]) {
-		box_muller(o1[2], o1[3], g0, g1);
-		x = make_double4_32a(g3 * sT, g0 * sT, g1 * sT, 0.0);
-	}
-	return x;
+	if(!redraw) return x;
+	const double sT = par[SP_SQRTT];
+	return which == 0 ? make_double4_32a(p0.x * sT, p0.y * sT, p1.x * sT, 0.0) :
+			make_double4_32a(p0.y * sT, p1.x * sT, p1.y * sT, 0.0);
 }
 
 // Bussi: from the sums of v, |v|^2 and |L|^2 over system sy, the new running kinetic energy
