@@ -188,9 +188,9 @@ typedef struct oxgb_md_settings {
 	int cells_auto_optimisation;/* cells_auto_optimisation */
 	int max_neigh;              /* neighbour-row capacity; 0 = sized from the first build */
 	int steps_per_graph;        /* MD steps captured per CUDA graph launch (0 = 16) */
-	int list_rebuild_node;      /* 0: the list rebuild is a device-side IF node of the step graph;
-	                               1: the rebuild kernels are launched every step and return at once
-	                               while the list is fresh (same results; kernel nodes profilable) */
+	int list_rebuild_node;      /* kept for callers that set it (0 or 1, the same): the list rebuild is one
+	                               kernel, launched every step, that returns at once while the list is
+	                               fresh */
 	int sort_every;             /* CUDA_sort_every (CUDABaseBackend.cu:263-281): every sort_every-th
 	                               list rebuild stores the nucleotides in cell order, on the device
 	                               (0: never).  Forces, Brownian and NVE trajectories are bit-identical
@@ -216,12 +216,11 @@ typedef struct oxgb_md_settings {
 	int list_kernel;            /* OXGB_LIST_AUTO (default), _WARP, _THREAD or _GROUP4/8/16 (below) */
 } oxgb_md_settings;
 enum { OXGB_SORT_HILBERT = 0, OXGB_SORT_CELLS = 1 };
-/* oxgb_md_settings.list_kernel: the neighbour-row kernel of the list build.  All give the same
- * rows entry for entry; which is faster depends on how many candidates a nucleotide's 27 cells hold
- * and on how many nucleotides a build covers.  AUTO: timed by the autotuner (md.autotune), else
- * WARP; WARP: a warp per nucleotide, lanes over the candidates; THREAD: a thread per nucleotide,
- * coalesced stores into the column-major rows; GROUP4 / GROUP8 / GROUP16: 4, 8 or 16 lanes per
- * nucleotide over its candidates */
+/* oxgb_md_settings.list_kernel: the lanes per nucleotide of the list build's row phase.  All give the
+ * same rows entry for entry; which is faster depends on how many candidates a nucleotide's 27 cells hold
+ * and on how many nucleotides a build covers.  AUTO: timed by the autotuner (md.autotune), else as many
+ * as keep the chip busy for the mean system; WARP: 32; GROUP16: 16; THREAD, GROUP4, GROUP8: 16 too (the
+ * names of earlier forms) */
 enum { OXGB_LIST_AUTO = 0, OXGB_LIST_WARP = 1, OXGB_LIST_THREAD = 2, OXGB_LIST_GROUP4 = 3, OXGB_LIST_GROUP8 = 4,
 	OXGB_LIST_GROUP16 = 5 };
 
@@ -383,7 +382,7 @@ int oxgb_md_set_force_shape(oxgb_md *h, int k);
 /* the shape table itself: shape k's nucleotides per pair-block warp queue, non-bonded lanes per
  * nucleotide and register cap (OXGB_E_INVALID past the last shape) */
 int oxgb_force_shape_table(int k, int *pair_npw, int *nb_lanes, int *nb_min_blocks);
-/* the neighbour-row kernel the engine's list builds use: OXGB_LIST_WARP, _THREAD or _GROUP4/8/16 */
+/* the lanes per nucleotide of the engine's list builds: OXGB_LIST_WARP, _THREAD or _GROUP4/8/16 */
 int oxgb_md_list_kernel(oxgb_md *h, int *kernel);
 /* device pointers (for zero-copy callers): FP64 positions, velocities, angular momenta and
  * quaternions (double4 each), FP32 forces and torques (float4; double4 in double precision) */

@@ -3,9 +3,9 @@
 // (src/CUDA/Backends/MD_CUDABackend.cu:567-619): first half kick + drift + rotation, list
 // rebuild when any nucleotide moved more than the skin, forces + second half kick, thermostat.
 // Each step is captured once into a CUDA graph (steps_per_graph steps per graph); the list
-// rebuild is a device-side IF conditional node driven by the staleness flag the first-step
-// kernel raises, so a run of many steps needs no host synchronisation at all (the reference
-// synchronises several times per step).
+// rebuild is one kernel that returns at once unless the first-step kernel has raised the staleness
+// flag, so a run of many steps needs no host synchronisation at all (the reference synchronises
+// several times per step).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -64,6 +64,7 @@ static int status_to_code(int st) {
 	if(st & OXGB_ERR_FENE) return OXGB_E_FENE;
 	if(st & OXGB_ERR_NEIGH_OVERFLOW) return OXGB_E_NEIGH_OVERFLOW;
 	if(st & OXGB_ERR_CELL) return OXGB_E_NONFINITE;
+	if(st & OXGB_ERR_SYNC) return OXGB_E_CUDA;
 	return OXGB_OK;
 }
 
@@ -73,6 +74,7 @@ static std::string status_message(int st) {
 	if(st & OXGB_ERR_NEIGH_OVERFLOW) m += "a neighbour row overflowed its capacity (raise max_neigh); ";
 	if(st & OXGB_ERR_NONFINITE) m += "non-finite or huge coordinates (the simulation exploded); ";
 	if(st & OXGB_ERR_CELL) m += "cell index out of range; ";
+	if(st & OXGB_ERR_SYNC) m += "a list build did not complete; ";
 	return m;
 }
 
@@ -209,6 +211,8 @@ struct ListBuffers {
 	int n_side = 0, n_cells = 0, max_nb = 0, N = 0;
 	int *cell_of = nullptr, *cell_count = nullptr, *cell_start = nullptr, *cell_cursor = nullptr, *cell_list = nullptr;
 	int *cell_tmp = nullptr, *scan_part = nullptr;
+	float4 *spos = nullptr, *sback = nullptr, *sa1 = nullptr;  // in cell order (the last two with dh)
+	ListSync *sync = nullptr;
 	int *nb = nullptr, *nnb = nullptr;
 	// engine only (dh set before alloc): the Debye-Hueckel rows, the pairs of the full rows whose
 	// backbone sites are within the Debye-Hueckel cutoff plus twice the skin, same capacity
@@ -228,17 +232,27 @@ struct ListBuffers {
 		CK(cudaMalloc(&cell_cursor, sizeof(int) * n_cells));
 		CK(cudaMalloc(&cell_list, sizeof(int) * std::max(N, 1)));
 		CK(cudaMalloc(&cell_tmp, sizeof(int) * std::max(N, 1)));
-		CK(cudaMalloc(&scan_part, sizeof(int) * (scan_tiles(n_cells) + 1)));
+		CK(cudaMalloc(&scan_part, sizeof(int) * LIST_MAX_BLOCKS));
+		CK(cudaMalloc(&spos, sizeof(float4) * std::max(N, 1)));
+		CK(cudaMalloc(&sync, sizeof(ListSync)));
 		CK(cudaMalloc(&nb, sizeof(int) * (size_t) std::max(N, 1) * max_nb));
 		CK(cudaMalloc(&nnb, sizeof(int) * std::max(N, 1)));
 		if(dh) {
 			CK(cudaMalloc(&dh_nb, sizeof(int) * (size_t) std::max(N, 1) * max_nb));
 			CK(cudaMalloc(&dh_n, sizeof(int) * std::max(N, 1)));
+			CK(cudaMalloc(&sback, sizeof(float4) * std::max(N, 1)));
+			CK(cudaMalloc(&sa1, sizeof(float4) * std::max(N, 1)));
 		}
+		// (complete before any stream's build)
+		CK(cudaMemset(cell_count, 0, sizeof(int) * n_cells));
+		CK(cudaMemset(sync, 0, sizeof(ListSync)));
+		CK(cudaStreamSynchronize(nullptr));
 		return OXGB_OK;
 	}
 	void free_all() {
-		for(int **p : {&cell_of, &cell_count, &cell_start, &cell_cursor, &cell_list, &cell_tmp, &scan_part, &nb, &nnb, &dh_nb, &dh_n}) {
+		for(void **p : {(void **) &cell_of, (void **) &cell_count, (void **) &cell_start, (void **) &cell_cursor, (void **) &cell_list,
+					(void **) &cell_tmp, (void **) &scan_part, (void **) &nb, (void **) &nnb, (void **) &dh_nb, (void **) &dh_n,
+					(void **) &spos, (void **) &sback, (void **) &sa1, (void **) &sync}) {
 			if(*p) cudaFree(*p);
 			*p = nullptr;
 		}
@@ -333,6 +347,10 @@ static ListArgs list_args(ListBuffers &lb, int N, const float4 *pos, float box, 
 	a.cell_list = lb.cell_list;
 	a.cell_tmp = lb.cell_tmp;
 	a.scan_part = lb.scan_part;
+	a.spos = lb.spos;
+	a.sback = lb.sback;
+	a.sa1 = lb.sa1;
+	a.sync = lb.sync;
 	a.nb = lb.nb;
 	a.nnb = lb.nnb;
 	a.max_nb = lb.max_nb;
@@ -344,11 +362,18 @@ static ListArgs list_args(ListBuffers &lb, int N, const float4 *pos, float box, 
 	return a;
 }
 
+// Lanes per nucleotide of a list build's rows where the caller leaves the choice: 32 while the chip has
+// threads to spare
+static int default_list_kind(long long n) { return n * 32 > 150000 ? OXGB_LIST_GROUP16 : OXGB_LIST_WARP; }
+
 extern "C" int oxgb_verlet_update(oxgb_verlet *h, const void *d_poss, void *d_list_poss, const void *d_bonds, void *stream) {
 	if(!h || !d_poss || !d_list_poss || !d_bonds) return fail(OXGB_E_INVALID, "null argument");
 	ListArgs a = list_args(h->lb, h->N, (const float4 *) d_poss, (float) h->box, h->rverlet, (const int2 *) d_bonds,
 			(float4 *) d_list_poss, h->d_status, h->d_flag, 0);
 	a.col_major = 1;  // matrix_neighs[k * N + i], the layout NEXT_NEIGHBOUR reads
+	a.n_systems = 1;
+	a.local_cells = list_local_cells(h->N, h->lb.n_cells);
+	a.list_kind = default_list_kind(h->N);
 	CK(launch_list_build(a, (cudaStream_t) stream));
 	return OXGB_OK;
 }
@@ -421,7 +446,7 @@ struct oxgb_md {
 	TermRadii radii{};
 	int *status = nullptr, *flag = nullptr;
 	long long *step = nullptr;
-	double *esplit = nullptr, *sums = nullptr, *bussi_partials = nullptr, *bussi_state = nullptr;
+	double *esplit = nullptr, *sums = nullptr, *bussi_partials = nullptr, *bussi_state = nullptr, *bussi_draws = nullptr;
 	long long *bussi_stamp = nullptr, *open_step = nullptr;
 	unsigned *bussi_done = nullptr, *bussi_prep_done = nullptr;
 	double *bussi_tot = nullptr;
@@ -435,14 +460,13 @@ struct oxgb_md {
 	int ext_n = 0;
 	bool energies_fresh = false;  // Fe / Te hold the forces and energies of the current state
 
-	cudaStream_t stream = nullptr, side = nullptr, noise = nullptr;
-	cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_first = nullptr;
+	cudaStream_t stream = nullptr, noise = nullptr;
+	cudaEvent_t ev_join = nullptr, ev_first = nullptr;
 	float4 *bussi_vf = nullptr, *bussi_Lf = nullptr;  // Bussi: half-kicked v, L in FP32 (mixed)
 	double *h_stage = nullptr, *d_stage = nullptr;   // the state in the caller's layout: pinned host, device
 	int *d_bad = nullptr;                             // lowest nucleotide with a bad quaternion
 	cudaGraphExec_t gexec = nullptr;
 	int graph_steps = 0;
-	bool conditional_ok = true;
 	// shape of the MD step's force kernels (force_shape_of) and its measured launch time
 	int shape = 0;
 	double shape_us = 0.0;
@@ -454,13 +478,13 @@ struct oxgb_md {
 	int *d_id = nullptr, *d_slot = nullptr, *d_perm = nullptr, *d_inv = nullptr;
 	int2 *bonds0 = nullptr;
 	unsigned char *sort_scratch = nullptr;
-	int *d_cell_hil = nullptr, *d_hcount = nullptr, *d_hstart = nullptr, *d_hcursor = nullptr;  // Hilbert order
+	int *d_cell_hil = nullptr, *d_hcount = nullptr, *d_hstart = nullptr;  // Hilbert order
 	int list_kind = OXGB_LIST_WARP;  // neighbour-row kernel (OXGB_LIST_*: chosen at creation or by the autotuner)
 	bool sorting() const { return md.sort_every > 0; }
 
 	void free_layout() {
 		for(void **p : {(void **) &d_sys_nside, (void **) &d_sys_cell0, (void **) &d_cell_sys, (void **) &d_sys_box,
-					(void **) &d_sys_rv2, (void **) &d_sys_dh2, (void **) &d_cell_hil, (void **) &d_hcount, (void **) &d_hstart, (void **) &d_hcursor}) {
+					(void **) &d_sys_rv2, (void **) &d_sys_dh2, (void **) &d_cell_hil, (void **) &d_hcount, (void **) &d_hstart}) {
 			if(*p) cudaFree(*p);
 			*p = nullptr;
 		}
@@ -473,15 +497,13 @@ struct oxgb_md {
 					(void *) fback, (void *) fa1lo, (void *) fbacklo, (void *) site_back, (void *) site_base, (void *) list_pos, (void *) list_a1, (void *) list_back, (void *) bonds, F, T, Fe, Te, bond_f,
 					bond_tp, bond_tq, edge_acc, d_tab, (void *) d_sys, (void *) d_sys_off, (void *) d_sys_stale, (void *) d_chunk_sys,
 					(void *) d_chunk_first, (void *) d_sys_chunk0, (void *) d_sys_par, (void *) d_sys_seed, (void *) status,
-					(void *) flag, (void *) step, (void *) esplit, (void *) sums, (void *) bussi_partials, (void *) bussi_state,
+					(void *) flag, (void *) step, (void *) esplit, (void *) sums, (void *) bussi_partials, (void *) bussi_state, (void *) bussi_draws,
 					(void *) bussi_stamp, (void *) open_step, (void *) bussi_done, (void *) bussi_prep_done, (void *) bussi_tot, (void *) bussi_fpart, (void *) term_max, ext_rec, (void *) ext_nuc, (void *) ext_off, (void *) grp_off, (void *) grp_mem, (void *) d_rebuilds})
 			if(p) cudaFree(p);
 		lb.free_all();
 		tl.free_all();
 		if(stream) cudaStreamDestroy(stream);
-		if(side) cudaStreamDestroy(side);
 		if(noise) cudaStreamDestroy(noise);
-		if(ev_fork) cudaEventDestroy(ev_fork);
 		if(ev_join) cudaEventDestroy(ev_join);
 		if(ev_first) cudaEventDestroy(ev_first);
 		if(bussi_vf) cudaFree(bussi_vf);
@@ -512,6 +534,7 @@ static ThermoArgs thermo_args(oxgb_md *h, int step_offset = 0, bool engine_step 
 	t.sys_chunk0 = h->d_sys_chunk0;
 	t.bussi_partials = h->bussi_partials;
 	t.bussi_state = h->bussi_state;
+	t.bussi_draws = h->bussi_draws;
 	t.bussi_stamp = h->bussi_stamp;
 	t.bussi_done = h->bussi_done;
 	t.bussi_prep_done = h->bussi_prep_done;
@@ -751,7 +774,6 @@ static int layout_cells(oxgb_md *h) {
 		CK(cudaMalloc(&h->d_cell_hil, sizeof(int) * n_cells));
 		CK(cudaMalloc(&h->d_hcount, sizeof(int) * (n_cells + 1)));
 		CK(cudaMalloc(&h->d_hstart, sizeof(int) * (n_cells + 1)));
-		CK(cudaMalloc(&h->d_hcursor, sizeof(int) * (n_cells + 1)));
 		CK(cudaMemcpy(h->d_cell_hil, cell_hil.data(), sizeof(int) * n_cells, cudaMemcpyHostToDevice));
 	}
 	return OXGB_OK;
@@ -805,8 +827,7 @@ extern "C" int oxgb_md_create(int n_systems, const int *offsets, const double *b
 		delete h;
 		return fail(OXGB_E_INVALID, "list_kernel must be OXGB_LIST_AUTO, _WARP, _THREAD or _GROUP4/8/16");
 	}
-	h->list_kind = h->md.list_kernel == OXGB_LIST_AUTO ? OXGB_LIST_WARP : h->md.list_kernel;
-	h->conditional_ok = h->md.list_rebuild_node == 0;
+	h->list_kind = h->md.list_kernel == OXGB_LIST_AUTO ? default_list_kind(N / n_systems) : h->md.list_kernel;
 	h->dbl = md->precision == OXGB_PRECISION_DOUBLE;
 	h->rcut.assign(n_systems, 0.0);
 	h->rverlet.assign(n_systems, 0.f);
@@ -839,9 +860,7 @@ extern "C" int oxgb_md_create(int n_systems, const int *offsets, const double *b
 	for(int k = 0; k < n_systems; k++) seeds[k] = h->md.seed + (unsigned long long) k;
 
 	if(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
-			cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking) != cudaSuccess ||
 			cudaStreamCreateWithFlags(&h->noise, cudaStreamNonBlocking) != cudaSuccess ||
-			cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
 			cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming) != cudaSuccess ||
 			cudaEventCreateWithFlags(&h->ev_first, cudaEventDisableTiming) != cudaSuccess)
 		return bail(fail(OXGB_E_CUDA, "stream creation failed"));
@@ -896,6 +915,7 @@ extern "C" int oxgb_md_create(int n_systems, const int *offsets, const double *b
 		ok &= cudaMalloc(&h->bussi_Lf, sizeof(float4) * (size_t) N) == cudaSuccess;
 	}
 	ok &= cudaMalloc(&h->bussi_state, sizeof(double) * 16 * n_systems) == cudaSuccess;
+	ok &= cudaMalloc(&h->bussi_draws, sizeof(double) * 4 * n_systems * h->md.steps_per_graph) == cudaSuccess;
 	ok &= cudaMalloc(&h->bussi_stamp, sizeof(long long)) == cudaSuccess;
 	ok &= cudaMalloc(&h->bussi_done, sizeof(unsigned) * n_systems) == cudaSuccess;
 	ok &= cudaMalloc(&h->bussi_prep_done, sizeof(unsigned) * n_systems) == cudaSuccess;
@@ -1033,6 +1053,10 @@ static ListArgs md_list_args(oxgb_md *h, int check_flag) {
 	a.sys_dh2 = h->n_systems > 1 ? h->d_sys_dh2 : nullptr;
 	a.sys_stale = h->d_sys_stale;
 	a.n_systems = h->n_systems;
+	a.sys_off = h->d_sys_off;
+	a.local_cells = !h->sorting();
+	for(int k = 0; k < h->n_systems && a.local_cells; k++)
+		a.local_cells = list_local_cells(h->offsets[k + 1] - h->offsets[k], h->cell0[k + 1] - h->cell0[k]);
 	a.n_cells_total = h->cell0[h->n_systems];
 	a.fa1 = h->fa1;
 	a.fback = h->fback;
@@ -1067,7 +1091,6 @@ static ListArgs md_list_args(oxgb_md *h, int check_flag) {
 		a.cell_hil = h->d_cell_hil;
 		a.hcount = h->d_hcount;
 		a.hstart = h->d_hstart;
-		a.hcursor = h->d_hcursor;
 	}
 	return a;
 }
@@ -1178,7 +1201,7 @@ static int autotune_shape(oxgb_md *h) {
 				if(h->offsets[k + 1] - h->offsets[k] > h->offsets[only + 1] - h->offsets[only]) only = k;
 		}
 		double best_list = 1e30;
-		for(int v = OXGB_LIST_WARP; v <= OXGB_LIST_GROUP16; v++) {
+		for(int v : {OXGB_LIST_GROUP16, OXGB_LIST_WARP}) {
 			h->list_kind = v;
 			int rc = build_list_now(h, only);
 			if(rc) return rc;
@@ -1413,23 +1436,16 @@ extern "C" int oxgb_md_get_state(oxgb_md *h, double *pos, double *quat, double *
 	return OXGB_OK;
 }
 
-// The Bussi draws depend only on (seed, step): they run on a second stream (a parallel branch
-// of the step graph) beside the first step, the list rebuild and the force kernels, and join
-// before the Bussi update.
-static cudaError_t fork_noise(oxgb_md *h, const StepArgs &sa) {
-	if(sa.th.thermostat != OXGB_THERMOSTAT_BUSSI) return cudaSuccess;
-	cudaError_t e = cudaEventRecord(h->ev_fork, h->stream);
-	if(e == cudaSuccess) e = cudaStreamWaitEvent(h->noise, h->ev_fork, 0);
-	if(e == cudaSuccess) e = launch_bussi_noise(sa, h->noise);
-	return e;
-}
-
-// after the first step of a Bussi step: the FP64 sums of the half-kicked state, on the side
-// branch (after the draws) while the main branch builds lists and evaluates forces
-static cudaError_t bussi_after_first_step(oxgb_md *h, const StepArgs &sa) {
+// A Bussi step's side branch, from the list build on and beside the force kernels: the FP64 sums of the
+// half-kicked state, and at the first of `steps` steps captured together the draws of all of them (they
+// depend only on the seed and the step).  It starts after the list build because a cooperative kernel
+// waits until the chip holds no other: beside the first step, the draws kept the build of a 96-system
+// batch waiting for 33 us in every step.
+static cudaError_t bussi_side_branch(oxgb_md *h, const StepArgs &sa, int steps) {
 	if(sa.th.thermostat != OXGB_THERMOSTAT_BUSSI) return cudaSuccess;
 	cudaError_t e = cudaEventRecord(h->ev_first, h->stream);
 	if(e == cudaSuccess) e = cudaStreamWaitEvent(h->noise, h->ev_first, 0);
+	if(e == cudaSuccess && sa.th.step_offset == 0) e = launch_bussi_noise(sa, steps, h->noise);
 	if(e == cudaSuccess) e = launch_bussi_prep(sa, h->n_chunks, h->dbl, h->noise);
 	if(e == cudaSuccess) e = cudaEventRecord(h->ev_join, h->noise);
 	return e;
@@ -1443,43 +1459,14 @@ static cudaError_t bussi_after_forces(oxgb_md *h, const StepArgs &sa) {
 	return e;
 }
 
-// one MD step on h->stream (captured into the graph at position k)
-static int enqueue_step(oxgb_md *h, cudaGraph_t capturing, int k) {
+// one MD step on h->stream, the k-th of `steps` captured together
+static int enqueue_step(oxgb_md *h, int k, int steps) {
 	StepArgs sa = step_args(h, k);
-	CK(fork_noise(h, sa));
 	CK(launch_first_step(sa, h->dbl, h->stream));
-	// the side branch reads the state: after the rebuild when a rebuild may move nucleotides
-	if(!h->sorting()) CK(bussi_after_first_step(h, sa));
-	ListArgs la = md_list_args(h, h->conditional_ok ? 0 : 1);
-	if(h->conditional_ok) {
-		cudaGraphConditionalHandle hc;
-		CK(cudaGraphConditionalHandleCreate(&hc, capturing, 0, cudaGraphCondAssignDefault));
-		CK(launch_set_conditional(h->flag, hc, h->stream));
-		cudaStreamCaptureStatus cs;
-		const cudaGraphNode_t *deps = nullptr;
-		size_t ndeps = 0;
-		cudaGraph_t g;
-		CK(cudaStreamGetCaptureInfo(h->stream, &cs, nullptr, &g, &deps, nullptr, &ndeps));
-		cudaGraphNodeParams cp{};
-		cp.type = cudaGraphNodeTypeConditional;
-		cp.conditional.handle = hc;
-		cp.conditional.type = cudaGraphCondTypeIf;
-		cp.conditional.size = 1;
-		cudaGraphNode_t node;
-		CK(cudaGraphAddNode(&node, g, deps, nullptr, ndeps, &cp));
-		cudaGraph_t body = cp.conditional.phGraph_out[0];
-		CK(cudaStreamBeginCaptureToGraph(h->side, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-		cudaError_t e1 = launch_list_build(la, h->side);
-		cudaGraph_t tmp;
-		cudaError_t e2 = cudaStreamEndCapture(h->side, &tmp);
-		CK(e1);
-		CK(e2);
-		CK(cudaStreamUpdateCaptureDependencies(h->stream, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
-	}
-	else {
-		CK(launch_list_build(la, h->stream));
-	}
-	if(h->sorting()) CK(bussi_after_first_step(h, sa));
+	ListArgs la = md_list_args(h, 1);
+	la.pdl = 1;
+	CK(launch_list_build(la, h->stream));
+	CK(bussi_side_branch(h, sa, steps));
 	ForceArgs fa = force_args(h, k, true);
 	CK(launch_forces_split(fa, h->dbl, false, false, h->stream));
 	CK(bussi_after_forces(h, sa));
@@ -1492,38 +1479,31 @@ static int build_graph(oxgb_md *h) {
 		h->gexec = nullptr;
 	}
 	const int K = h->md.steps_per_graph;
-	for(int attempt = 0; attempt < 2; attempt++) {
-		cudaGraph_t g;
-		CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeRelaxed));
-		cudaStreamCaptureStatus cs;
-		cudaGraph_t cap;
-		CK(cudaStreamGetCaptureInfo(h->stream, &cs, nullptr, &cap, nullptr, nullptr, nullptr));
-		int rc = OXGB_OK;
-		for(int k = 0; k < K && rc == OXGB_OK; k++) rc = enqueue_step(h, cap, k);
-		if(rc == OXGB_OK) {
-			StepArgs sa = step_args(h);
-			cudaError_t e = launch_step_advance(sa, K, h->stream);
-			if(e != cudaSuccess) rc = fail(OXGB_E_CUDA, cudaGetErrorString(e));
-		}
-		cudaError_t ee = cudaStreamEndCapture(h->stream, &g);
-		if(rc == OXGB_OK && ee == cudaSuccess) {
-			cudaError_t ie = cudaGraphInstantiate(&h->gexec, g, 0);
-			cudaGraphDestroy(g);
-			if(ie == cudaSuccess) {
-				h->graph_steps = K;
-				return OXGB_OK;
-			}
-			rc = fail(OXGB_E_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(ie));
-		}
-		else if(ee == cudaSuccess) {
-			cudaGraphDestroy(g);
-		}
-		cudaGetLastError();
-		if(!h->conditional_ok) return rc ? rc : fail(OXGB_E_CUDA, "graph capture failed");
-		// fall back to always-launched rebuild kernels that exit early on a fresh list
-		h->conditional_ok = false;
+	cudaGraph_t g;
+	CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeRelaxed));
+	int rc = OXGB_OK;
+	for(int k = 0; k < K && rc == OXGB_OK; k++) rc = enqueue_step(h, k, K);
+	if(rc == OXGB_OK) {
+		StepArgs sa = step_args(h);
+		cudaError_t e = launch_step_advance(sa, K, h->stream);
+		if(e != cudaSuccess) rc = fail(OXGB_E_CUDA, cudaGetErrorString(e));
 	}
-	return fail(OXGB_E_CUDA, "graph capture failed");
+	cudaError_t ee = cudaStreamEndCapture(h->stream, &g);
+	if(rc == OXGB_OK && ee == cudaSuccess) {
+		cudaError_t ie = cudaGraphInstantiate(&h->gexec, g, 0);
+		cudaGraphDestroy(g);
+		if(ie == cudaSuccess) {
+			h->graph_steps = K;
+			return OXGB_OK;
+		}
+		h->gexec = nullptr;
+		rc = fail(OXGB_E_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(ie));
+	}
+	else if(ee == cudaSuccess) {
+		cudaGraphDestroy(g);
+	}
+	cudaGetLastError();
+	return rc ? rc : fail(OXGB_E_CUDA, "graph capture failed");
 }
 
 extern "C" int oxgb_md_run(oxgb_md *h, int nsteps, int sync) {
@@ -1540,16 +1520,9 @@ extern "C" int oxgb_md_run(oxgb_md *h, int nsteps, int sync) {
 	}
 	// remainder, eagerly
 	for(; done < nsteps; done++) {
+		const int rc = enqueue_step(h, 0, 1);
+		if(rc) return rc;
 		StepArgs sa = step_args(h);
-		CK(fork_noise(h, sa));
-		CK(launch_first_step(sa, h->dbl, h->stream));
-		if(!h->sorting()) CK(bussi_after_first_step(h, sa));
-		ListArgs la = md_list_args(h, 1);
-		CK(launch_list_build(la, h->stream));
-		if(h->sorting()) CK(bussi_after_first_step(h, sa));
-		ForceArgs fa = force_args(h, 0, true);
-		CK(launch_forces_split(fa, h->dbl, false, false, h->stream));
-		CK(bussi_after_forces(h, sa));
 		CK(launch_step_advance(sa, 1, h->stream));
 	}
 	// the last step's second half kick and thermostat, so that the state is complete whenever

@@ -1132,7 +1132,11 @@ __device__ __forceinline__ void edge_block(const ForceArgs &a, const Loader &ld,
 // edge blocks.  G: groups of 32 nucleotides per pair block.
 template <typename R, class Loader, bool SPLIT, bool ENERGY, int G, bool EDGE = false, int K = 4>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? OXGB_PAIR_MINB : 1) k_bonded_pairs(ForceArgs a, Loader ld, int pair_blocks) {
-	pdl_trigger();  // the non-bonded kernel may start (it waits before reading these results)
+	// launched programmatically after the list build, it reads nothing before that is complete; nor may
+	// the non-bonded kernel start before (it reads the lists and mirrors at once, and waits only for
+	// these results)
+	pdl_wait();
+	pdl_trigger();
 	const int b = blockIdx.x;
 	const int bonded_blocks = (a.N + BONDS_PER_BLOCK - 1) / BONDS_PER_BLOCK;
 	if(b < pair_blocks) pair_block<R, Loader, SPLIT, ENERGY, G>(a, ld, b);
@@ -1718,7 +1722,8 @@ static void launch_split_t(const ForceArgs &a, Loader ld, cudaStream_t s, cudaEv
 	// (use_edge) one edge block per 128 / K nucleotides
 	const int pair_blocks = (a.N + PAIR_GROUP * G - 1) / (PAIR_GROUP * G);
 	const int edge_blocks = EDGE ? nonbonded_blocks(a.N, K) : 0;
-	k_bonded_pairs<R, Loader, SPLIT, ENERGY, G, EDGE, K><<<pair_blocks + blocks + edge_blocks, tpb, 0, s>>>(a, ld, pair_blocks);
+	launch_after(k_bonded_pairs<R, Loader, SPLIT, ENERGY, G, EDGE, K>, dim3(pair_blocks + blocks + edge_blocks), dim3(tpb), 0, s, a, ld,
+			pair_blocks);
 	// the non-bonded kernel starts its Debye-Hueckel and excluded-volume work while the tail of
 	// the bonded and pair blocks runs; the external forces follow it the same way
 	if(wait) cudaStreamWaitEvent(s, wait, 0);

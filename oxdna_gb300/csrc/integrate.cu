@@ -366,10 +366,10 @@ __global__ void __launch_bounds__(64, 16) k_first_step(StepArgs a) {
 
 // ---------------------------------------------------------------- thermostats
 
-// the Bussi draws of the current step for system blockIdx.x: warp 0 translational (channel 0),
-// warp 1 rotational (channel 1)
+// the Bussi draws of the blockIdx.y-th step from this one on for system blockIdx.x: warp 0
+// translational (channel 0), warp 1 rotational (channel 1)
 __global__ void k_bussi_noise(StepArgs a) {
-	const long long s = step_of(a.th);
+	const long long s = step_of(a.th) + blockIdx.y;
 	const int sy = blockIdx.x;
 	if(s % a.th.newtonian_steps != 0 || (threadIdx.x & 31) != 0) return;
 	const int w = threadIdx.x >> 5;
@@ -379,8 +379,9 @@ __global__ void k_bussi_noise(StepArgs a) {
 	rs.init(a.th.sys_seed[sy], s, (unsigned) w);
 	double sum, rr;
 	bussi_draws(rs, w == 0 ? 3 * (n - 1) : 3 * n, sum, rr);
-	a.th.bussi_state[16 * sy + 8 + 2 * w] = sum;
-	a.th.bussi_state[16 * sy + 9 + 2 * w] = rr;
+	double *to = a.th.bussi_draws + 4 * ((size_t) blockIdx.y * a.th.n_systems + sy) + 2 * w;
+	to[0] = sum;
+	to[1] = rr;
 }
 
 // ---------------------------------------------------------------- Bussi kinetic sums
@@ -732,11 +733,6 @@ __global__ void __launch_bounds__(256) k_system_sums(StepArgs a, double *out) {
 	}
 }
 
-__global__ void k_set_conditional(const int *flag, cudaGraphConditionalHandle h) {
-	pdl_wait();  // launched after the first step, which raises the flag
-	if(threadIdx.x == 0 && blockIdx.x == 0) cudaGraphSetConditional(h, *flag != 0 ? 1u : 0u);
-}
-
 // ---------------------------------------------------------------- launchers
 
 static inline int blocks_for(int N, int tpb) { return N > 0 ? (N + tpb - 1) / tpb : 1; }
@@ -749,8 +745,8 @@ cudaError_t launch_first_step(const StepArgs &a, bool double_forces, cudaStream_
 	return launch_after(k_first_step<float4>, dim3(blocks_for(a.N, 32)), dim3(64), 0, s, a);
 }
 
-cudaError_t launch_bussi_noise(const StepArgs &a, cudaStream_t s) {
-	k_bussi_noise<<<a.th.n_systems, 64, 0, s>>>(a);
+cudaError_t launch_bussi_noise(const StepArgs &a, int steps, cudaStream_t s) {
+	k_bussi_noise<<<dim3(a.th.n_systems, steps), 64, 0, s>>>(a);
 	return cudaGetLastError();
 }
 
@@ -775,10 +771,6 @@ cudaError_t launch_step_flush(const StepArgs &a, bool double_forces, cudaStream_
 	else k_step_flush<float4><<<blocks_for(a.N, 256), 256, 0, s>>>(a);
 	k_step_flush_clear<<<1, 32, 0, s>>>(a);
 	return cudaGetLastError();
-}
-
-cudaError_t launch_set_conditional(const int *flag, cudaGraphConditionalHandle h, cudaStream_t s) {
-	return launch_after(k_set_conditional, dim3(1), dim3(32), 0, s, flag, h);
 }
 
 cudaError_t launch_make_mirrors(const StepArgs &a, cudaStream_t s) {

@@ -11,6 +11,7 @@
 #define OXGB_ERR_NEIGH_OVERFLOW 2  /* a neighbour row exceeded its capacity */
 #define OXGB_ERR_NONFINITE 4       /* a non-finite or huge coordinate */
 #define OXGB_ERR_CELL 8            /* cell index out of range */
+#define OXGB_ERR_SYNC 16           /* a list build's blocks did not meet at their barrier */
 
 namespace oxgb {
 
@@ -82,8 +83,9 @@ struct ThermoArgs {
 	                                       // |F|^2, L.T, |T|^2) go to bussi_fpart
 	float4 *bussi_vf, *bussi_Lf;           // [N] half-kicked v and L rounded to FP32 (mixed precision)
 	double *bussi_state;                   // [n_systems * 16]: K_t, K_r, factor_t, factor_r,
-	                                       // vcom x y z, -, then the step's draws: sum_t, rr_t,
-	                                       // sum_r, rr_r
+	                                       // vcom x y z
+	double *bussi_draws;                   // [steps per graph][n_systems * 4] the draws of a step: sum_t,
+	                                       // rr_t, sum_r, rr_r
 	unsigned *bussi_done;                  // [n_systems] chunks arrived in this step's sums (0 between steps)
 	unsigned *bussi_prep_done;             // the same for the sums of the half-kicked state
 	double *bussi_tot;                     // [n_systems * 8] system totals of the half-kicked state
@@ -177,6 +179,12 @@ int nonbonded_blocks(int N, int lanes);
 int force_shape_count();
 void force_shape_of(int k, int *npw, int *lanes, int *minb);
 
+// the grid barrier of a list build (zero before the first one)
+struct ListSync {
+	unsigned count, gen;
+};
+constexpr int LIST_MAX_BLOCKS = 1024;
+
 struct ListArgs {
 	int N;
 	const float4 *pos;      // FP32 positions the list is built from (hi part)
@@ -185,12 +193,18 @@ struct ListArgs {
 	int n_side;             // cells per side
 	const int2 *bonds;
 	int *cell_of;           // [N]
-	int *cell_count;        // [n_cells]
+	int *cell_count;        // [n_cells], zero between builds (and before the first)
 	int *cell_start;        // [n_cells + 1]
 	int *cell_cursor;       // [n_cells]
 	int *cell_list;         // [N] particles by cell, by caller's index within a cell
 	int *cell_tmp;          // [N] scatter target before the ordering
-	int *scan_part;         // [scan_tiles(n_cells) + 1]
+	int *scan_part;         // [LIST_MAX_BLOCKS]
+	float4 *spos, *sback, *sa1;  // [N] positions (w: nucleotide), backbone offsets and a1 in the order of
+	                        // cell_list; the last two with term lists or Debye-Hueckel rows (else null)
+	ListSync *sync;
+	int pdl;                // launched programmatically after the kernel before it
+	int local_cells;        // every system is small: its cells are filled by one block (never when sorting)
+	const int *sys_off;     // [n_systems + 1] first nucleotide of each system (null: one system)
 	int *nb, *nnb;          // [N * max_nb], [N]
 	int max_nb;
 	float4 *list_pos;       // positions at this build
@@ -244,12 +258,10 @@ struct ListArgs {
 	unsigned char *scratch; // [N * SORT_BYTES]
 	// Hilbert order of the cells (null: row-major cell order): cell c of the global numbering is
 	// the cell_hil[c]-th of its system's cells along a Hilbert curve (plus the system's first
-	// cell); hcount / hstart / hcursor [n_cells + 1] are the counts and the exclusive scan in that
-	// order.  hilbert_pass marks the argument copy that runs the scan kernels on them.
+	// cell); hcount / hstart [n_cells + 1] are the counts and the exclusive scan in that order
 	const int *cell_hil;
-	int *hcount, *hstart, *hcursor;
-	int hilbert_pass;
-	int list_kind;          // neighbour-row kernel: OXGB_LIST_WARP, _THREAD or _GROUP4/8/16
+	int *hcount, *hstart;
+	int list_kind;          // lanes per nucleotide of the rows: OXGB_LIST_*
 };
 
 // bytes per nucleotide of the sort's staging buffer: 4 FP64 vectors, 9 vectors of 32 bits, bonds,
@@ -257,10 +269,15 @@ struct ListArgs {
 #define SORT_MIRRORS 9
 #define SORT_BYTES (4 * 32 + SORT_MIRRORS * 16 + 8 + 4 + 4)
 
-// full rebuild: cells (counting sort, deterministic order) then neighbour rows
+// A system's cells are filled by one block up to this many nucleotides (four of a thread's at once) and
+// cells (4096 at a time, a few microseconds each); beyond, by the grid in phases, whose four barriers take
+// about 2.5 us each
+constexpr int LIST_LOCAL_N = 4096;
+inline bool list_local_cells(long long n, long long cells) { return n <= LIST_LOCAL_N && cells <= 16384; }
+
+// the build, one cooperative launch: cells (counting sort, deterministic order) then neighbour rows; with
+// check_flag it returns at once while the lists are fresh
 cudaError_t launch_list_build(const ListArgs &a, cudaStream_t s);
-// size of ListArgs::scan_part is scan_tiles(n_cells) + 1
-int scan_tiles(int n_cells);
 
 struct StepArgs {
 	int N;
@@ -286,9 +303,8 @@ struct StepArgs {
 // first half of an MD step: completes a pending half kick and the previous step's thermostat,
 // then half kick, drift, rotation, FP32 mirrors and the list-staleness flags
 cudaError_t launch_first_step(const StepArgs &a, bool double_forces, cudaStream_t s);
-// the Bussi draws of the current step, per system (they do not depend on the state: they run
-// beside the step)
-cudaError_t launch_bussi_noise(const StepArgs &a, cudaStream_t s);
+// the Bussi draws of `steps` steps from this one on, per system (they do not depend on the state)
+cudaError_t launch_bussi_noise(const StepArgs &a, int steps, cudaStream_t s);
 // Bussi kinetic-energy sums of the half-kicked state (after the first step, beside the forces)
 // and of the force terms with the per-system update (after the forces); n_chunks chunks of up to
 // 256 nucleotides
@@ -305,7 +321,6 @@ cudaError_t launch_step_flush(const StepArgs &a, bool double_forces, cudaStream_
 // check_only that is all that is written)
 cudaError_t launch_unpack_state(const StepArgs &a, const double *in, int *bad, bool check_only, cudaStream_t s);
 cudaError_t launch_pack_state(const StepArgs &a, double *out, cudaStream_t s);
-cudaError_t launch_set_conditional(const int *flag, cudaGraphConditionalHandle h, cudaStream_t s);
 // refresh the FP32 mirrors from the FP64 state (after a host upload)
 cudaError_t launch_make_mirrors(const StepArgs &a, cudaStream_t s);
 // velocities and angular momenta of nucleotides lo .. hi - 1 times f

@@ -1,22 +1,22 @@
 // Verlet-list build that allocates no device memory.
 //
-// oxgb_verlet_build_noalloc runs the same kernels as oxgb_verlet_update (lists.cu): counting
-// sort into cells, then one warp per nucleotide over the 27 neighbouring cells.  Their scratch
+// oxgb_verlet_build_noalloc runs the same kernel as oxgb_verlet_update (lists.cu): counting
+// sort into cells, then the rows over the 27 neighbouring cells.  Its scratch
 // (cell of every nucleotide, the cell segments, the per-cell counts, starts and cursors, the
-// scan tiles, the status word) lives in the file-scope device arrays below instead of buffers
+// block sums, the positions in cell order, the barrier, the status word) lives in the file-scope device arrays below instead of buffers
 // owned by an oxgb_verlet handle.  The caller owns every output buffer.
 //
 // Limits: N <= OXGB_NOALLOC_MAX_N nucleotides and at most OXGB_NOALLOC_MAX_CELLS cells (the
 // cell grid follows the same sizing rule as the handle-based list); larger requests are
-// rejected before anything is launched.  The scratch is ~1.2 MB of device memory per device,
+// rejected before anything is launched.  The scratch is ~2.3 MB of device memory per device,
 // set aside when the module is loaded.
 //
 // The host finds the scratch with cudaGetSymbolAddress, once per device (with that device
 // current), and checks on every call that the module was not reloaded since; the first call
 // on a device may load the module, so it should come before any stream capture.  Calls on one device share the scratch: two calls
 // that overlap in time (different streams or threads) race and must be serialised by the
-// caller.  Each call clears what must start at zero (the status word; the cell counts are
-// zeroed by the build itself), so consecutive calls never see each other's leftovers.
+// caller.  Each call clears what must start at zero (the status word; the cell counts are left at
+// zero by the build itself), so consecutive calls never see each other's leftovers.
 #include "kernels.h"
 #include "params.h"
 
@@ -31,7 +31,6 @@ std::string list_status_message(int st);
 
 constexpr int NOALLOC_MAX_N = OXGB_NOALLOC_MAX_N;
 constexpr int NOALLOC_MAX_CELLS = OXGB_NOALLOC_MAX_CELLS;
-constexpr int NOALLOC_TILES = (NOALLOC_MAX_CELLS + 2047) / 2048 + 1;  // scan_tiles(max) + 1
 
 static __device__ __align__(256) int g_cell_of[NOALLOC_MAX_N];
 static __device__ __align__(256) int g_cell_tmp[NOALLOC_MAX_N];
@@ -39,11 +38,15 @@ static __device__ __align__(256) int g_cell_list[NOALLOC_MAX_N];
 static __device__ __align__(256) int g_cell_count[NOALLOC_MAX_CELLS];
 static __device__ __align__(256) int g_cell_start[NOALLOC_MAX_CELLS + 1];
 static __device__ __align__(256) int g_cell_cursor[NOALLOC_MAX_CELLS];
-static __device__ __align__(256) int g_scan_part[NOALLOC_TILES];
+static __device__ __align__(256) int g_scan_part[LIST_MAX_BLOCKS];
+static __device__ __align__(256) float4 g_spos[NOALLOC_MAX_N];
+static __device__ __align__(256) ListSync g_sync;
 static __device__ __align__(256) int g_status[2];  // status word, rebuild flag
 
 struct Scratch {
 	int *cell_of, *cell_tmp, *cell_list, *cell_count, *cell_start, *cell_cursor, *scan_part, *status;
+	float4 *spos;
+	ListSync *sync;
 };
 
 static std::mutex g_scratch_mutex;
@@ -82,6 +85,10 @@ static cudaError_t scratch_of_current_device(Scratch &out) {
 		s.cell_cursor = (int *) p;
 		if((e = cudaGetSymbolAddress(&p, g_scan_part)) != cudaSuccess) return e;
 		s.scan_part = (int *) p;
+		if((e = cudaGetSymbolAddress(&p, g_spos)) != cudaSuccess) return e;
+		s.spos = (float4 *) p;
+		if((e = cudaGetSymbolAddress(&p, g_sync)) != cudaSuccess) return e;
+		s.sync = (ListSync *) p;
 		if((e = cudaGetSymbolAddress(&p, g_status)) != cudaSuccess) return e;
 		s.status = (int *) p;
 		g_scratch[dev] = s;
@@ -132,6 +139,8 @@ extern "C" int oxgb_verlet_build_noalloc(int N, double box, double rcut, double 
 	a.cell_list = sc.cell_list;
 	a.cell_tmp = sc.cell_tmp;
 	a.scan_part = sc.scan_part;
+	a.spos = sc.spos;
+	a.sync = sc.sync;
 	a.nb = d_matrix_neighs;
 	a.nnb = d_number_neighs;
 	a.max_nb = max_neigh;
@@ -141,6 +150,8 @@ extern "C" int oxgb_verlet_build_noalloc(int N, double box, double rcut, double 
 	a.check_flag = 0;
 	a.rebuilds = nullptr;
 	a.col_major = 1;
+	a.n_systems = 1;
+	a.local_cells = list_local_cells(N, n_cells);
 	e = launch_list_build(a, s);
 	if(e != cudaSuccess) return set_error(OXGB_E_CUDA, std::string("list build: ") + cudaGetErrorString(e));
 	int st = 0;

@@ -212,12 +212,13 @@ static __device__ __noinline__ double4_32a brownian_redraw_warp(const ThermoArgs
 static __device__ void bussi_update(const ThermoArgs &t, int sy, long long s, int which, const double sum[5]) {
 	const double *par = t.sys_par + sy * SP_STRIDE;
 	double *st = t.bussi_state + 16 * sy;
+	const double *dr = t.bussi_draws + 4 * ((size_t) t.step_offset * t.n_systems + sy);
 	if(which == 0) {
 		const double inv_n = par[SP_INVN];
 		const double n = (double) (t.sys_off[sy + 1] - t.sys_off[sy]);
 		const double vc[3] = {sum[0] * inv_n, sum[1] * inv_n, sum[2] * inv_n};
 		const double Kt_now = 0.5 * (sum[3] - n * (vc[0] * vc[0] + vc[1] * vc[1] + vc[2] * vc[2]));
-		update_K(st[0], par[SP_1MC], par[SP_A], par[SP_B], __ldcg(st + 8), __ldcg(st + 9));
+		update_K(st[0], par[SP_1MC], par[SP_A], par[SP_B], __ldcg(dr), __ldcg(dr + 1));
 		st[2] = sqrt(st[0]) * rsqrt(Kt_now);
 		st[4] = vc[0];
 		st[5] = vc[1];
@@ -225,7 +226,7 @@ static __device__ void bussi_update(const ThermoArgs &t, int sy, long long s, in
 	}
 	else {
 		const double Kr_now = 0.5 * sum[4];
-		update_K(st[1], par[SP_1MC], par[SP_A], par[SP_B], __ldcg(st + 10), __ldcg(st + 11));
+		update_K(st[1], par[SP_1MC], par[SP_A], par[SP_B], __ldcg(dr + 2), __ldcg(dr + 3));
 		st[3] = sqrt(st[1]) * rsqrt(Kr_now);
 	}
 }
