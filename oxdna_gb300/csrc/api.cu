@@ -148,9 +148,9 @@ extern "C" int oxgb_dna2_compute_forces(oxgb_dna2 *h, int N, double box, const v
 		int rc = dna2_upload(h, box);
 		if(rc) return rc;
 	}
-	ForceArgs a{};
+	RefArgs a{};
 	a.N = N;
-	a.pos_hi = (const float4 *) d_poss;
+	a.pos = (const float4 *) d_poss;
 	a.quat = (const float4 *) d_orientations;
 	a.bonds = (const int2 *) d_bonds;
 	a.nb = d_matrix_neighs;
@@ -158,8 +158,8 @@ extern "C" int oxgb_dna2_compute_forces(oxgb_dna2 *h, int N, double box, const v
 	a.max_nb = max_neigh;
 	a.nb_stride_i = stride_i;
 	a.nb_stride_k = stride_k;
-	a.forces = d_forces;
-	a.torques = d_torques;
+	a.forces = (float4 *) d_forces;
+	a.torques = (float4 *) d_torques;
 	a.table = h->d_tab;
 	a.status = h->d_status;
 	CK(launch_forces_reference_layout(a, (cudaStream_t) stream));

@@ -1,19 +1,12 @@
-// oxDNA2 force and torque kernel: one warp per nucleotide.
+// oxDNA2 force and torque kernels.
 //
-// Lanes stride over the nucleotide's neighbour row (full list: every pair is seen from both
-// ends, so no atomics and a fixed summation order); lanes 0 and 1 also take the 3' and 5'
-// bonded pairs.  Each lane accumulates its pair forces, lab-frame torques and energies with
-// compensated (Kahan) sums, the warp combines them with an error-free TwoSum butterfly, and
-// lane 0 rotates the torque into the body frame and writes the result.  Replaces the
+// The engine's (mixed and FP64) evaluate bonds and pair terms once per pair, in blocks of their own
+// (k_bonded_pairs), and Debye-Hueckel and the excluded volume from each end of a nucleotide's rows
+// (k_nonbonded_*), with no atomics and a fixed summation order.  The reference layout (float4 positions
+// with btype/index packed in w, float4 quaternions, int2 bonds and a neighbour matrix of any stride) has
+// a kernel of its own, which accumulates into forces and torques initialised by the caller, exactly the
+// contract of CUDABaseInteraction::compute_forces (k_forces_reference, at the end).  They replace the
 // reference's thread-per-nucleotide dna_forces (src/CUDA/Interactions/CUDA_DNA.cuh:832-904).
-//
-// Three instantiations:
-//  * FP32 "mixed" path: positions as a hi/lo float pair so that pair separations keep ~1e-7
-//    absolute accuracy in boxes of side 200+, quaternions in FP32, FP32 pair math;
-//  * FP64 path: the same physics in double, for parity against the FP64 oracle;
-//  * reference layout: float4 positions with btype/index packed in w, float4 quaternions,
-//    int2 bonds and a neighbour matrix of any stride, accumulating into forces and torques
-//    initialised by the caller, exactly the contract of CUDABaseInteraction::compute_forces.
 #include "kernels.h"
 #include "split.cuh"
 
@@ -37,23 +30,6 @@ struct KahanV {
 	}
 };
 
-// sum over the warp of (s - c) pairs with TwoSum at every butterfly level; all lanes get it
-template <typename R>
-__device__ __forceinline__ R warp_sum_comp(R s, R c) {
-	R err = -c;
-#pragma unroll
-	for(int off = 16; off > 0; off >>= 1) {
-		const R so = __shfl_xor_sync(0xffffffffu, s, off);
-		const R eo = __shfl_xor_sync(0xffffffffu, err, off);
-		const R t = s + so;
-		const R bp = t - s;
-		const R e2 = (s - (t - bp)) + (so - bp);
-		s = t;
-		err += eo + e2;
-	}
-	return s + err;
-}
-
 __device__ __forceinline__ int ref_type_of_btype(int bt) {
 	return (bt > 0) ? (bt & 3) : 3 - ((3 - bt) & 3);
 }
@@ -64,6 +40,26 @@ template <typename R>
 __device__ __forceinline__ const DNA2Table<R> &table_of(const ForceArgs &a, int sy) {
 	return reinterpret_cast<const DNA2Table<R> *>(a.table)[sy];
 }
+
+// Debye-Hueckel of a pair in FP32 (dh_sites): the force on p over the vector from p's backbone site to
+// q's, and the energy, at squared distance r2 < rc2; cut: the end charges' factor.  1 / r by a Newton step
+// on the approximate reciprocal square root, both branches evaluated (a third of the pairs is inside
+// the smoothing range, so a warp takes both anyway).
+struct DebyeF {
+	float rc, rc2, rhigh, mk, pre, b, half;
+	__device__ __forceinline__ explicit DebyeF(const DNA2Table<float> &P)
+		: rc(P.dh_rc), rc2(P.dh_rc * P.dh_rc), rhigh(P.dh_rhigh), mk(P.dh_minus_kappa), pre(P.dh_prefactor), b(P.dh_b),
+		  half(P.dh_half_charged_ends ? 0.5f : 1.f) {}
+	__device__ __forceinline__ float force(float r2, float cut, float &e) const {
+		float v = rsqrtf(r2);
+		v = v * fmaf(-0.5f * r2 * v, v, 1.5f);
+		const float r = r2 * v;
+		const float ex = pre * m_exp(mk * r), g = b * (r - rc);
+		const bool in = r < rhigh;
+		e = cut * (in ? ex * v : g * (r - rc));
+		return -((in ? ex * (v - mk) * v : -2.f * g) * cut) * v;
+	}
+};
 
 // ---------------------------------------------------------------- particle loaders
 
@@ -162,6 +158,7 @@ struct LoadDouble {
 
 struct LoadRef {
 	const float4 *pos, *quat;
+	__device__ __forceinline__ NoRefine refine(int, int) const { return NoRefine{}; }
 	__device__ __forceinline__ void load(int i, const DNA2Table<float> &P, const int2 b, Nuc<float> &n, float4 &hi,
 			float4 &lo) const {
 		hi = pos[i];
@@ -177,7 +174,7 @@ struct LoadRef {
 			const DNA2Table<float> &P) const {
 		float d[3] = {qh.x - ph.x, qh.y - ph.y, qh.z - ph.z};
 #pragma unroll
-		for(int k = 0; k < 3; k++) d[k] = fmaf(-rintf(d[k] / P.box_hi), P.box_hi, d[k]);
+		for(int k = 0; k < 3; k++) d[k] = fmaf(-rintf(d[k] * P.inv_box), P.box_hi, d[k]);
 		return Sep<float>{v3<float>{d[0], d[1], d[2]}, v3<float>{0.f, 0.f, 0.f}};
 	}
 	__device__ __forceinline__ Sep<float> diff(const float4 &ph, const float4 &, const float4 &qh, const float4 &) const {
@@ -195,137 +192,6 @@ template <>
 struct Vec4Of<double> {
 	using T = double4_32a;
 };
-
-// ---------------------------------------------------------------- the kernel
-
-template <typename R, class Loader, bool SPLIT, bool ACCUMULATE>
-__global__ void __launch_bounds__(128) k_forces(ForceArgs a, Loader ld) {
-	using V4 = typename Vec4Of<R>::T;
-	const DNA2Table<R> &P = table_of<R>(a, 0);
-
-	const int lane = threadIdx.x & 31;
-	const int warps_per_block = blockDim.x >> 5;
-	const int gw = blockIdx.x * warps_per_block + (threadIdx.x >> 5);
-	const int nw = gridDim.x * warps_per_block;
-	V4 *F4 = reinterpret_cast<V4 *>(a.forces);
-	V4 *T4 = reinterpret_cast<V4 *>(a.torques);
-
-	for(int i = gw; i < a.N; i += nw) {
-		const int2 bi = a.bonds[i];
-		Nuc<R> p;
-		V4 ph, pl;
-		ld.load(i, P, bi, p, ph, pl);
-
-		KahanV<R> F{}, T{};
-		R E = R(0), Ec = R(0), Eh = R(0), Ehc = R(0);
-		R split[N_TERMS];
-		if(SPLIT) {
-#pragma unroll
-			for(int k = 0; k < N_TERMS; k++) split[k] = R(0);
-		}
-
-		// bonded pairs: lane 0 the 3' neighbour (p = i), lane 1 the 5' neighbour (q = i)
-		if(lane < 2) {
-			const int j = (lane == 0) ? bi.x : bi.y;
-			if(j >= 0) {
-				const int2 bj = a.bonds[j];
-				Nuc<R> q;
-				V4 qh, ql;
-				ld.load(j, P, bj, q, qh, ql);
-				PairOut<R> o{};
-				bool ok;
-				if(lane == 0) ok = bonded<R, SPLIT, false>(P, p, q, ld.diff(ph, pl, qh, ql), o);
-				else ok = bonded<R, SPLIT, true>(P, q, p, ld.diff(qh, ql, ph, pl), o);
-				if(!ok) atomicOr(a.status, OXGB_ERR_FENE);
-				F.add(o.F);
-				T.add(o.T);
-				KahanV<R>::kadd(E, Ec, o.E);
-				if(SPLIT) {
-#pragma unroll
-					for(int k = 0; k < N_TERMS; k++) split[k] += o.split[k];
-				}
-			}
-		}
-
-		const int nn = a.nnb[i];
-		if(nn > a.max_nb) atomicOr(a.status, OXGB_ERR_NEIGH_OVERFLOW);
-		const int nlim = nn < a.max_nb ? nn : a.max_nb;
-		const long long row = (long long) i * a.nb_stride_i;
-		for(int k = lane; k < nlim; k += 32) {
-			const int j = a.nb[row + (long long) k * a.nb_stride_k];
-			if(j == i || j == bi.x || j == bi.y) continue;
-			const int2 bj = a.bonds[j];
-			Nuc<R> q;
-			V4 qh, ql;
-			ld.load(j, P, bj, q, qh, ql);
-			PairOut<R> o{};
-			nonbonded_p<R, SPLIT>(P, p, q, ld.sep(ph, pl, qh, ql, P), o);
-			F.add(o.F);
-			T.add(o.T);
-			KahanV<R>::kadd(E, Ec, o.E);
-			KahanV<R>::kadd(Eh, Ehc, o.Ehb);
-			if(SPLIT) {
-#pragma unroll
-				for(int k2 = 0; k2 < N_TERMS; k2++) split[k2] += o.split[k2];
-			}
-		}
-
-		const R fx = warp_sum_comp(F.s.x, F.c.x), fy = warp_sum_comp(F.s.y, F.c.y), fz = warp_sum_comp(F.s.z, F.c.z);
-		const R tx = warp_sum_comp(T.s.x, T.c.x), ty = warp_sum_comp(T.s.y, T.c.y), tz = warp_sum_comp(T.s.z, T.c.z);
-		const R e = warp_sum_comp(E, Ec), eh = warp_sum_comp(Eh, Ehc);
-		if(SPLIT) {
-#pragma unroll
-			for(int k = 0; k < N_TERMS; k++) split[k] = warp_sum_comp(split[k], R(0));
-		}
-		if(lane == 0) {
-			const v3<R> tl{tx, ty, tz};
-			// body frame: components along a1, a2, a3
-			const R bx = dot(p.a1, tl), by = dot(p.a2, tl), bz = dot(p.a3, tl);
-			V4 fo, to;
-			if(ACCUMULATE) {
-				fo = F4[i];
-				to = T4[i];
-				fo.x += fx;
-				fo.y += fy;
-				fo.z += fz;
-				fo.w += e;
-				to.x += bx;
-				to.y += by;
-				to.z += bz;
-				to.w = eh;
-			}
-			else {
-				fo.x = fx;
-				fo.y = fy;
-				fo.z = fz;
-				fo.w = e;
-				to.x = bx;
-				to.y = by;
-				to.z = bz;
-				to.w = eh;
-			}
-			F4[i] = fo;
-			T4[i] = to;
-			if(SPLIT) {
-#pragma unroll
-				for(int k = 0; k < N_TERMS; k++) atomicAdd(a.esplit + k, 0.5 * (double) split[k]);
-			}
-		}
-	}
-}
-
-// ---------------------------------------------------------------- host launchers
-
-static int grid_for(int N, int warps_per_block) {
-	const int blocks = (N + warps_per_block - 1) / warps_per_block;
-	return blocks > 0 ? blocks : 1;
-}
-
-cudaError_t launch_forces_reference_layout(const ForceArgs &a, cudaStream_t s) {
-	LoadRef ld{a.pos_hi, a.quat};
-	k_forces<float, LoadRef, false, true><<<grid_for(a.N, 4), 128, 0, s>>>(a, ld);
-	return cudaGetLastError();
-}
 
 // FFS order parameters on the reference layout (hb_op_precalc, near_hb_op_precalc and
 // dist_op_precalc, src/CUDA/Interactions/CUDA_DNA.cuh:910-1067): one thread per listed pair
@@ -393,9 +259,8 @@ cudaError_t launch_order_params(int mode, const float4 *poss, const float4 *quat
 
 // ====================================================================== split path
 //
-// The warp-per-nucleotide kernel above leaves most lanes idle: a nucleotide has ~20-30
-// neighbours, only a few of them close enough for hydrogen bonding, cross or coaxial
-// stacking, and the two bonded pairs ran on two lanes.  The split path instead
+// A nucleotide has ~20-30 neighbours, only a few of them close enough for hydrogen bonding, cross or
+// coaxial stacking.  The split path
 //  * evaluates every bonded pair once, one thread per bond, for both nucleotides;
 //  * runs the non-bonded terms one thread per nucleotide, one loop per term over the term
 //    lists of the Verlet build (full rows for Debye-Hueckel, centre-close pairs for the
@@ -553,6 +418,12 @@ template <>
 __device__ __forceinline__ void load_axes<SplitMixed, float>(const SplitMixed &ld, int j, const DNA2Table<float> &, Nuc<float> &n,
 		float4 &h, float4 &l) {
 	ld.axes(j, n, h, l);
+}
+
+template <>
+__device__ __forceinline__ void load_axes<LoadRef, float>(const LoadRef &ld, int j, const DNA2Table<float> &P, Nuc<float> &n,
+		float4 &h, float4 &l) {
+	ld.load(j, P, make_int2(0, 0), n, h, l);
 }
 
 // Bonded block b: 64 bonds (owner p, partner q = n3[p]), a pair of threads each, in different warps:
@@ -783,9 +654,8 @@ static_assert(sizeof(PairItem<float>) == 63 * 4, "an odd number of words");
 
 // stage 2 of item m of pair (i, j), term 0 hydrogen bonding, 1 cross stacking, 2 coaxial stacking
 template <typename R, class Loader>
-__device__ __forceinline__ void pair_radial(const ForceArgs &a, const Loader &ld, int i, int j, int term, PairItem<R> &m) {
+__device__ __forceinline__ void pair_radial(const DNA2Table<R> &P, const Loader &ld, int i, int j, int term, PairItem<R> &m) {
 	using V4 = typename Vec4Of<R>::T;
-	const DNA2Table<R> &P = table_of<R>(a, a.sys ? a.sys[i] : 0);
 	Nuc<R> p, q;
 	V4 ph, pl, qh, ql;
 	load_axes<Loader, R>(ld, i, P, p, ph, pl);
@@ -952,7 +822,8 @@ __device__ __forceinline__ void pair_block(const ForceArgs &a, const Loader &ld,
 			while(c1 < n && (queue[c1].y & (1 << 18))) c1--;
 			for(int m = threadIdx.x; m < c1 - c0; m += 128) {
 				const int2 w = queue[c0 + m];
-				pair_radial<R, Loader>(a, ld, first + (w.y >> 19), w.x, (w.y >> 16) & 3, item[m]);
+				const int i = first + (w.y >> 19);
+				pair_radial<R, Loader>(table_of<R>(a, a.sys ? a.sys[i] : 0), ld, i, w.x, (w.y >> 16) & 3, item[m]);
 			}
 			__syncthreads();
 			for(int m0 = warp * 4; m0 < c1 - c0; m0 += 16) {  // warp-uniform: four items at a time
@@ -1344,9 +1215,8 @@ __global__ void __launch_bounds__(128, MINB) k_nonbonded_mixed(ForceArgs a, Spli
 		// the torque is taken once from the sum.
 		const int ndh = live ? min(a.dh_n[i], a.max_nb) : 0;
 		{
-			const float rc = P.dh_rc, rc2 = rc * rc, rh = P.dh_rhigh, mk = P.dh_minus_kappa, pre = P.dh_prefactor, b = P.dh_b;
-			const float half = P.dh_half_charged_ends ? 0.5f : 1.f;
-			const float pcut = back.w != 0.f ? half : 1.f;
+			const DebyeF D(P);
+			const float pcut = back.w != 0.f ? D.half : 1.f;
 			KahanV<float> f{};
 			int4 qn = pk;
 			int k = sub;
@@ -1358,19 +1228,11 @@ __global__ void __launch_bounds__(128, MINB) k_nonbonded_mixed(ForceArgs a, Spli
 				if(k + 2 * K < ndh) jn = a.dh_nb[(long long) (k + 2 * K) * N + i];
 				const float x = (float) (q.x - pk.x), y = (float) (q.y - pk.y), z = (float) (q.z - pk.z);
 				const float r2 = (x * x + y * y + z * z) * u2;
-				if(r2 < rc2) {
-					// 1 / r with a Newton step on the approximate reciprocal square root
-					float v = rsqrtf(r2);
-					v = v * fmaf(-0.5f * r2 * v, v, 1.5f);
-					const float r = r2 * v, cut = pcut * (q.w ? half : 1.f);
-					const float ex = pre * m_exp(mk * r), g = b * (r - rc);
-					const bool in = r < rh;
-					// -dE/dr / r, on p along its distance from q
-					const float fm = in ? ex * (v - mk) * v : -2.f * g;
-					const float s = -(fm * cut) * (v * unit);
+				if(r2 < D.rc2) {
+					float e;
+					const float s = D.force(r2, pcut * (q.w ? D.half : 1.f), e) * unit;
 					f.add(v3<float>{x * s, y * s, z * s});
 					if(ENERGY) {
-						const float e = cut * (in ? ex * v : g * (r - rc));
 						KahanV<float>::kadd(acc.E, acc.Ec, e);
 						if(SPLIT) acc.split[T_DH] += e;
 					}
@@ -1711,6 +1573,218 @@ __global__ void k_external(ForceArgs a) {
 	f.y += fy;
 	f.z += fz;
 	F[i] = f;
+}
+
+// ====================================================================== reference layout
+//
+// K lanes per nucleotide over its row of the neighbour matrix, every pair from both ends (the rows are
+// full, and a partner's share would need atomics).  A lane builds its partner's frame from the quaternion
+// (two 16-byte gathers per partner), evaluates Debye-Hueckel, screens the excluded volume (evaluated in
+// the rare case of a contact) and the pair terms; pairs with live terms go to the warp's queue, an item
+// per term, which the warp takes through the stages of the pair blocks: a lane per item, then eight lanes
+// per item.  The block's bonds, both sides of each nucleotide, are evaluated by two full warps, stacking by
+// one and FENE with the excluded volume by the other.  Sums are compensated and their order is fixed.
+//
+// Latency of the dependent chains bounds it.  40,000 duplex nucleotides: 65 us per call, 43 M warp
+// instructions; with a warp per nucleotide, each pair's terms on the lane that found it and the two bonds
+// on two lanes, where most lanes waited for the few on a long branch, 371 us.  Error of the forces against
+// 64 bits (24 states of 12,000 duplex nucleotides): 1.350e-6, that kernel's 1.353e-6.
+constexpr int REF_QUEUE = 64 + 3 * 32, REF_CHUNK = 16;
+
+// the plain excluded volume of a pair with a site pair in contact: force and torque on p, energy (rare,
+// out of line: the loop keeps its registers)
+__device__ __noinline__ float4 ev_pair_call(v3<float> r, v3<float> pa1, v3<float> pback, v3<float> qa1, v3<float> qback, float3 *T) {
+	Nuc<float> p, q;
+	p.base = pa1 * float(OXM_POS_BASE), p.back = pback;
+	q.base = qa1 * float(OXM_POS_BASE), q.back = qback;
+	PairOut<float> o{};
+	pair_ev<float, false>(p, q, Sep<float>{r, v3<float>{0.f, 0.f, 0.f}}, o);
+	*T = make_float3(o.T.x, o.T.y, o.T.z);
+	return make_float4(o.F.x, o.F.y, o.F.z, o.E);
+}
+
+template <int K>
+__global__ void __launch_bounds__(128, 4) k_forces_reference(RefArgs a) {
+	constexpr int NB = 128 / K, NW = 32 / K;  // nucleotides of a block, of a warp
+	__shared__ int2 queues[4][REF_QUEUE];      // partner; term | nucleotide of the warp << 2
+	__shared__ PairItem<float> items[4][REF_CHUNK];
+	__shared__ float bond[2][2 * NB][7];       // [stacking, backbone][nucleotide and side]: force, torque, energy
+	const LoadRef ld{a.pos, a.quat};
+	const DNA2Table<float> &P = *a.table;
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = threadIdx.x % K;
+	const int first = blockIdx.x * NB, wfirst = first + warp * NW;
+	const int i_raw = first + (int) threadIdx.x / K;
+	const bool live = i_raw < a.N;
+	const int i = live ? i_raw : a.N - 1;
+
+	// the block's bonds: side 0 of nucleotide u its 3' bond (u is p), side 1 its 5' bond (u is q)
+	if(warp < 2 && lane < 2 * NB) {
+		const int u = first + (lane >> 1), side = lane & 1;
+		const int2 bu = u < a.N ? a.bonds[u] : make_int2(-1, -1);
+		const int p = side ? bu.y : u, q = side ? u : bu.x;
+		float *out = bond[warp][lane];
+#pragma unroll
+		for(int k = 0; k < 7; k++) out[k] = 0.f;
+		if(p >= 0 && q >= 0) {
+			Nuc<float> np, nq;
+			float4 ph, pl, qh, ql;
+			ld.load(p, P, make_int2(0, 0), np, ph, pl);
+			ld.load(q, P, make_int2(0, 0), nq, qh, ql);
+			BondOut<float> o;
+			o.f = o.tp = o.tq = v3<float>{0.f, 0.f, 0.f};
+			o.split[0] = o.split[1] = o.split[2] = 0.f;
+			if(warp == 0) bonded_stacking(P, np, nq, ld.diff(ph, pl, qh, ql), o);
+			else if(!bonded_backbone(P, np, nq, ld.diff(ph, pl, qh, ql), o)) atomicOr(a.status, OXGB_ERR_FENE);
+			const float s = side ? 1.f : -1.f;
+			const v3<float> t = side ? o.tq : o.tp;
+			out[0] = s * o.f.x, out[1] = s * o.f.y, out[2] = s * o.f.z;
+			out[3] = t.x, out[4] = t.y, out[5] = t.z;
+			out[6] = o.split[0] + o.split[1] + o.split[2];
+		}
+	}
+
+	Nuc<float> p;
+	float4 ph, pl;
+	const int2 bi = a.bonds[i];
+	ld.load(i, P, bi, p, ph, pl);
+	SplitAcc<float, false, true> acc{};
+	KahanV<float> dh{};
+	const DebyeF D(P);
+	const float pcut = p.is_end ? D.half : 1.f;
+	int2 *queue = queues[warp];
+	PairItem<float> *item = items[warp];
+	int n = 0;  // queued items (warp-uniform)
+	// stages 2 to 4 of all queued items; the first lane of a nucleotide adds its items in order
+	auto drain = [&]() {
+		__syncwarp();
+		for(int c0 = 0; c0 < n; c0 += REF_CHUNK) {
+			const int m = min(n - c0, REF_CHUNK);
+			if(lane < m) {
+				const int2 w = queue[c0 + lane];
+				pair_radial<float, LoadRef>(P, ld, wfirst + (w.y >> 2), w.x, w.y & 3, item[lane]);
+			}
+			__syncwarp();
+			for(int m0 = 0; m0 < m; m0 += 4) {
+				const int v = min(m0 + lane / 8, m - 1);
+				pair_angles<float>(queue[c0 + v].y & 3, item[v]);
+				__syncwarp();
+			}
+			// the sums of an item by a lane, over the item's first words
+			if(lane < m) {
+				const int term = queue[c0 + lane].y & 3;
+				PairItem<float> &x = item[lane];
+				v3<float> f, t;
+				const float e = pair_sums<float>(term, x, f, t);
+				const v3<float> T = t - cross(v3<float>{x.axes[0], x.axes[1], x.axes[2]} * (term == 2 ? float(OXM_POS_STACK) : float(OXM_POS_BASE)), f);
+				const bool on = e != 0.f;
+				float *o = x.axes;
+				o[0] = on ? -f.x : 0.f, o[1] = on ? -f.y : 0.f, o[2] = on ? -f.z : 0.f;
+				o[3] = on ? T.x : 0.f, o[4] = on ? T.y : 0.f, o[5] = on ? T.z : 0.f;
+				o[6] = e;
+			}
+			__syncwarp();
+			for(int v = 0; v < m; v++) {
+				const int2 w = queue[c0 + v];
+				if((w.y >> 2) == lane / K && sub == v % K) {
+					const float *o = item[v].axes;
+					acc.F.add(v3<float>{o[0], o[1], o[2]});
+					acc.T.add(v3<float>{o[3], o[4], o[5]});
+					KahanV<float>::kadd(acc.E, acc.Ec, o[6]);
+					if((w.y & 3) == 0) KahanV<float>::kadd(acc.Eh, acc.Ehc, o[6]);
+				}
+			}
+			__syncwarp();
+		}
+		n = 0;
+	};
+	const int nn = live ? a.nnb[i] : 0;
+	if(nn > a.max_nb && sub == 0) atomicOr(a.status, OXGB_ERR_NEIGH_OVERFLOW);
+	const int nlim = min(nn, a.max_nb);
+	const long long row = (long long) i * a.nb_stride_i;
+	int longest = nlim;
+#pragma unroll
+	for(int off = 16; off >= K; off >>= 1) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, off));
+	for(int k0 = 0; k0 < longest; k0 += K) {  // warp-uniform
+		const int k = k0 + sub;
+		int j = -1, mask = 0;
+		if(k < nlim) j = a.nb[row + (long long) k * a.nb_stride_k];
+		if(j >= 0 && j != i && j != bi.x && j != bi.y) {
+			Nuc<float> q;
+			float4 qh, ql;
+			// (only Debye-Hueckel's end charges need a partner's bonds)
+			ld.load(j, P, a.bonds[j], q, qh, ql);
+			const v3<float> r = ld.sep(ph, pl, qh, ql, P).hi;
+			if(dot(r, r) < P.rcut2) {
+				const v3<float> rb = r + q.back - p.back;
+				const float rb2 = dot(rb, rb);
+				if(rb2 < D.rc2) {
+					float e;
+					dh.add(rb * D.force(rb2, pcut * (q.is_end ? D.half : 1.f), e));
+					KahanV<float>::kadd(acc.E, acc.Ec, e);
+				}
+				if(ev_contact(p, q, r)) {
+					float3 t;
+					const float4 fe = ev_pair_call(r, p.a1, p.back, q.a1, q.back, &t);
+					acc.F.add(v3<float>{fe.x, fe.y, fe.z});
+					acc.T.add(v3<float>{t.x, t.y, t.z});
+					KahanV<float>::kadd(acc.E, acc.Ec, fe.w);
+				}
+				mask = live_terms(p, q, r);
+			}
+		}
+		// the round's items, in the lanes' order
+		if(__any_sync(0xffffffffu, mask != 0)) {
+			int incl = __popc(mask);
+#pragma unroll
+			for(int off = 1; off < 32; off <<= 1) {
+				const int u = __shfl_up_sync(0xffffffffu, incl, off);
+				if(lane >= off) incl += u;
+			}
+			int at = n + incl - __popc(mask);
+			for(int left = mask; left; left &= left - 1) queue[at++] = make_int2(j, (__ffs(left) - 1) | (lane / K) << 2);
+			n += __shfl_sync(0xffffffffu, incl, 31);
+			if(n > REF_QUEUE - 3 * 32) drain();
+		}
+	}
+	drain();
+	const v3<float> fs{dh.s.x - dh.c.x, dh.s.y - dh.c.y, dh.s.z - dh.c.z};
+	acc.F.add(fs);
+	acc.T.add(cross(p.back, fs));
+	__syncthreads();
+	if(sub < 2) {
+#pragma unroll
+		for(int part = 0; part < 2; part++) {
+			const float *o = bond[part][2 * ((int) threadIdx.x / K) + sub];
+			acc.F.add(v3<float>{o[0], o[1], o[2]});
+			acc.T.add(v3<float>{o[3], o[4], o[5]});
+			KahanV<float>::kadd(acc.E, acc.Ec, o[6]);
+		}
+	}
+	const float fx = group_sum_comp<float, K>(acc.F.s.x, acc.F.c.x), fy = group_sum_comp<float, K>(acc.F.s.y, acc.F.c.y),
+			fz = group_sum_comp<float, K>(acc.F.s.z, acc.F.c.z);
+	const v3<float> tl{group_sum_comp<float, K>(acc.T.s.x, acc.T.c.x), group_sum_comp<float, K>(acc.T.s.y, acc.T.c.y),
+			group_sum_comp<float, K>(acc.T.s.z, acc.T.c.z)};
+	const float e = group_sum_comp<float, K>(acc.E, acc.Ec), eh = group_sum_comp<float, K>(acc.Eh, acc.Ehc);
+	if(sub == 0 && live) {
+		float4 fo = a.forces[i], to = a.torques[i];
+		fo.x += fx, fo.y += fy, fo.z += fz, fo.w += e;
+		// body frame: components along a1, a2, a3
+		to.x += dot(p.a1, tl), to.y += dot(p.a2, tl), to.z += dot(p.a3, tl), to.w = eh;
+		a.forces[i] = fo;
+		a.torques[i] = to;
+	}
+}
+
+cudaError_t launch_forces_reference_layout(const RefArgs &a, cudaStream_t s) {
+	// as many lanes per nucleotide as one resident wave of blocks holds (4 of 128 threads on each of 152
+	// SMs): more lanes shorten the row loops, a second wave doubles the time.  32 / 16 / 8 lanes, us per
+	// call: 1,000 nucleotides 10.3 / 12.3 / 12.3, 2,400: 12.3 / 12.3 / 14.3, 4,000: 18.5 / 14.4 / 14.4,
+	// 6,000: 26.6 / 22.1 / 16.4, 40,000: 137 / 101 / 65.
+	constexpr int wave = 152 * 4 * 128;
+	if((long long) a.N * 32 <= wave) k_forces_reference<32><<<(a.N + 3) / 4, 128, 0, s>>>(a);
+	else if((long long) a.N * 16 <= wave) k_forces_reference<16><<<(a.N + 7) / 8, 128, 0, s>>>(a);
+	else k_forces_reference<8><<<(a.N + 15) / 16, 128, 0, s>>>(a);
+	return cudaGetLastError();
 }
 
 template <typename R, class Loader, bool SPLIT, bool ENERGY, int G = 1, int K = OXGB_NB_LANES, int NBMINB = OXGB_NB_MINB,

@@ -103,7 +103,6 @@ struct ForceArgs {
 	int N;
 	const float4 *pos_hi, *pos_lo;         // FP32 mirrors (w of pos_hi: btype<<22 | index, w of pos_lo: type)
 	const float4 *fa1, *fa3;               // FP32 body axes a1, a3 (rounded once from FP64)
-	const float4 *quat;                    // reference layout only: FP32 quaternions
 	const double4_32a *posd, *quatd;          // FP64 state
 	const int2 *bonds;                    // (n3, n5), -1 if none
 	const int *nb, *nnb;                  // neighbour rows and counts
@@ -161,7 +160,19 @@ struct ForceArgs {
 // nucleotides whose owned pair-term entries are kept together (ForceArgs::own)
 constexpr int PAIR_GROUP = 32;
 
-cudaError_t launch_forces_reference_layout(const ForceArgs &a, cudaStream_t s);
+// the reference's device layout (oxgb_dna2_compute_forces): element k of row i at
+// nb[i * nb_stride_i + k * nb_stride_k]
+struct RefArgs {
+	int N, max_nb;
+	const float4 *pos, *quat;
+	const int2 *bonds;
+	const int *nb, *nnb;
+	long long nb_stride_i, nb_stride_k;
+	float4 *forces, *torques;
+	const DNA2Table<float> *table;
+	int *status;
+};
+cudaError_t launch_forces_reference_layout(const RefArgs &a, cudaStream_t s);
 // FFS order parameters of listed pairs on the reference layout (mode 0 hydrogen-bonding energy,
 // 1 nearly-bonded flag, 2 base-base distance)
 cudaError_t launch_order_params(int mode, const float4 *poss, const float4 *quat, const int *op1, const int *op2, int n,
