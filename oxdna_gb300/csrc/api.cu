@@ -427,6 +427,7 @@ struct oxgb_md {
 	bool have_topology = false, have_state = false;
 
 	double4_32a *posd = nullptr, *veld = nullptr, *Ld = nullptr, *quatd = nullptr;
+	double4_32a *frame64 = nullptr;  // FP64 engine: frames (write_frame64)
 	float4 *pos_hi = nullptr, *pos_lo = nullptr, *fa1 = nullptr, *fa3 = nullptr, *fback = nullptr, *list_pos = nullptr;
 	float4 *fa1lo = nullptr, *fbacklo = nullptr;  // remainders of fa1 / fback (FP32 engines)
 	int4 *site_back = nullptr, *site_base = nullptr;  // fixed-point sites (FP32 engines)
@@ -493,7 +494,7 @@ struct oxgb_md {
 	~oxgb_md() {
 		if(gexec) cudaGraphExecDestroy(gexec);
 		free_layout();
-		for(void *p : {(void *) posd, (void *) veld, (void *) Ld, (void *) quatd, (void *) pos_hi, (void *) pos_lo, (void *) fa1, (void *) fa3,
+		for(void *p : {(void *) posd, (void *) veld, (void *) Ld, (void *) quatd, (void *) frame64, (void *) pos_hi, (void *) pos_lo, (void *) fa1, (void *) fa3,
 					(void *) fback, (void *) fa1lo, (void *) fbacklo, (void *) site_back, (void *) site_base, (void *) list_pos, (void *) list_a1, (void *) list_back, (void *) bonds, F, T, Fe, Te, bond_f,
 					bond_tp, bond_tq, edge_acc, d_tab, (void *) d_sys, (void *) d_sys_off, (void *) d_sys_stale, (void *) d_chunk_sys,
 					(void *) d_chunk_first, (void *) d_sys_chunk0, (void *) d_sys_par, (void *) d_sys_seed, (void *) status,
@@ -558,6 +559,7 @@ static StepArgs step_args(oxgb_md *h, int step_offset = 0) {
 	a.vel = h->veld;
 	a.angmom = h->Ld;
 	a.quat = h->quatd;
+	a.frame64 = h->frame64;
 	a.pos_hi = h->pos_hi;
 	a.pos_lo = h->pos_lo;
 	a.fa1 = h->fa1;
@@ -594,6 +596,7 @@ static ForceArgs force_args(oxgb_md *h, int step_offset = 0, bool engine_step = 
 	a.fa3 = h->fa3;
 	a.posd = h->posd;
 	a.quatd = h->quatd;
+	a.frame64 = h->frame64;
 	a.bonds = h->bonds;
 	a.nb = h->lb.nb;
 	a.nnb = h->lb.nnb;
@@ -881,6 +884,7 @@ extern "C" int oxgb_md_create(int n_systems, const int *offsets, const double *b
 		ok &= cudaMalloc(&h->site_back, sizeof(int4) * N) == cudaSuccess;
 		ok &= cudaMalloc(&h->site_base, sizeof(int4) * N) == cudaSuccess;
 	}
+	else ok &= cudaMalloc(&h->frame64, 4 * sizeof(double4_32a) * N) == cudaSuccess;
 	ok &= cudaMalloc(&h->list_a1, sizeof(float4) * N) == cudaSuccess;
 	ok &= cudaMalloc(&h->list_back, sizeof(float4) * N) == cudaSuccess;
 	ok &= cudaMalloc(&h->bond_f, v4 * N) == cudaSuccess;
@@ -1083,6 +1087,7 @@ static ListArgs md_list_args(oxgb_md *h, int check_flag) {
 		a.perm = h->d_perm;
 		a.inv = h->d_inv;
 		a.st[0] = h->posd, a.st[1] = h->veld, a.st[2] = h->Ld, a.st[3] = h->quatd;
+		a.frame64 = h->frame64;
 		a.mir[0] = h->pos_hi, a.mir[1] = h->pos_lo, a.mir[2] = h->fa1, a.mir[3] = h->fa3, a.mir[4] = h->fback;
 		a.mir[5] = h->fa1lo, a.mir[6] = h->fbacklo;
 		a.mir[7] = reinterpret_cast<float4 *>(h->site_back), a.mir[8] = reinterpret_cast<float4 *>(h->site_base);
@@ -1112,6 +1117,8 @@ static int build_list_now(oxgb_md *h, int only = -1) {
 // an MD step runs (no energies), so that a state evolves the same whatever the caller asks for
 // in between; evaluations with energies (and the per-term split) go to Fe / Te.
 static int compute_forces_now(oxgb_md *h) {
+	// (the FP64 state may have been written through oxgb_md_device_buffers; the FP64 kernels read its frames)
+	if(h->dbl) CK(launch_make_mirrors(step_args(h), h->stream));
 	ForceArgs fa = force_args(h);
 	CK(launch_forces_split(fa, h->dbl, false, false, h->stream));
 	h->energies_fresh = false;
@@ -1241,6 +1248,7 @@ static int autotune_shape(oxgb_md *h) {
 }
 
 static int compute_energies_now(oxgb_md *h, bool split) {
+	if(h->dbl) CK(launch_make_mirrors(step_args(h), h->stream));  // (as in compute_forces_now)
 	ForceArgs fa = force_args(h, 0, false, true);
 	if(split) CK(cudaMemsetAsync(h->esplit, 0, sizeof(double) * 8 * h->n_systems, h->stream));
 	CK(launch_forces_split(fa, h->dbl, split, true, h->stream));

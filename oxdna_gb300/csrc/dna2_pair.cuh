@@ -131,6 +131,26 @@ OXGB_HD void make_sites(Nuc<R> &n) {
 	n.base = (sizeof(R) == 4) ? n.a1 * R(OXM_POS_BASE) : n.stack * R((double) OXM_POS_BASE / (double) OXM_POS_STACK);
 }
 
+// The FP64 engine's frame of every nucleotide, kept beside the FP32 mirrors (arrays of N, one after the
+// other: a1, a2, a3, backbone offset with the strand-end flag in w).  Nucleotide i's from its quaternion,
+// with the products and sums spelt out, so that whoever fills it gets the same bits.
+template <class V4>
+OXGB_HD void write_frame64(V4 *frame, long long N, int i, const V4 &q, bool is_end) {
+	auto f = [](double a, double b, double c) { return m_fma(a, b, c); };
+	const double d = f(q.z, q.z, -(q.w * q.w)), s = f(q.z, q.z, q.w * q.w);
+	const double u = f(q.x, q.x, -(q.y * q.y)), t = f(q.x, q.x, q.y * q.y);
+	const double xy = q.x * q.y, xz = q.x * q.z, yz = q.y * q.z;
+	V4 a1, a2, a3, b;
+	a1.x = u - d, a1.y = 2.0 * f(q.z, q.w, xy), a1.z = 2.0 * f(-q.y, q.w, xz), a1.w = 0.0;
+	a2.x = 2.0 * f(-q.z, q.w, xy), a2.y = -(u + d), a2.z = 2.0 * f(q.x, q.w, yz), a2.w = 0.0;
+	a3.x = 2.0 * f(q.y, q.w, xz), a3.y = 2.0 * f(-q.x, q.w, yz), a3.z = s - t, a3.w = 0.0;
+	b.x = f(a1.x, OXM_POS_MM_BACK1, a2.x * OXM_POS_MM_BACK2);
+	b.y = f(a1.y, OXM_POS_MM_BACK1, a2.y * OXM_POS_MM_BACK2);
+	b.z = f(a1.z, OXM_POS_MM_BACK1, a2.z * OXM_POS_MM_BACK2);
+	b.w = is_end ? 1.0 : 0.0;
+	frame[i] = a1, frame[N + i] = a2, frame[2 * N + i] = a3, frame[3 * N + i] = b;
+}
+
 // centre-centre separation of a pair as an unevaluated sum hi + lo: the FP32 path carries the
 // low part so that the stiff site-site vectors keep ~ulp accuracy; the other paths have lo = 0
 template <typename R>
@@ -795,11 +815,30 @@ template <typename R>
 OXGB_HD bool dh_sites(const DNA2Table<R> &P, const v3<R> &rback, bool p_end, bool q_end, v3<R> &f, R &e) {
 	const R rb2 = dot(rback, rback);
 	if(!(rb2 < P.dh_rc * P.dh_rc)) return false;
-	const R rmod = m_sqrt(rb2);
-	if(!(rmod < P.dh_rc)) return false;
 	R cut = R(1);
 	if(P.dh_half_charged_ends && p_end) cut *= R(0.5);
 	if(P.dh_half_charged_ends && q_end) cut *= R(0.5);
+	if constexpr(sizeof(R) == 8) {
+		// one reciprocal square root instead of a square root and three divisions, each some ten operations
+		// of the FP64 pipe, which is what bounds the FP64 kernels
+		const R v = m_rsqrt(rb2), r = rb2 * v;
+		if(!(r < P.dh_rc)) return false;
+		R s;
+		if(r < P.dh_rhigh) {
+			const R ex = P.dh_prefactor * m_exp(P.dh_minus_kappa * r) * cut * v;
+			e = ex;
+			s = ex * (P.dh_minus_kappa - v) * v;
+		}
+		else {
+			const R g = P.dh_b * (r - P.dh_rc) * cut;
+			e = g * (r - P.dh_rc);
+			s = R(2) * g * v;
+		}
+		f = rback * s;
+		return true;
+	}
+	const R rmod = m_sqrt(rb2);
+	if(!(rmod < P.dh_rc)) return false;
 	const v3<R> rd = rback * (R(1) / rmod);
 	R en, fm;
 	if(rmod < P.dh_rhigh) {
@@ -921,6 +960,42 @@ OXGB_HD bool bonded_backbone(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R
 	return ok;
 }
 
+// Stacking in its short form, from w and |w| between the unmodified backbone sites (POS_BACK along a1), and
+// direction and distance of the stacking sites: each factor's derivative acts where its argument lives,
+// theta5, theta6 and the radial part on the stacking sites, phi1 and phi2 on the sites of w.  bonded_stacking
+// writes the phi terms out in the stacking-site vector, as DNAInteraction.cpp:600-690 does: the same
+// forces in some 150 more operations.  Used in FP64, whose pipe bounds those kernels; in FP32 the two forms
+// round differently where factors cancel and the operations are not what bounds a bond.
+template <typename R>
+OXGB_HD void bonded_stacking_short(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R> &q, const v3<R> &w, R wm, const v3<R> &rd,
+		R rs, BondOut<R> &b) {
+	const R iw = R(1) / wm, ir = R(1) / rs;
+	const v3<R> wd = w * iw;
+	const R c4 = dot(p.a3, q.a3), c5 = dot(p.a3, rd), c6 = dot(q.a3, rd), cp1 = dot(p.a2, wd), cp2 = dot(q.a2, wd);
+	const v3<R> x4 = cross(p.a3, q.a3), x5 = cross(p.a3, rd), x6 = cross(q.a3, rd);
+	static_assert(sizeof(R) == 8, "f4_both takes the sine from the cosine");
+	R F, FD, g4, d4, g5, d5, g6, d6, h1, h1d, h2, h2d;
+	f1_both(P, rs, OXM_F1_ST, q.type, p.type, F, FD, R(0));
+	f4_both(c4, R(0), OXM_F4_ST_T4, g4, d4);
+	f4_both(-c5, R(0), OXM_F4_ST_T5, g5, d5);
+	f4_both(-c6, R(0), OXM_F4_ST_T5, g6, d6);
+	f5_both(cp1, OXM_F5_PHI1, h1, h1d);
+	f5_both(cp2, OXM_F5_PHI2, h2, h2d);
+	const R g = g4 * g5 * g6, h = h1 * h2, e = F * g * h;
+	b.split[2] = e;
+	if(e != R(0)) {
+		const R Fh = F * h, Fg = F * g;
+		const R e4 = Fh * d4 * g5 * g6, e5 = Fh * g4 * d5 * g6, e6 = Fh * g4 * g5 * d6;
+		const R k1 = Fg * h1d * h2, k2 = Fg * h1 * h2d;
+		// on q's stacking site, and on q's end of w
+		const v3<R> fs = (p.a3 - rd * c5) * (e5 * ir) + (q.a3 - rd * c6) * (e6 * ir) - rd * (FD * g * h);
+		const v3<R> fw = (wd * cp1 - p.a2) * (k1 * iw) + (wd * cp2 - q.a2) * (k2 * iw);
+		b.f += fs + fw;
+		b.tp += x5 * e5 - x4 * e4 - cross(p.a2, wd) * k1 - cross(p.stack, fs) - cross(p.a1, fw) * R(OXM_POS_BACK);
+		b.tq += x6 * e6 + x4 * e4 - cross(q.a2, wd) * k2 + cross(q.stack, fs) + cross(q.a1, fw) * R(OXM_POS_BACK);
+	}
+}
+
 // stacking, added to b
 template <typename R, class X = NoRefine>
 OXGB_HD void bonded_stacking(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R> &q, const Sep<R> &sep, BondOut<R> &b,
@@ -935,6 +1010,10 @@ OXGB_HD void bonded_stacking(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R
 	R rl = R(0);
 	if constexpr(X::on && sizeof(R) == 4) rl = site_dist_remainder(sep, p, xr.lo(0), q, xr.lo(1), true, rsm);
 	const v3<R> rd = rstack * (R(1) / rsm);
+	if constexpr(sizeof(R) == 8) {
+		bonded_stacking_short(P, p, q, rbackref, rbr, rd, rsm, b);
+		return;
+	}
 	const R c4 = dot(a3, b3), c5 = dot(a3, rd), c6 = -dot(b3, rd);
 	const R cp1 = dot(a2, rbackref) / rbr, cp2 = dot(b2, rbackref) / rbr;
 	R F1, F1D, g4, d4, g5, d5, g6, d6, h1, h1d, h2, h2d;

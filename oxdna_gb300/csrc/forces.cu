@@ -129,33 +129,6 @@ struct LoadMixed {
 	}
 };
 
-struct LoadDouble {
-	const double4_32a *pos, *quat;
-	const float4 *meta;  // pos_hi of the mixed layout: w carries btype; lo.w carries the type
-	const float4 *meta_lo;
-	__device__ __forceinline__ void load(int i, const DNA2Table<double> &P, const int2 b, Nuc<double> &n, double4_32a &ps,
-			double4_32a &unused) const {
-		ps = pos[i];
-		const double4_32a q = quat[i];
-		quat_frame(q.x, q.y, q.z, q.w, n.a1, n.a2, n.a3);
-		make_sites(n);
-		n.btype = __float_as_int(meta[i].w) >> 22;
-		n.type = __float_as_int(meta_lo[i].w) & 7;
-		n.is_end = (b.x < 0 || b.y < 0);
-	}
-	__device__ __forceinline__ Sep<double> sep(const double4_32a &p, const double4_32a &, const double4_32a &q, const double4_32a &,
-			const DNA2Table<double> &P) const {
-		double d[3] = {q.x - p.x, q.y - p.y, q.z - p.z};
-		const double L = P.box_hi + P.box_lo;
-#pragma unroll
-		for(int k = 0; k < 3; k++) d[k] = d[k] - rint(d[k] / L) * L;
-		return Sep<double>{v3<double>{d[0], d[1], d[2]}, v3<double>{0., 0., 0.}};
-	}
-	__device__ __forceinline__ Sep<double> diff(const double4_32a &p, const double4_32a &, const double4_32a &q, const double4_32a &) const {
-		return Sep<double>{v3<double>{q.x - p.x, q.y - p.y, q.z - p.z}, v3<double>{0., 0., 0.}};
-	}
-};
-
 struct LoadRef {
 	const float4 *pos, *quat;
 	__device__ __forceinline__ NoRefine refine(int, int) const { return NoRefine{}; }
@@ -365,26 +338,74 @@ struct SplitMixed {
 	}
 };
 
+// The FP64 engine.  Its kernels are bound by the FP64 pipe (one warp instruction in some 16 cycles), so
+// what they need in FP64 is read, not made: the frames are kept (write_frame64; made by every reader, a
+// frame was 40 of the 180 FP64 operations of a Debye-Hueckel pair), the periodic image is picked by a
+// product and a rounding addition instead of a division per axis (45 operations of a pair, now 12: the
+// same integer but for separations within an ulp of half a box, twice the range of any listed pair), and
+// pairs that a conservative test can dismiss are dismissed in FP32, on the mirrors that the list build uses.
+// 4,000 duplex nucleotides, k_bonded_pairs and k_nonbonded_split: 68.7 and 46.1 us with frames and
+// quotients per reader, 55.7 and 27.8 us so (526,000 and 497,000 FP64 warp instructions, then 380,000 and
+// 267,000).
 struct SplitDouble {
-	const double4_32a *pos, *quat;
-	const float4 *meta, *meta_lo;
-	const int2 *bonds;
+	const double4_32a *pos, *frame;
+	long long N;
+	SplitMixed screen;  // the FP32 mirrors
 	__device__ __forceinline__ NoRefine refine(int, int) const { return NoRefine{}; }
 	__device__ __forceinline__ Sep<double> sep(const double4_32a &p, const double4_32a &, const double4_32a &q,
 			const double4_32a &, const DNA2Table<double> &P) const {
-		return LoadDouble{}.sep(p, p, q, q, P);
+		double d[3] = {q.x - p.x, q.y - p.y, q.z - p.z};
+		const double L = P.box_hi + P.box_lo;
+#pragma unroll
+		for(int k = 0; k < 3; k++) {
+			constexpr double magic = 6755399441055744.0;  // 1.5 * 2^52
+			const double m = __dsub_rn(__fma_rn(d[k], P.inv_box, magic), magic);
+			d[k] = __fma_rn(-m, L, d[k]);
+		}
+		return Sep<double>{v3<double>{d[0], d[1], d[2]}, v3<double>{0., 0., 0.}};
 	}
 	__device__ __forceinline__ Sep<double> sep_soft(const double4_32a &p, const double4_32a &, const double4_32a &q,
 			const double4_32a &, const DNA2Table<double> &P) const {
-		return LoadDouble{}.sep(p, p, q, q, P);
+		return sep(p, p, q, q, P);
 	}
 	__device__ __forceinline__ Sep<double> diff(const double4_32a &p, const double4_32a &, const double4_32a &q,
 			const double4_32a &) const {
-		return LoadDouble{}.diff(p, p, q, q);
+		return Sep<double>{v3<double>{q.x - p.x, q.y - p.y, q.z - p.z}, v3<double>{0., 0., 0.}};
+	}
+	__device__ __forceinline__ void types(int j, Nuc<double> &n) const {
+		n.btype = __float_as_int(screen.hi[j].w) >> 22;
+		n.type = __float_as_int(screen.lo[j].w) & 7;
+	}
+	__device__ __forceinline__ void back(int j, Nuc<double> &n, double4_32a &h) const {
+		h = pos[j];
+		const double4_32a b = frame[3 * N + j];
+		n.back = v3<double>{b.x, b.y, b.z};
+		n.is_end = b.w != 0.0;
+	}
+	__device__ __forceinline__ void axes(int j, Nuc<double> &n, double4_32a &h) const {
+		h = pos[j];
+		const double4_32a x1 = frame[j], x3 = frame[2 * N + j];
+		n.a1 = v3<double>{x1.x, x1.y, x1.z};
+		n.a3 = v3<double>{x3.x, x3.y, x3.z};
+		n.stack = n.a1 * double(OXM_POS_STACK);
+		n.base = n.stack * ((double) OXM_POS_BASE / (double) OXM_POS_STACK);
+		types(j, n);
+	}
+	__device__ __forceinline__ void full(int j, Nuc<double> &n, double4_32a &h) const {
+		axes(j, n, h);
+		back(j, n, h);
+		const double4_32a x2 = frame[N + j];
+		n.a2 = v3<double>{x2.x, x2.y, x2.z};
+	}
+	// the box as the FP32 separation reads it
+	__device__ __forceinline__ static DNA2Table<float> screen_box(const DNA2Table<double> &P) {
+		DNA2Table<float> f;
+		const double L = P.box_hi + P.box_lo;
+		f.box_hi = (float) L, f.box_lo = (float) (L - (double) f.box_hi), f.inv_box = 1.f / f.box_hi;
+		return f;
 	}
 };
 
-// FP64 loads need the table (for the base-site ratio), so the double loader takes it explicitly
 template <class Loader, typename R>
 __device__ __forceinline__ void load_full(const Loader &ld, int j, const DNA2Table<R> &P, Nuc<R> &n,
 		typename Vec4Of<R>::T &h, typename Vec4Of<R>::T &l);
@@ -394,25 +415,31 @@ __device__ __forceinline__ void load_full<SplitMixed, float>(const SplitMixed &l
 	ld.full(j, n, h, l);
 }
 template <>
-__device__ __forceinline__ void load_full<SplitDouble, double>(const SplitDouble &ld, int j, const DNA2Table<double> &P,
-		Nuc<double> &n, double4_32a &h, double4_32a &l) {
-	LoadDouble{ld.pos, ld.quat, ld.meta, ld.meta_lo}.load(j, P, ld.bonds[j], n, h, l);
+__device__ __forceinline__ void load_full<SplitDouble, double>(const SplitDouble &ld, int j, const DNA2Table<double> &,
+		Nuc<double> &n, double4_32a &h, double4_32a &) {
+	ld.full(j, n, h);
 }
 template <class Loader, typename R>
 __device__ __forceinline__ void load_dh(const Loader &ld, int j, const DNA2Table<R> &P, Nuc<R> &n, typename Vec4Of<R>::T &h,
-		typename Vec4Of<R>::T &l) {
-	load_full<Loader, R>(ld, j, P, n, h, l);
-}
+		typename Vec4Of<R>::T &l);
 template <>
 __device__ __forceinline__ void load_dh<SplitMixed, float>(const SplitMixed &ld, int j, const DNA2Table<float> &, Nuc<float> &n,
 		float4 &h, float4 &l) {
 	ld.dh(j, n, h, l);
 }
+template <>
+__device__ __forceinline__ void load_dh<SplitDouble, double>(const SplitDouble &ld, int j, const DNA2Table<double> &, Nuc<double> &n,
+		double4_32a &h, double4_32a &) {
+	ld.back(j, n, h);
+}
 
 template <class Loader, typename R>
 __device__ __forceinline__ void load_axes(const Loader &ld, int j, const DNA2Table<R> &P, Nuc<R> &n, typename Vec4Of<R>::T &h,
-		typename Vec4Of<R>::T &l) {
-	load_full<Loader, R>(ld, j, P, n, h, l);
+		typename Vec4Of<R>::T &l);
+template <>
+__device__ __forceinline__ void load_axes<SplitDouble, double>(const SplitDouble &ld, int j, const DNA2Table<double> &, Nuc<double> &n,
+		double4_32a &h, double4_32a &) {
+	ld.axes(j, n, h);
 }
 template <>
 __device__ __forceinline__ void load_axes<SplitMixed, float>(const SplitMixed &ld, int j, const DNA2Table<float> &, Nuc<float> &n,
@@ -600,6 +627,28 @@ __device__ __forceinline__ void angular_factor(const Angular<R> &k, R c, R sn, R
 	fd = -dsin;
 }
 
+// the same in FP64 at angle t, with the sine's square and inverse
+__device__ __forceinline__ void angular_factor_fp64(const Angular<double> &k, double t, double s2, double inv, double &f, double &fd) {
+	const double tt0 = t - k.t0, ad = fabs(tt0), far = k.tc - ad, at = s2 > 1e-8 ? inv : 1.0;
+	double dsin = 0.0;  // -df/dt / sin
+	f = 0.0;
+	if(ad < k.tc) {
+		const bool outer = ad > k.ts;
+		f = outer ? k.b * far * far : 1.0 - k.a * ad * ad;
+		// (on the axis itself |t - t0| / sin is 1 where t0 is 0 or pi)
+		const double lin = 2.0 * (outer ? k.b * far * inv : k.a * (s2 > 1e-8 ? ad : 1.0) * at);
+		dsin = copysign(lin, tt0);
+	}
+	if(k.harm != 0.0) {
+		const double h = t - (double) OXM_CXST_THETA1_SB;
+		if(h >= 0.0) {
+			f += k.harm * h * h;
+			dsin -= 2.0 * k.harm * (s2 > 1e-8 ? h : 1.0) * at;
+		}
+	}
+	fd = dsin;
+}
+
 // Which terms of pair (p, q) can be non-zero: 1 hydrogen bonding, 2 cross stacking, 4 coaxial stacking.
 // Distance windows (a little wider than the terms' own, for the plain FP32 separation) and the support
 // of every angular factor in its cosine; the terms themselves are zero outside them.
@@ -642,7 +691,7 @@ constexpr int PAIR_QUEUE = 512 + 3 * 128;  // items waiting (a round of screenin
 template <typename R>
 struct PairItem {
 	R axes[12];            // a1, a3 of p; a1, a3 of q
-	R rd[3], r, F, FD;     // site direction and distance, radial factor and its derivative
+	R rd[3], r, F, FD;     // site direction and distance (FP64: its inverse), radial factor and its derivative
 	R d[6];                // centre separation, hi and lo
 	R g[6];                // the angular factors
 	// a vector and its coefficient: the torque axes X of lanes 0 and 3, the force directions of lanes
@@ -665,7 +714,8 @@ __device__ __forceinline__ void pair_radial(const DNA2Table<R> &P, const Loader 
 	p.stack = p.a1 * R(OXM_POS_STACK), q.stack = q.a1 * R(OXM_POS_STACK);
 	const v3<R> rs = stack ? site_vec(d, q.stack, p.stack) : site_vec(d, q.base, p.base);
 	const R r = m_sqrt(dot(rs, rs));
-	const v3<R> rd = rs * (R(1) / r);
+	const R ir = R(1) / r;
+	const v3<R> rd = rs * ir;
 	R rl = R(0);
 	const auto x = ld.refine(i, j);
 	if constexpr(decltype(x)::on) rl = site_dist_remainder(d, p, x.lo(0), q, x.lo(1), stack, r);
@@ -682,7 +732,7 @@ __device__ __forceinline__ void pair_radial(const DNA2Table<R> &P, const Loader 
 #pragma unroll
 	for(int k = 0; k < 4; k++) m.axes[3 * k] = ax[k].x, m.axes[3 * k + 1] = ax[k].y, m.axes[3 * k + 2] = ax[k].z;
 	m.rd[0] = rd.x, m.rd[1] = rd.y, m.rd[2] = rd.z;
-	m.r = r, m.F = F, m.FD = FD;
+	m.r = sizeof(R) == 8 ? ir : r, m.F = F, m.FD = FD;
 	m.d[0] = d.hi.x, m.d[1] = d.hi.y, m.d[2] = d.hi.z, m.d[3] = d.lo.x, m.d[4] = d.lo.y, m.d[5] = d.lo.z;
 }
 
@@ -699,14 +749,29 @@ __device__ __forceinline__ void pair_angles(int term, PairItem<R> &m) {
 	const R *pv = v_rd ? m.rd : m.axes + (sub == 3 ? 9 : 6);
 	const v3<R> u{pu[0], pu[1], pu[2]}, v{pv[0], pv[1], pv[2]};
 	const v3<R> X = cross(u, v);
-	const R cs = s * dot(u, v), sn = m_sqrt(dot(X, X));
+	const R cs = s * dot(u, v);
 	R g, D;
-	angular_factor(c, cs, sn, g, D);
-	if(c.both != R(0)) {
-		R g2, D2;
-		angular_factor(c, -cs, sn, g2, D2);
-		g += g2;
-		D -= D2;
+	if constexpr(sizeof(R) == 8) {
+		// one reciprocal square root for the sine and its inverse, and one angle for both directions: the
+		// divisions and the second arctangent are half of a factor's operations on the FP64 pipe
+		const R s2 = dot(X, X), inv = m_rsqrt(s2), theta = m_atan2(s2 > R(0) ? s2 * inv : R(0), cs);
+		angular_factor_fp64(c, theta, s2, inv, g, D);
+		if(c.both != R(0)) {
+			R g2, D2;
+			angular_factor_fp64(c, R(3.14159265358979323846) - theta, s2, inv, g2, D2);
+			g += g2;
+			D -= D2;
+		}
+	}
+	else {
+		const R sn = m_sqrt(dot(X, X));
+		angular_factor(c, cs, sn, g, D);
+		if(c.both != R(0)) {
+			R g2, D2;
+			angular_factor(c, -cs, sn, g2, D2);
+			g += g2;
+			D -= D2;
+		}
 	}
 	// F g0 .. g5 with this lane's D in the place of its g, a product from the left
 	R z = m.F;
@@ -724,7 +789,7 @@ __device__ __forceinline__ void pair_angles(int term, PairItem<R> &m) {
 	}
 	const v3<R> w = u_q ? u + v * cs : u - v * cs;
 	R *o = m.push[sub < 3 ? sub - 1 : sub - 2];
-	o[0] = w.x, o[1] = w.y, o[2] = w.z, o[3] = (u_q ? z : -z) / m.r;
+	o[0] = w.x, o[1] = w.y, o[2] = w.z, o[3] = sizeof(R) == 8 ? (u_q ? z : -z) * m.r : (u_q ? z : -z) / m.r;
 	if(!u_q) {
 		const v3<R> y = cross(v, u);
 		R *t = m.twist[sub < 3 ? 0 : 1];
@@ -757,7 +822,14 @@ __device__ __forceinline__ R pair_sums(int term, const PairItem<R> &m, v3<R> &f,
 	return e;
 }
 
-// Pair block b (128 threads): the entries owned by G groups of 32 nucleotides, in the four stages above
+// Blocks of a group of 32 nucleotides: in FP64, where the groups of the systems it is used for do not
+// fill the chip's pipes evenly, two (about 32 items each, the least that fills a warp of stages 2 and 4).
+// With angular_factor_fp64, 4,000 duplex nucleotides: 55.7 -> 34.8 us.
+template <typename R>
+constexpr int PAIR_PARTS = sizeof(R) == 8 ? 2 : 1;
+
+// Pair block b (128 threads): the entries owned by G groups of 32 nucleotides, or its part of one group's,
+// in the four stages above
 template <typename R, class Loader, bool SPLIT, bool ENERGY, int G>
 __device__ __forceinline__ void pair_block(const ForceArgs &a, const Loader &ld, int b) {
 	using V4 = typename Vec4Of<R>::T;
@@ -766,20 +838,23 @@ __device__ __forceinline__ void pair_block(const ForceArgs &a, const Loader &ld,
 	__shared__ int wcount[4];
 	const long long N = a.N;
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	const int g0 = b * G, first = g0 * PAIR_GROUP, groups = (a.N + PAIR_GROUP - 1) / PAIR_GROUP;
+	constexpr int PARTS = PAIR_PARTS<R>;
+	static_assert(PARTS == 1 || G == 1, "parts of one group");
+	const int g0 = b / PARTS * G, first = g0 * PAIR_GROUP, groups = (a.N + PAIR_GROUP - 1) / PAIR_GROUP;
 	int start[G + 1];  // the groups' entries, one after the other
 	start[0] = 0;
 #pragma unroll
 	for(int g = 0; g < G; g++) start[g + 1] = start[g] + (g0 + g < groups ? a.own_n[g0 + g] : 0);
 	V4 *res = reinterpret_cast<V4 *>(a.pt_res);
+	const int lo = start[G] * (b % PARTS) / PARTS, hi = start[G] * (b % PARTS + 1) / PARTS;
 	int n = 0;  // queued items (block-uniform)
-	bool more = start[G] > 0;
-	for(int r0 = 0; more; r0 += 128) {
+	bool more = hi > lo;
+	for(int r0 = lo; more; r0 += 128) {
 		// stage 1
 		int mask = 0, i0 = 0;
 		int2 it = make_int2(0, 0);
 		const int r = r0 + (int) threadIdx.x;
-		if(r < start[G]) {
+		if(r < hi) {
 			int g = 0;
 #pragma unroll
 			for(int u = 1; u < G; u++) g += r >= start[u];
@@ -790,12 +865,20 @@ __device__ __forceinline__ void pair_block(const ForceArgs &a, const Loader &ld,
 			it = a.own[(long long) (g0 + g) * PAIR_GROUP * a.pt_cap + (r - base)];
 			i0 = first + g * PAIR_GROUP + (it.y >> 16);
 			it.y &= 0xffff;
-			Nuc<R> p, q;
-			V4 ph, pl, qh, ql;
 			const DNA2Table<R> &P = table_of<R>(a, a.sys ? a.sys[i0] : 0);
-			load_axes<Loader, R>(ld, i0, P, p, ph, pl);
-			load_axes<Loader, R>(ld, it.x, P, q, qh, ql);
-			mask = live_terms(p, q, ld.sep(ph, pl, qh, ql, P).plain());
+			Nuc<float> p, q;
+			float4 ph, pl, qh, ql;
+			if constexpr(sizeof(R) == 8) {
+				const DNA2Table<float> B = ld.screen_box(P);
+				ld.screen.axes(i0, p, ph, pl);
+				ld.screen.axes(it.x, q, qh, ql);
+				mask = live_terms(p, q, ld.screen.sep(ph, pl, qh, ql, B).plain());
+			}
+			else {
+				load_axes<Loader, R>(ld, i0, P, p, ph, pl);
+				load_axes<Loader, R>(ld, it.x, P, q, qh, ql);
+				mask = live_terms(p, q, ld.sep(ph, pl, qh, ql, P).plain());
+			}
 		}
 		int incl = __popc(mask);
 #pragma unroll
@@ -805,7 +888,7 @@ __device__ __forceinline__ void pair_block(const ForceArgs &a, const Loader &ld,
 		}
 		if(lane == 31) wcount[warp] = incl;
 		__syncthreads();
-		more = r0 + 128 < start[G];
+		more = r0 + 128 < hi;
 		int at = n + incl - __popc(mask);
 #pragma unroll
 		for(int w = 0; w < 4; w++) {
@@ -1144,8 +1227,16 @@ __global__ void __launch_bounds__(128, 1) k_nonbonded_split(ForceArgs a, Loader 
 		}
 		// excluded volume over centre-close pairs (use_edge: the edge blocks did it)
 		const int nev = (live && !EDGE) ? min(a.ev_n[i], a.ev_cap) : 0;
+		const DNA2Table<float> B = ld.screen_box(P);
+		Nuc<float> sp;
+		float4 sph, spl;
+		ld.screen.full(i, sp, sph, spl);
 		for(int k = sub; k < nev; k += K) {
 			const int j = a.ev_nb[(long long) k * N + i];
+			Nuc<float> sq;
+			float4 sqh, sql;
+			ld.screen.full(j, sq, sqh, sql);
+			if(!ev_contact(sp, sq, ld.screen.sep(sph, spl, sqh, sql, B).plain())) continue;
 			Nuc<R> q;
 			V4 qh, ql;
 			load_full<Loader, R>(ld, j, P, q, qh, ql);
@@ -1794,7 +1885,7 @@ static void launch_split_t(const ForceArgs &a, Loader ld, cudaStream_t s, cudaEv
 	const int blocks = a.N > 0 ? (a.N + BONDS_PER_BLOCK - 1) / BONDS_PER_BLOCK : 1;
 	// pair blocks of G groups of 32 nucleotides, then one bonded block per 64 nucleotides, then
 	// (use_edge) one edge block per 128 / K nucleotides
-	const int pair_blocks = (a.N + PAIR_GROUP * G - 1) / (PAIR_GROUP * G);
+	const int pair_blocks = (a.N + PAIR_GROUP * G - 1) / (PAIR_GROUP * G) * PAIR_PARTS<R>;
 	const int edge_blocks = EDGE ? nonbonded_blocks(a.N, K) : 0;
 	launch_after(k_bonded_pairs<R, Loader, SPLIT, ENERGY, G, EDGE, K>, dim3(pair_blocks + blocks + edge_blocks), dim3(tpb), 0, s, a, ld,
 			pair_blocks);
@@ -1830,15 +1921,19 @@ static void launch_edge(const ForceArgs &a, Loader ld, bool split, bool energy, 
 	else launch_split_t<R, Loader, false, false, G, K, MB, true>(a, ld, s, wait);
 }
 
+static SplitDouble double_loader(const ForceArgs &a) {
+	return SplitDouble{a.posd, a.frame64, a.N, SplitMixed{a.pos_hi, a.pos_lo, a.fa1, a.fa3, a.fback, nullptr, nullptr}};
+}
+
 cudaError_t launch_forces_split(const ForceArgs &a, bool dbl, bool split, bool energy, cudaStream_t s, cudaEvent_t wait) {
 	if(a.edge) {
-		if(dbl) launch_edge<double, SplitDouble>(a, SplitDouble{a.posd, a.quatd, a.pos_hi, a.pos_lo, a.bonds}, split, energy, s, wait);
+		if(dbl) launch_edge<double, SplitDouble>(a, double_loader(a), split, energy, s, wait);
 		else launch_edge<float, SplitMixed>(a, SplitMixed{a.pos_hi, a.pos_lo, a.fa1, a.fa3, a.fback, a.fa1lo, a.fbacklo}, split, energy,
 				s, wait);
 		return cudaGetLastError();
 	}
 	if(dbl) {
-		SplitDouble ld{a.posd, a.quatd, a.pos_hi, a.pos_lo, a.bonds};
+		const SplitDouble ld = double_loader(a);
 		if(split) launch_split_t<double, SplitDouble, true, true>(a, ld, s, wait);
 		else if(energy) launch_split_t<double, SplitDouble, false, true>(a, ld, s, wait);
 		else launch_split_t<double, SplitDouble, false, false>(a, ld, s, wait);

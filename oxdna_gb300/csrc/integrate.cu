@@ -62,9 +62,10 @@ __device__ __forceinline__ void mirror_sites(const StepArgs &a, int i, const Fix
 	a.site_base[i] = make_int4(c.x + fixed_round(a1.x * sb), c.y + fixed_round(a1.y * sb), c.z + fixed_round(a1.z * sb), 0);
 }
 
-// returns a1 and the backbone offset (w: the strand-end flag); with a.fa1lo also the remainders of a1 and the backbone
-// offset (exact value = mirror + remainder to ~2^-46), which the force kernels use for the stiff
+// returns a1 and the backbone offset (w: the strand-end flag) and with F64 keeps the FP64 engine's frame;
+// with a.fa1lo also the remainders of a1 and the backbone offset (exact value = mirror + remainder to ~2^-46), which the force kernels use for the stiff
 // radial factors and excluded-volume contacts
+template <bool F64>
 __device__ __forceinline__ void mirror_frame(const StepArgs &a, int i, const double4_32a &q, float3 &a1o, float4 &backo) {
 	float qh[4], ql[4], a1[3], a3[3], bk[3], a1l[3], bkl[3];
 	split_rn(q.x, qh[0], ql[0]);
@@ -82,6 +83,7 @@ __device__ __forceinline__ void mirror_frame(const StepArgs &a, int i, const dou
 	// the strand-end flag rides in w
 	const int2 bd = a.bonds[i];
 	backo = make_float4(bk[0], bk[1], bk[2], (bd.x < 0 || bd.y < 0) ? 1.f : 0.f);
+	if(F64 && a.frame64) write_frame64(a.frame64, a.N, i, q, bd.x < 0 || bd.y < 0);
 	a.fback[i] = backo;
 	a1o = make_float3(a1[0], a1[1], a1[2]);
 }
@@ -109,7 +111,7 @@ __global__ void k_make_mirrors(StepArgs a) {
 	float3 a1, hi, lo;
 	float4 bk;
 	mirror_position(a, i, a.pos[i], hi, lo);
-	mirror_frame(a, i, a.quat[i], a1, bk);
+	mirror_frame<true>(a, i, a.quat[i], a1, bk);
 	if(a.site_back) {
 		const FixedBox b = fixed_box(a, a.th.sys[i]);
 		mirror_sites(a, i, b, fixed_centre(b, hi, lo), a1, bk);
@@ -297,7 +299,7 @@ __global__ void __launch_bounds__(64, 16) k_first_step(StepArgs a) {
 			const double4_32a qd = widen4(q.x, q.y, q.z, q.w);
 			a.angmom[i] = x;
 			a.quat[i] = qd;
-			mirror_frame(a, i, qd, fa1, fbk);
+			mirror_frame<!SITES>(a, i, qd, fa1, fbk);
 		}
 		}
 	}
@@ -339,7 +341,7 @@ __global__ void __launch_bounds__(64, 16) k_first_step(StepArgs a) {
 			if(!(sizeof(V4) == sizeof(float4) && rotate_small(q.x, q.y, q.z, q.w, x.x, x.y, x.z, 0.5 * a.dt))) rotate(q, x, a.dt);
 			a.angmom[i] = x;
 			a.quat[i] = q;
-			mirror_frame(a, i, q, fa1, fbk);
+			mirror_frame<!SITES>(a, i, q, fa1, fbk);
 		}
 	}
 	// (ahead of the wait for the frame)

@@ -104,6 +104,7 @@ struct ForceArgs {
 	const float4 *pos_hi, *pos_lo;         // FP32 mirrors (w of pos_hi: btype<<22 | index, w of pos_lo: type)
 	const float4 *fa1, *fa3;               // FP32 body axes a1, a3 (rounded once from FP64)
 	const double4_32a *posd, *quatd;          // FP64 state
+	const double4_32a *frame64;               // FP64 engine: frames (write_frame64)
 	const int2 *bonds;                    // (n3, n5), -1 if none
 	const int *nb, *nnb;                  // neighbour rows and counts
 	const int *dh_nb, *dh_n;              // Debye-Hueckel rows (engine; null: the full rows)
@@ -263,6 +264,7 @@ struct ListArgs {
 	int *id, *slot;         // [N] caller's index of each slot, and its inverse
 	int *perm, *inv;        // [N] scratch: old slot of new slot k, new slot of old slot
 	double4_32a *st[4];     // FP64 state: positions, velocities, angular momenta, quaternions
+	double4_32a *frame64;   // FP64 engine: frames, made anew from the sorted quaternions (null: none)
 	float4 *mir[9];         // mirrors: pos_hi, pos_lo, fa1, fa3, fback, fa1lo, fbacklo, site_back, site_base
 	                        // (any may be null)
 	int2 *bonds_rw;         // the bonds the rows exclude (the array of `bonds`)
@@ -294,6 +296,7 @@ struct StepArgs {
 	int N;
 	double dt;
 	double4_32a *pos, *vel, *angmom, *quat;   // FP64 state
+	double4_32a *frame64;                     // FP64 engine: frames (write_frame64; null: none)
 	int f32;                               // backend_precision = float: FP32 integration, the state kept FP32-representable
 	float4 *pos_hi, *pos_lo, *fa1, *fa3;  // FP32 mirrors written by the first step
 	const void *forces, *torques;         // float4 (mixed) or double4_32a (double)

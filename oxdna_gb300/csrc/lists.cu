@@ -375,6 +375,7 @@ __device__ __forceinline__ void phase_sort_scatter(const ListArgs &a) {
 #pragma unroll
 		for(int t = 0; t < SORT_MIRRORS; t++)
 			if(a.mir[t]) a.mir[t][k] = sf[t * N + k];
+		if(a.frame64) write_frame64(a.frame64, N, k, sd[3 * N + k], sb[k].x < 0 || sb[k].y < 0);
 		a.bonds_rw[k] = sb[k];
 		const int id = si[k];
 		a.id[k] = id;

@@ -67,6 +67,11 @@ OXGB_HD v3<R> cross(v3<R> a, v3<R> b) {
 // force kernels are not compiled with fast-math), the double ones the double functions
 OXGB_HD float m_sqrt(float x) { return sqrtf(x); }
 OXGB_HD double m_sqrt(double x) { return sqrt(x); }
+#ifdef __CUDA_ARCH__
+OXGB_HD double m_rsqrt(double x) { return rsqrt(x); }
+#else
+OXGB_HD double m_rsqrt(double x) { return 1.0 / sqrt(x); }
+#endif
 OXGB_HD float m_exp(float x) { return expf(x); }
 OXGB_HD double m_exp(double x) { return exp(x); }
 OXGB_HD float m_expm1(float x) { return expm1f(x); }
