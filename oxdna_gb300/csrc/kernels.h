@@ -283,10 +283,11 @@ struct ListArgs {
 #define SORT_BYTES (4 * 32 + SORT_MIRRORS * 16 + 8 + 4 + 4)
 
 // A system's cells are filled by one block up to this many nucleotides (four of a thread's at once) and
-// cells (4096 at a time, a few microseconds each); beyond, by the grid in phases, whose four barriers take
-// about 2.5 us each
+// cells (counts in shared memory, sixteen of a thread's at once): 3 us for 24 nucleotides, 6 for 1,000, 11
+// for some thousand; beyond, by the grid in phases, 20 us for 40,000, half of it four barriers
 constexpr int LIST_LOCAL_N = 4096;
-inline bool list_local_cells(long long n, long long cells) { return n <= LIST_LOCAL_N && cells <= 16384; }
+constexpr int LIST_LOCAL_CELLS = 16384;
+inline bool list_local_cells(long long n, long long cells) { return n <= LIST_LOCAL_N && cells <= LIST_LOCAL_CELLS; }
 
 // the build, one cooperative launch: cells (counting sort, deterministic order) then neighbour rows; with
 // check_flag it returns at once while the lists are fresh

@@ -69,6 +69,8 @@ __device__ __forceinline__ bool rebuilt(const ListArgs &a, int s) { return !a.sy
 // 40,000 duplex nucleotides 75 / 47.7 -> 62 / 38; 250,000 strand nucleotides 230 / 117.5 -> 172 / 107;
 // the plain list of 120,000 (no term lists) 97.3 -> 62.6.
 constexpr int LIST_TPB = 1024;
+// shared memory of a block that fills a whole system's cells (system_cells): padded counts, nucleotides
+constexpr int LIST_LOCAL_SMEM = (LIST_LOCAL_CELLS + LIST_LOCAL_CELLS / 16 + 2 + LIST_LOCAL_N) * (int) sizeof(int);
 
 __device__ __forceinline__ bool grid_sync(ListSync *y) {
 	if(gridDim.x == 1) {
@@ -263,49 +265,69 @@ __device__ __forceinline__ void phase_rank(const ListArgs &a, bool copy) {
 	}
 }
 
-// A system's cells by one block, with block barriers only (ListArgs::local_cells): counts, segments from
-// the system's first nucleotide on, scatter and ranks.  For systems of a few thousand nucleotides this
-// saves four grid barriers of about 2.5 us, and a batch's systems go side by side.
+// A system's cells by one block, with block barriers only (ListArgs::local_cells; no cell-order storage):
+// counts, segments from the system's first nucleotide on, scatter and ranks.  For systems of a few thousand
+// nucleotides this saves four grid barriers of about 2.5 us, and a batch's systems go side by side.  The
+// counts, starts and scattered nucleotides stay in shared memory: through global memory each of the five
+// dependent passes waited for L2 (rebuilds of two or so systems of a batch of 96, cells: 18 us; so: 11).
 __device__ __forceinline__ void system_cells(const ListArgs &a, int s) {
+	extern __shared__ int local_smem[];
+	__shared__ int wt[32];
+	int *cnt = local_smem, *tmp = cnt + LIST_LOCAL_CELLS + LIST_LOCAL_CELLS / 16 + 2;
+	auto at = [](int c) { return c + (c >> 4); };  // (threads take runs of up to 16 cells: padded to miss bank conflicts)
 	const int i0 = a.sys_off ? a.sys_off[s] : 0, i1 = a.sys_off ? a.sys_off[s + 1] : a.N;
 	const CellGeo g = cell_geo(a, s);
-	const int c0 = g.cell0, c1 = c0 + g.n * g.n * g.n, t = threadIdx.x;
+	const int cells = g.n * g.n * g.n, t = threadIdx.x;
 	constexpr int Q = LIST_LOCAL_N / LIST_TPB;  // nucleotides of a thread, whose loads overlap
-	int c[Q], at[Q];
+	float4 r[Q];
+	int c[Q], rank[Q];
 #pragma unroll
 	for(int q = 0; q < Q; q++) {
 		const int i = i0 + t + q * LIST_TPB;
-		c[q] = c0;
-		if(i < i1) c[q] = cell_at(a, g, a.pos[i]);
+		if(i < i1) r[q] = a.pos[i];
 	}
+	for(int k = t; k < cells; k += LIST_TPB) cnt[at(k)] = 0;
+	__syncthreads();
 #pragma unroll
 	for(int q = 0; q < Q; q++) {
 		const int i = i0 + t + q * LIST_TPB;
-		at[q] = 0;
+		c[q] = rank[q] = 0;
 		if(i < i1) {
-			a.cell_of[i] = c[q];
-			at[q] = atomicAdd(a.cell_count + c[q], 1);
+			const int cell = cell_at(a, g, r[q]);
+			a.cell_of[i] = cell;
+			c[q] = cell - g.cell0;
+			rank[q] = atomicAdd(cnt + at(c[q]), 1);
 		}
 	}
 	__syncthreads();
-	block_scan(c0, c1, i0, [&](int c) { return __ldcg(a.cell_count + c); }, [&](int c, int start) {
-		a.cell_start[c] = start;
-		a.cell_count[c] = 0;
-	});
-	// (the next system's first cell starts there too)
-	if(t == 0) a.cell_start[c1] = i1;
+	{
+		const int w = (cells + LIST_TPB - 1) / LIST_TPB, lo = min(t * w, cells), hi = min(lo + w, cells);
+		int sum = 0;
+		for(int k = lo; k < hi; k++) sum += cnt[at(k)];
+		int run = block_incl_scan(sum, wt) - sum;
+		for(int k = lo; k < hi; k++) {
+			const int n = cnt[at(k)];
+			cnt[at(k)] = run;
+			run += n;
+		}
+		if(t == 0) cnt[at(cells)] = i1 - i0;
+	}
 	__syncthreads();
+	// (the next system's first cell starts where this one's last ends)
+	for(int k = t; k <= cells; k += LIST_TPB) a.cell_start[g.cell0 + k] = i0 + cnt[at(k)];
 #pragma unroll
 	for(int q = 0; q < Q; q++) {
 		const int i = i0 + t + q * LIST_TPB;
-		if(i < i1) a.cell_tmp[a.cell_start[c[q]] + at[q]] = i;
+		if(i < i1) tmp[cnt[at(c[q])] + rank[q]] = i;
 	}
 	__syncthreads();
 #pragma unroll
 	for(int q = 0; q < Q; q++) {
 		const int i = i0 + t + q * LIST_TPB;
 		if(i >= i1) continue;
-		const int b = a.cell_start[c[q]], p = b + rank_in_cell(a, b, a.cell_start[c[q] + 1], id_of(a, i));
+		const int b = cnt[at(c[q])], e = cnt[at(c[q] + 1)];
+		int p = i0 + b;
+		for(int k = b; k < e; k++) p += tmp[k] < i;
 		a.cell_list[p] = i;
 		sorted_copy(a, p, i);
 	}
@@ -389,6 +411,47 @@ __device__ __forceinline__ void phase_sorted_copies(const ListArgs &a) {
 		if(rebuilt(a, sys_of(a, p))) sorted_copy(a, p, a.cell_list[p]);
 }
 
+// ---------------------------------------------------------------- the nucleotides to rebuild
+
+// The nucleotides of the systems to rebuild, one system after the other, so that a build of a few systems
+// of a batch is dealt over the whole grid (going through all nucleotides and skipping the others, two
+// systems of a batch of 96 landed on 40 of 152 SMs and each group of lanes skipped a dozen nucleotides:
+// 21 us for their rows; so: 12.6).  For batches of up to a block's threads; else all nucleotides, tested.
+struct StaleSystems {
+	int n, total;
+	int first[LIST_TPB], end[LIST_TPB];
+};
+struct Stale {
+	int n, total;  // systems (0: all nucleotides), nucleotides
+	const int *first, *end;
+	// the v-th nucleotide
+	__device__ __forceinline__ int operator[](int v) const {
+		if(n == 0) return v;
+		int lo = 0, hi = n - 1;  // the first system whose end exceeds v
+		while(lo < hi) {
+			const int m = (lo + hi) / 2;
+			if(end[m] > v) hi = m;
+			else lo = m + 1;
+		}
+		return first[lo] + v - (lo > 0 ? end[lo - 1] : 0);
+	}
+};
+
+__device__ __forceinline__ Stale list_stale_systems(const ListArgs &a, StaleSystems &y) {
+	if(a.n_systems < 2 || !a.sys || !a.sys_stale || !a.sys_off || a.n_systems > LIST_TPB) return Stale{0, a.N, nullptr, nullptr};
+	__shared__ int wt[32];
+	const int s = threadIdx.x;
+	const bool on = s < a.n_systems && rebuilt(a, s);
+	const int first = on ? a.sys_off[s] : 0, size = on ? a.sys_off[s + 1] - first : 0;
+	const int k = block_incl_scan(on, wt);
+	__syncthreads();
+	const int end = block_incl_scan(size, wt);
+	if(on) y.first[k - 1] = first, y.end[k - 1] = end;
+	if(s == LIST_TPB - 1) y.n = k, y.total = end;
+	__syncthreads();
+	return Stale{y.n, y.total, y.first, y.end};
+}
+
 // ---------------------------------------------------------------- phases: rows
 
 // A listed pair can have hydrogen bonding or cross stacking before the next rebuild only if its base
@@ -450,7 +513,7 @@ __device__ __forceinline__ void put(int *rows, bool col_major, long long N, int 
 // warp reach those tests at different times and run them one after the other: 120 M warp instructions
 // for 250,000 nucleotides.)
 template <int K>
-__device__ __forceinline__ void phase_rows(const ListArgs &a) {
+__device__ __forceinline__ void phase_rows(const ListArgs &a, const Stale &stale) {
 	constexpr int G = LIST_TPB / K;
 	__shared__ int2 kept[G][2 * K + 1];  // (place in the cell-sorted order, nucleotide); odd stride
 	const int lane = threadIdx.x & 31, sub = lane % K, grp = (int) threadIdx.x / K;
@@ -458,7 +521,11 @@ __device__ __forceinline__ void phase_rows(const ListArgs &a) {
 	const unsigned below = ((1u << lane) - 1u) & gmask;
 	const bool terms = a.ev_nb != nullptr, dhl = a.dh_nb != nullptr;
 	const long long N = a.N;
-	for(int i = blockIdx.x * G + grp; i < a.N; i += gridDim.x * G) {  // group-uniform
+	// neighbouring nucleotides to the groups of a block (their rows' entries share sectors); where every
+	// group gets one at most, to different blocks
+	const int total_n = stale.total, stride = gridDim.x * G;
+	for(int v = total_n <= stride ? grp * gridDim.x + blockIdx.x : blockIdx.x * G + grp; v < total_n; v += stride) {  // group-uniform
+		const int i = stale[v];
 		const int sy = sys_of(a, i);
 		if(!rebuilt(a, sy)) continue;
 		const CellGeo g = cell_geo(a, sy);
@@ -644,6 +711,8 @@ __global__ void __launch_bounds__(LIST_TPB, 1) k_list_build(ListArgs a, int n_ce
 	pdl_trigger();  // (every block is running: the next kernel's blocks wait for this one's end)
 	pdl_wait();
 	if(a.check_flag && *(volatile const int *) a.flag == 0) return;
+	__shared__ StaleSystems stale_systems;
+	const Stale stale = list_stale_systems(a, stale_systems);
 	if(a.local_cells) {
 		for(int k = blockIdx.x; k < a.n_systems; k += gridDim.x)
 			if(rebuilt(a, k)) system_cells(a, k);
@@ -688,7 +757,7 @@ __global__ void __launch_bounds__(LIST_TPB, 1) k_list_build(ListArgs a, int n_ce
 			}
 		}
 	}
-	phase_rows<K>(a);
+	phase_rows<K>(a, stale);
 	if(a.own) {
 		if(!grid_sync(a.sync)) goto failed;
 		phase_own(a);
@@ -727,7 +796,10 @@ static cudaError_t launch_build(const ListArgs &a, int n_cells, cudaStream_t s) 
 	if(sms[dev].load() == 0) {
 		int n = 0, per = 0;
 		if((e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-		if((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_list_build<K>, LIST_TPB, 0)) != cudaSuccess) return e;
+		if((e = cudaFuncSetAttribute(k_list_build<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, LIST_LOCAL_SMEM)) != cudaSuccess)
+			return e;
+		if((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_list_build<K>, LIST_TPB, LIST_LOCAL_SMEM)) != cudaSuccess)
+			return e;
 		if(per < 1) return cudaErrorCooperativeLaunchTooLarge;
 		sms[dev].store(std::min(n, LIST_MAX_BLOCKS));
 	}
@@ -736,6 +808,7 @@ static cudaError_t launch_build(const ListArgs &a, int n_cells, cudaStream_t s) 
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = dim3(blocks > 0 ? blocks : 1);
 	cfg.blockDim = dim3(LIST_TPB);
+	cfg.dynamicSmemBytes = a.local_cells ? LIST_LOCAL_SMEM : 0;
 	cfg.stream = s;
 	cudaLaunchAttribute at[2];
 	at[0].id = cudaLaunchAttributeCooperative;

@@ -41,3 +41,27 @@ def test_partial_rebuilds_of_a_batch_match_the_systems_alone(sizes):
     # systems were rebuilt apart from each other
     assert builds < alone
     b.close()
+
+
+def test_batches_beyond_a_blocks_systems_match_the_systems_alone():
+    # more systems than a block has threads: the rows go through all nucleotides and test each
+    one = [G.system_for_config(1, seed=70 + k, scale=40 / 40000.0) for k in range(3)]
+    n = 1030
+    kw = dict(dt=0.003, thermostat="john", newtonian_steps=7, pt=0.2, verlet_skin=0.03)
+    s = [one[k % 3] for k in range(n)]
+    b = MDSystem([x.box for x in s], [x.top for x in s], [dna2_settings(x.T, 0.5) for x in s], md_settings(seed=5, **kw))
+    b.set_state(*[np.concatenate(x) for x in zip(*[(x.pos, x.quats(), x.vel, x.L) for x in s])])
+    b.run(41)
+    sb, rows_b = b.get_state(), b.neighbours()
+    for k in (0, 511, 1023, 1024, 1029):
+        m = MDSystem(s[k].box, s[k].top, dna2_settings(s[k].T, 0.5), md_settings(seed=5 + k, **kw))
+        m.set_state(s[k].pos, s[k].quats(), s[k].vel, s[k].L)
+        m.run(41)
+        sm, rows = m.get_state(), m.neighbours()
+        lo, hi = b.offsets[k], b.offsets[k + 1]
+        for key in ("pos", "quat", "vel", "Lmom"):
+            assert np.array_equal(sb[key][lo:hi], sm[key]), (k, key)
+        assert np.array_equal(rows_b[0][lo:hi], rows[0]), k
+        m.close()
+    assert b.info()["rebuilds"] >= 2
+    b.close()
