@@ -449,8 +449,7 @@ struct oxgb_md {
 	long long *step = nullptr;
 	double *esplit = nullptr, *sums = nullptr, *bussi_partials = nullptr, *bussi_state = nullptr, *bussi_draws = nullptr;
 	long long *bussi_stamp = nullptr, *open_step = nullptr;
-	unsigned *bussi_done = nullptr, *bussi_prep_done = nullptr;
-	double *bussi_tot = nullptr;
+	unsigned *bussi_done = nullptr;
 	float2 *bussi_fpart = nullptr;
 	int *term_max = nullptr;
 	void *ext_rec = nullptr;              // external forces grouped by nucleotide
@@ -463,7 +462,6 @@ struct oxgb_md {
 
 	cudaStream_t stream = nullptr, noise = nullptr;
 	cudaEvent_t ev_join = nullptr, ev_first = nullptr;
-	float4 *bussi_vf = nullptr, *bussi_Lf = nullptr;  // Bussi: half-kicked v, L in FP32 (mixed)
 	double *h_stage = nullptr, *d_stage = nullptr;   // the state in the caller's layout: pinned host, device
 	int *d_bad = nullptr;                             // lowest nucleotide with a bad quaternion
 	cudaGraphExec_t gexec = nullptr;
@@ -499,7 +497,7 @@ struct oxgb_md {
 					bond_tp, bond_tq, edge_acc, d_tab, (void *) d_sys, (void *) d_sys_off, (void *) d_sys_stale, (void *) d_chunk_sys,
 					(void *) d_chunk_first, (void *) d_sys_chunk0, (void *) d_sys_par, (void *) d_sys_seed, (void *) status,
 					(void *) flag, (void *) step, (void *) esplit, (void *) sums, (void *) bussi_partials, (void *) bussi_state, (void *) bussi_draws,
-					(void *) bussi_stamp, (void *) open_step, (void *) bussi_done, (void *) bussi_prep_done, (void *) bussi_tot, (void *) bussi_fpart, (void *) term_max, ext_rec, (void *) ext_nuc, (void *) ext_off, (void *) grp_off, (void *) grp_mem, (void *) d_rebuilds})
+					(void *) bussi_stamp, (void *) open_step, (void *) bussi_done, (void *) bussi_fpart, (void *) term_max, ext_rec, (void *) ext_nuc, (void *) ext_off, (void *) grp_off, (void *) grp_mem, (void *) d_rebuilds})
 			if(p) cudaFree(p);
 		lb.free_all();
 		tl.free_all();
@@ -507,8 +505,6 @@ struct oxgb_md {
 		if(noise) cudaStreamDestroy(noise);
 		if(ev_join) cudaEventDestroy(ev_join);
 		if(ev_first) cudaEventDestroy(ev_first);
-		if(bussi_vf) cudaFree(bussi_vf);
-		if(bussi_Lf) cudaFree(bussi_Lf);
 		if(h_stage) cudaFreeHost(h_stage);
 		if(d_stage) cudaFree(d_stage);
 		if(d_bad) cudaFree(d_bad);
@@ -538,11 +534,7 @@ static ThermoArgs thermo_args(oxgb_md *h, int step_offset = 0, bool engine_step 
 	t.bussi_draws = h->bussi_draws;
 	t.bussi_stamp = h->bussi_stamp;
 	t.bussi_done = h->bussi_done;
-	t.bussi_prep_done = h->bussi_prep_done;
-	t.bussi_tot = h->bussi_tot;
 	t.bussi_fpart = h->bussi_fpart;
-	t.bussi_vf = h->bussi_vf;
-	t.bussi_Lf = h->bussi_Lf;
 	t.open_step = engine_step ? h->open_step : nullptr;
 	t.step_base = h->step;
 	t.step_offset = step_offset;
@@ -913,17 +905,11 @@ extern "C" int oxgb_md_create(int n_systems, const int *offsets, const double *b
 	ok &= cudaMalloc(&h->step, sizeof(long long)) == cudaSuccess;
 	ok &= cudaMalloc(&h->esplit, sizeof(double) * 8 * n_systems) == cudaSuccess;
 	ok &= cudaMalloc(&h->sums, sizeof(double) * 4 * h->n_chunks) == cudaSuccess;
-	ok &= cudaMalloc(&h->bussi_partials, sizeof(double) * 16 * h->n_chunks) == cudaSuccess;
-	if(md->thermostat == OXGB_THERMOSTAT_BUSSI && !h->dbl) {
-		ok &= cudaMalloc(&h->bussi_vf, sizeof(float4) * (size_t) N) == cudaSuccess;
-		ok &= cudaMalloc(&h->bussi_Lf, sizeof(float4) * (size_t) N) == cudaSuccess;
-	}
+	ok &= cudaMalloc(&h->bussi_partials, sizeof(double) * 8 * h->n_chunks) == cudaSuccess;
 	ok &= cudaMalloc(&h->bussi_state, sizeof(double) * 16 * n_systems) == cudaSuccess;
 	ok &= cudaMalloc(&h->bussi_draws, sizeof(double) * 4 * n_systems * h->md.steps_per_graph) == cudaSuccess;
 	ok &= cudaMalloc(&h->bussi_stamp, sizeof(long long)) == cudaSuccess;
 	ok &= cudaMalloc(&h->bussi_done, sizeof(unsigned) * n_systems) == cudaSuccess;
-	ok &= cudaMalloc(&h->bussi_prep_done, sizeof(unsigned) * n_systems) == cudaSuccess;
-	ok &= cudaMalloc(&h->bussi_tot, sizeof(double) * 8 * n_systems) == cudaSuccess;
 	ok &= cudaMalloc(&h->bussi_fpart, sizeof(float2) * 8 * h->n_chunks) == cudaSuccess;
 	ok &= cudaMallocHost(&h->h_stage, sizeof(double) * 13 * (size_t) N) == cudaSuccess;
 	ok &= cudaMalloc(&h->d_stage, sizeof(double) * 13 * (size_t) N) == cudaSuccess;
@@ -950,7 +936,6 @@ extern "C" int oxgb_md_create(int n_systems, const int *offsets, const double *b
 	ok &= cudaMemcpy(h->d_sys_seed, seeds.data(), sizeof(unsigned long long) * n_systems, cudaMemcpyHostToDevice) == cudaSuccess;
 	ok &= cudaMemset(h->d_sys_stale, 0, sizeof(int) * n_systems) == cudaSuccess;
 	ok &= cudaMemset(h->bussi_done, 0, sizeof(unsigned) * n_systems) == cudaSuccess;
-	ok &= cudaMemset(h->bussi_prep_done, 0, sizeof(unsigned) * n_systems) == cudaSuccess;
 	ok &= cudaMemset(h->status, 0, sizeof(int)) == cudaSuccess;
 	ok &= cudaMemset(h->flag, 0, sizeof(int)) == cudaSuccess;
 	ok &= cudaMemset(h->step, 0, sizeof(long long)) == cudaSuccess;
@@ -1444,25 +1429,23 @@ extern "C" int oxgb_md_get_state(oxgb_md *h, double *pos, double *quat, double *
 	return OXGB_OK;
 }
 
-// A Bussi step's side branch, from the list build on and beside the force kernels: the FP64 sums of the
-// half-kicked state, and at the first of `steps` steps captured together the draws of all of them (they
-// depend only on the seed and the step).  It starts after the list build because a cooperative kernel
+// Bussi: at the first of `steps` steps captured together, from its list build on and beside its force
+// kernels, the draws of all of them (they depend only on the seed and the step).  The branch starts after the list build because a cooperative kernel
 // waits until the chip holds no other: beside the first step, the draws kept the build of a 96-system
 // batch waiting for 33 us in every step.
 static cudaError_t bussi_side_branch(oxgb_md *h, const StepArgs &sa, int steps) {
-	if(sa.th.thermostat != OXGB_THERMOSTAT_BUSSI) return cudaSuccess;
+	if(sa.th.thermostat != OXGB_THERMOSTAT_BUSSI || sa.th.step_offset != 0) return cudaSuccess;
 	cudaError_t e = cudaEventRecord(h->ev_first, h->stream);
 	if(e == cudaSuccess) e = cudaStreamWaitEvent(h->noise, h->ev_first, 0);
-	if(e == cudaSuccess && sa.th.step_offset == 0) e = launch_bussi_noise(sa, steps, h->noise);
-	if(e == cudaSuccess) e = launch_bussi_prep(sa, h->n_chunks, h->dbl, h->noise);
+	if(e == cudaSuccess) e = launch_bussi_noise(sa, steps, h->noise);
 	if(e == cudaSuccess) e = cudaEventRecord(h->ev_join, h->noise);
 	return e;
 }
 
-// after the forces of a Bussi step: join the side branch, then the force sums and the update
+// after the forces of a Bussi step: join the side branch, then the kinetic sums and the update
 static cudaError_t bussi_after_forces(oxgb_md *h, const StepArgs &sa) {
 	if(sa.th.thermostat != OXGB_THERMOSTAT_BUSSI) return cudaSuccess;
-	cudaError_t e = cudaStreamWaitEvent(h->stream, h->ev_join, 0);
+	cudaError_t e = sa.th.step_offset == 0 ? cudaStreamWaitEvent(h->stream, h->ev_join, 0) : cudaSuccess;
 	if(e == cudaSuccess) e = launch_bussi_reduce(sa, h->n_chunks, h->dbl, h->stream);
 	return e;
 }

@@ -11,9 +11,9 @@
 // update runs on the device (its gamma deviate uses the same algorithm as the reference).
 // The second half kick of a step and its thermostat are deferred to the next first step (or
 // to the flush at the end of a run), where they run one thread per nucleotide next to the
-// first half kick; the Bussi sums run beside (k_bussi_prep) and after (k_bussi_sums, with the update) the forces, and its
-// draws on a parallel branch of the step graph (k_bussi_noise).  No FP64 work is left in the force
-// kernels, whose lanes are mostly idle at the epilogue.
+// first half kick; the Bussi sums run after the forces (k_bussi_sums, with the update), and its draws, those of
+// all steps of a graph at once, on a parallel branch of the step graph (k_bussi_noise).  No FP64 work is
+// left in the mixed engine's force kernels, whose lanes are mostly idle at the epilogue.
 #include "split.cuh"
 #include "thermo.cuh"
 
@@ -391,9 +391,7 @@ __global__ void k_bussi_noise(StepArgs a) {
 // The update of step s needs, per system, the sums of v, |v|^2 and |L|^2 over the completed
 // momenta v + h F and L + h T (h = dt / 2).  They are split as
 //   sum (v + h F)^2 = sum v^2 + 2 h sum v.F + h^2 sum F^2   (and likewise for L, T):
-// the FP64 sums of the half-kicked state (k_bussi_prep) depend only on the first step and run on
-// a side branch of the step graph while the force kernels run (they use the FP64 pipe, which
-// the FP32 force kernels leave idle); the force terms (k_bussi_sums) are FP32 products of the
+// the FP64 sums of the half-kicked state depend only on the first step; the force terms are FP32 products of the
 // FP32 forces with the FP32-rounded momenta, summed with compensation, a correction of relative
 // size h |F| / |v| to sums that stay FP64.  Both sums run over the same chunks (up to 256
 // nucleotides of one system, aligned to the system's first nucleotide), so a system reduces the
@@ -430,12 +428,15 @@ __device__ __forceinline__ T warp_transpose_sum8(const T (&x)[8], Add add) {
 	return add(t, shfl_xor(t, 1));
 }
 
-// the 8 per-thread values of a block summed in a fixed order into red[0..7] (a 256-thread block)
-__device__ __forceinline__ void block_sum8(const double (&x)[8], double *red) {
+// the 8 per-thread values of a block's first nw warps summed in a fixed order into red[0..7] (a 256-thread
+// block)
+__device__ __forceinline__ void block_sum8(const double (&x)[8], double *red, int nw = 8) {
 	__shared__ double part[8][8];
-	const double t = warp_transpose_sum8(x, [](double p, double q) { return p + q; });
-	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-	if((lane & 3) == 0) part[lane >> 2][w] = t;
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+	if(w < nw) {
+		const double t = warp_transpose_sum8(x, [](double p, double q) { return p + q; });
+		if((lane & 3) == 0) part[lane >> 2][w] = t;
+	}
 	__syncthreads();
 	if(threadIdx.x < 8) {
 		double r = 0;
@@ -462,115 +463,86 @@ __device__ __forceinline__ void block_sum8f(const CompF (&x)[8], float2 *out) {
 	if(threadIdx.x < 8) out[threadIdx.x] = make_float2(r.s, r.e);
 }
 
-// the same into doubles (threads 0..7)
-__device__ __forceinline__ void block_sum8(const CompF (&x)[8], double *red) {
-	const CompF r = block_sum8_comp(x);
-	if(threadIdx.x < 8) red[threadIdx.x] = widen(r.s) + widen(r.e);
-}
-
-// Bussi step s, after the first step: per chunk, the FP64 sums of the half-kicked v, |v|^2 and
-// |L|^2 (and, in mixed precision, v and L rounded to FP32 for the force terms)
-template <typename V4>
-__global__ void __launch_bounds__(256) k_bussi_prep(StepArgs a) {
-	const long long s = step_of(a.th);
-	if(s % a.th.newtonian_steps != 0) return;
-	const int c = blockIdx.x;
-	const int sy = a.th.chunk_sys[c];
-	const int i = a.th.chunk_first[c] + threadIdx.x;
-	double x[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-	if(i < a.th.sys_off[sy + 1]) {
-		const double4_32a v = a.vel[i], L = a.angmom[i];
-		x[0] = v.x;
-		x[1] = v.y;
-		x[2] = v.z;
-		x[3] = v.x * v.x + v.y * v.y + v.z * v.z;
-		x[4] = L.x * L.x + L.y * L.y + L.z * L.z;
-		if(sizeof(V4) == sizeof(float4)) {
-			a.th.bussi_vf[i] = make_float4(narrow(v.x), narrow(v.y), narrow(v.z), 0.f);
-			a.th.bussi_Lf[i] = make_float4(narrow(L.x), narrow(L.y), narrow(L.z), 0.f);
-		}
-	}
-	block_sum8(x, a.th.bussi_partials + 16 * c);
-	// the block that brings a system's last chunk sums them (fixed order) into the system's
-	// totals, still on the side branch
-	__shared__ int last;
-	if(threadIdx.x < 8) __threadfence();
-	__syncthreads();
-	if(threadIdx.x == 0) {
-		const unsigned nc = (unsigned) (a.th.sys_chunk0[sy + 1] - a.th.sys_chunk0[sy]);
-		last = atomicAdd(a.th.bussi_prep_done + sy, 1u) == nc - 1u;
-		if(last) a.th.bussi_prep_done[sy] = 0u;
-	}
-	__syncthreads();
-	if(!last) return;
-	__threadfence();
+// The rescaling of system sy from its chunks' sums, reduced by the block in a fixed chunk order (the result
+// does not depend on which block runs it); translation on thread 0 and rotation on thread 32 (two warps: the
+// chains overlap).  Every step waits for this, so it is one load of the chunks and one reduction, of the five
+// completed sums, over the warps that have chunks.
+__device__ __forceinline__ void bussi_system_update(const StepArgs &a, int sy) {
+	__shared__ double kin[8];
 	const int c0 = a.th.sys_chunk0[sy], nc = a.th.sys_chunk0[sy + 1] - c0;
-	double y[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-	for(int b = threadIdx.x; b < nc; b += blockDim.x) {
-		const double *p = a.th.bussi_partials + 16 * (c0 + b);
-#pragma unroll
-		for(int k = 0; k < 5; k++) y[k] += __ldcg(p + k);
+	const int which = threadIdx.x >> 5;
+	double root = 0.0, inv_n = 0.0, n = 0.0;
+	if(threadIdx.x == 0 || threadIdx.x == 32) {
+		root = __ldcg(a.th.bussi_state + 16 * sy + 8 + which);
+		inv_n = a.th.sys_par[sy * SP_STRIDE + SP_INVN];
+		n = (double) (a.th.sys_off[sy + 1] - a.th.sys_off[sy]);
 	}
-	__syncthreads();  // the block's scratch is reused
-	block_sum8(y, a.th.bussi_tot + 8 * sy);
-}
-
-// the update of system sy: the totals of the half-kicked state (k_bussi_prep) and the force
-// terms of its chunks, reduced by the block in a fixed chunk order as compensated float pairs
-// (the result does not depend on which block runs it); translation on thread 0 and rotation on
-// thread 32 (two warps: the chains overlap)
-__device__ __forceinline__ void bussi_system_update(const StepArgs &a, int sy, long long s) {
-	__shared__ double tot[8];
-	const int c0 = a.th.sys_chunk0[sy], nc = a.th.sys_chunk0[sy + 1] - c0;
-	CompF y[8];
-#pragma unroll
-	for(int k = 0; k < 8; k++) y[k] = CompF{0.f, 0.f};
-	for(int b = threadIdx.x; b < nc; b += blockDim.x) {
-		const float2 *p = a.th.bussi_fpart + 8 * (c0 + b);
-#pragma unroll
-		for(int k = 0; k < 7; k++) {
-			const float2 v = __ldcg(p + k);
-			y[k] = comp_add(y[k], CompF{v.x, v.y});
-		}
-	}
-	__syncthreads();  // the block's scratch is reused
-	block_sum8(y, tot);
-	__syncthreads();
-	if(threadIdx.x != 0 && threadIdx.x != 32) return;
-	const double *x = a.th.bussi_tot + 8 * sy;
 	const double h = 0.5 * a.dt;
-	const double sum[5] = {__ldcg(x) + h * tot[0], __ldcg(x + 1) + h * tot[1], __ldcg(x + 2) + h * tot[2],
-			__ldcg(x + 3) + 2.0 * h * tot[3] + h * h * tot[4], __ldcg(x + 4) + 2.0 * h * tot[5] + h * h * tot[6]};
-	bussi_update(a.th, sy, s, threadIdx.x == 0 ? 0 : 1, sum);
+	double x[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+	for(int b = threadIdx.x; b < nc; b += blockDim.x) {
+		const double *q = a.th.bussi_partials + 8 * (c0 + b);
+		const float2 *p = a.th.bussi_fpart + 8 * (c0 + b);
+		double k[5], f[7];
+#pragma unroll
+		for(int u = 0; u < 5; u++) k[u] = __ldcg(q + u);
+#pragma unroll
+		for(int u = 0; u < 7; u++) {
+			const float2 v = __ldcg(p + u);
+			f[u] = widen(v.x) + widen(v.y);
+		}
+#pragma unroll
+		for(int u = 0; u < 3; u++) x[u] += k[u] + h * f[u];
+		x[3] += k[3] + 2.0 * h * f[3] + h * h * f[4];
+		x[4] += k[4] + 2.0 * h * f[5] + h * h * f[6];
+	}
+	__syncthreads();  // the block's scratch is reused
+	block_sum8(x, kin, min((nc + 31) >> 5, 8));
+	__syncthreads();
+	if(threadIdx.x == 0 || threadIdx.x == 32) bussi_factor(a.th, sy, which, kin, root, inv_n, n);
 }
 
-// Bussi step s, after its forces: per chunk the sums of F, v.F, |F|^2, L.T and |T|^2 (FP32
-// products, compensated sums; FP64 in double precision).  The block that brings a system's last
-// chunk (a per-system arrival counter) makes that system's update, so there is no separate
-// update launch.
+// Bussi step s, after its forces.  Before it waits for them: per chunk, the FP64 sums of the half-kicked
+// v, |v|^2 and |L|^2 and the system's new kinetic energies, beside the tail of the force kernels.  Then the sums of F, v.F, |F|^2, L.T and |T|^2
+// (FP32 products with the FP32-rounded momenta, compensated sums; FP64 in double precision).  The block that
+// brings a system's last chunk (a per-system arrival counter) makes that system's update, so there is no
+// separate update launch.
+//
+// What bounds it is the chain from the forces to the rescaling: 40,000 nucleotides, 1 us for the chunks'
+// sums, 0.8 for the arrivals, 4.1 for the last block's (5.2 with the kinetic energies' update and a reduction of
+// force terms apart from it; the arithmetic is a chain of FP64 operations).  The FP64 sums were a kernel on a
+// side branch of the step graph, joined before this one in every step: 57.2 us per step, 56.1 so; a batch of
+// 96 systems 108.7 and 107.1.
 template <typename V4>
 __global__ void __launch_bounds__(256) k_bussi_sums(StepArgs a) {
-	pdl_wait();  // launched after the force kernels
-	pdl_trigger();
 	const long long s = step_of(a.th);
-	if(s % a.th.newtonian_steps != 0) return;
+	const bool due = s % a.th.newtonian_steps == 0;
 	const int c = blockIdx.x;
 	const int sy = a.th.chunk_sys[c];
 	const int i = a.th.chunk_first[c] + threadIdx.x;
-	const bool live = i < a.th.sys_off[sy + 1];
+	const bool live = due && i < a.th.sys_off[sy + 1];
+	double4_32a v = make_double4_32a(0., 0., 0., 0.), L = v;
+	if(live) v = a.vel[i], L = a.angmom[i];  // (the first step's, complete before the force kernels began)
+	if(due) {
+		if(c == a.th.sys_chunk0[sy] && (threadIdx.x == 0 || threadIdx.x == 32)) bussi_advance(a.th, sy, threadIdx.x >> 5);
+		const double x[8] = {v.x, v.y, v.z, v.x * v.x + v.y * v.y + v.z * v.z, L.x * L.x + L.y * L.y + L.z * L.z, 0, 0, 0};
+		block_sum8(x, a.th.bussi_partials + 8 * c);
+	}
+	pdl_wait();  // launched after the force kernels
+	pdl_trigger();
+	if(!due) return;
 	if(sizeof(V4) == sizeof(float4)) {
 		CompF x[8];
 #pragma unroll
 		for(int k = 0; k < 8; k++) x[k] = CompF{0.f, 0.f};
 		if(live) {
 			const float4 F = reinterpret_cast<const float4 *>(a.forces)[i], T = reinterpret_cast<const float4 *>(a.torques)[i];
-			const float4 v = a.th.bussi_vf[i], L = a.th.bussi_Lf[i];
+			const float3 vf = make_float3(narrow(v.x), narrow(v.y), narrow(v.z)), Lf = make_float3(narrow(L.x), narrow(L.y), narrow(L.z));
 			x[0].s = F.x;
 			x[1].s = F.y;
 			x[2].s = F.z;
-			x[3].s = v.x * F.x + v.y * F.y + v.z * F.z;
+			x[3].s = vf.x * F.x + vf.y * F.y + vf.z * F.z;
 			x[4].s = F.x * F.x + F.y * F.y + F.z * F.z;
-			x[5].s = L.x * T.x + L.y * T.y + L.z * T.z;
+			x[5].s = Lf.x * T.x + Lf.y * T.y + Lf.z * T.z;
 			x[6].s = T.x * T.x + T.y * T.y + T.z * T.z;
 		}
 		block_sum8f(x, a.th.bussi_fpart + 8 * c);
@@ -580,7 +552,6 @@ __global__ void __launch_bounds__(256) k_bussi_sums(StepArgs a) {
 		if(live) {
 			const double4_32a F = reinterpret_cast<const double4_32a *>(a.forces)[i],
 							  T = reinterpret_cast<const double4_32a *>(a.torques)[i];
-			const double4_32a v = a.vel[i], L = a.angmom[i];
 			x[0] = F.x;
 			x[1] = F.y;
 			x[2] = F.z;
@@ -591,6 +562,7 @@ __global__ void __launch_bounds__(256) k_bussi_sums(StepArgs a) {
 		}
 		// FP64 sums, kept as float pairs like the mixed-precision ones (hi + lo carries 48 bits)
 		__shared__ double red[8];
+		__syncthreads();  // (the block's scratch is reused)
 		block_sum8(x, red);
 		__syncthreads();
 		if(threadIdx.x < 8) {
@@ -600,11 +572,14 @@ __global__ void __launch_bounds__(256) k_bussi_sums(StepArgs a) {
 		}
 	}
 	__shared__ int last;
-	if(threadIdx.x < 8) __threadfence();  // the partials are visible device-wide before this block arrives
 	__syncthreads();
 	if(threadIdx.x == 0) {
 		const unsigned nc = (unsigned) (a.th.sys_chunk0[sy + 1] - a.th.sys_chunk0[sy]);
-		last = atomicAdd(a.th.bussi_done + sy, 1u) == nc - 1u;
+		// released after and acquired before the block's barriers: the partials of every chunk that
+		// arrived are visible to the block that arrives last
+		unsigned old;
+		asm volatile("atom.add.acq_rel.gpu.u32 %0, [%1], 1;" : "=r"(old) : "l"(a.th.bussi_done + sy) : "memory");
+		last = old == nc - 1u;
 		if(last) {
 			a.th.bussi_done[sy] = 0u;  // every chunk has arrived: ready for the next step
 			// the next first step applies the rescaling of step s (every system updates at the same steps)
@@ -613,8 +588,7 @@ __global__ void __launch_bounds__(256) k_bussi_sums(StepArgs a) {
 	}
 	__syncthreads();
 	if(!last) return;
-	__threadfence();
-	bussi_system_update(a, sy, s);
+	bussi_system_update(a, sy);
 }
 
 __global__ void k_step_advance(StepArgs a, int K) {
@@ -749,12 +723,6 @@ cudaError_t launch_first_step(const StepArgs &a, bool double_forces, cudaStream_
 
 cudaError_t launch_bussi_noise(const StepArgs &a, int steps, cudaStream_t s) {
 	k_bussi_noise<<<dim3(a.th.n_systems, steps), 64, 0, s>>>(a);
-	return cudaGetLastError();
-}
-
-cudaError_t launch_bussi_prep(const StepArgs &a, int n_chunks, bool double_forces, cudaStream_t s) {
-	if(double_forces) k_bussi_prep<double4_32a><<<n_chunks, 256, 0, s>>>(a);
-	else k_bussi_prep<float4><<<n_chunks, 256, 0, s>>>(a);
 	return cudaGetLastError();
 }
 

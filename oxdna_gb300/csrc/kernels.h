@@ -78,17 +78,14 @@ struct ThermoArgs {
 	// Bussi: the kinetic sums run over chunks of up to 256 nucleotides of one system
 	const int *chunk_sys, *chunk_first;    // [chunks]
 	const int *sys_chunk0;                 // [n_systems + 1] first chunk of each system
-	double *bussi_partials;                // [chunks * 16] per-chunk sums 0-4 of the half-kicked
+	double *bussi_partials;                // [chunks * 8] per-chunk sums 0-4 of the half-kicked
 	                                       // state (v, |v|^2, |L|^2); the force terms (F, v.F,
 	                                       // |F|^2, L.T, |T|^2) go to bussi_fpart
-	float4 *bussi_vf, *bussi_Lf;           // [N] half-kicked v and L rounded to FP32 (mixed precision)
 	double *bussi_state;                   // [n_systems * 16]: K_t, K_r, factor_t, factor_r,
 	                                       // vcom x y z
 	double *bussi_draws;                   // [steps per graph][n_systems * 4] the draws of a step: sum_t,
 	                                       // rr_t, sum_r, rr_r
 	unsigned *bussi_done;                  // [n_systems] chunks arrived in this step's sums (0 between steps)
-	unsigned *bussi_prep_done;             // the same for the sums of the half-kicked state
-	double *bussi_tot;                     // [n_systems * 8] system totals of the half-kicked state
 	float2 *bussi_fpart;                   // [chunks * 8] per-chunk force-term sums as float pairs
 	long long *bussi_stamp;                // step of the last Bussi update (OXGB_NO_STEP: none)
 	long long *open_step;                  // step whose second half kick is pending
@@ -323,7 +320,6 @@ cudaError_t launch_bussi_noise(const StepArgs &a, int steps, cudaStream_t s);
 // Bussi kinetic-energy sums of the half-kicked state (after the first step, beside the forces)
 // and of the force terms with the per-system update (after the forces); n_chunks chunks of up to
 // 256 nucleotides
-cudaError_t launch_bussi_prep(const StepArgs &a, int n_chunks, bool double_forces, cudaStream_t s);
 cudaError_t launch_bussi_reduce(const StepArgs &a, int n_chunks, bool double_forces, cudaStream_t s);
 // id[k] = slot[k] = k: the caller's order (cell-order storage undone)
 cudaError_t launch_identity_order(int *id, int *slot, int N, cudaStream_t s);

@@ -206,29 +206,31 @@ static __device__ __noinline__ double4_32a brownian_redraw_warp(const ThermoArgs
 			make_double4_32a(p0.y * sT, p1.x * sT, p1.y * sT, 0.0);
 }
 
-// Bussi: from the sums of v, |v|^2 and |L|^2 over system sy, the new running kinetic energy
-// (with the draws of this step) and the rescaling factor of one kind of motion: which = 0
-// translation (about the centre-of-mass velocity), 1 rotation.  The two run on two threads.
-static __device__ void bussi_update(const ThermoArgs &t, int sy, long long s, int which, const double sum[5]) {
+// Bussi: the new running kinetic energy of one kind of motion of system sy (which = 0 translation, 1
+// rotation) from this step's draws, and its square root.  It needs no sums, so it is off the chain from the
+// forces to the rescaling.
+static __device__ void bussi_advance(const ThermoArgs &t, int sy, int which) {
 	const double *par = t.sys_par + sy * SP_STRIDE;
 	double *st = t.bussi_state + 16 * sy;
-	const double *dr = t.bussi_draws + 4 * ((size_t) t.step_offset * t.n_systems + sy);
+	const double *dr = t.bussi_draws + 4 * ((size_t) t.step_offset * t.n_systems + sy) + 2 * which;
+	update_K(st[which], par[SP_1MC], par[SP_A], par[SP_B], __ldcg(dr), __ldcg(dr + 1));
+	st[8 + which] = sqrt(st[which]);
+}
+
+// the rescaling factor of one kind of motion (translation: about the centre-of-mass velocity) from the sums
+// of v, |v|^2 and |L|^2 over system sy; root: bussi_advance's, inv_n: 1 / n
+static __device__ __forceinline__ void bussi_factor(const ThermoArgs &t, int sy, int which, const double sum[5], double root,
+		double inv_n, double n) {
+	double *st = t.bussi_state + 16 * sy;
 	if(which == 0) {
-		const double inv_n = par[SP_INVN];
-		const double n = (double) (t.sys_off[sy + 1] - t.sys_off[sy]);
 		const double vc[3] = {sum[0] * inv_n, sum[1] * inv_n, sum[2] * inv_n};
 		const double Kt_now = 0.5 * (sum[3] - n * (vc[0] * vc[0] + vc[1] * vc[1] + vc[2] * vc[2]));
-		update_K(st[0], par[SP_1MC], par[SP_A], par[SP_B], __ldcg(dr), __ldcg(dr + 1));
-		st[2] = sqrt(st[0]) * rsqrt(Kt_now);
+		st[2] = root * rsqrt(Kt_now);
 		st[4] = vc[0];
 		st[5] = vc[1];
 		st[6] = vc[2];
 	}
-	else {
-		const double Kr_now = 0.5 * sum[4];
-		update_K(st[1], par[SP_1MC], par[SP_A], par[SP_B], __ldcg(dr + 2), __ldcg(dr + 3));
-		st[3] = sqrt(st[1]) * rsqrt(Kr_now);
-	}
+	else st[3] = root * rsqrt(0.5 * sum[4]);
 }
 
 // one kind of motion of bussi_rescale (which = 0: the velocity, 1: the angular momentum)
