@@ -207,21 +207,36 @@ __device__ __forceinline__ double4_32a round4(const double4_32a &v) {
 	return widen4(narrow(v.x), narrow(v.y), narrow(v.z), narrow(v.w));
 }
 
-// First half of step s, two warps per 32 nucleotides: warp 0 of a block the translation (second
-// half kick and thermostat of step s - 1, half kick, drift, position mirror), warp 1 the
+// First half of step s, two warps per 32 nucleotides: the first the translation (second
+// half kick and thermostat of step s - 1, half kick, drift, position mirror), the second the
 // rotation (the same for the angular momentum, rotation, frame mirror).  The chains of FP64
 // operations are half as long and twice as many warps hide them; a warp never diverges on the
 // kind of motion.  What needs both, the sites and the staleness test, is done by the translation warp,
 // whose own chain is the shorter one.
 // (capped at 64 registers, 16 blocks per SM: measured in alternating runs, the 250k MD step
 // 138.7 -> 136.9 us and the 256-system batch 263.4 -> 261.3 us against the uncapped 80)
-template <typename V4, bool F32 = false>
-__global__ void __launch_bounds__(64, 16) k_first_step(StepArgs a) {
-	__shared__ float3 s_a1[32];
-	__shared__ float4 s_back[32];
-	const int lane = threadIdx.x & 31;
-	const bool rot = threadIdx.x >= 32;
-	const int i = blockIdx.x * 32 + lane;
+// Named barrier 1 + pair of W pairs of warps: arrive or, with WAIT, wait too.  The numbers are immediates: with
+// a computed one a block takes all 16 barriers, and the SM has them for half of the blocks only.
+template <int W, bool WAIT>
+__device__ __forceinline__ void pair_barrier(int pair) {
+	if constexpr(W > 1) {
+		if(pair != W - 1) {
+			pair_barrier<W - 1, WAIT>(pair);
+			return;
+		}
+	}
+	if(WAIT) asm volatile("bar.sync %0, 64;" ::"n"(W) : "memory");
+	else asm volatile("bar.arrive %0, 64;" ::"n"(W) : "memory");
+}
+
+// W: pairs of warps per block, which share their Brownian redraws (launch_first_step)
+template <typename V4, bool F32, bool BROWNIAN, int W>
+__global__ void __launch_bounds__(64 * W, 16 / W) k_first_step(StepArgs a) {
+	__shared__ float3 s_a1[W][32];
+	__shared__ float4 s_back[W][32];
+	const int lane = threadIdx.x & 31, pair = (threadIdx.x >> 5) % W;
+	const bool rot = threadIdx.x >= 32 * W;
+	const int i = (blockIdx.x * W + pair) * 32 + lane;
 	const bool live = i < a.N;
 	float3 r32 = make_float3(0.f, 0.f, 0.f), r32l = r32, fa1 = r32;
 	float4 fbk = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -248,11 +263,26 @@ __global__ void __launch_bounds__(64, 16) k_first_step(StepArgs a) {
 	// read before waiting for it, and only its outputs (the forces, the Bussi update) after.
 	// Otherwise (the first step of a graph or a single step, which may follow any kernel that
 	// writes the state) everything is read after the wait.
+	// The previous step's redraws depend on nothing but the seed, the step and the caller's index.
 	const bool early = a.th.step_offset > 0;
-	if(early) load_state();
+	bool redraw = false;
+	double4_32a fresh;
+	auto draws = [&]() {
+		__shared__ RedrawPool<W> pool;
+		const long long sp = step_of(a.th) - 1;
+		if(sp % a.th.newtonian_steps == 0)
+			redraw = brownian_redraws(a.th, pool, sy, live ? (a.th.id ? a.th.id[i] : i) - a.th.sys_off[sy] : 0, sp, rot, live, fresh);
+	};
+	if(early) {
+		load_state();
+		if(BROWNIAN) draws();
+	}
 	pdl_wait();
 	pdl_trigger();
-	if(!early) load_state();
+	if(!early) {
+		load_state();
+		if(BROWNIAN) draws();
+	}
 	if constexpr(F32) {
 		if(live) {
 		// backend_precision = float (CUDA_MD.cuh:11-60,556-578): the kicks, the drift and the
@@ -262,7 +292,6 @@ __global__ void __launch_bounds__(64, 16) k_first_step(StepArgs a) {
 		const float dt = (float) a.dt, hdt = 0.5f * dt;
 		const bool complete = *a.th.open_step == s - 1;
 		const long long sp = s - 1;
-		const bool brownian = complete && a.th.thermostat == 1 && sp % a.th.newtonian_steps == 0;
 		const bool bussi = complete && a.th.thermostat == 2 && *a.th.bussi_stamp == sp;
 		const V4 G = reinterpret_cast<const V4 *>(rot ? a.torques : a.forces)[i];
 		const float gx = (float) G.x, gy = (float) G.y, gz = (float) G.z;
@@ -271,10 +300,9 @@ __global__ void __launch_bounds__(64, 16) k_first_step(StepArgs a) {
 			u.x += gx * hdt;
 			u.y += gy * hdt;
 			u.z += gz * hdt;
-			if(brownian || bussi) {
+			if(redraw || bussi) {
 				x = widen4(u.x, u.y, u.z, 0.f);
-				if(brownian) x = brownian_redraw_warp(a.th, sy, (a.th.id ? a.th.id[i] : i) - a.th.sys_off[sy], sp, rot ? 1 : 0,
-						min(a.N - (int) blockIdx.x * 32, 32), x);
+				if(redraw) x = fresh;
 				else bussi_rescale_part(a.th, sy, rot ? 1 : 0, x);
 				u = make_float3(narrow(x.x), narrow(x.y), narrow(x.z));
 			}
@@ -310,7 +338,6 @@ __global__ void __launch_bounds__(64, 16) k_first_step(StepArgs a) {
 		// that a state is the same whether or not a run ended at that step)
 		const bool complete = *a.th.open_step == s - 1;
 		const long long sp = s - 1;
-		const bool brownian = complete && a.th.thermostat == 1 && sp % a.th.newtonian_steps == 0;
 		const bool bussi = complete && a.th.thermostat == 2 && *a.th.bussi_stamp == sp;
 		const V4 G = reinterpret_cast<const V4 *>(rot ? a.torques : a.forces)[i];
 		const double gx = widen(G.x), gy = widen(G.y), gz = widen(G.z);
@@ -318,8 +345,7 @@ __global__ void __launch_bounds__(64, 16) k_first_step(StepArgs a) {
 			x.x = fma(gx, hdt, x.x);
 			x.y = fma(gy, hdt, x.y);
 			x.z = fma(gz, hdt, x.z);
-			if(brownian) x = brownian_redraw_warp(a.th, sy, (a.th.id ? a.th.id[i] : i) - a.th.sys_off[sy], sp, rot ? 1 : 0,
-						min(a.N - (int) blockIdx.x * 32, 32), x);
+			if(redraw) x = fresh;
 			else if(bussi) bussi_rescale_part(a.th, sy, rot ? 1 : 0, x);
 		}
 		x.x = fma(gx, hdt, x.x);
@@ -346,17 +372,17 @@ __global__ void __launch_bounds__(64, 16) k_first_step(StepArgs a) {
 	}
 	// (ahead of the wait for the frame)
 	if(SITES && live && !rot) centre = fixed_centre(fb, r32, r32l);
-	// the rotation warp posts its frame and leaves (named barrier 1: arrive, no wait)
+	// the rotation warp posts its frame and leaves (named barrier 1 + pair: arrive, no wait)
 	if(rot) {
-		s_a1[lane] = fa1;
-		s_back[lane] = fbk;
-		asm volatile("bar.arrive 1, 64;" ::: "memory");
+		s_a1[pair][lane] = fa1;
+		s_back[pair][lane] = fbk;
+		pair_barrier<W, false>(pair);
 		return;
 	}
-	asm volatile("bar.sync 1, 64;" ::: "memory");
+	pair_barrier<W, true>(pair);
 	if(!live) return;
-	fa1 = s_a1[lane];
-	fbk = s_back[lane];
+	fa1 = s_a1[pair][lane];
+	fbk = s_back[pair][lane];
 	if(SITES) mirror_sites(a, i, fb, centre, fa1, fbk);
 	// Verlet list staleness (CUDA_mixed.cuh:68, extended to the interaction sites for the term
 	// lists), per system
@@ -714,11 +740,35 @@ __global__ void __launch_bounds__(256) k_system_sums(StepArgs a, double *out) {
 static inline int blocks_for(int N, int tpb) { return N > 0 ? (N + tpb - 1) / tpb : 1; }
 
 cudaError_t launch_first_step(const StepArgs &a, bool double_forces, cudaStream_t s) {
-	// two-warp blocks of 32 nucleotides: the FP64 work (1/64 of the FP32 rate) spreads evenly over
-	// the SMs
-	if(double_forces) return launch_after(k_first_step<double4_32a>, dim3(blocks_for(a.N, 32)), dim3(64), 0, s, a);
-	if(a.f32) return launch_after(k_first_step<float4, true>, dim3(blocks_for(a.N, 32)), dim3(64), 0, s, a);
-	return launch_after(k_first_step<float4>, dim3(blocks_for(a.N, 32)), dim3(64), 0, s, a);
+	const bool brownian = a.th.thermostat == 1;
+	// double and float engines: two-warp blocks of 32 nucleotides, so that the FP64 work (1/64 of the FP32
+	// rate) spreads evenly over the SMs
+	const dim3 grid(blocks_for(a.N, 32)), block(64);
+	if(double_forces)
+		return brownian ? launch_after(k_first_step<double4_32a, false, true, 1>, grid, block, 0, s, a) :
+				launch_after(k_first_step<double4_32a, false, false, 1>, grid, block, 0, s, a);
+	if(a.f32)
+		return brownian ? launch_after(k_first_step<float4, true, true, 1>, grid, block, 0, s, a) :
+				launch_after(k_first_step<float4, true, false, 1>, grid, block, 0, s, a);
+	// mixed engine: two pairs of warps per block.  One, two, four, us per step: 40,000 duplex nucleotides 53.8,
+	// 52.6, 53.4, 250,000 strand nucleotides 106.8, 104.7, 105.8, a batch of 96 systems 109.3, 108.2, 108.1,
+	// 1,000 duplex nucleotides 17.2, 17.2, 18.3.
+	const dim3 grid2(blocks_for(a.N, 64)), block2(128);
+	if(!brownian) return launch_after(k_first_step<float4, false, false, 2>, grid2, block2, 0, s, a);
+	// Where redraws come in (nearly) every step, the FP64 pipes they load want the blocks spread evenly, but
+	// blocks launched ahead pile up on the SMs that the kernel before leaves first.  If one wave holds the
+	// grid, a block asks for as much shared memory as leaves room for no more than an even share: 32,000
+	// nucleotides, a tenth redrawn in every step, 30.6 -> 26.8 us per step.  (Without redraws, 40,000 nucleotides, it
+	// costs 1.5 us: changing the split of the SM's memory between kernels is not free.)
+	const int share = (int) (grid2.x + 151) / 152;
+	size_t room = 0;
+	if(a.th.newtonian_steps <= 2 && share < 8) {
+		room = ((228 * 1024 / (share + 1) - 8192) / 128 + 1) * 128;  // (8 KB: its static memory)
+		const cudaError_t e = cudaFuncSetAttribute(k_first_step<float4, false, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+				227 * 1024 - 16384);
+		if(e != cudaSuccess) return e;
+	}
+	return launch_after(k_first_step<float4, false, true, 2>, grid2, block2, room, s, a);
 }
 
 cudaError_t launch_bussi_noise(const StepArgs &a, int steps, cudaStream_t s) {

@@ -160,50 +160,60 @@ static __device__ __noinline__ void brownian_redraw(const ThermoArgs &t, int sy,
 	}
 }
 
-// One kind of motion of brownian_redraw (which = 0: the velocity, 1: the angular momentum) for a warp
-// whose lanes 0 .. n - 1 call it, with the same draws; returns x, redrawn or not.  A redraw takes two
-// pairs of normal deviates, each a logarithm, a square root, a sine and a cosine on the slow FP64 pipe,
-// which takes as long for one lane as for all: so the pairs of the lanes that redraw (a tenth of them at
-// most, commonly a hundredth) are dealt to the warp's lanes and made in one pass, and a warp without a
-// redraw makes none.  (Each lane made its own two pairs, one of them drawn or not: a first step that
-// redraws a tenth of 32,000 nucleotides took 28 us.)
-static __device__ __noinline__ double4_32a brownian_redraw_warp(const ThermoArgs &t, int sy, int i_local, long long s, int which,
-		int n, double4_32a x) {
-	const double *par = t.sys_par + sy * SP_STRIDE;
-	const unsigned long long seed = t.sys_seed[sy];
-	const unsigned lanes = n == 32 ? 0xffffffffu : (1u << n) - 1u, lane = threadIdx.x & 31;
+// The redraws of a block of W pairs of warps, warp w < W the velocities of 32 nucleotides and warp w + W
+// their angular momenta (`rot`), with the same draws as brownian_redraw: whether this lane's is redrawn, and
+// to what (g).  A redraw takes two pairs of normal deviates, each a logarithm, a square root, a sine and a
+// cosine on the slow FP64 pipe, some 150 operations that take as long for one lane as for all: so the pairs of
+// the lanes that redraw (a tenth of them at most, commonly a hundredth) are dealt to all threads.  The whole
+// block calls, ahead of its wait for the forces.  Measured for 32,000 nucleotides of which a tenth is redrawn
+// in every step, us per step: dealt over a warp and after the wait 45.1, over one pair of warps and before it
+// 35.4, over two pairs 30.6, four 31.0.
+template <int W>
+struct RedrawPool {
+	uint2 key[128 * W];
+	double2 dev[128 * W];
+	int count[2 * W];
+};
+
+template <int W>
+static __device__ __noinline__ bool brownian_redraws(const ThermoArgs &t, RedrawPool<W> &y, int sy, int i_local, long long s, bool rot,
+		bool live, double4_32a &g) {
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	unsigned o0[4], o1[4];
-	const unsigned k0 = (unsigned) seed, k1 = (unsigned) (seed >> 32);
-	const unsigned s0 = (unsigned) s, s1 = (unsigned) ((unsigned long long) s >> 32);
-	philox(k0, k1, s0, s1, RNG_BROWNIAN, (unsigned) (2 * i_local), o0);
-	const bool redraw = which == 0 ? drawn(o0[0], par[SP_PT]) : drawn(o0[1], par[SP_PR]);
-	const unsigned who = __ballot_sync(lanes, redraw);
-	if(who == 0u) return x;
-	philox(k0, k1, s0, s1, RNG_BROWNIAN, (unsigned) (2 * i_local + 1), o1);
-	// the two pairs of a nucleotide: velocity g0 g1 | g2 -, angular momentum - g3 | g4 g5
-	const unsigned a0 = which == 0 ? o0[2] : o1[0], b0 = which == 0 ? o0[3] : o1[1];
-	const unsigned a1 = which == 0 ? o1[0] : o1[2], b1 = which == 0 ? o1[1] : o1[3];
-	const int pairs = 2 * __popc(who), mine = 2 * __popc(who & ((1u << lane) - 1u));
-	double2 p0 = make_double2(0.0, 0.0), p1 = p0;
-	for(int q0 = 0; q0 < pairs; q0 += n) {
-		const int q = q0 + (int) lane;
-		const int src = q < pairs ? (int) __fns(who, 0u, q / 2 + 1) : 0;
-		const unsigned u0 = __shfl_sync(lanes, a0, src), v0 = __shfl_sync(lanes, b0, src);
-		const unsigned u1 = __shfl_sync(lanes, a1, src), v1 = __shfl_sync(lanes, b1, src);
-		double2 g = make_double2(0.0, 0.0);
-		if(q < pairs) g = box_muller(q & 1 ? u1 : u0, q & 1 ? v1 : v0);
-#pragma unroll
-		for(int h = 0; h < 2; h++) {
-			const int at = mine + h - q0;  // the lane that made this lane's pair h
-			const bool here = redraw && at >= 0 && at < n;
-			const double gx = __shfl_sync(lanes, g.x, here ? at : 0), gy = __shfl_sync(lanes, g.y, here ? at : 0);
-			if(here) (h == 0 ? p0 : p1) = make_double2(gx, gy);
-		}
+	bool redraw = false;
+	if(live) {
+		const double *par = t.sys_par + sy * SP_STRIDE;
+		const unsigned long long seed = t.sys_seed[sy];
+		const unsigned k0 = (unsigned) seed, k1 = (unsigned) (seed >> 32);
+		const unsigned s0 = (unsigned) s, s1 = (unsigned) ((unsigned long long) s >> 32);
+		philox(k0, k1, s0, s1, RNG_BROWNIAN, (unsigned) (2 * i_local), o0);
+		redraw = rot ? drawn(o0[1], par[SP_PR]) : drawn(o0[0], par[SP_PT]);
+		if(redraw) philox(k0, k1, s0, s1, RNG_BROWNIAN, (unsigned) (2 * i_local + 1), o1);
 	}
-	if(!redraw) return x;
-	const double sT = par[SP_SQRTT];
-	return which == 0 ? make_double4_32a(p0.x * sT, p0.y * sT, p1.x * sT, 0.0) :
-			make_double4_32a(p0.y * sT, p1.x * sT, p1.y * sT, 0.0);
+	const unsigned who = __ballot_sync(0xffffffffu, redraw);
+	if(lane == 0) y.count[warp] = __popc(who);
+	__syncthreads();
+	int total = 0, at = 0;
+#pragma unroll
+	for(int w = 0; w < 2 * W; w++) {
+		if(w == warp) at = total;
+		total += y.count[w];
+	}
+	if(total == 0) return false;  // (block-uniform)
+	at = 2 * (at + __popc(who & ((1u << lane) - 1u)));
+	// the two pairs of a nucleotide: velocity g0 g1 | g2 -, angular momentum - g3 | g4 g5
+	if(redraw) {
+		y.key[at] = rot ? make_uint2(o1[0], o1[1]) : make_uint2(o0[2], o0[3]);
+		y.key[at + 1] = rot ? make_uint2(o1[2], o1[3]) : make_uint2(o1[0], o1[1]);
+	}
+	__syncthreads();
+	for(int q = threadIdx.x; q < 2 * total; q += 64 * W) y.dev[q] = box_muller(y.key[q].x, y.key[q].y);
+	__syncthreads();
+	if(!redraw) return false;
+	const double sT = t.sys_par[sy * SP_STRIDE + SP_SQRTT];
+	const double2 p0 = y.dev[at], p1 = y.dev[at + 1];
+	g = rot ? make_double4_32a(p0.y * sT, p1.x * sT, p1.y * sT, 0.0) : make_double4_32a(p0.x * sT, p0.y * sT, p1.x * sT, 0.0);
+	return true;
 }
 
 // Bussi: the new running kinetic energy of one kind of motion of system sy (which = 0 translation, 1
