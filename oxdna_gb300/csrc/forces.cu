@@ -968,10 +968,13 @@ __device__ __forceinline__ void pair_block(const ForceArgs &a, const Loader &ld,
 	}
 }
 
-// minimum resident blocks per SM asked of the register allocator for the bonded/pair kernel
-#ifndef OXGB_PAIR_MINB
-#define OXGB_PAIR_MINB 5
-#endif
+// Minimum resident blocks per SM asked of the register allocator for the bonded/pair kernel (80 registers).
+// Its warps wait for one another's stages, so residency pays until registers spill.  5, 6, 7, 8 blocks, us per
+// step at the blocks' sizes of launch_md_shape: 40,000 duplex nucleotides 40.9, 39.7, 40.5, 40.8; 160,000
+// 128, 123.3, 124.6, 128.0; 250,000 strand nucleotides 105, 101.0, 99.2, 102.4; batch of 96 systems 88, 81.7, 84.7,
+// 88.5.
+// (with the edge blocks, whose registers would spill, 5)
+constexpr int PAIR_MINB = 6;
 
 
 // compensated sum over the K lanes of a group (TwoSum at every level); every lane of the group
@@ -1085,7 +1088,7 @@ __device__ __forceinline__ void edge_block(const ForceArgs &a, const Loader &ld,
 // costliest, dispatched first), then the bonded blocks, which fill the tail, and with use_edge the
 // edge blocks.  G: groups of 32 nucleotides per pair block.
 template <typename R, class Loader, bool SPLIT, bool ENERGY, int G, bool EDGE = false, int K = 4>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? OXGB_PAIR_MINB : 1) k_bonded_pairs(ForceArgs a, Loader ld, int pair_blocks) {
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? (EDGE ? 5 : PAIR_MINB) : 1) k_bonded_pairs(ForceArgs a, Loader ld, int pair_blocks) {
 	// launched programmatically after the list build, it reads nothing before that is complete; nor may
 	// the non-bonded kernel start before (it reads the lists and mirrors at once, and waits only for
 	// these results)
@@ -1413,7 +1416,7 @@ int nonbonded_blocks(int N, int lanes) {
 }
 
 // The shapes of the MD step's force kernels (engine, mixed and float precision) the autotuner
-// chooses among: nucleotides per pair-block warp queue, lanes per nucleotide in the non-bonded
+// chooses among: the pair blocks' size (32: three groups, 16: six, see launch_md_shape), lanes per nucleotide in the non-bonded
 // kernel and the resident blocks per SM its register cap asks for.  Shape 0 is the default, the
 // best of hand sweeps on the 40k and 250k workloads.
 struct ForceShapeDef {
@@ -1901,15 +1904,19 @@ static void launch_split_t(const ForceArgs &a, Loader ld, cudaStream_t s, cudaEv
 	if(a.ext_n > 0) launch_after(k_external<typename Vec4Of<R>::T>, dim3((a.ext_n + tpb - 1) / tpb), dim3(tpb), 0, s, a);
 }
 
-#ifndef OXGB_PAIR_WIDE_N
-#define OXGB_PAIR_WIDE_N 100000
-#endif
-// the MD step's kernels (mixed / float engine) in shape k of FORCE_SHAPES
+// The MD step's kernels (mixed / float engine) in shape k of FORCE_SHAPES.  A pair block takes one group of
+// 32 nucleotides while that leaves the chip a few blocks per SM, three (shapes of 32) or six (16) where there
+// are more groups than run at a time: strands have few live pairs, and a block with a handful is all latency;
+// duplexes lose little, since three groups' items still go through the stages together.  1, 2, 3, 4, 6 groups, us
+// per step: 40,000 duplex nucleotides 39.7, 41.8, 49.5, 55.1, 69.1, 80,000: 64.8, 68.2, 65.9, 68.8, 83.0, 160,000: 126.5,
+// 125.2, 123.3, 126.8, 121.9; strands, 60,000: 32.5, 31.3, 30.0, 30.0, 30.2, 250,000: 111.0, 103.6, 101.0, 99.5, 98.2; batch
+// of 96 systems (70,000) 85.1, 86.1, 81.7, 88.9, 102.3.
+constexpr int PAIR_WIDE_N = 65000;
 template <int k>
 static void launch_md_shape(const ForceArgs &a, const SplitMixed &ld, cudaStream_t s, cudaEvent_t wait) {
 	constexpr ForceShapeDef d = FORCE_SHAPES[k];
-	if(a.N < OXGB_PAIR_WIDE_N) launch_split_t<float, SplitMixed, false, false, 1, d.lanes, d.minb>(a, ld, s, wait);
-	else launch_split_t<float, SplitMixed, false, false, d.npw / 8, d.lanes, d.minb>(a, ld, s, wait);
+	if(a.N < PAIR_WIDE_N) launch_split_t<float, SplitMixed, false, false, 1, d.lanes, d.minb>(a, ld, s, wait);
+	else launch_split_t<float, SplitMixed, false, false, d.npw == 32 ? 3 : 6, d.lanes, d.minb>(a, ld, s, wait);
 }
 
 // use_edge: the default shape with the edge blocks
