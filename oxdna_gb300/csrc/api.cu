@@ -462,6 +462,8 @@ struct oxgb_md {
 
 	cudaStream_t stream = nullptr, noise = nullptr;
 	cudaEvent_t ev_join = nullptr, ev_first = nullptr;
+	int *h_word = nullptr;       // pinned: integers read back (4 used), then h_split
+	double *h_split = nullptr;   // [8 * n_systems] energies by term
 	double *h_stage = nullptr, *d_stage = nullptr;   // the state in the caller's layout: pinned host, device
 	int *d_bad = nullptr;                             // lowest nucleotide with a bad quaternion
 	cudaGraphExec_t gexec = nullptr;
@@ -506,6 +508,7 @@ struct oxgb_md {
 		if(ev_join) cudaEventDestroy(ev_join);
 		if(ev_first) cudaEventDestroy(ev_first);
 		if(h_stage) cudaFreeHost(h_stage);
+		if(h_word) cudaFreeHost(h_word);
 		if(d_stage) cudaFree(d_stage);
 		if(d_bad) cudaFree(d_bad);
 		for(void *p : {(void *) d_id, (void *) d_slot, (void *) d_perm, (void *) d_inv, (void *) bonds0, (void *) sort_scratch})
@@ -912,6 +915,8 @@ extern "C" int oxgb_md_create(int n_systems, const int *offsets, const double *b
 	ok &= cudaMalloc(&h->bussi_done, sizeof(unsigned) * n_systems) == cudaSuccess;
 	ok &= cudaMalloc(&h->bussi_fpart, sizeof(float2) * 8 * h->n_chunks) == cudaSuccess;
 	ok &= cudaMallocHost(&h->h_stage, sizeof(double) * 13 * (size_t) N) == cudaSuccess;
+	ok &= cudaMallocHost(&h->h_word, 64 + sizeof(double) * 8 * n_systems) == cudaSuccess;
+	if(ok) h->h_split = reinterpret_cast<double *>(h->h_word + 16);
 	ok &= cudaMalloc(&h->d_stage, sizeof(double) * 13 * (size_t) N) == cudaSuccess;
 	ok &= cudaMalloc(&h->d_bad, sizeof(int)) == cudaSuccess;
 	ok &= cudaMalloc(&h->open_step, sizeof(long long)) == cudaSuccess;
@@ -1247,9 +1252,9 @@ static int ensure_energies(oxgb_md *h) {
 }
 
 static int read_status(oxgb_md *h) {
-	int st = 0;
-	CK(cudaMemcpyAsync(&st, h->status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+	CK(cudaMemcpyAsync(h->h_word, h->status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
 	CK(cudaStreamSynchronize(h->stream));
+	const int st = h->h_word[0];
 	if(st) {
 		CK(cudaMemsetAsync(h->status, 0, sizeof(int), h->stream));
 		CK(cudaStreamSynchronize(h->stream));
@@ -1265,8 +1270,8 @@ static int size_and_build_list(oxgb_md *h) {
 	if(h->md.max_neigh > 0) return read_status(h);
 	// the longest rows of any build so far (kept on the device by the list build: four integers
 	// to read rather than the counts of every nucleotide)
-	int tm[4];
-	CK(cudaMemcpyAsync(tm, h->term_max, sizeof(tm), cudaMemcpyDeviceToHost, h->stream));
+	int *tm = h->h_word;
+	CK(cudaMemcpyAsync(tm, h->term_max, 4 * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
 	CK(cudaStreamSynchronize(h->stream));
 	const int mx = tm[3];
 	int want = ((std::max(64, mx + mx / 2 + 32) + 31) / 32) * 32;
@@ -1301,6 +1306,7 @@ static int size_and_build_list(oxgb_md *h) {
 	}
 	else {
 		CK(cudaMemsetAsync(h->status, 0, sizeof(int), h->stream));
+		return OXGB_OK;
 	}
 	return read_status(h);
 }
@@ -1315,12 +1321,21 @@ struct CopyJob {
 	size_t bytes;
 };
 
+// run(k, parts) for every part of a job of `total` bytes, by a thread each when it is large
+template <class Run>
+static void parallel_parts(size_t total, const Run &run) {
+	const unsigned hw = std::thread::hardware_concurrency();
+	const int parts = (int) std::min<size_t>(std::min(8u, hw > 0 ? hw : 1u), total / (2u << 20) + 1);
+	std::vector<std::thread> pool;
+	for(int k = 1; k < parts; k++) pool.emplace_back(run, k, parts);
+	run(0, parts);
+	for(std::thread &th : pool) th.join();
+}
+
 static void staged_copy(const std::vector<CopyJob> &jobs) {
 	size_t total = 0;
 	for(const CopyJob &j : jobs) total += j.bytes;
-	const unsigned hw = std::thread::hardware_concurrency();
-	const int T = (int) std::min<size_t>(std::min(8u, hw > 0 ? hw : 1u), total / (2u << 20) + 1);
-	auto run = [&](int t) {
+	parallel_parts(total, [&](int t, int T) {
 		// thread t copies bytes [t total / T, (t + 1) total / T) of the concatenated jobs
 		const size_t lo = total * t / T, hi = total * (t + 1) / T;
 		size_t base = 0;
@@ -1329,15 +1344,7 @@ static void staged_copy(const std::vector<CopyJob> &jobs) {
 			if(a < b) std::memcpy((char *) j.dst + (a - base), (const char *) j.src + (a - base), b - a);
 			base += j.bytes;
 		}
-	};
-	if(T <= 1) {
-		run(0);
-		return;
-	}
-	std::vector<std::thread> pool;
-	for(int t = 1; t < T; t++) pool.emplace_back(run, t);
-	run(0);
-	for(std::thread &th : pool) th.join();
+	});
 }
 
 extern "C" int oxgb_md_set_state(oxgb_md *h, const double *pos, const double *quat, const double *vel, const double *L) {
@@ -1348,22 +1355,20 @@ extern "C" int oxgb_md_set_state(oxgb_md *h, const double *pos, const double *qu
 	double *st = h->h_stage;
 	staged_copy({{st, pos, sizeof(double) * 3 * N}, {st + 3 * N, quat, sizeof(double) * 4 * N},
 			{st + 7 * N, vel, sizeof(double) * 3 * N}, {st + 10 * N, L, sizeof(double) * 3 * N}});
-	const int none = INT_MAX;
-	CK(cudaMemcpyAsync(h->d_bad, &none, sizeof(int), cudaMemcpyHostToDevice, h->stream));
+	CK(cudaMemsetAsync(h->d_bad, 0x7f, sizeof(int), h->stream));  // above any nucleotide
 	CK(cudaMemcpyAsync(h->d_stage, st, sizeof(double) * 13 * N, cudaMemcpyHostToDevice, h->stream));
 	StepArgs sa = step_args(h);
 	// checked before anything is written, so that a rejected state leaves the current one
 	CK(launch_unpack_state(sa, h->d_stage, h->d_bad, true, h->stream));
-	int bad = INT_MAX;
-	CK(cudaMemcpyAsync(&bad, h->d_bad, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+	CK(cudaMemcpyAsync(h->h_word, h->d_bad, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
 	CK(cudaStreamSynchronize(h->stream));
-	if(bad != INT_MAX) return fail(OXGB_E_INVALID, "quaternion of nucleotide " + std::to_string(bad) + " is not normalisable");
+	const int bad = h->h_word[0];
+	if(bad < h->N) return fail(OXGB_E_INVALID, "quaternion of nucleotide " + std::to_string(bad) + " is not normalisable");
 	if(h->sorting()) {
 		const int rc0 = caller_order(h);
 		if(rc0) return rc0;
 	}
-	CK(launch_unpack_state(sa, h->d_stage, h->d_bad, false, h->stream));
-	if(clear_pending(h)) return fail(OXGB_E_CUDA, "upload");  // a new state: nothing pending
+	CK(launch_unpack_state(sa, h->d_stage, h->d_bad, false, h->stream));  // a new state: nothing pending
 	CK(launch_make_mirrors(sa, h->stream));
 	int rc = size_and_build_list(h);
 	if(rc) return rc;
@@ -1527,7 +1532,8 @@ extern "C" int oxgb_md_run(oxgb_md *h, int nsteps, int sync) {
 	return OXGB_OK;
 }
 
-static int download_forces(oxgb_md *h, const void *dF, const void *dT, double *F, double *T, double *E);
+static int download_forces(oxgb_md *h, const void *dF, const void *dT, double *F, double *T, double *E, double *Es = nullptr,
+		bool check = false);
 
 extern "C" int oxgb_md_compute_forces(oxgb_md *h, double *F, double *T, double *E, double *E_split) {
 	if(!h || !h->have_state) return fail(OXGB_E_INVALID, "no state");
@@ -1537,12 +1543,7 @@ extern "C" int oxgb_md_compute_forces(oxgb_md *h, double *F, double *T, double *
 	if(rc) return rc;
 	rc = compute_energies_now(h, true);
 	if(rc) return rc;
-	rc = read_status(h);
-	if(rc) return rc;
-	rc = download_forces(h, h->Fe, h->Te, F, T, E);
-	if(rc) return rc;
-	if(E_split) CK(cudaMemcpy(E_split, h->esplit, sizeof(double) * 8 * h->n_systems, cudaMemcpyDeviceToHost));
-	return OXGB_OK;
+	return download_forces(h, h->Fe, h->Te, F, T, E, E_split, true);
 }
 
 extern "C" int oxgb_md_get_forces(oxgb_md *h, double *F, double *T, double *E) {
@@ -1551,13 +1552,11 @@ extern "C" int oxgb_md_get_forces(oxgb_md *h, double *F, double *T, double *E) {
 		int rc = ensure_energies(h);
 		if(rc) return rc;
 	}
-	CK(cudaStreamSynchronize(h->stream));
 	int rc = download_forces(h, h->F, h->T, F, T, nullptr);
 	if(rc == OXGB_OK && E) rc = download_forces(h, h->Fe, h->Te, nullptr, nullptr, E);
 	return rc;
 }
 
-// F, T from the device buffers dF, dT and E from the w of dF (any output may be NULL)
 // the caller's index of every slot (the identity unless the engine stores in cell order)
 static int storage_order(oxgb_md *h, std::vector<int> &id) {
 	id.resize(h->N);
@@ -1570,29 +1569,45 @@ static int storage_order(oxgb_md *h, std::vector<int> &id) {
 	return OXGB_OK;
 }
 
-static int download_forces(oxgb_md *h, const void *dF, const void *dT, double *F, double *T, double *E) {
+// nucleotides lo .. hi - 1 of downloaded forces f (w: energy) and torques t into the caller's arrays
+template <class V4>
+static void put_forces(const V4 *f, const V4 *t, const int *id, int lo, int hi, double *F, double *T, double *E) {
+	for(int i = lo; i < hi; i++) {
+		const size_t o = id ? (size_t) id[i] : (size_t) i;
+		if(F) F[3 * o] = f[i].x, F[3 * o + 1] = f[i].y, F[3 * o + 2] = f[i].z;
+		if(T) T[3 * o] = t[i].x, T[3 * o + 1] = t[i].y, T[3 * o + 2] = t[i].z;
+		if(E) E[o] = f[i].w;
+	}
+}
+
+// F, T from the device buffers dF, dT, E from the w of dF and Es, the energies by term (any output may be
+// NULL), with the status: everything into pinned memory and one wait, then the caller's layout, by several
+// threads when large
+static int download_forces(oxgb_md *h, const void *dF, const void *dT, double *F, double *T, double *E, double *Es,
+		bool check) {
 	const int N = h->N;
 	std::vector<int> id;
-	const int rc = storage_order(h, id);
-	if(rc) return rc;
-	auto put = [&](int i, double fx, double fy, double fz, double fw, double tx, double ty, double tz) {
-		const size_t o = (size_t) id[i];
-		if(F) F[3 * o] = fx, F[3 * o + 1] = fy, F[3 * o + 2] = fz;
-		if(T) T[3 * o] = tx, T[3 * o + 1] = ty, T[3 * o + 2] = tz;
-		if(E) E[o] = fw;
-	};
-	if(h->dbl) {
-		std::vector<double4_32a> f(N), t(N);
-		CK(cudaMemcpy(f.data(), dF, sizeof(double4_32a) * N, cudaMemcpyDeviceToHost));
-		CK(cudaMemcpy(t.data(), dT, sizeof(double4_32a) * N, cudaMemcpyDeviceToHost));
-		for(int i = 0; i < N; i++) put(i, f[i].x, f[i].y, f[i].z, f[i].w, t[i].x, t[i].y, t[i].z);
+	if(h->sorting()) {
+		const int rc = storage_order(h, id);
+		if(rc) return rc;
 	}
-	else {
-		std::vector<float4> f(N), t(N);
-		CK(cudaMemcpy(f.data(), dF, sizeof(float4) * N, cudaMemcpyDeviceToHost));
-		CK(cudaMemcpy(t.data(), dT, sizeof(float4) * N, cudaMemcpyDeviceToHost));
-		for(int i = 0; i < N; i++) put(i, f[i].x, f[i].y, f[i].z, f[i].w, t[i].x, t[i].y, t[i].z);
+	const size_t v4 = h->dbl ? sizeof(double4_32a) : sizeof(float4);
+	char *f = (char *) h->h_stage, *t = f + v4 * N;
+	if(F || E) CK(cudaMemcpyAsync(f, dF, v4 * N, cudaMemcpyDeviceToHost, h->stream));
+	if(T) CK(cudaMemcpyAsync(t, dT, v4 * N, cudaMemcpyDeviceToHost, h->stream));
+	if(Es) CK(cudaMemcpyAsync(h->h_split, h->esplit, sizeof(double) * 8 * h->n_systems, cudaMemcpyDeviceToHost, h->stream));
+	if(check) {
+		const int rc = read_status(h);
+		if(rc) return rc;
 	}
+	else CK(cudaStreamSynchronize(h->stream));
+	if(Es) std::memcpy(Es, h->h_split, sizeof(double) * 8 * h->n_systems);
+	parallel_parts((size_t) N * 7 * sizeof(double), [&](int k, int parts) {
+		const int lo = (int) ((long long) N * k / parts), hi = (int) ((long long) N * (k + 1) / parts);
+		const int *order = id.empty() ? nullptr : id.data();
+		if(h->dbl) put_forces((const double4_32a *) f, (const double4_32a *) t, order, lo, hi, F, T, E);
+		else put_forces((const float4 *) f, (const float4 *) t, order, lo, hi, F, T, E);
+	});
 	return OXGB_OK;
 }
 

@@ -661,6 +661,7 @@ __global__ void k_unpack_state(StepArgs a, const double *in, int *bad, int check
 		n = 1.0;
 	}
 	if(check_only) return;
+	if(i == 0) *a.th.open_step = *a.th.bussi_stamp = OXGB_NO_STEP;  // nothing is pending in a new state
 	double4_32a P = make_double4_32a(p[0], p[1], p[2], 0.0);
 	double4_32a Q = make_double4_32a(__ddiv_rn(q[0], n), __ddiv_rn(q[1], n), __ddiv_rn(q[2], n), __ddiv_rn(q[3], n));
 	double4_32a V = make_double4_32a(v[0], v[1], v[2], 0.0), M = make_double4_32a(l[0], l[1], l[2], 0.0);
