@@ -453,6 +453,19 @@ __device__ __forceinline__ void load_axes<LoadRef, float>(const LoadRef &ld, int
 	ld.load(j, P, make_int2(0, 0), n, h, l);
 }
 
+// A term's energies of a warp (0: none) into system sy's sum.  All terms of all nucleotides meet at eight
+// addresses per system, where atomics go one after the other: a warp in one system, nearly all of them, adds
+// up first.  The whole warp calls.  (An atomic per bond and lane made an upload and evaluation of 10,000
+// nucleotides 481 us long, 399 so.)
+__device__ __forceinline__ void add_split(double *esplit, int sy, int term, double e) {
+	if(__all_sync(0xffffffffu, sy == __shfl_sync(0xffffffffu, sy, 0))) {
+#pragma unroll
+		for(int off = 16; off > 0; off >>= 1) e += __shfl_xor_sync(0xffffffffu, e, off);
+		if((threadIdx.x & 31) != 0) return;
+	}
+	if(e != 0.0) atomicAdd(esplit + 8 * sy + term, e);
+}
+
 // Bonded block b: 64 bonds (owner p, partner q = n3[p]), a pair of threads each, in different warps:
 // the first half of the block evaluates the stacking, the second half FENE and the bonded excluded
 // volume, joined through shared memory.  One thread for all of a bond is a dependent chain twice as
@@ -471,6 +484,7 @@ __device__ __forceinline__ void bonded_block(const ForceArgs &a, const Loader &l
 	const int q = p < a.N ? a.bonds[p].x : -1;
 	BondOut<R> o;
 	o.f = o.tp = o.tq = v3<R>{R(0), R(0), R(0)};
+	o.split[0] = o.split[1] = o.split[2] = R(0);
 	if(q >= 0) {
 		const int sy = a.sys ? a.sys[p] : 0;
 		const DNA2Table<R> &P = table_of<R>(a, sy);
@@ -483,15 +497,18 @@ __device__ __forceinline__ void bonded_block(const ForceArgs &a, const Loader &l
 			const R v[10] = {o.f.x, o.f.y, o.f.z, o.tp.x, o.tp.y, o.tp.z, o.tq.x, o.tq.y, o.tq.z, o.split[0] + o.split[1]};
 #pragma unroll
 			for(int k = 0; k < (ENERGY ? 10 : 9); k++) part[t][k] = v[k];
-			if(SPLIT) {
-				atomicAdd(a.esplit + 8 * sy + T_FENE, (double) o.split[0]);
-				atomicAdd(a.esplit + 8 * sy + T_BEXC, (double) o.split[1]);
-			}
 		}
 		else {
 			bonded_stacking(P, np, nq, ld.diff(ph, pl, qh, ql), o, ld.refine(p, q));
-			if(SPLIT) atomicAdd(a.esplit + 8 * sy + T_STCK, (double) o.split[2]);
 		}
+	}
+	if(SPLIT) {
+		const int sy = a.sys ? a.sys[min(p, a.N - 1)] : 0;
+		if(backbone) {
+			add_split(a.esplit, sy, T_FENE, (double) o.split[0]);
+			add_split(a.esplit, sy, T_BEXC, (double) o.split[1]);
+		}
+		else add_split(a.esplit, sy, T_STCK, (double) o.split[2]);
 	}
 	__syncthreads();
 	if(q >= 0 && !backbone) {
@@ -1070,10 +1087,9 @@ __device__ __forceinline__ void edge_block(const ForceArgs &a, const Loader &ld,
 		acc.add(o);
 		partner(j, -o.F, cross_accurate(sp, o.F) - o.T, o.E);
 	}
-	if(SPLIT && live) {
+	if(SPLIT) {
 #pragma unroll
-		for(int k = 0; k < N_TERMS; k++)
-			if(acc.split[k] != R(0)) atomicAdd(a.esplit + 8 * sy + k, (double) acc.split[k]);
+		for(int k = 0; k < N_TERMS; k++) add_split(a.esplit, sy, k, live ? (double) acc.split[k] : 0.0);
 	}
 	const R fx = group_sum_comp<R, K>(acc.F.s.x, acc.F.c.x), fy = group_sum_comp<R, K>(acc.F.s.y, acc.F.c.y),
 			fz = group_sum_comp<R, K>(acc.F.s.z, acc.F.c.z);
@@ -1253,10 +1269,9 @@ __global__ void __launch_bounds__(128, 1) k_nonbonded_split(ForceArgs a, Loader 
 		pdl_wait();
 		pdl_trigger();
 		gather_results<R, ENERGY, K, EDGE>(a, i, sub, live, a.bonds[i], acc);
-		if(SPLIT && live) {
+		if(SPLIT) {
 #pragma unroll
-			for(int k = 0; k < N_TERMS; k++)
-				if(acc.split[k] != R(0)) atomicAdd(a.esplit + 8 * sy + k, 0.5 * (double) acc.split[k]);
+			for(int k = 0; k < N_TERMS; k++) add_split(a.esplit, sy, k, live ? 0.5 * (double) acc.split[k] : 0.0);
 		}
 
 		const R fx = group_sum_comp<R, K>(acc.F.s.x, acc.F.c.x), fy = group_sum_comp<R, K>(acc.F.s.y, acc.F.c.y),
@@ -1381,10 +1396,9 @@ __global__ void __launch_bounds__(128, MINB) k_nonbonded_mixed(ForceArgs a, Spli
 				acc.add(o);
 			}
 		}
-		if(SPLIT && live) {
+		if(SPLIT) {
 #pragma unroll
-			for(int k = 0; k < N_TERMS; k++)
-				if(acc.split[k] != 0.f) atomicAdd(a.esplit + 8 * sy + k, 0.5 * (double) acc.split[k]);
+			for(int k = 0; k < N_TERMS; k++) add_split(a.esplit, sy, k, live ? 0.5 * (double) acc.split[k] : 0.0);
 		}
 	}
 	// the axes of the body frame, before the wait for the pair and bond results
