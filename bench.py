@@ -59,7 +59,7 @@ WORKLOADS = {
 }
 
 
-# dram__bytes_read.sum + dram__bytes_write.sum of k_bonded_pairs + k_nonbonded_split per force
+# dram__bytes_read.sum + dram__bytes_write.sum of k_bonded_pairs + k_nonbonded_mixed per force
 # launch (the MD step's variant, autotuned shape 4), from the one-kernel ncu --set full captures
 # summarised in profiles/k_*_{plain40k,large250k}.md (cold caches)
 FORCE_TRAFFIC = {"plain40k": 8.596992e6 + 22.528e3 + 21.910528e6 + 0.0,
@@ -677,7 +677,7 @@ def roofline_of(ox, L, _abi, sysm, stream, torch, systems, peak, traffic=None):
             "frac": achieved / peak, "traffic": traffic,
             "traffic_note": "DRAM bytes (read + write) of one launch of the two force kernels, from an ncu "
                             "--set full capture with cold caches; the timed launches find their data in L2",
-            "kernel": "k_bonded_pairs + k_nonbonded_split (FP32 pair math)",
+            "kernel": "k_bonded_pairs + k_nonbonded_mixed (FP32 pair math)",
             "flops_per_launch": flops, "sfu_per_launch": sfu, "launch_ms": t_force * 1e3,
             "unordered_pairs_listed": pairs, "unordered_pairs_in_cutoff": in_range,
             "flop_count": "every bond and every unordered pair once (partner torque included), "
@@ -804,19 +804,12 @@ def plain_run(args, name, rank, world, torch, ox, _abi, peak):
                       "what": "per step: oxgb_md_set_state from host arrays (upload, list build, forces), M MD "
                               "steps, oxgb_md_get_state into the same host arrays every step; wall clock"}
         assert np.all(np.isfinite(got["pos"]))
-    # our kernels in the timed region: per MD step the first step, the bonded + pair kernel and
-    # the non-bonded kernel, the Bussi draws and sums (the last block of a system makes its
-    # update), and either the rebuild condition (conditional node: 10 list kernels per rebuild)
-    # or the 10 list kernels themselves (kernel node: they return at once unless a system is
-    # stale); per graph of 25 steps the step advance; per run the 2-kernel flush
-    per_step = 3 + (2 if wl["thermostat"] == "bussi" else 0)
-    if args.list_node == "conditional":
-        per_step += 1
-        list_launches = rebuilds * 10
-    else:
-        per_step += 10
-        list_launches = 0
-    out["gpu_launches"] = int(steps_total * per_step + list_launches + (steps_total // 25) + 2 * args.steps)
+    # our kernels in the timed region: per MD step the first step, the list build (which returns at once
+    # unless a system is stale), the bonded + pair kernel, the non-bonded kernel and the Bussi sums (the last
+    # block of a system makes its update); per graph of 25 steps the Bussi draws and the step advance; per run
+    # the 2-kernel flush
+    bussi = 1 if wl["thermostat"] == "bussi" else 0
+    out["gpu_launches"] = int(steps_total * (4 + bussi) + (steps_total // 25) * (1 + bussi) + 2 * args.steps)
     out["_system"] = s
     sysm.close()
     return out
@@ -876,8 +869,8 @@ def main():
     ap.add_argument("--batched-only", action="store_true",
                     help="only the batched engine (no plain workloads, no one-at-a-time comparison): profiling")
     ap.add_argument("--list-node", default="conditional", choices=["conditional", "kernel"],
-                    help="list rebuild as a conditional graph node, or as always-launched kernels that "
-                         "return at once on a fresh list (what a kernel-level profiler can see)")
+                    help="kept: either way the list rebuild is one kernel per step that returns at once on "
+                         "a fresh list")
     ap.add_argument("--sort-every", type=int, default=None,
                     help="store nucleotides in cell order every k-th list rebuild (default: the workload's)")
     ap.add_argument("--precision-study", action="store_true",

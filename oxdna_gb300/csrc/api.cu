@@ -480,7 +480,7 @@ struct oxgb_md {
 	int2 *bonds0 = nullptr;
 	unsigned char *sort_scratch = nullptr;
 	int *d_cell_hil = nullptr, *d_hcount = nullptr, *d_hstart = nullptr;  // Hilbert order
-	int list_kind = OXGB_LIST_WARP;  // neighbour-row kernel (OXGB_LIST_*: chosen at creation or by the autotuner)
+	int list_kind = OXGB_LIST_WARP;  // lanes of the rows (OXGB_LIST_WARP or _GROUP16: chosen at creation or by the autotuner)
 	bool sorting() const { return md.sort_every > 0; }
 
 	void free_layout() {
@@ -1181,14 +1181,10 @@ static int autotune_shape(oxgb_md *h) {
 			best = k;
 		}
 	}
-	// the neighbour-row kernel: both build the same rows from the current positions (a rebuild
-	// is idempotent); not timed when sorting, where extra builds would move the sort schedule.
-	// A single system rebuilds whole, so that is what is timed; a batch rebuilds a few of its
-	// systems at a time (each its own staleness), nearly every step, so a rebuild of its largest
-	// system alone is timed: there a nucleotide's serial walk over its 27 cells (the thread
-	// kernel) is latency that no other work hides (measured on the 256-system batch: the warp
-	// kernel 291 us per MD step, the thread kernel 374 us, although the thread kernel rebuilds
-	// the whole batch faster)
+	// the lanes per nucleotide of the rows, 16 or 32: both build the same rows from the current positions (a
+	// rebuild is idempotent); not timed when sorting, where extra builds would move the sort schedule.
+	// A single system rebuilds whole, so that is what is timed; a batch rebuilds a few of its systems at a
+	// time (each its own staleness), nearly every step, so a rebuild of its largest system alone is timed
 	int list_kind = -1;
 	if(h->md.list_kernel == OXGB_LIST_AUTO && !h->sorting()) {
 		int only = -1;

@@ -868,16 +868,6 @@ OXGB_HD void pair_dh(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R> &q, co
 	}
 }
 
-template <typename R, bool SPLIT>
-OXGB_HD void nonbonded_p(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R> &q, const Sep<R> &sep, PairOut<R> &o) {
-	const v3<R> r = sep.plain();
-	if(dot(r, r) >= P.rcut2) return;
-	pair_ev<R, SPLIT>(p, q, sep, o);
-	pair_base<R, SPLIT>(P, p, q, sep, o);
-	pair_stack<R, SPLIT>(p, q, sep, o);
-	pair_dh<R, SPLIT>(P, p, q, r, o);
-}
-
 // ---------------------------------------------------------------- bonded pair
 
 // p is the nucleotide whose 3' neighbour is q, r = q.centre - p.centre (no periodic image).
@@ -1083,25 +1073,6 @@ OXGB_HD bool bonded_both(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R> &q
 	const bool ok = bonded_backbone(P, p, q, sep, b, xr);
 	bonded_stacking(P, p, q, sep, b, xr);
 	b.E = b.split[0] + b.split[1] + b.split[2];
-	return ok;
-}
-
-// one side of a bonded pair: QSIDE selects q (force +f, torque tq) or p (force -f, torque tp)
-template <typename R, bool SPLIT, bool QSIDE>
-OXGB_HD bool bonded(const DNA2Table<R> &P, const Nuc<R> &p, const Nuc<R> &q, const Sep<R> &sep, PairOut<R> &o) {
-	BondOut<R> b;
-	const bool ok = bonded_both(P, p, q, sep, b);
-	if(QSIDE) {
-		o.F += b.f;
-		o.T += b.tq;
-	}
-	else {
-		o.F -= b.f;
-		o.T += b.tp;
-	}
-	add_e<R, SPLIT>(o, T_FENE, b.split[0]);
-	add_e<R, SPLIT>(o, T_BEXC, b.split[1]);
-	add_e<R, SPLIT>(o, T_STCK, b.split[2]);
 	return ok;
 }
 

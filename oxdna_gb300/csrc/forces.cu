@@ -64,20 +64,6 @@ struct DebyeF {
 // ---------------------------------------------------------------- particle loaders
 
 struct LoadMixed {
-	const float4 *pos_hi, *pos_lo, *fa1, *fa3;
-	__device__ __forceinline__ void load(int i, const DNA2Table<float> &P, const int2 b, Nuc<float> &n, float4 &hi,
-			float4 &lo) const {
-		hi = __ldg(pos_hi + i);
-		lo = __ldg(pos_lo + i);
-		const float4 x1 = __ldg(fa1 + i), x3 = __ldg(fa3 + i);
-		n.a1 = v3<float>{x1.x, x1.y, x1.z};
-		n.a3 = v3<float>{x3.x, x3.y, x3.z};
-		n.a2 = cross(n.a3, n.a1);
-		make_sites(n);
-		n.btype = __float_as_int(hi.w) >> 22;
-		n.type = __float_as_int(lo.w) & 7;
-		n.is_end = (b.x < 0 || b.y < 0);
-	}
 	// minimum image of q - p as hi + lo.  The image m = round(d / box) of a listed pair
 	// (|q - p| < r_verlet, far below box / 2) has d / box at least 0.4 from a half-integer, so
 	// the product with an approximate inverse rounds to the same integer as the quotient;
@@ -1897,7 +1883,7 @@ cudaError_t launch_forces_reference_layout(const RefArgs &a, cudaStream_t s) {
 
 template <typename R, class Loader, bool SPLIT, bool ENERGY, int G = 1, int K = OXGB_NB_LANES, int NBMINB = OXGB_NB_MINB,
 		bool EDGE = false>
-static void launch_split_t(const ForceArgs &a, Loader ld, cudaStream_t s, cudaEvent_t wait) {
+static void launch_split_t(const ForceArgs &a, Loader ld, cudaStream_t s) {
 	const int tpb = 128;
 	const int blocks = a.N > 0 ? (a.N + BONDS_PER_BLOCK - 1) / BONDS_PER_BLOCK : 1;
 	// pair blocks of G groups of 32 nucleotides, then one bonded block per 64 nucleotides, then
@@ -1908,13 +1894,11 @@ static void launch_split_t(const ForceArgs &a, Loader ld, cudaStream_t s, cudaEv
 			pair_blocks);
 	// the non-bonded kernel starts its Debye-Hueckel and excluded-volume work while the tail of
 	// the bonded and pair blocks runs; the external forces follow it the same way
-	if(wait) cudaStreamWaitEvent(s, wait, 0);
 	auto nonbonded = [] {
 		if constexpr(sizeof(R) == 4) return &k_nonbonded_mixed<SPLIT, ENERGY, K, NBMINB, EDGE>;
 		else return &k_nonbonded_split<R, Loader, SPLIT, ENERGY, K, EDGE>;
 	}();
-	if(wait) nonbonded<<<nonbonded_blocks(a.N, K), tpb, 0, s>>>(a, ld);
-	else launch_after(nonbonded, dim3(nonbonded_blocks(a.N, K)), dim3(tpb), 0, s, a, ld);
+	launch_after(nonbonded, dim3(nonbonded_blocks(a.N, K)), dim3(tpb), 0, s, a, ld);
 	if(a.ext_n > 0) launch_after(k_external<typename Vec4Of<R>::T>, dim3((a.ext_n + tpb - 1) / tpb), dim3(tpb), 0, s, a);
 }
 
@@ -1927,51 +1911,50 @@ static void launch_split_t(const ForceArgs &a, Loader ld, cudaStream_t s, cudaEv
 // of 96 systems (70,000) 85.1, 86.1, 81.7, 88.9, 102.3.
 constexpr int PAIR_WIDE_N = 65000;
 template <int k>
-static void launch_md_shape(const ForceArgs &a, const SplitMixed &ld, cudaStream_t s, cudaEvent_t wait) {
+static void launch_md_shape(const ForceArgs &a, const SplitMixed &ld, cudaStream_t s) {
 	constexpr ForceShapeDef d = FORCE_SHAPES[k];
-	if(a.N < PAIR_WIDE_N) launch_split_t<float, SplitMixed, false, false, 1, d.lanes, d.minb>(a, ld, s, wait);
-	else launch_split_t<float, SplitMixed, false, false, d.npw == 32 ? 3 : 6, d.lanes, d.minb>(a, ld, s, wait);
+	if(a.N < PAIR_WIDE_N) launch_split_t<float, SplitMixed, false, false, 1, d.lanes, d.minb>(a, ld, s);
+	else launch_split_t<float, SplitMixed, false, false, d.npw == 32 ? 3 : 6, d.lanes, d.minb>(a, ld, s);
 }
 
 // use_edge: the default shape with the edge blocks
 template <typename R, class Loader>
-static void launch_edge(const ForceArgs &a, Loader ld, bool split, bool energy, cudaStream_t s, cudaEvent_t wait) {
+static void launch_edge(const ForceArgs &a, Loader ld, bool split, bool energy, cudaStream_t s) {
 	constexpr int G = 1, K = OXGB_NB_LANES, MB = OXGB_NB_MINB;
-	if(split) launch_split_t<R, Loader, true, true, G, K, MB, true>(a, ld, s, wait);
-	else if(energy) launch_split_t<R, Loader, false, true, G, K, MB, true>(a, ld, s, wait);
-	else launch_split_t<R, Loader, false, false, G, K, MB, true>(a, ld, s, wait);
+	if(split) launch_split_t<R, Loader, true, true, G, K, MB, true>(a, ld, s);
+	else if(energy) launch_split_t<R, Loader, false, true, G, K, MB, true>(a, ld, s);
+	else launch_split_t<R, Loader, false, false, G, K, MB, true>(a, ld, s);
 }
 
 static SplitDouble double_loader(const ForceArgs &a) {
 	return SplitDouble{a.posd, a.frame64, a.N, SplitMixed{a.pos_hi, a.pos_lo, a.fa1, a.fa3, a.fback, nullptr, nullptr}};
 }
 
-cudaError_t launch_forces_split(const ForceArgs &a, bool dbl, bool split, bool energy, cudaStream_t s, cudaEvent_t wait) {
+cudaError_t launch_forces_split(const ForceArgs &a, bool dbl, bool split, bool energy, cudaStream_t s) {
 	if(a.edge) {
-		if(dbl) launch_edge<double, SplitDouble>(a, double_loader(a), split, energy, s, wait);
-		else launch_edge<float, SplitMixed>(a, SplitMixed{a.pos_hi, a.pos_lo, a.fa1, a.fa3, a.fback, a.fa1lo, a.fbacklo}, split, energy,
-				s, wait);
+		if(dbl) launch_edge<double, SplitDouble>(a, double_loader(a), split, energy, s);
+		else launch_edge<float, SplitMixed>(a, SplitMixed{a.pos_hi, a.pos_lo, a.fa1, a.fa3, a.fback, a.fa1lo, a.fbacklo}, split, energy, s);
 		return cudaGetLastError();
 	}
 	if(dbl) {
 		const SplitDouble ld = double_loader(a);
-		if(split) launch_split_t<double, SplitDouble, true, true>(a, ld, s, wait);
-		else if(energy) launch_split_t<double, SplitDouble, false, true>(a, ld, s, wait);
-		else launch_split_t<double, SplitDouble, false, false>(a, ld, s, wait);
+		if(split) launch_split_t<double, SplitDouble, true, true>(a, ld, s);
+		else if(energy) launch_split_t<double, SplitDouble, false, true>(a, ld, s);
+		else launch_split_t<double, SplitDouble, false, false>(a, ld, s);
 	}
 	else {
 		SplitMixed ld{a.pos_hi, a.pos_lo, a.fa1, a.fa3, a.fback, a.fa1lo, a.fbacklo};
-		if(split) launch_split_t<float, SplitMixed, true, true>(a, ld, s, wait);
-		else if(energy) launch_split_t<float, SplitMixed, false, true>(a, ld, s, wait);
+		if(split) launch_split_t<float, SplitMixed, true, true>(a, ld, s);
+		else if(energy) launch_split_t<float, SplitMixed, false, true>(a, ld, s);
 		else {
 			static_assert(N_FORCE_SHAPES == 6, "one case per shape");
 			switch(a.shape) {
-			case 1: launch_md_shape<1>(a, ld, s, wait); break;
-			case 2: launch_md_shape<2>(a, ld, s, wait); break;
-			case 3: launch_md_shape<3>(a, ld, s, wait); break;
-			case 4: launch_md_shape<4>(a, ld, s, wait); break;
-			case 5: launch_md_shape<5>(a, ld, s, wait); break;
-			default: launch_md_shape<0>(a, ld, s, wait); break;
+			case 1: launch_md_shape<1>(a, ld, s); break;
+			case 2: launch_md_shape<2>(a, ld, s); break;
+			case 3: launch_md_shape<3>(a, ld, s); break;
+			case 4: launch_md_shape<4>(a, ld, s); break;
+			case 5: launch_md_shape<5>(a, ld, s); break;
+			default: launch_md_shape<0>(a, ld, s); break;
 			}
 		}
 	}

@@ -175,12 +175,10 @@ cudaError_t launch_forces_reference_layout(const RefArgs &a, cudaStream_t s);
 // 1 nearly-bonded flag, 2 base-base distance)
 cudaError_t launch_order_params(int mode, const float4 *poss, const float4 *quat, const int *op1, const int *op2, int n,
 		const void *table, float *val, bool *flag, cudaStream_t s);
-// split path: bonded pairs (one thread per bond, both sides), then non-bonded terms (one
-// thread per nucleotide, one loop per term list) with the bonded results gathered in its epilogue
-// wait: an event the non-bonded kernel waits for, or null
+// the engine's forces: bonds and pair terms once per pair (k_bonded_pairs), then Debye-Hueckel and excluded
+// volume from each nucleotide's rows, which gathers their results (k_nonbonded_*)
 // energy = false: forces and torques only (w of F and T left 0), what an MD step needs
-cudaError_t launch_forces_split(const ForceArgs &a, bool dbl, bool split, bool energy, cudaStream_t s,
-		cudaEvent_t wait = nullptr);
+cudaError_t launch_forces_split(const ForceArgs &a, bool dbl, bool split, bool energy, cudaStream_t s);
 // blocks of the split non-bonded kernel for N nucleotides at `lanes` lanes per nucleotide
 int nonbonded_blocks(int N, int lanes);
 // shapes of the MD step's force kernels (mixed / float engine, ForceArgs::shape): how many, and

@@ -43,7 +43,8 @@ def dna2_settings(T: float, salt: float = 0.5, average: bool = True, seq: Option
     return s
 
 
-# the neighbour-row kernels of the list build (OXGB_LIST_*): identical rows, different speeds
+# the lanes per nucleotide of the list build's rows (OXGB_LIST_*): identical rows, different speeds; "warp" is 32,
+# "group16" and all others 16
 LIST_KERNELS = {"auto": 0, "warp": 1, "thread": 2, "group4": 3, "group8": 4, "group16": 5}
 
 
