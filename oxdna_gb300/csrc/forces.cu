@@ -452,14 +452,14 @@ __device__ __forceinline__ void add_split(double *esplit, int sy, int term, doub
 	if(e != 0.0) atomicAdd(esplit + 8 * sy + term, e);
 }
 
-// Bonded block b: 64 bonds (owner p, partner q = n3[p]), a pair of threads each, in different warps:
+// Bonded block b of TPB threads: TPB / 2 bonds (owner p, partner q = n3[p]), a pair of threads each, in different warps:
 // the first half of the block evaluates the stacking, the second half FENE and the bonded excluded
 // volume, joined through shared memory.  One thread for all of a bond is a dependent chain twice as
 // long, and as long as that chain is what a launch lasts where the chip is not full.
-constexpr int BONDS_PER_BLOCK = 64;
 
-template <typename R, class Loader, bool SPLIT, bool ENERGY>
+template <typename R, class Loader, bool SPLIT, bool ENERGY, int TPB>
 __device__ __forceinline__ void bonded_block(const ForceArgs &a, const Loader &ld, int b) {
+	constexpr int BONDS_PER_BLOCK = TPB / 2;
 	using V4 = typename Vec4Of<R>::T;
 	__shared__ R part[BONDS_PER_BLOCK][11];  // force, torques, energy of the backbone part (an odd number of words)
 	const int t = threadIdx.x & (BONDS_PER_BLOCK - 1);
@@ -688,7 +688,6 @@ __device__ __forceinline__ int live_terms(const Nuc<R> &p, const Nuc<R> &q, cons
 }
 
 constexpr int PAIR_CHUNK = 64;             // items taken through stages 2 to 4 at a time
-constexpr int PAIR_QUEUE = 512 + 3 * 128;  // items waiting (a round of screening adds at most 3 x 128)
 
 // one item between the stages (an odd number of words apart: no bank conflicts)
 template <typename R>
@@ -831,14 +830,15 @@ __device__ __forceinline__ R pair_sums(int term, const PairItem<R> &m, v3<R> &f,
 template <typename R>
 constexpr int PAIR_PARTS = sizeof(R) == 8 ? 2 : 1;
 
-// Pair block b (128 threads): the entries owned by G groups of 32 nucleotides, or its part of one group's,
+// Pair block b (TPB threads): the entries owned by G groups of 32 nucleotides, or its part of one group's,
 // in the four stages above
-template <typename R, class Loader, bool SPLIT, bool ENERGY, int G>
+template <typename R, class Loader, bool SPLIT, bool ENERGY, int G, int TPB>
 __device__ __forceinline__ void pair_block(const ForceArgs &a, const Loader &ld, int b) {
+	constexpr int PAIR_QUEUE = 7 * TPB;  // items waiting (a round of screening adds at most 3 x TPB)
 	using V4 = typename Vec4Of<R>::T;
 	__shared__ int2 queue[PAIR_QUEUE];  // partner; k | m << 8 | term << 16 | further term of the pair << 18 | i - first << 19
 	__shared__ PairItem<R> item[PAIR_CHUNK];
-	__shared__ int wcount[4];
+	__shared__ int wcount[TPB / 32];
 	const long long N = a.N;
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	constexpr int PARTS = PAIR_PARTS<R>;
@@ -852,7 +852,7 @@ __device__ __forceinline__ void pair_block(const ForceArgs &a, const Loader &ld,
 	const int lo = start[G] * (b % PARTS) / PARTS, hi = start[G] * (b % PARTS + 1) / PARTS;
 	int n = 0;  // queued items (block-uniform)
 	bool more = hi > lo;
-	for(int r0 = lo; more; r0 += 128) {
+	for(int r0 = lo; more; r0 += TPB) {
 		// stage 1
 		int mask = 0, i0 = 0;
 		int2 it = make_int2(0, 0);
@@ -891,34 +891,34 @@ __device__ __forceinline__ void pair_block(const ForceArgs &a, const Loader &ld,
 		}
 		if(lane == 31) wcount[warp] = incl;
 		__syncthreads();
-		more = r0 + 128 < hi;
+		more = r0 + TPB < hi;
 		int at = n + incl - __popc(mask);
 #pragma unroll
-		for(int w = 0; w < 4; w++) {
+		for(int w = 0; w < TPB / 32; w++) {
 			if(w < warp) at += wcount[w];
 			n += wcount[w];
 		}
 		for(int left = mask, k = 0; left; left &= left - 1, k++)
 			queue[at + k] = make_int2(it.x, it.y | (__ffs(left) - 1) << 16 | (k > 0 ? 1 << 18 : 0) | (i0 - first) << 19);
 		__syncthreads();
-		if(more && n <= PAIR_QUEUE - 3 * 128) continue;
+		if(more && n <= PAIR_QUEUE - 3 * TPB) continue;
 		for(int c0 = 0; c0 < n;) {
 			// the next chunk ends with a whole pair
 			int c1 = min(n, c0 + PAIR_CHUNK);
 			while(c1 < n && (queue[c1].y & (1 << 18))) c1--;
-			for(int m = threadIdx.x; m < c1 - c0; m += 128) {
+			for(int m = threadIdx.x; m < c1 - c0; m += TPB) {
 				const int2 w = queue[c0 + m];
 				const int i = first + (w.y >> 19);
 				pair_radial<R, Loader>(table_of<R>(a, a.sys ? a.sys[i] : 0), ld, i, w.x, (w.y >> 16) & 3, item[m]);
 			}
 			__syncthreads();
-			for(int m0 = warp * 4; m0 < c1 - c0; m0 += 16) {  // warp-uniform: four items at a time
+			for(int m0 = warp * 4; m0 < c1 - c0; m0 += TPB / 8) {  // warp-uniform: four items at a time
 				// (lanes without an item repeat the last one: the same values, written again)
 				const int m = min(m0 + lane / 8, c1 - c0 - 1);
 				pair_angles<R>((queue[c0 + m].y >> 16) & 3, item[m]);
 			}
 			__syncthreads();
-			for(int m = threadIdx.x; m < c1 - c0; m += 128) {
+			for(int m = threadIdx.x; m < c1 - c0; m += TPB) {
 				const int2 w = queue[c0 + m];
 				if(w.y & (1 << 18)) continue;  // taken with the pair's first item
 				const int i = first + (w.y >> 19), j = w.x, k = w.y & 255, mj = (w.y >> 8) & 255;
@@ -1089,17 +1089,17 @@ __device__ __forceinline__ void edge_block(const ForceArgs &a, const Loader &ld,
 // result buffers), so they share one launch: blocks 0 .. pair_blocks - 1 are pair blocks (the
 // costliest, dispatched first), then the bonded blocks, which fill the tail, and with use_edge the
 // edge blocks.  G: groups of 32 nucleotides per pair block.
-template <typename R, class Loader, bool SPLIT, bool ENERGY, int G, bool EDGE = false, int K = 4>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? (EDGE ? 5 : PAIR_MINB) : 1) k_bonded_pairs(ForceArgs a, Loader ld, int pair_blocks) {
+template <typename R, class Loader, bool SPLIT, bool ENERGY, int G, int TPB = 128, bool EDGE = false, int K = 4>
+__global__ void __launch_bounds__(TPB, sizeof(R) == 4 ? (EDGE ? 5 : PAIR_MINB) * 128 / TPB : 1) k_bonded_pairs(ForceArgs a, Loader ld, int pair_blocks) {
 	// launched programmatically after the list build, it reads nothing before that is complete; nor may
 	// the non-bonded kernel start before (it reads the lists and mirrors at once, and waits only for
 	// these results)
 	pdl_wait();
 	pdl_trigger();
 	const int b = blockIdx.x;
-	const int bonded_blocks = (a.N + BONDS_PER_BLOCK - 1) / BONDS_PER_BLOCK;
-	if(b < pair_blocks) pair_block<R, Loader, SPLIT, ENERGY, G>(a, ld, b);
-	else if(!EDGE || b < pair_blocks + bonded_blocks) bonded_block<R, Loader, SPLIT, ENERGY>(a, ld, b - pair_blocks);
+	const int bonded_blocks = (a.N + TPB / 2 - 1) / (TPB / 2);
+	if(b < pair_blocks) pair_block<R, Loader, SPLIT, ENERGY, G, TPB>(a, ld, b);
+	else if(!EDGE || b < pair_blocks + bonded_blocks) bonded_block<R, Loader, SPLIT, ENERGY, TPB>(a, ld, b - pair_blocks);
 	else if constexpr(EDGE) edge_block<R, Loader, SPLIT, ENERGY, K>(a, ld, b - pair_blocks - bonded_blocks);
 }
 
@@ -1882,15 +1882,15 @@ cudaError_t launch_forces_reference_layout(const RefArgs &a, cudaStream_t s) {
 }
 
 template <typename R, class Loader, bool SPLIT, bool ENERGY, int G = 1, int K = OXGB_NB_LANES, int NBMINB = OXGB_NB_MINB,
-		bool EDGE = false>
+		bool EDGE = false, int TPB = 128>
 static void launch_split_t(const ForceArgs &a, Loader ld, cudaStream_t s) {
 	const int tpb = 128;
-	const int blocks = a.N > 0 ? (a.N + BONDS_PER_BLOCK - 1) / BONDS_PER_BLOCK : 1;
-	// pair blocks of G groups of 32 nucleotides, then one bonded block per 64 nucleotides, then
-	// (use_edge) one edge block per 128 / K nucleotides
+	const int blocks = a.N > 0 ? (a.N + TPB / 2 - 1) / (TPB / 2) : 1;
+	// pair blocks of G groups of 32 nucleotides, then one bonded block per TPB / 2 nucleotides, then
+	// (use_edge) one edge block per TPB / K nucleotides
 	const int pair_blocks = (a.N + PAIR_GROUP * G - 1) / (PAIR_GROUP * G) * PAIR_PARTS<R>;
-	const int edge_blocks = EDGE ? nonbonded_blocks(a.N, K) : 0;
-	launch_after(k_bonded_pairs<R, Loader, SPLIT, ENERGY, G, EDGE, K>, dim3(pair_blocks + blocks + edge_blocks), dim3(tpb), 0, s, a, ld,
+	const int edge_blocks = EDGE ? (int) (((long long) a.N * K + TPB - 1) / TPB) : 0;
+	launch_after(k_bonded_pairs<R, Loader, SPLIT, ENERGY, G, TPB, EDGE, EDGE ? K : 4>, dim3(pair_blocks + blocks + edge_blocks), dim3(TPB), 0, s, a, ld,
 			pair_blocks);
 	// the non-bonded kernel starts its Debye-Hueckel and excluded-volume work while the tail of
 	// the bonded and pair blocks runs; the external forces follow it the same way
@@ -1910,10 +1910,16 @@ static void launch_split_t(const ForceArgs &a, Loader ld, cudaStream_t s) {
 // 125.2, 123.3, 126.8, 121.9; strands, 60,000: 32.5, 31.3, 30.0, 30.0, 30.2, 250,000: 111.0, 103.6, 101.0, 99.5, 98.2; batch
 // of 96 systems (70,000) 85.1, 86.1, 81.7, 88.9, 102.3.
 constexpr int PAIR_WIDE_N = 65000;
+// Blocks of 256 threads instead of 128 where one resident wave (three per SM) holds them all: a group's
+// stages are then half as many rounds long, which is what the launch lasts where the chip is not full.  64, 128,
+// 256 threads, us per step: 24 nucleotides 18.1, 16.7, 14.9, 1,000 duplex nucleotides 20.4, 17.0, 15.6; 128 and 256: 5,000:
+// 22.4, 19.3, 8,000: 22.8, 20.1, 12,000: 24.1, 23.4, 16,000: 25.2, 27.8; 10,000 strand nucleotides 17.4, 17.6.
+constexpr bool pair_small(int N) { return N / 32 + N / 128 <= 3 * 152; }
 template <int k>
 static void launch_md_shape(const ForceArgs &a, const SplitMixed &ld, cudaStream_t s) {
 	constexpr ForceShapeDef d = FORCE_SHAPES[k];
-	if(a.N < PAIR_WIDE_N) launch_split_t<float, SplitMixed, false, false, 1, d.lanes, d.minb>(a, ld, s);
+	if(pair_small(a.N)) launch_split_t<float, SplitMixed, false, false, 1, d.lanes, d.minb, false, 256>(a, ld, s);
+	else if(a.N < PAIR_WIDE_N) launch_split_t<float, SplitMixed, false, false, 1, d.lanes, d.minb>(a, ld, s);
 	else launch_split_t<float, SplitMixed, false, false, d.npw == 32 ? 3 : 6, d.lanes, d.minb>(a, ld, s);
 }
 
