@@ -1323,7 +1323,13 @@ static void parallel_parts(size_t total, const Run &run) {
 	const unsigned hw = std::thread::hardware_concurrency();
 	const int parts = (int) std::min<size_t>(std::min(8u, hw > 0 ? hw : 1u), total / (2u << 20) + 1);
 	std::vector<std::thread> pool;
-	for(int k = 1; k < parts; k++) pool.emplace_back(run, k, parts);
+	int started = 1;
+	try {
+		for(; started < parts; started++) pool.emplace_back(run, started, parts);
+	}
+	catch(...) {  // no thread to be had: its part and the rest here
+	}
+	for(int k = started; k < parts; k++) run(k, parts);
 	run(0, parts);
 	for(std::thread &th : pool) th.join();
 }
