@@ -160,6 +160,10 @@ int oxgb_verlet_build_noalloc(int N, double box, double rcut, double skin, int c
 /* device pointers of the neighbour rows (int[N * max_neigh]) and counts (int[N]) */
 int oxgb_verlet_buffers(oxgb_verlet *h, int **d_matrix_neighs, int **d_number_neighs, int *max_neigh, int *n_cells_side);
 int oxgb_verlet_status(oxgb_verlet *h);
+/* polls of its barrier before a list build gives up (0: the default, some seconds; below 0: none), for
+ * trying out the error path: the build and those after it return with OXGB_E_CUDA in the status, and the
+ * first build after that status was read is whole again.  No counterpart in the reference. */
+int oxgb_verlet_set_list_wait(oxgb_verlet *h, int polls);
 int oxgb_verlet_destroy(oxgb_verlet *h);
 
 /* ------------------------------------------------------------------ MD backend layer */
@@ -384,6 +388,9 @@ int oxgb_md_set_force_shape(oxgb_md *h, int k);
 int oxgb_force_shape_table(int k, int *pair_npw, int *nb_lanes, int *nb_min_blocks);
 /* the lanes per nucleotide of the engine's list builds: OXGB_LIST_WARP, _THREAD or _GROUP4/8/16 */
 int oxgb_md_list_kernel(oxgb_md *h, int *kernel);
+/* the same for an engine's list builds (oxgb_verlet_set_list_wait); with cell-order storage a build that
+ * gave up takes the state with it, and the next one has to be set */
+int oxgb_md_set_list_wait(oxgb_md *h, int polls);
 /* device pointers (for zero-copy callers): FP64 positions, velocities, angular momenta and
  * quaternions (double4 each), FP32 forces and torques (float4; double4 in double precision) */
 int oxgb_md_device_buffers(oxgb_md *h, void **pos, void **vel, void **L, void **quat, void **F, void **T);

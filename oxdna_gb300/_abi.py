@@ -111,6 +111,8 @@ SIGNATURES = {
     "oxgb_md_set_force_shape": (C.c_int, [_VP, C.c_int]),
     "oxgb_force_shape_table": (C.c_int, [C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "oxgb_md_list_kernel": (C.c_int, [_VP, C.POINTER(C.c_int)]),
+    "oxgb_md_set_list_wait": (C.c_int, [_VP, C.c_int]),
+    "oxgb_verlet_set_list_wait": (C.c_int, [_VP, C.c_int]),
     "oxgb_md_set_temperature": (C.c_int, [_VP, C.c_int, C.c_double]),
     "oxgb_md_neighbours": (C.c_int, [_VP, _VP, _VP, C.c_int, _VP, _VP]),
     "oxgb_md_info": (C.c_int, [_VP, C.POINTER(C.c_longlong), C.POINTER(C.c_longlong), C.POINTER(C.c_int)]),

@@ -60,11 +60,11 @@ extern "C" void oxgb_md_default_settings(oxgb_md_settings *s) {
 }
 
 static int status_to_code(int st) {
+	if(st & OXGB_ERR_SYNC) return OXGB_E_CUDA;  // (first: forces from unfinished lists may raise the others)
 	if(st & OXGB_ERR_NONFINITE) return OXGB_E_NONFINITE;
 	if(st & OXGB_ERR_FENE) return OXGB_E_FENE;
 	if(st & OXGB_ERR_NEIGH_OVERFLOW) return OXGB_E_NEIGH_OVERFLOW;
 	if(st & OXGB_ERR_CELL) return OXGB_E_NONFINITE;
-	if(st & OXGB_ERR_SYNC) return OXGB_E_CUDA;
 	return OXGB_OK;
 }
 
@@ -214,6 +214,7 @@ struct ListBuffers {
 	float4 *spos = nullptr, *sback = nullptr, *sa1 = nullptr;  // in cell order (the last two with dh)
 	ListSync *sync = nullptr;
 	int *nb = nullptr, *nnb = nullptr;
+	int wait_polls = LIST_WAIT_POLLS;
 	// engine only (dh set before alloc): the Debye-Hueckel rows, the pairs of the full rows whose
 	// backbone sites are within the Debye-Hueckel cutoff plus twice the skin, same capacity
 	bool dh = false;
@@ -243,11 +244,18 @@ struct ListBuffers {
 			CK(cudaMalloc(&sback, sizeof(float4) * std::max(N, 1)));
 			CK(cudaMalloc(&sa1, sizeof(float4) * std::max(N, 1)));
 		}
+		// rows that no build has written are empty, not whatever the memory held
+		CK(cudaMemset(nnb, 0, sizeof(int) * std::max(N, 1)));
+		if(dh) CK(cudaMemset(dh_n, 0, sizeof(int) * std::max(N, 1)));
 		// (complete before any stream's build)
-		CK(cudaMemset(cell_count, 0, sizeof(int) * n_cells));
-		CK(cudaMemset(sync, 0, sizeof(ListSync)));
+		CK(reset(nullptr));
 		CK(cudaStreamSynchronize(nullptr));
 		return OXGB_OK;
+	}
+	// what a build starts from: before the first one, and after one that gave up at its barrier
+	cudaError_t reset(cudaStream_t s) {
+		const cudaError_t e = cudaMemsetAsync(cell_count, 0, sizeof(int) * n_cells, s);
+		return e != cudaSuccess ? e : cudaMemsetAsync(sync, 0, sizeof(ListSync), s);
 	}
 	void free_all() {
 		for(void **p : {(void **) &cell_of, (void **) &cell_count, (void **) &cell_start, (void **) &cell_cursor, (void **) &cell_list,
@@ -282,6 +290,7 @@ struct TermLists {
 		CK(cudaMalloc(&pt_res, 2 * v4 * (size_t) N * pt_cap));
 		CK(cudaMalloc(&pt_live, sizeof(unsigned long long) * words * N));
 		CK(cudaMemsetAsync(pt_live, 0, sizeof(unsigned long long) * words * N, s));
+		for(int *n : {ev_n, pt_n, own_n}) CK(cudaMemsetAsync(n, 0, sizeof(int) * N, s));  // as ListBuffers' counts
 		return OXGB_OK;
 	}
 	void free_all() {
@@ -351,6 +360,7 @@ static ListArgs list_args(ListBuffers &lb, int N, const float4 *pos, float box, 
 	a.sback = lb.sback;
 	a.sa1 = lb.sa1;
 	a.sync = lb.sync;
+	a.wait_polls = lb.wait_polls;
 	a.nb = lb.nb;
 	a.nnb = lb.nnb;
 	a.max_nb = lb.max_nb;
@@ -392,7 +402,19 @@ extern "C" int oxgb_verlet_status(oxgb_verlet *h) {
 	int st = 0;
 	CK(cudaMemcpy(&st, h->d_status, sizeof(int), cudaMemcpyDeviceToHost));
 	CK(cudaMemset(h->d_status, 0, sizeof(int)));
+	if(st & OXGB_ERR_SYNC) {
+		CK(h->lb.reset(nullptr));
+		CK(cudaStreamSynchronize(nullptr));
+	}
 	if(st) return fail(status_to_code(st), status_message(st));
+	return OXGB_OK;
+}
+
+static int wait_polls(int polls) { return polls > 0 ? polls : polls == 0 ? LIST_WAIT_POLLS : 0; }
+
+extern "C" int oxgb_verlet_set_list_wait(oxgb_verlet *h, int polls) {
+	if(!h) return fail(OXGB_E_INVALID, "null handle");
+	h->lb.wait_polls = wait_polls(polls);
 	return OXGB_OK;
 }
 
@@ -462,7 +484,7 @@ struct oxgb_md {
 
 	cudaStream_t stream = nullptr, noise = nullptr;
 	cudaEvent_t ev_join = nullptr, ev_first = nullptr;
-	int *h_word = nullptr;       // pinned: integers read back (4 used), then h_split
+	int *h_word = nullptr;       // pinned: integers read back (5 used), then h_split
 	double *h_split = nullptr;   // [8 * n_systems] energies by term
 	double *h_stage = nullptr, *d_stage = nullptr;   // the state in the caller's layout: pinned host, device
 	int *d_bad = nullptr;                             // lowest nucleotide with a bad quaternion
@@ -1142,6 +1164,8 @@ static int ilog2(long long v) {
 	return k;
 }
 
+static int read_status(oxgb_md *h);
+
 static int autotune_shape(oxgb_md *h) {
 	if(h->dbl || h->tuned) return OXGB_OK;
 	const auto key = std::make_tuple(h->md.precision, ilog2(h->N), ilog2(h->N / h->n_systems));
@@ -1221,6 +1245,9 @@ static int autotune_shape(oxgb_md *h) {
 	}
 	cudaEventDestroy(e0);
 	cudaEventDestroy(e1);
+	CK(cudaMemcpyAsync(h->h_word, h->status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+	CK(cudaStreamSynchronize(h->stream));
+	if(h->h_word[0] & OXGB_ERR_SYNC) return read_status(h);  // (nothing was timed)
 	h->shape = best;
 	h->shape_us = best_us;
 	h->tuned = true;
@@ -1253,6 +1280,14 @@ static int read_status(oxgb_md *h) {
 	const int st = h->h_word[0];
 	if(st) {
 		CK(cudaMemsetAsync(h->status, 0, sizeof(int), h->stream));
+		if(st & OXGB_ERR_SYNC) {
+			// a list build gave up: the next one starts clean and builds every system.  With cell-order storage
+			// it may have stopped between the two halves of a move, so a new state is needed
+			CK(h->lb.reset(h->stream));
+			CK(cudaMemsetAsync(h->d_sys_stale, 1, sizeof(int) * h->n_systems, h->stream));
+			CK(cudaMemsetAsync(h->flag, 1, sizeof(int), h->stream));
+			if(h->sorting()) h->have_state = false;
+		}
 		CK(cudaStreamSynchronize(h->stream));
 		return fail(status_to_code(st), status_message(st));
 	}
@@ -1268,7 +1303,10 @@ static int size_and_build_list(oxgb_md *h) {
 	// to read rather than the counts of every nucleotide)
 	int *tm = h->h_word;
 	CK(cudaMemcpyAsync(tm, h->term_max, 4 * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+	CK(cudaMemcpyAsync(tm + 4, h->status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
 	CK(cudaStreamSynchronize(h->stream));
+	// (rows too short for this capacity are the reason to size them; a build that gave up is an error)
+	if(tm[4] & OXGB_ERR_SYNC) return read_status(h);
 	const int mx = tm[3];
 	int want = ((std::max(64, mx + mx / 2 + 32) + 31) / 32) * 32;
 	auto cap_of = [](int m) { return ((std::max(16, m + m / 2 + 8) + 7) / 8) * 8; };
@@ -1402,6 +1440,17 @@ extern "C" int oxgb_md_set_force_shape(oxgb_md *h, int k) {
 extern "C" int oxgb_md_list_kernel(oxgb_md *h, int *kernel) {
 	if(!h || !kernel) return fail(OXGB_E_INVALID, "null argument");
 	*kernel = h->list_kind;
+	return OXGB_OK;
+}
+
+extern "C" int oxgb_md_set_list_wait(oxgb_md *h, int polls) {
+	if(!h) return fail(OXGB_E_INVALID, "null handle");
+	h->lb.wait_polls = wait_polls(polls);
+	if(h->gexec) {  // part of the captured launches
+		CK(cudaStreamSynchronize(h->stream));
+		cudaGraphExecDestroy(h->gexec);
+		h->gexec = nullptr;
+	}
 	return OXGB_OK;
 }
 

@@ -186,10 +186,12 @@ int nonbonded_blocks(int N, int lanes);
 int force_shape_count();
 void force_shape_of(int k, int *npw, int *lanes, int *minb);
 
-// the grid barrier of a list build (zero before the first one)
+// the grid barrier of a list build (zero before the first one), and whether a build gave up at it: until the
+// host has cleared this and the cell counts, later builds return at once with OXGB_ERR_SYNC
 struct ListSync {
-	unsigned count, gen;
+	unsigned count, gen, failed;
 };
+constexpr int LIST_WAIT_POLLS = 4000000;  // some seconds
 constexpr int LIST_MAX_BLOCKS = 1024;
 
 struct ListArgs {
@@ -209,6 +211,7 @@ struct ListArgs {
 	float4 *spos, *sback, *sa1;  // [N] positions (w: nucleotide), backbone offsets and a1 in the order of
 	                        // cell_list; the last two with term lists or Debye-Hueckel rows (else null)
 	ListSync *sync;
+	int wait_polls;         // polls of a barrier before a build gives up (LIST_WAIT_POLLS)
 	int pdl;                // launched programmatically after the kernel before it
 	int local_cells;        // every system is small: its cells are filled by one block (never when sorting)
 	const int *sys_off;     // [n_systems + 1] first nucleotide of each system (null: one system)

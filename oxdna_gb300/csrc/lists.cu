@@ -63,7 +63,10 @@ __device__ __forceinline__ bool rebuilt(const ListArgs &a, int s) { return !a.sy
 // nucleotides: 21.7 us per step with it, 12.7 without; 250,000: 117.5 and 106.6).  A kernel that reads
 // the flag and returns costs about 1 us.  The launch is cooperative (the driver keeps all its blocks
 // resident together), the arrival count is reset by the last block to arrive, and a wait that should not
-// end gives up after some seconds, flags the build and lets every block leave.
+// end gives up after some seconds, flags the build and lets every block leave.  A block that leaves so is
+// missing at every later barrier, so no block gets beyond the phase after that one, and what a phase reads
+// was written in full.  It leaves arrivals and cell counts behind, on which no build may start: `failed`
+// keeps later ones out until the host has cleared them (ListBuffers::reset).
 //
 // Measured, a rebuild / a step without one, before and now (us): 24 nucleotides 30 / 21.7 -> 11 / 14;
 // 40,000 duplex nucleotides 75 / 47.7 -> 62 / 38; 250,000 strand nucleotides 230 / 117.5 -> 172 / 107;
@@ -72,7 +75,8 @@ constexpr int LIST_TPB = 1024;
 // shared memory of a block that fills a whole system's cells (system_cells): padded counts, nucleotides
 constexpr int LIST_LOCAL_SMEM = (LIST_LOCAL_CELLS + LIST_LOCAL_CELLS / 16 + 2 + LIST_LOCAL_N) * (int) sizeof(int);
 
-__device__ __forceinline__ bool grid_sync(ListSync *y) {
+__device__ __forceinline__ bool grid_sync(const ListArgs &a) {
+	ListSync *y = a.sync;
 	if(gridDim.x == 1) {
 		__syncthreads();
 		return true;
@@ -90,9 +94,12 @@ __device__ __forceinline__ bool grid_sync(ListSync *y) {
 		}
 		else {
 			unsigned now = gen;
-			for(int it = 0; now == gen && it < 4000000; it++)
+			for(int it = 0; now == gen && it < a.wait_polls; it++)
 				asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(now) : "l"(&y->gen) : "memory");
-			if(now == gen) ok = 0;
+			if(now == gen) {
+				ok = 0;
+				y->failed = 1;
+			}
 		}
 	}
 	__syncthreads();
@@ -706,82 +713,88 @@ __device__ __forceinline__ void phase_own(const ListArgs &a) {
 
 // ---------------------------------------------------------------- the build
 
+// the phases of a build; false if a barrier gave up
 template <int K>
-__global__ void __launch_bounds__(LIST_TPB, 1) k_list_build(ListArgs a, int n_cells) {
-	pdl_trigger();  // (every block is running: the next kernel's blocks wait for this one's end)
-	pdl_wait();
-	if(a.check_flag && *(volatile const int *) a.flag == 0) return;
+__device__ __forceinline__ bool list_phases(const ListArgs &a, int n_cells) {
 	__shared__ StaleSystems stale_systems;
 	const Stale stale = list_stale_systems(a, stale_systems);
 	if(a.local_cells) {
 		for(int k = blockIdx.x; k < a.n_systems; k += gridDim.x)
 			if(rebuilt(a, k)) system_cells(a, k);
-		if(!grid_sync(a.sync)) goto failed;
+		if(!grid_sync(a)) return false;
 	}
 	else {
 		phase_count(a);
-		if(!grid_sync(a.sync)) goto failed;
+		if(!grid_sync(a)) return false;
 		phase_block_sum(a, n_cells, [&](int c) { return cell_size(a, c); });
-		if(!grid_sync(a.sync)) goto failed;
+		if(!grid_sync(a)) return false;
 		phase_scan(a, n_cells, [&](int c) { return cell_size(a, c); }, [&](int c, int start) {
 			a.cell_start[c] = start;
 			if(c == n_cells) return;
 			a.cell_cursor[c] = start;
 			a.cell_count[c] = 0;  // for the next build (cells of systems that are not rebuilt hold zero)
 		});
-		if(!grid_sync(a.sync)) goto failed;
+		if(!grid_sync(a)) return false;
 		phase_scatter(a);
-		if(!grid_sync(a.sync)) goto failed;
+		if(!grid_sync(a)) return false;
 		{
 			const bool sorting = sort_now(a);
 			phase_rank(a, !sorting);
-			if(!grid_sync(a.sync)) goto failed;
+			if(!grid_sync(a)) return false;
 			if(sorting) {
 				if(a.cell_hil) {
 					for(int c = blockIdx.x * LIST_TPB + threadIdx.x; c < n_cells; c += gridDim.x * LIST_TPB)
 						a.hcount[a.cell_hil[c]] = a.cell_start[c + 1] - a.cell_start[c];
-					if(!grid_sync(a.sync)) goto failed;
+					if(!grid_sync(a)) return false;
 					phase_block_sum(a, n_cells, [&](int c) { return a.hcount[c]; });
-					if(!grid_sync(a.sync)) goto failed;
+					if(!grid_sync(a)) return false;
 					phase_scan(a, n_cells, [&](int c) { return a.hcount[c]; }, [&](int c, int start) { a.hstart[c] = start; });
-					if(!grid_sync(a.sync)) goto failed;
+					if(!grid_sync(a)) return false;
 				}
 				phase_sort_perm(a);
-				if(!grid_sync(a.sync)) goto failed;
+				if(!grid_sync(a)) return false;
 				phase_sort_gather(a);
-				if(!grid_sync(a.sync)) goto failed;
+				if(!grid_sync(a)) return false;
 				phase_sort_scatter(a);
-				if(!grid_sync(a.sync)) goto failed;
+				if(!grid_sync(a)) return false;
 				phase_sorted_copies(a);
-				if(!grid_sync(a.sync)) goto failed;
+				if(!grid_sync(a)) return false;
 			}
 		}
 	}
 	phase_rows<K>(a, stale);
 	if(a.own) {
-		if(!grid_sync(a.sync)) goto failed;
+		if(!grid_sync(a)) return false;
 		phase_own(a);
 	}
-	// the last block to finish counts the build and clears the requests
-	{
-		__shared__ int last;
-		__syncthreads();
-		if(threadIdx.x == 0) {
-			__threadfence();
-			last = gridDim.x == 1 || atomicAdd(&a.sync->count, 1u) == gridDim.x - 1;
-			if(last) a.sync->count = 0;
-		}
-		__syncthreads();
-		if(!last) return;
-		if(a.sys_stale)
-			for(int s = threadIdx.x; s < a.n_systems; s += LIST_TPB) a.sys_stale[s] = 0;
-		if(threadIdx.x != 0) return;
-		if(a.rebuilds) *a.rebuilds += 1;
-		*a.flag = 0;
+	return true;
+}
+
+template <int K>
+__global__ void __launch_bounds__(LIST_TPB, 1) k_list_build(ListArgs a, int n_cells) {
+	pdl_trigger();  // (every block is running: the next kernel's blocks wait for this one's end)
+	pdl_wait();
+	if(a.check_flag && *(volatile const int *) a.flag == 0) return;
+	const bool barred = __syncthreads_or(threadIdx.x == 0 && *(volatile const unsigned *) &a.sync->failed != 0);
+	if(barred || !list_phases<K>(a, n_cells)) {
+		if(threadIdx.x == 0) atomicOr(a.status, OXGB_ERR_SYNC);
+		return;
 	}
-	return;
-failed:
-	if(threadIdx.x == 0) atomicOr(a.status, OXGB_ERR_SYNC);
+	// the last block to finish counts the build and clears the requests
+	__shared__ int last;
+	__syncthreads();
+	if(threadIdx.x == 0) {
+		__threadfence();
+		last = gridDim.x == 1 || atomicAdd(&a.sync->count, 1u) == gridDim.x - 1;
+		if(last) a.sync->count = 0;
+	}
+	__syncthreads();
+	if(!last) return;
+	if(a.sys_stale)
+		for(int s = threadIdx.x; s < a.n_systems; s += LIST_TPB) a.sys_stale[s] = 0;
+	if(threadIdx.x != 0) return;
+	if(a.rebuilds) *a.rebuilds += 1;
+	*a.flag = 0;
 }
 
 template <int K>

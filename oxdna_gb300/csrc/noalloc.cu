@@ -15,8 +15,8 @@
 // current), and checks on every call that the module was not reloaded since; the first call
 // on a device may load the module, so it should come before any stream capture.  Calls on one device share the scratch: two calls
 // that overlap in time (different streams or threads) race and must be serialised by the
-// caller.  Each call clears what must start at zero (the status word; the cell counts are left at
-// zero by the build itself), so consecutive calls never see each other's leftovers.
+// caller.  Each call clears what must start at zero (the status word, the barrier, the cell counts), so
+// consecutive calls never see each other's leftovers.
 #include "kernels.h"
 #include "params.h"
 
@@ -40,13 +40,16 @@ static __device__ __align__(256) int g_cell_start[NOALLOC_MAX_CELLS + 1];
 static __device__ __align__(256) int g_cell_cursor[NOALLOC_MAX_CELLS];
 static __device__ __align__(256) int g_scan_part[LIST_MAX_BLOCKS];
 static __device__ __align__(256) float4 g_spos[NOALLOC_MAX_N];
-static __device__ __align__(256) ListSync g_sync;
-static __device__ __align__(256) int g_status[2];  // status word, rebuild flag
+struct Words {  // what starts at zero on every call
+	int status, flag;
+	ListSync sync;
+};
+static __device__ __align__(256) Words g_words;
 
 struct Scratch {
-	int *cell_of, *cell_tmp, *cell_list, *cell_count, *cell_start, *cell_cursor, *scan_part, *status;
+	int *cell_of, *cell_tmp, *cell_list, *cell_count, *cell_start, *cell_cursor, *scan_part;
 	float4 *spos;
-	ListSync *sync;
+	Words *words;
 };
 
 static std::mutex g_scratch_mutex;
@@ -54,7 +57,7 @@ static Scratch g_scratch[64];
 static bool g_scratch_ok[64];
 
 // device addresses of the scratch arrays on the current device: looked up together once per
-// device; every later call looks up the status word's address alone (cheap once the module is
+// device; every later call looks up the address of the words alone (cheap once the module is
 // loaded) and redoes the whole lookup if it moved, which happens when a device reset or a new
 // primary context has loaded the module again
 static cudaError_t scratch_of_current_device(Scratch &out) {
@@ -65,8 +68,8 @@ static cudaError_t scratch_of_current_device(Scratch &out) {
 	std::lock_guard<std::mutex> lock(g_scratch_mutex);
 	if(g_scratch_ok[dev]) {
 		void *p = nullptr;
-		if((e = cudaGetSymbolAddress(&p, g_status)) != cudaSuccess) return e;
-		if((int *) p != g_scratch[dev].status) g_scratch_ok[dev] = false;
+		if((e = cudaGetSymbolAddress(&p, g_words)) != cudaSuccess) return e;
+		if((Words *) p != g_scratch[dev].words) g_scratch_ok[dev] = false;
 	}
 	if(!g_scratch_ok[dev]) {
 		Scratch s{};
@@ -87,10 +90,8 @@ static cudaError_t scratch_of_current_device(Scratch &out) {
 		s.scan_part = (int *) p;
 		if((e = cudaGetSymbolAddress(&p, g_spos)) != cudaSuccess) return e;
 		s.spos = (float4 *) p;
-		if((e = cudaGetSymbolAddress(&p, g_sync)) != cudaSuccess) return e;
-		s.sync = (ListSync *) p;
-		if((e = cudaGetSymbolAddress(&p, g_status)) != cudaSuccess) return e;
-		s.status = (int *) p;
+		if((e = cudaGetSymbolAddress(&p, g_words)) != cudaSuccess) return e;
+		s.words = (Words *) p;
 		g_scratch[dev] = s;
 		g_scratch_ok[dev] = true;
 	}
@@ -122,8 +123,10 @@ extern "C" int oxgb_verlet_build_noalloc(int N, double box, double rcut, double 
 	cudaError_t e = scratch_of_current_device(sc);
 	if(e != cudaSuccess) return set_error(OXGB_E_CUDA, std::string("scratch lookup: ") + cudaGetErrorString(e));
 	cudaStream_t s = (cudaStream_t) stream;
-	// status word and rebuild flag start at zero on every call
-	e = cudaMemsetAsync(sc.status, 0, 2 * sizeof(int), s);
+	// whatever the call before left (it may have overlapped another one, or given up at its barrier)
+	e = cudaMemsetAsync(sc.words, 0, sizeof(Words), s);
+	const bool local = list_local_cells(N, n_cells);
+	if(e == cudaSuccess && !local) e = cudaMemsetAsync(sc.cell_count, 0, sizeof(int) * n_cells, s);
 	if(e != cudaSuccess) return set_error(OXGB_E_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
 	ListArgs a{};
 	a.N = N;
@@ -140,22 +143,23 @@ extern "C" int oxgb_verlet_build_noalloc(int N, double box, double rcut, double 
 	a.cell_tmp = sc.cell_tmp;
 	a.scan_part = sc.scan_part;
 	a.spos = sc.spos;
-	a.sync = sc.sync;
+	a.sync = &sc.words->sync;
+	a.wait_polls = LIST_WAIT_POLLS;
 	a.nb = d_matrix_neighs;
 	a.nnb = d_number_neighs;
 	a.max_nb = max_neigh;
 	a.list_pos = (float4 *) d_list_poss;
-	a.status = sc.status;
-	a.flag = sc.status + 1;
+	a.status = &sc.words->status;
+	a.flag = &sc.words->flag;
 	a.check_flag = 0;
 	a.rebuilds = nullptr;
 	a.col_major = 1;
 	a.n_systems = 1;
-	a.local_cells = list_local_cells(N, n_cells);
+	a.local_cells = local;
 	e = launch_list_build(a, s);
 	if(e != cudaSuccess) return set_error(OXGB_E_CUDA, std::string("list build: ") + cudaGetErrorString(e));
 	int st = 0;
-	e = cudaMemcpyAsync(&st, sc.status, sizeof(int), cudaMemcpyDeviceToHost, s);
+	e = cudaMemcpyAsync(&st, &sc.words->status, sizeof(int), cudaMemcpyDeviceToHost, s);
 	if(e == cudaSuccess) e = cudaStreamSynchronize(s);
 	if(e != cudaSuccess) return set_error(OXGB_E_CUDA, std::string("status read: ") + cudaGetErrorString(e));
 	if(st) return set_error(list_status_code(st), list_status_message(st));
