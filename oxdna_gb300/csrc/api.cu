@@ -1486,9 +1486,9 @@ extern "C" int oxgb_md_get_state(oxgb_md *h, double *pos, double *quat, double *
 }
 
 // Bussi: at the first of `steps` steps captured together, from its list build on and beside its force
-// kernels, the draws of all of them (they depend only on the seed and the step).  The branch starts after the list build because a cooperative kernel
-// waits until the chip holds no other: beside the first step, the draws kept the build of a 96-system
-// batch waiting for 33 us in every step.
+// kernels, the draws of all of them (they depend only on the seed and the step).  The branch starts after the list
+// build because the build's blocks take whole SMs: beside the first step, the draws of a 96-system batch held
+// its build back by 33 us in every step (measured when a build needed all SMs at once).
 static cudaError_t bussi_side_branch(oxgb_md *h, const StepArgs &sa, int steps) {
 	if(sa.th.thermostat != OXGB_THERMOSTAT_BUSSI || sa.th.step_offset != 0) return cudaSuccess;
 	cudaError_t e = cudaEventRecord(h->ev_first, h->stream);

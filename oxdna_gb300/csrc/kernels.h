@@ -186,13 +186,15 @@ int nonbonded_blocks(int N, int lanes);
 int force_shape_count();
 void force_shape_of(int k, int *npw, int *lanes, int *minb);
 
-// the grid barrier of a list build (zero before the first one), and whether a build gave up at it: until the
-// host has cleared this and the cell counts, later builds return at once with OXGB_ERR_SYNC
+// the blocks of a list build (all zero before the first one), each counter in a line of its own: who takes part
+// (roll, done, members; lists.cu), the members' barrier (count, gen), and the blocks that have left.  After a build
+// that gave up at a wait the roll stays closed: until the host has cleared this and the cell counts, later builds
+// return at once with OXGB_ERR_SYNC
 struct ListSync {
-	unsigned count, gen, failed;
+	unsigned roll, pad0[31], done, members, pad1[30], count, gen, pad2[30], left, pad3[31];
 };
 constexpr int LIST_WAIT_POLLS = 4000000;  // some seconds
-constexpr int LIST_MAX_BLOCKS = 1024;
+constexpr int LIST_MAX_BLOCKS = 1024;   // (roll and left count to 16,383)
 
 struct ListArgs {
 	int N;
@@ -211,7 +213,7 @@ struct ListArgs {
 	float4 *spos, *sback, *sa1;  // [N] positions (w: nucleotide), backbone offsets and a1 in the order of
 	                        // cell_list; the last two with term lists or Debye-Hueckel rows (else null)
 	ListSync *sync;
-	int wait_polls;         // polls of a barrier before a build gives up (LIST_WAIT_POLLS)
+	int wait_polls;         // polls of a wait before a build gives up (LIST_WAIT_POLLS)
 	int pdl;                // launched programmatically after the kernel before it
 	int local_cells;        // every system is small: its cells are filled by one block (never when sorting)
 	const int *sys_off;     // [n_systems + 1] first nucleotide of each system (null: one system)
@@ -287,7 +289,7 @@ constexpr int LIST_LOCAL_N = 4096;
 constexpr int LIST_LOCAL_CELLS = 16384;
 inline bool list_local_cells(long long n, long long cells) { return n <= LIST_LOCAL_N && cells <= LIST_LOCAL_CELLS; }
 
-// the build, one cooperative launch: cells (counting sort, deterministic order) then neighbour rows; with
+// the build, one launch: cells (counting sort, deterministic order) then neighbour rows; with
 // check_flag it returns at once while the lists are fresh
 cudaError_t launch_list_build(const ListArgs &a, cudaStream_t s);
 

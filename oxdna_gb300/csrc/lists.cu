@@ -5,7 +5,7 @@
 // CUDASimpleVerletList.cu:231-289).  Cells are filled by a counting sort (count, scan,
 // scatter, then each particle placed by the rank of its caller's index within its cell), so there is no
 // per-cell capacity to overflow and the neighbour order is deterministic run to run.  All of a build is
-// one cooperative kernel, whose phases are separated by grid barriers.  The geometry is the
+// one kernel, whose phases are separated by barriers of the blocks that run.  The geometry is the
 // reference's fp32 geometry: cell coordinate ((x/L - floor(x/L)) * (1 - FLT_EPSILON)) * n and
 // minimum-image squared distance against r_verlet^2, with IEEE division and the fused
 // multiply-adds written out, so that oracle/dna2_oracle.c (oxo_verlet_f32) reproduces the
@@ -56,28 +56,112 @@ __device__ __forceinline__ CellGeo cell_geo(const ListArgs &a, int s) {
 __device__ __forceinline__ bool rebuilt(const ListArgs &a, int s) { return !a.sys_stale || a.sys_stale[s] != 0; }
 
 
-// ---------------------------------------------------------------- the grid barrier
+// ---------------------------------------------------------------- the blocks of a build
 //
 // One build is one launch: as a graph node of its own per phase it was a conditional (IF) node holding
 // ten kernels, and that node alone cost 9 to 11 us per MD step whether the lists were stale or not (24
 // nucleotides: 21.7 us per step with it, 12.7 without; 250,000: 117.5 and 106.6).  A kernel that reads
-// the flag and returns costs about 1 us.  The launch is cooperative (the driver keeps all its blocks
-// resident together), the arrival count is reset by the last block to arrive, and a wait that should not
-// end gives up after some seconds, flags the build and lets every block leave.  A block that leaves so is
-// missing at every later barrier, so no block gets beyond the phase after that one, and what a phase reads
-// was written in full.  It leaves arrivals and cell counts behind, on which no build may start: `failed`
-// keeps later ones out until the host has cleared them (ListBuffers::reset).
+// the flag and returns costs about 1 us.
 //
-// Measured, a rebuild / a step without one, before and now (us): 24 nucleotides 30 / 21.7 -> 11 / 14;
+// Its phases are separated by barriers, so no block may wait for one that is not running: beside another
+// program's kernel (a block here takes a whole SM's registers) some start when the others have finished.  A
+// cooperative launch, which starts all blocks or none, had every build wait for whatever else the GPU ran:
+// 40,000 nucleotides beside one-block kernels of 0.2 and 2 ms on another stream, 214 and 449 us per step
+// (alone 53), a list of 16,000 1,948 us (alone 35); without it 53 to 54, and 37.  So the blocks that run share the
+// work, which takes a build of the whole grid about 1 us more.  The first phase is
+// cut into as many items as the grid has blocks, each taken by whichever block asks for one; who asks before
+// the last item is done is a member of the build, and the later phases and their barriers are the members'
+// alone (their number changes no result).  A block that starts later finds the roll closed and leaves.  The
+// last block of the grid to leave clears the barrier, the requests and the flag, which so stand for every
+// block of the launch alike.
+//
+// A wait that should not end gives up after some seconds, flags the build and lets its block leave.  Such a
+// block is missing at every later barrier, so no block gets beyond the phase after that one, and what a phase
+// reads was written in full.  Its cell counts stay behind, on which no build may start: the roll stays closed to
+// later ones until the host has cleared them (ListBuffers::reset).
+//
+// Measured, a rebuild / a step without one, before the one launch and now (us): 24 nucleotides 30 / 21.7 -> 11 / 14;
 // 40,000 duplex nucleotides 75 / 47.7 -> 62 / 38; 250,000 strand nucleotides 230 / 117.5 -> 172 / 107;
-// the plain list of 120,000 (no term lists) 97.3 -> 62.6.
+// the plain list of 120,000 (no term lists) 97.3 -> 64.
 constexpr int LIST_TPB = 1024;
 // shared memory of a block that fills a whole system's cells (system_cells): padded counts, nucleotides
 constexpr int LIST_LOCAL_SMEM = (LIST_LOCAL_CELLS + LIST_LOCAL_CELLS / 16 + 2 + LIST_LOCAL_N) * (int) sizeof(int);
 
-__device__ __forceinline__ bool grid_sync(const ListArgs &a) {
+// this block's number among the members, and how many they are (0: not a member); in shared memory, read where
+// needed (the rows have no register to spare)
+struct Member {
+	int id, n;
+};
+
+// ListSync::roll: closed | a build gave up | arrivals << 16 | items taken; left: blocks that gave up << 16 | blocks
+constexpr unsigned ROLL_CLOSED = 0x80000000u, ROLL_FAILED = 0x40000000u, ROLL_ONE = 0x10000u;
+
+__device__ __forceinline__ int roll_arrivals(unsigned roll) { return (int) ((roll & (ROLL_FAILED - 1)) >> 16); }
+
+// (thread 0) polls *at until it is not `from`; false if the wait ran out
+__device__ __forceinline__ bool poll(const ListArgs &a, const unsigned *at, unsigned from, unsigned &now) {
+	now = from;
+	for(int it = 0; now == from && it < a.wait_polls; it++) asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(now) : "l"(at) : "memory");
+	return now != from;
+}
+
+// The first phase, item(k) for k = 0 .. gridDim.x - 1, and the roll; false if the wait ran out.  meanwhile(): work
+// of every block, done while its arrival is on the way.
+template <class Item, class Work>
+__device__ __forceinline__ bool first_phase(const ListArgs &a, volatile Member &me, const Item &item, const Work &meanwhile) {
+	const unsigned grid = gridDim.x;
+	if(grid == 1) {
+		meanwhile();
+		item(0);
+		if(threadIdx.x == 0) me.id = 0, me.n = 1;
+		__syncthreads();
+		return true;
+	}
 	ListSync *y = a.sync;
-	if(gridDim.x == 1) {
+	__shared__ unsigned taken;
+	__shared__ int ok;
+	unsigned k = 0;
+	if(threadIdx.x == 0) k = atomicAdd(&y->roll, ROLL_ONE + 1);
+	meanwhile();
+	if(threadIdx.x == 0) {
+		taken = k;
+		me.id = roll_arrivals(k);
+		me.n = 0;
+	}
+	__syncthreads();
+	k = taken;
+	if(k & ROLL_CLOSED) return !(k & ROLL_FAILED);
+	unsigned closer = 0;  // (thread 0: the members, once this block has closed the roll)
+	for(k &= ROLL_ONE - 1; k < grid; k = taken & (ROLL_ONE - 1)) {
+		item((int) k);
+		__syncthreads();  // (everyone has read `taken`, too)
+		if(threadIdx.x == 0) {
+			unsigned roll, done;
+			asm volatile("atom.add.relaxed.gpu.u32 %0, [%1], 1;" : "=r"(roll) : "l"(&y->roll) : "memory");
+			asm volatile("atom.add.acq_rel.gpu.u32 %0, [%1], 1;" : "=r"(done) : "l"(&y->done) : "memory");
+			taken = roll;
+			if(done == grid - 1) {
+				// (all have arrived, commonly; else nobody may any more)
+				closer = roll_arrivals(roll);
+				if(closer < grid) closer = roll_arrivals(atomicOr(&y->roll, ROLL_CLOSED));
+				asm volatile("st.release.gpu.u32 [%0], %1;" ::"l"(&y->members), "r"(closer) : "memory");
+			}
+		}
+		__syncthreads();
+	}
+	if(threadIdx.x == 0) {
+		ok = 1;
+		if(closer == 0) ok = poll(a, &y->members, 0, closer);
+		me.n = (int) closer;
+	}
+	__syncthreads();
+	return ok != 0;
+}
+
+// the members' barrier; false if the wait ran out
+__device__ __forceinline__ bool members_sync(const ListArgs &a, const volatile Member &me) {
+	ListSync *y = a.sync;
+	if(me.n == 1) {
 		__syncthreads();
 		return true;
 	}
@@ -88,19 +172,11 @@ __device__ __forceinline__ bool grid_sync(const ListArgs &a) {
 		asm volatile("ld.relaxed.gpu.u32 %0, [%1];" : "=r"(gen) : "l"(&y->gen) : "memory");
 		asm volatile("atom.add.acq_rel.gpu.u32 %0, [%1], 1;" : "=r"(old) : "l"(&y->count) : "memory");
 		ok = 1;
-		if(old == gridDim.x - 1) {
+		if(old == (unsigned) me.n - 1) {
 			asm volatile("st.relaxed.gpu.u32 [%0], 0;" ::"l"(&y->count) : "memory");
 			asm volatile("red.add.release.gpu.u32 [%0], 1;" ::"l"(&y->gen) : "memory");
 		}
-		else {
-			unsigned now = gen;
-			for(int it = 0; now == gen && it < a.wait_polls; it++)
-				asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(now) : "l"(&y->gen) : "memory");
-			if(now == gen) {
-				ok = 0;
-				y->failed = 1;
-			}
-		}
+		else ok = poll(a, &y->gen, gen, gen);
 	}
 	__syncthreads();
 	return ok != 0;
@@ -132,9 +208,9 @@ __device__ __forceinline__ int block_incl_scan(int v, int *warp_tot) {
 
 
 // this block's share of n items: a contiguous range
-__device__ __forceinline__ void block_share(int n, int &lo, int &hi) {
-	lo = (int) ((long long) n * blockIdx.x / gridDim.x);
-	hi = (int) ((long long) n * (blockIdx.x + 1) / gridDim.x);
+__device__ __forceinline__ void block_share(const volatile Member &me, int n, int &lo, int &hi) {
+	lo = (int) ((long long) n * me.id / me.n);
+	hi = (int) ((long long) n * (me.id + 1) / me.n);
 }
 
 // the cell of a nucleotide at r in a system of geometry g
@@ -155,9 +231,9 @@ __device__ __forceinline__ int cell_at(const ListArgs &a, const CellGeo &g, cons
 }
 
 // the cell of every nucleotide of the systems to rebuild, and their numbers (cell_count is zero between
-// builds)
-__device__ __forceinline__ void phase_count(const ListArgs &a) {
-	for(int i = blockIdx.x * LIST_TPB + threadIdx.x; i < a.N; i += gridDim.x * LIST_TPB) {
+// builds): the item-th of gridDim.x parts
+__device__ __forceinline__ void phase_count(const ListArgs &a, int item) {
+	for(int i = item * LIST_TPB + threadIdx.x; i < a.N; i += gridDim.x * LIST_TPB) {
 		const int s = sys_of(a, i);
 		if(!rebuilt(a, s)) continue;
 		const int c = cell_at(a, cell_geo(a, s), a.pos[i]);
@@ -173,15 +249,15 @@ __device__ __forceinline__ int cell_size(const ListArgs &a, int c) {
 	return __ldcg(a.cell_count + c);  // (counted by atomics: not through L1)
 }
 
-// sum of f(c) over this block's share of the cells, to scan_part[blockIdx.x]
+// sum of f(c) over this block's share of the cells, to scan_part[me.id]
 template <class F>
-__device__ __forceinline__ void phase_block_sum(const ListArgs &a, int n_cells, const F &f) {
+__device__ __forceinline__ void phase_block_sum(const ListArgs &a, const volatile Member &me, int n_cells, const F &f) {
 	__shared__ int wt[32];
 	int lo, hi, v = 0;
-	block_share(n_cells, lo, hi);
+	block_share(me, n_cells, lo, hi);
 	for(int c = lo + threadIdx.x; c < hi; c += LIST_TPB) v += f(c);
 	const int incl = block_incl_scan(v, wt);
-	if(threadIdx.x == LIST_TPB - 1) a.scan_part[blockIdx.x] = incl;
+	if(threadIdx.x == LIST_TPB - 1) a.scan_part[me.id] = incl;
 }
 
 // exclusive scan by one block of f(c) over the cells lo .. hi - 1, from `carry`: put(c, sum below c);
@@ -213,11 +289,11 @@ __device__ __forceinline__ int block_scan(int lo, int hi, int carry, const F &f,
 // exclusive scan of f(c), after phase_block_sum and a barrier: put(c, sum of f below c) for every cell
 // of the block's share; the block of the last cell calls put(n_cells, total)
 template <class F, class P>
-__device__ __forceinline__ void phase_scan(const ListArgs &a, int n_cells, const F &f, const P &put) {
+__device__ __forceinline__ void phase_scan(const ListArgs &a, const volatile Member &me, int n_cells, const F &f, const P &put) {
 	__shared__ int wt[32], before;
 	int lo, hi, v = 0;
-	block_share(n_cells, lo, hi);
-	for(int b = threadIdx.x; b < (int) blockIdx.x; b += LIST_TPB) v += a.scan_part[b];
+	block_share(me, n_cells, lo, hi);
+	for(int b = threadIdx.x; b < me.id; b += LIST_TPB) v += a.scan_part[b];
 	v = block_incl_scan(v, wt);
 	if(threadIdx.x == LIST_TPB - 1) before = v;
 	__syncthreads();
@@ -226,8 +302,8 @@ __device__ __forceinline__ void phase_scan(const ListArgs &a, int n_cells, const
 }
 
 // particles into their cells' segments, in arbitrary order (cell_tmp)
-__device__ __forceinline__ void phase_scatter(const ListArgs &a) {
-	for(int i = blockIdx.x * LIST_TPB + threadIdx.x; i < a.N; i += gridDim.x * LIST_TPB) {
+__device__ __forceinline__ void phase_scatter(const ListArgs &a, const volatile Member &me) {
+	for(int i = me.id * LIST_TPB + threadIdx.x; i < a.N; i += me.n * LIST_TPB) {
 		if(!rebuilt(a, sys_of(a, i))) continue;
 		a.cell_tmp[atomicAdd(a.cell_cursor + a.cell_of[i], 1)] = i;
 	}
@@ -262,8 +338,8 @@ __device__ __forceinline__ int rank_in_cell(const ListArgs &a, int b, int e, int
 }
 
 // each particle's rank by caller's index within its cell gives the deterministic order (cell_list)
-__device__ __forceinline__ void phase_rank(const ListArgs &a, bool copy) {
-	for(int i = blockIdx.x * LIST_TPB + threadIdx.x; i < a.N; i += gridDim.x * LIST_TPB) {
+__device__ __forceinline__ void phase_rank(const ListArgs &a, const volatile Member &me, bool copy) {
+	for(int i = me.id * LIST_TPB + threadIdx.x; i < a.N; i += me.n * LIST_TPB) {
 		if(!rebuilt(a, sys_of(a, i))) continue;
 		const int c = a.cell_of[i], b = a.cell_start[c];
 		const int p = b + rank_in_cell(a, b, a.cell_start[c + 1], id_of(a, i));
@@ -353,8 +429,8 @@ __device__ __forceinline__ bool sort_now(const ListArgs &a) {
 // New slot k takes old slot perm[k] (rebuilt systems; the others stay): cell_list[k], or with the
 // Hilbert order the nucleotide whose cell is at that position along the curve (hstart, the scan of the
 // cells' sizes in that order), at its rank within the cell
-__device__ __forceinline__ void phase_sort_perm(const ListArgs &a) {
-	for(int p = blockIdx.x * LIST_TPB + threadIdx.x; p < a.N; p += gridDim.x * LIST_TPB) {
+__device__ __forceinline__ void phase_sort_perm(const ListArgs &a, const volatile Member &me) {
+	for(int p = me.id * LIST_TPB + threadIdx.x; p < a.N; p += me.n * LIST_TPB) {
 		int from = p, to = p;
 		if(rebuilt(a, sys_of(a, p))) {
 			from = a.cell_list[p];
@@ -369,13 +445,13 @@ __device__ __forceinline__ void phase_sort_perm(const ListArgs &a) {
 }
 
 // everything of old slot perm[k] into the staging buffer at k; bonds renumbered
-__device__ __forceinline__ void phase_sort_gather(const ListArgs &a) {
+__device__ __forceinline__ void phase_sort_gather(const ListArgs &a, const volatile Member &me) {
 	const long long N = a.N;
 	double4_32a *sd = reinterpret_cast<double4_32a *>(a.scratch);
 	float4 *sf = reinterpret_cast<float4 *>(a.scratch + 4 * 32 * N);
 	int2 *sb = reinterpret_cast<int2 *>(a.scratch + (4 * 32 + SORT_MIRRORS * 16) * N);
 	int *si = reinterpret_cast<int *>(a.scratch + (4 * 32 + SORT_MIRRORS * 16 + 8) * N);
-	for(int k = blockIdx.x * LIST_TPB + threadIdx.x; k < a.N; k += gridDim.x * LIST_TPB) {
+	for(int k = me.id * LIST_TPB + threadIdx.x; k < a.N; k += me.n * LIST_TPB) {
 		const int from = a.perm[k];
 #pragma unroll
 		for(int t = 0; t < 4; t++) sd[t * N + k] = a.st[t][from];
@@ -392,13 +468,13 @@ __device__ __forceinline__ void phase_sort_gather(const ListArgs &a) {
 }
 
 // the staging buffer back into the arrays, and the inverse map
-__device__ __forceinline__ void phase_sort_scatter(const ListArgs &a) {
+__device__ __forceinline__ void phase_sort_scatter(const ListArgs &a, const volatile Member &me) {
 	const long long N = a.N;
 	const double4_32a *sd = reinterpret_cast<const double4_32a *>(a.scratch);
 	const float4 *sf = reinterpret_cast<const float4 *>(a.scratch + 4 * 32 * N);
 	const int2 *sb = reinterpret_cast<const int2 *>(a.scratch + (4 * 32 + SORT_MIRRORS * 16) * N);
 	const int *si = reinterpret_cast<const int *>(a.scratch + (4 * 32 + SORT_MIRRORS * 16 + 8) * N);
-	for(int k = blockIdx.x * LIST_TPB + threadIdx.x; k < a.N; k += gridDim.x * LIST_TPB) {
+	for(int k = me.id * LIST_TPB + threadIdx.x; k < a.N; k += me.n * LIST_TPB) {
 #pragma unroll
 		for(int t = 0; t < 4; t++) a.st[t][k] = sd[t * N + k];
 #pragma unroll
@@ -413,8 +489,8 @@ __device__ __forceinline__ void phase_sort_scatter(const ListArgs &a) {
 	}
 }
 
-__device__ __forceinline__ void phase_sorted_copies(const ListArgs &a) {
-	for(int p = blockIdx.x * LIST_TPB + threadIdx.x; p < a.N; p += gridDim.x * LIST_TPB)
+__device__ __forceinline__ void phase_sorted_copies(const ListArgs &a, const volatile Member &me) {
+	for(int p = me.id * LIST_TPB + threadIdx.x; p < a.N; p += me.n * LIST_TPB)
 		if(rebuilt(a, sys_of(a, p))) sorted_copy(a, p, a.cell_list[p]);
 }
 
@@ -425,12 +501,8 @@ __device__ __forceinline__ void phase_sorted_copies(const ListArgs &a) {
 // systems of a batch of 96 landed on 40 of 152 SMs and each group of lanes skipped a dozen nucleotides:
 // 21 us for their rows; so: 12.6).  For batches of up to a block's threads; else all nucleotides, tested.
 struct StaleSystems {
-	int n, total;
-	int first[LIST_TPB], end[LIST_TPB];
-};
-struct Stale {
 	int n, total;  // systems (0: all nucleotides), nucleotides
-	const int *first, *end;
+	int first[LIST_TPB], end[LIST_TPB];
 	// the v-th nucleotide
 	__device__ __forceinline__ int operator[](int v) const {
 		if(n == 0) return v;
@@ -444,8 +516,12 @@ struct Stale {
 	}
 };
 
-__device__ __forceinline__ Stale list_stale_systems(const ListArgs &a, StaleSystems &y) {
-	if(a.n_systems < 2 || !a.sys || !a.sys_stale || !a.sys_off || a.n_systems > LIST_TPB) return Stale{0, a.N, nullptr, nullptr};
+// into shared memory; a barrier has to follow
+__device__ __forceinline__ void list_stale_systems(const ListArgs &a, StaleSystems &y) {
+	if(a.n_systems < 2 || !a.sys || !a.sys_stale || !a.sys_off || a.n_systems > LIST_TPB) {
+		if(threadIdx.x == 0) y.n = 0, y.total = a.N;
+		return;
+	}
 	__shared__ int wt[32];
 	const int s = threadIdx.x;
 	const bool on = s < a.n_systems && rebuilt(a, s);
@@ -455,8 +531,6 @@ __device__ __forceinline__ Stale list_stale_systems(const ListArgs &a, StaleSyst
 	const int end = block_incl_scan(size, wt);
 	if(on) y.first[k - 1] = first, y.end[k - 1] = end;
 	if(s == LIST_TPB - 1) y.n = k, y.total = end;
-	__syncthreads();
-	return Stale{y.n, y.total, y.first, y.end};
 }
 
 // ---------------------------------------------------------------- phases: rows
@@ -520,7 +594,7 @@ __device__ __forceinline__ void put(int *rows, bool col_major, long long N, int 
 // warp reach those tests at different times and run them one after the other: 120 M warp instructions
 // for 250,000 nucleotides.)
 template <int K>
-__device__ __forceinline__ void phase_rows(const ListArgs &a, const Stale &stale) {
+__device__ __forceinline__ void phase_rows(const ListArgs &a, const volatile Member &me, const StaleSystems &stale) {
 	constexpr int G = LIST_TPB / K;
 	__shared__ int2 kept[G][2 * K + 1];  // (place in the cell-sorted order, nucleotide); odd stride
 	const int lane = threadIdx.x & 31, sub = lane % K, grp = (int) threadIdx.x / K;
@@ -530,8 +604,7 @@ __device__ __forceinline__ void phase_rows(const ListArgs &a, const Stale &stale
 	const long long N = a.N;
 	// neighbouring nucleotides to the groups of a block (their rows' entries share sectors); where every
 	// group gets one at most, to different blocks
-	const int total_n = stale.total, stride = gridDim.x * G;
-	for(int v = total_n <= stride ? grp * gridDim.x + blockIdx.x : blockIdx.x * G + grp; v < total_n; v += stride) {  // group-uniform
+	for(int v = stale.total <= me.n * G ? grp * me.n + me.id : me.id * G + grp; v < stale.total; v += me.n * G) {  // group-uniform
 		const int i = stale[v];
 		const int sy = sys_of(a, i);
 		if(!rebuilt(a, sy)) continue;
@@ -669,12 +742,12 @@ __device__ __forceinline__ void phase_rows(const ListArgs &a, const Stale &stale
 // search of the partner's list reads four entries at a time (a serial walk is a chain of dependent
 // loads).  Their order within the group does not matter to the results.  A group that straddles systems
 // is rebuilt if one of them is: the other lists are as they were.
-__device__ __forceinline__ void phase_own(const ListArgs &a) {
+__device__ __forceinline__ void phase_own(const ListArgs &a, const volatile Member &me) {
 	constexpr int T = 4 * PAIR_GROUP, B = LIST_TPB / T;  // threads of a group, groups of a block
 	__shared__ int count[B];
 	const long long N = a.N;
 	const int w = (int) threadIdx.x / T, t = (int) threadIdx.x % T, groups = (a.N + PAIR_GROUP - 1) / PAIR_GROUP;
-	for(int g0 = blockIdx.x * B; g0 < groups; g0 += gridDim.x * B) {
+	for(int g0 = me.id * B; g0 < groups; g0 += me.n * B) {
 		const int g = g0 + w, i = g * PAIR_GROUP + t / 4;
 		if(t == 0) count[w] = 0;
 		__syncthreads();
@@ -713,80 +786,84 @@ __device__ __forceinline__ void phase_own(const ListArgs &a) {
 
 // ---------------------------------------------------------------- the build
 
-// the phases of a build; false if a barrier gave up
+// the phases of a build; false if a wait ran out
 template <int K>
 __device__ __forceinline__ bool list_phases(const ListArgs &a, int n_cells) {
-	__shared__ StaleSystems stale_systems;
-	const Stale stale = list_stale_systems(a, stale_systems);
-	if(a.local_cells) {
-		for(int k = blockIdx.x; k < a.n_systems; k += gridDim.x)
+	__shared__ StaleSystems stale;
+	__shared__ volatile Member me;
+	const bool joined = first_phase(a, me, [&](int item) {
+		if(!a.local_cells) return phase_count(a, item);
+		for(int k = item; k < a.n_systems; k += gridDim.x)
 			if(rebuilt(a, k)) system_cells(a, k);
-		if(!grid_sync(a)) return false;
-	}
-	else {
-		phase_count(a);
-		if(!grid_sync(a)) return false;
-		phase_block_sum(a, n_cells, [&](int c) { return cell_size(a, c); });
-		if(!grid_sync(a)) return false;
-		phase_scan(a, n_cells, [&](int c) { return cell_size(a, c); }, [&](int c, int start) {
+	}, [&] { list_stale_systems(a, stale); });
+	if(!joined) return false;
+	if(me.n == 0) return true;
+	if(!a.local_cells) {
+		auto sync = [&] { return members_sync(a, me); };
+		phase_block_sum(a, me, n_cells, [&](int c) { return cell_size(a, c); });
+		if(!sync()) return false;
+		phase_scan(a, me, n_cells, [&](int c) { return cell_size(a, c); }, [&](int c, int start) {
 			a.cell_start[c] = start;
 			if(c == n_cells) return;
 			a.cell_cursor[c] = start;
 			a.cell_count[c] = 0;  // for the next build (cells of systems that are not rebuilt hold zero)
 		});
-		if(!grid_sync(a)) return false;
-		phase_scatter(a);
-		if(!grid_sync(a)) return false;
-		{
-			const bool sorting = sort_now(a);
-			phase_rank(a, !sorting);
-			if(!grid_sync(a)) return false;
-			if(sorting) {
-				if(a.cell_hil) {
-					for(int c = blockIdx.x * LIST_TPB + threadIdx.x; c < n_cells; c += gridDim.x * LIST_TPB)
-						a.hcount[a.cell_hil[c]] = a.cell_start[c + 1] - a.cell_start[c];
-					if(!grid_sync(a)) return false;
-					phase_block_sum(a, n_cells, [&](int c) { return a.hcount[c]; });
-					if(!grid_sync(a)) return false;
-					phase_scan(a, n_cells, [&](int c) { return a.hcount[c]; }, [&](int c, int start) { a.hstart[c] = start; });
-					if(!grid_sync(a)) return false;
-				}
-				phase_sort_perm(a);
-				if(!grid_sync(a)) return false;
-				phase_sort_gather(a);
-				if(!grid_sync(a)) return false;
-				phase_sort_scatter(a);
-				if(!grid_sync(a)) return false;
-				phase_sorted_copies(a);
-				if(!grid_sync(a)) return false;
+		if(!sync()) return false;
+		phase_scatter(a, me);
+		if(!sync()) return false;
+		const bool sorting = sort_now(a);
+		phase_rank(a, me, !sorting);
+		if(!sync()) return false;
+		if(sorting) {
+			if(a.cell_hil) {
+				for(int c = me.id * LIST_TPB + threadIdx.x; c < n_cells; c += me.n * LIST_TPB)
+					a.hcount[a.cell_hil[c]] = a.cell_start[c + 1] - a.cell_start[c];
+				if(!sync()) return false;
+				phase_block_sum(a, me, n_cells, [&](int c) { return a.hcount[c]; });
+				if(!sync()) return false;
+				phase_scan(a, me, n_cells, [&](int c) { return a.hcount[c]; }, [&](int c, int start) { a.hstart[c] = start; });
+				if(!sync()) return false;
 			}
+			phase_sort_perm(a, me);
+			if(!sync()) return false;
+			phase_sort_gather(a, me);
+			if(!sync()) return false;
+			phase_sort_scatter(a, me);
+			if(!sync()) return false;
+			phase_sorted_copies(a, me);
+			if(!sync()) return false;
 		}
 	}
-	phase_rows<K>(a, stale);
+	phase_rows<K>(a, me, stale);
 	if(a.own) {
-		if(!grid_sync(a)) return false;
-		phase_own(a);
+		if(!members_sync(a, me)) return false;
+		phase_own(a, me);
 	}
 	return true;
 }
 
 template <int K>
 __global__ void __launch_bounds__(LIST_TPB, 1) k_list_build(ListArgs a, int n_cells) {
-	pdl_trigger();  // (every block is running: the next kernel's blocks wait for this one's end)
+	pdl_trigger();  // (the next kernel's blocks wait for this one's end)
 	pdl_wait();
 	if(a.check_flag && *(volatile const int *) a.flag == 0) return;
-	const bool barred = __syncthreads_or(threadIdx.x == 0 && *(volatile const unsigned *) &a.sync->failed != 0);
-	if(barred || !list_phases<K>(a, n_cells)) {
-		if(threadIdx.x == 0) atomicOr(a.status, OXGB_ERR_SYNC);
-		return;
-	}
-	// the last block to finish counts the build and clears the requests
+	const bool whole = list_phases<K>(a, n_cells);
+	// the last block to leave clears the barrier, and after a whole build counts it and clears the requests
 	__shared__ int last;
 	__syncthreads();
 	if(threadIdx.x == 0) {
+		if(!whole) atomicOr(a.status, OXGB_ERR_SYNC);
 		__threadfence();
-		last = gridDim.x == 1 || atomicAdd(&a.sync->count, 1u) == gridDim.x - 1;
-		if(last) a.sync->count = 0;
+		last = 1;
+		if(gridDim.x > 1) {
+			const unsigned left = atomicAdd(&a.sync->left, whole ? 1u : ROLL_ONE + 1);
+			last = (left & (ROLL_ONE - 1)) == gridDim.x - 1;
+			if(last) {
+				if(!whole || left >= ROLL_ONE) last = 0;
+				a.sync->roll = last ? 0 : ROLL_CLOSED | ROLL_FAILED;
+				a.sync->done = a.sync->members = a.sync->count = a.sync->left = 0;
+			}
+		}
 	}
 	__syncthreads();
 	if(!last) return;
@@ -799,21 +876,17 @@ __global__ void __launch_bounds__(LIST_TPB, 1) k_list_build(ListArgs a, int n_ce
 
 template <int K>
 static cudaError_t launch_build(const ListArgs &a, int n_cells, cudaStream_t s) {
-	// all blocks resident together: one per SM (the occupancy of this kernel), fewer where the
-	// nucleotides do not fill them
+	// a block per SM (it takes the SM's registers), fewer where the nucleotides do not fill them
 	static std::atomic<int> sms[64];  // per device (whoever comes first; the same value)
 	int dev = 0;
 	cudaError_t e = cudaGetDevice(&dev);
 	if(e != cudaSuccess) return e;
 	if(dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
 	if(sms[dev].load() == 0) {
-		int n = 0, per = 0;
+		int n = 0;
 		if((e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
 		if((e = cudaFuncSetAttribute(k_list_build<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, LIST_LOCAL_SMEM)) != cudaSuccess)
 			return e;
-		if((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_list_build<K>, LIST_TPB, LIST_LOCAL_SMEM)) != cudaSuccess)
-			return e;
-		if(per < 1) return cudaErrorCooperativeLaunchTooLarge;
 		sms[dev].store(std::min(n, LIST_MAX_BLOCKS));
 	}
 	const long long threads = std::max((long long) a.N * K, (long long) n_cells / 8);
@@ -823,13 +896,11 @@ static cudaError_t launch_build(const ListArgs &a, int n_cells, cudaStream_t s) 
 	cfg.blockDim = dim3(LIST_TPB);
 	cfg.dynamicSmemBytes = a.local_cells ? LIST_LOCAL_SMEM : 0;
 	cfg.stream = s;
-	cudaLaunchAttribute at[2];
-	at[0].id = cudaLaunchAttributeCooperative;
-	at[0].val.cooperative = 1;
-	at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-	at[1].val.programmaticStreamSerializationAllowed = 1;
+	cudaLaunchAttribute at[1];
+	at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	at[0].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = at;
-	cfg.numAttrs = a.pdl ? 2 : 1;
+	cfg.numAttrs = a.pdl ? 1 : 0;
 	return cudaLaunchKernelEx(&cfg, k_list_build<K>, a, n_cells);
 }
 
