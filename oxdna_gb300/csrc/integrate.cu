@@ -394,11 +394,11 @@ __global__ void __launch_bounds__(64 * W, 16 / W) k_first_step(StepArgs a) {
 
 // ---------------------------------------------------------------- thermostats
 
-// the Bussi draws of the blockIdx.y-th step from this one on for system blockIdx.x: warp 0
-// translational (channel 0), warp 1 rotational (channel 1)
+// the Bussi draws of one system and step (step after step from this one on, systems together; one dimension, as
+// the grid's others hold 65,535): warp 0 translational (channel 0), warp 1 rotational (channel 1)
 __global__ void k_bussi_noise(StepArgs a) {
-	const long long s = step_of(a.th) + blockIdx.y;
-	const int sy = blockIdx.x;
+	const int k = blockIdx.x / a.th.n_systems, sy = blockIdx.x % a.th.n_systems;
+	const long long s = step_of(a.th) + k;
 	if(s % a.th.newtonian_steps != 0 || (threadIdx.x & 31) != 0) return;
 	const int w = threadIdx.x >> 5;
 	if(w > 1) return;
@@ -407,7 +407,7 @@ __global__ void k_bussi_noise(StepArgs a) {
 	rs.init(a.th.sys_seed[sy], s, (unsigned) w);
 	double sum, rr;
 	bussi_draws(rs, w == 0 ? 3 * (n - 1) : 3 * n, sum, rr);
-	double *to = a.th.bussi_draws + 4 * ((size_t) blockIdx.y * a.th.n_systems + sy) + 2 * w;
+	double *to = a.th.bussi_draws + 4 * ((size_t) k * a.th.n_systems + sy) + 2 * w;
 	to[0] = sum;
 	to[1] = rr;
 }
@@ -773,7 +773,7 @@ cudaError_t launch_first_step(const StepArgs &a, bool double_forces, cudaStream_
 }
 
 cudaError_t launch_bussi_noise(const StepArgs &a, int steps, cudaStream_t s) {
-	k_bussi_noise<<<dim3(a.th.n_systems, steps), 64, 0, s>>>(a);
+	k_bussi_noise<<<a.th.n_systems * steps, 64, 0, s>>>(a);
 	return cudaGetLastError();
 }
 
