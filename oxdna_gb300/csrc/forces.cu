@@ -1321,7 +1321,7 @@ __global__ void __launch_bounds__(128, MINB) k_nonbonded_mixed(ForceArgs a, Spli
 				const int4 q = qn;
 				if(k + K < ndh) qn = __ldg(a.site_back + jn);
 				if(k + 2 * K < ndh) jn = a.dh_nb[(long long) (k + 2 * K) * N + i];
-				const float x = (float) (q.x - pk.x), y = (float) (q.y - pk.y), z = (float) (q.z - pk.z);
+				const float x = (float) fixed_sep(q.x, pk.x), y = (float) fixed_sep(q.y, pk.y), z = (float) fixed_sep(q.z, pk.z);
 				const float r2 = (x * x + y * y + z * z) * u2;
 				if(r2 < D.rc2) {
 					float e;
@@ -1348,7 +1348,7 @@ __global__ void __launch_bounds__(128, MINB) k_nonbonded_mixed(ForceArgs a, Spli
 					t3 = float(EVc<3>::RC * EVc<3>::RC) * m * iu2;
 		static_assert(EVc<3>::RC == EVc<4>::RC, "one threshold for backbone-base");
 		auto sq = [](const int4 &p, const int4 &q) {
-			const float x = (float) (q.x - p.x), y = (float) (q.y - p.y), z = (float) (q.z - p.z);
+			const float x = (float) fixed_sep(q.x, p.x), y = (float) fixed_sep(q.y, p.y), z = (float) fixed_sep(q.z, p.z);
 			return x * x + y * y + z * z;
 		};
 		for(int w0 = 0; w0 < nev; w0 += 64 * K) {

@@ -47,19 +47,19 @@ __device__ __forceinline__ FixedBox fixed_box(const StepArgs &a, int sy) {
 }
 
 // a position (hi + lo) in fixed point
-__device__ __forceinline__ int3 fixed_centre(const FixedBox &b, float3 hi, float3 lo) {
-	return make_int3((int) fixed_coord(hi.x, lo.x, b.box_hi, b.box_lo, b.inv_box, b.s_hi, b.s_lo),
-			(int) fixed_coord(hi.y, lo.y, b.box_hi, b.box_lo, b.inv_box, b.s_hi, b.s_lo),
-			(int) fixed_coord(hi.z, lo.z, b.box_hi, b.box_lo, b.inv_box, b.s_hi, b.s_lo));
+__device__ __forceinline__ uint3 fixed_centre(const FixedBox &b, float3 hi, float3 lo) {
+	return make_uint3(fixed_coord(hi.x, lo.x, b.box_hi, b.box_lo, b.inv_box, b.s_hi, b.s_lo),
+			fixed_coord(hi.y, lo.y, b.box_hi, b.box_lo, b.inv_box, b.s_hi, b.s_lo),
+			fixed_coord(hi.z, lo.z, b.box_hi, b.box_lo, b.inv_box, b.s_hi, b.s_lo));
 }
 
 // the fixed-point backbone and base sites of nucleotide i, from its position, its FP32 backbone offset
 // and a1 (base site at 0.4 a1)
-__device__ __forceinline__ void mirror_sites(const StepArgs &a, int i, const FixedBox &b, int3 c, float3 a1, float4 back) {
+__device__ __forceinline__ void mirror_sites(const StepArgs &a, int i, const FixedBox &b, uint3 c, float3 a1, float4 back) {
 	const float s2 = 2.f * b.s_hi, sb = 0.4f * s2;
-	a.site_back[i] = make_int4(c.x + fixed_round(back.x * s2), c.y + fixed_round(back.y * s2), c.z + fixed_round(back.z * s2),
+	a.site_back[i] = make_int4(fixed_site(c.x, back.x * s2), fixed_site(c.y, back.y * s2), fixed_site(c.z, back.z * s2),
 			back.w != 0.f);
-	a.site_base[i] = make_int4(c.x + fixed_round(a1.x * sb), c.y + fixed_round(a1.y * sb), c.z + fixed_round(a1.z * sb), 0);
+	a.site_base[i] = make_int4(fixed_site(c.x, a1.x * sb), fixed_site(c.y, a1.y * sb), fixed_site(c.z, a1.z * sb), 0);
 }
 
 // returns a1 and the backbone offset (w: the strand-end flag) and with F64 keeps the FP64 engine's frame;
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(64 * W, 16 / W) k_first_step(StepArgs a) {
 	float4 lp, la1, lbk;
 	constexpr bool SITES = sizeof(V4) == sizeof(float4);  // (the double engine has no fixed-point sites)
 	FixedBox fb{};
-	int3 centre = make_int3(0, 0, 0);
+	uint3 centre = make_uint3(0, 0, 0);
 	auto load_state = [&]() {
 		if(live) {
 			sy = a.th.sys[i];

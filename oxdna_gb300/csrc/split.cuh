@@ -312,6 +312,11 @@ OXGB_HD unsigned fixed_coord(float hi, float lo, float box_hi, float box_lo, flo
 	return 2u * (unsigned) i + (unsigned) fixed_round(2.f * OXGB_FADD(OXGB_FSUB(p, (float) i), e));
 }
 
+// a coordinate c and an offset x, both in units, and the separation of two coordinates: modulo the box, so
+// unsigned (past a face the signed sum or difference would be undefined)
+OXGB_HD int fixed_site(unsigned c, float x) { return (int) (c + (unsigned) fixed_round(x)); }
+OXGB_HD int fixed_sep(int to, int from) { return (int) ((unsigned) to - (unsigned) from); }
+
 // The rotation of the unit quaternion q = (x, y, z, w) by the angle dt |L| about the body-frame
 // angular momentum L (hd = dt / 2): q <- q (x) (sin(t/2) L^, cos(t/2)), t = dt |L|, written
 // as q + c with the small correction c = q (x) (delta, eps), delta = k L, eps = cos(t/2) - 1,
