@@ -32,7 +32,8 @@ struct DNA2Table {
 	R box_hi, box_lo;  // box side as an unevaluated sum hi + lo (exact FP64 value)
 	R inv_box;         // about 1 / box_hi: picks the periodic image (an integer; see LoadMixed::sep)
 	R fix_hi, fix_lo;  // 2^31 / box side as hi + lo, and
-	R fix_unit;        // box side / 2^32: the units of the fixed-point sites (fixed_site)
+	R fix_unit, fix_unit_lo;  // box side / 2^32, the units of the fixed-point sites (fixed_site), as hi + lo, and
+	R fix_unit2, fix_unit2_lo;  // its square: a rounded one would scale every distance of the box alike
 	int dh_half_charged_ends, use_mbf, pad0, pad1;
 };
 

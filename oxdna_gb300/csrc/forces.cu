@@ -1302,7 +1302,7 @@ __global__ void __launch_bounds__(128, MINB) k_nonbonded_mixed(ForceArgs a, Spli
 	const int2 bi = a.bonds[i];
 	const float4 back = __ldg(ld.fback + i);
 	if(!EDGE) {
-		const float unit = P.fix_unit, u2 = unit * unit;
+		const float unit = P.fix_unit, unit_lo = P.fix_unit_lo, u2 = P.fix_unit2, u2_lo = P.fix_unit2_lo;
 		const int4 pk = __ldg(a.site_back + i);
 		// Debye-Hueckel (dh_sites) over its rows: the next partner's site is loaded before this
 		// partner's arithmetic, and the index after it one iteration earlier still.  The lever arm of
@@ -1322,10 +1322,10 @@ __global__ void __launch_bounds__(128, MINB) k_nonbonded_mixed(ForceArgs a, Spli
 				if(k + K < ndh) qn = __ldg(a.site_back + jn);
 				if(k + 2 * K < ndh) jn = a.dh_nb[(long long) (k + 2 * K) * N + i];
 				const float x = (float) fixed_sep(q.x, pk.x), y = (float) fixed_sep(q.y, pk.y), z = (float) fixed_sep(q.z, pk.z);
-				const float r2 = (x * x + y * y + z * z) * u2;
+				const float d2 = x * x + y * y + z * z, r2 = fmaf(d2, u2, d2 * u2_lo);
 				if(r2 < D.rc2) {
 					float e;
-					const float s = D.force(r2, pcut * (q.w ? D.half : 1.f), e) * unit;
+					const float s = D.force(r2, pcut * (q.w ? D.half : 1.f), e);  // (per unit: scaled after the sum)
 					f.add(v3<float>{x * s, y * s, z * s});
 					if(ENERGY) {
 						KahanV<float>::kadd(acc.E, acc.Ec, e);
@@ -1333,7 +1333,8 @@ __global__ void __launch_bounds__(128, MINB) k_nonbonded_mixed(ForceArgs a, Spli
 					}
 				}
 			}
-			const v3<float> fs{f.s.x - f.c.x, f.s.y - f.c.y, f.s.z - f.c.z};
+			const v3<float> fu{f.s.x - f.c.x, f.s.y - f.c.y, f.s.z - f.c.z};
+			const v3<float> fs{fmaf(fu.x, unit, fu.x * unit_lo), fmaf(fu.y, unit, fu.y * unit_lo), fmaf(fu.z, unit, fu.z * unit_lo)};
 			acc.F.add(fs);
 			acc.T.add(cross(v3<float>{back.x, back.y, back.z}, fs));
 		}

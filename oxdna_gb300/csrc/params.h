@@ -106,6 +106,7 @@ inline int build_table(const oxgb_dna2_settings &s, double box, DNA2Table<double
 	P.fix_hi = 2147483648.0 / box;
 	P.fix_lo = 0.0;
 	P.fix_unit = box / 4294967296.0;
+	P.fix_unit2 = P.fix_unit * P.fix_unit;
 	return 0;
 }
 
@@ -122,6 +123,8 @@ inline void to_float(const DNA2Table<double> &d, double box, DNA2Table<float> &f
 	f.box_lo = (float) (box - (double) f.box_hi);
 	f.inv_box = (float) (1.0 / (double) f.box_hi);
 	f.fix_lo = (float) (2147483648.0 / box - (double) f.fix_hi);
+	f.fix_unit_lo = (float) (d.fix_unit - (double) f.fix_unit);
+	f.fix_unit2_lo = (float) (d.fix_unit2 - (double) f.fix_unit2);
 }
 
 // pair-distance bounds of the force kernel's term lists: a term can only act within these
