@@ -453,6 +453,7 @@ struct oxgb_md {
 	float4 *pos_hi = nullptr, *pos_lo = nullptr, *fa1 = nullptr, *fa3 = nullptr, *fback = nullptr, *list_pos = nullptr;
 	float4 *fa1lo = nullptr, *fbacklo = nullptr;  // remainders of fa1 / fback (FP32 engines)
 	int4 *site_back = nullptr, *site_base = nullptr;  // fixed-point sites (FP32 engines)
+	bool fixed_sites = false;  // no box above FIXED_BOX_MAX: the force kernels read them
 	float4 *list_a1 = nullptr, *list_back = nullptr;
 	int2 *bonds = nullptr;
 	void *F = nullptr, *T = nullptr, *bond_f = nullptr, *bond_tp = nullptr, *bond_tq = nullptr;
@@ -634,8 +635,8 @@ static ForceArgs force_args(oxgb_md *h, int step_offset = 0, bool engine_step = 
 	a.fback = h->fback;
 	a.fa1lo = h->fa1lo;
 	a.fbacklo = h->fbacklo;
-	a.site_back = h->site_back;
-	a.site_base = h->site_base;
+	a.site_back = h->fixed_sites ? h->site_back : nullptr;
+	a.site_base = h->fixed_sites ? h->site_base : nullptr;
 	a.ev_nb = h->tl.ev_nb;
 	a.ev_n = h->tl.ev_n;
 	a.pt_nb = h->tl.pt_nb;
@@ -900,6 +901,7 @@ extern "C" int oxgb_md_create(int n_systems, const int *offsets, const double *b
 		ok &= cudaMalloc(&h->fbacklo, sizeof(float4) * N) == cudaSuccess;
 		ok &= cudaMalloc(&h->site_back, sizeof(int4) * N) == cudaSuccess;
 		ok &= cudaMalloc(&h->site_base, sizeof(int4) * N) == cudaSuccess;
+		h->fixed_sites = *std::max_element(h->box.begin(), h->box.end()) <= FIXED_BOX_MAX;
 	}
 	else ok &= cudaMalloc(&h->frame64, 4 * sizeof(double4_32a) * N) == cudaSuccess;
 	ok &= cudaMalloc(&h->list_a1, sizeof(float4) * N) == cudaSuccess;

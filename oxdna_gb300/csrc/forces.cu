@@ -1289,7 +1289,31 @@ __global__ void __launch_bounds__(128, 1) k_nonbonded_split(ForceArgs a, Loader 
 // separation is good to one unit, box / 2^32 (5e-8 in a box of 230, where the FP32 difference of the
 // hi parts is off by up to 3.8e-6): Debye-Hueckel's force slope is below 0.1, and the screen's margin
 // is 1e-4.  Contacts are evaluated from the mirrors, refined, as everywhere.
-template <bool SPLIT, bool ENERGY, int K, int MINB = OXGB_NB_MINB, bool EDGE = false>
+// A nucleotide's backbone site, as fixed point, or (FIXED = false), for boxes above FIXED_BOX_MAX, where the
+// unit is coarser than FP32 separations, as hi + lo position and offset, as good at any size of the box.
+template <bool FIXED>
+struct Partner {
+	int4 s;
+	__device__ __forceinline__ void load(const ForceArgs &a, const SplitMixed &, int j) { s = __ldg(a.site_back + j); }
+	__device__ __forceinline__ bool end() const { return s.w != 0; }
+	__device__ __forceinline__ float3 sep(const SplitMixed &, const Partner &q, const DNA2Table<float> &) const {
+		return make_float3((float) fixed_sep(q.s.x, s.x), (float) fixed_sep(q.s.y, s.y), (float) fixed_sep(q.s.z, s.z));
+	}
+};
+template <>
+struct Partner<false> {
+	float4 h, l, b;
+	__device__ __forceinline__ void load(const ForceArgs &, const SplitMixed &ld, int j) {
+		h = __ldg(ld.hi + j), l = __ldg(ld.lo + j), b = __ldg(ld.fback + j);
+	}
+	__device__ __forceinline__ bool end() const { return b.w != 0.f; }
+	__device__ __forceinline__ float3 sep(const SplitMixed &ld, const Partner &q, const DNA2Table<float> &P) const {
+		const v3<float> d = ld.sep(h, l, q.h, q.l, P).plain();
+		return make_float3(d.x + q.b.x - b.x, d.y + q.b.y - b.y, d.z + q.b.z - b.z);
+	}
+};
+
+template <bool SPLIT, bool ENERGY, int K, int MINB = OXGB_NB_MINB, bool EDGE = false, bool FIXED = true>
 __global__ void __launch_bounds__(128, MINB) k_nonbonded_mixed(ForceArgs a, SplitMixed ld) {
 	const long long N = a.N;
 	const int sub = threadIdx.x % K;
@@ -1303,7 +1327,8 @@ __global__ void __launch_bounds__(128, MINB) k_nonbonded_mixed(ForceArgs a, Spli
 	const float4 back = __ldg(ld.fback + i);
 	if(!EDGE) {
 		const float unit = P.fix_unit, unit_lo = P.fix_unit_lo, u2 = P.fix_unit2, u2_lo = P.fix_unit2_lo;
-		const int4 pk = __ldg(a.site_back + i);
+		Partner<FIXED> p;
+		p.load(a, ld, i);
 		// Debye-Hueckel (dh_sites) over its rows: the next partner's site is loaded before this
 		// partner's arithmetic, and the index after it one iteration earlier still.  The lever arm of
 		// every pair's torque on i is i's backbone offset, so the forces are summed (compensated) and
@@ -1313,19 +1338,19 @@ __global__ void __launch_bounds__(128, MINB) k_nonbonded_mixed(ForceArgs a, Spli
 			const DebyeF D(P);
 			const float pcut = back.w != 0.f ? D.half : 1.f;
 			KahanV<float> f{};
-			int4 qn = pk;
+			Partner<FIXED> qn = p;
 			int k = sub;
-			if(k < ndh) qn = __ldg(a.site_back + a.dh_nb[(long long) k * N + i]);
+			if(k < ndh) qn.load(a, ld, a.dh_nb[(long long) k * N + i]);
 			int jn = k + K < ndh ? a.dh_nb[(long long) (k + K) * N + i] : 0;
 			for(; k < ndh; k += K) {
-				const int4 q = qn;
-				if(k + K < ndh) qn = __ldg(a.site_back + jn);
+				const Partner<FIXED> q = qn;
+				if(k + K < ndh) qn.load(a, ld, jn);
 				if(k + 2 * K < ndh) jn = a.dh_nb[(long long) (k + 2 * K) * N + i];
-				const float x = (float) fixed_sep(q.x, pk.x), y = (float) fixed_sep(q.y, pk.y), z = (float) fixed_sep(q.z, pk.z);
-				const float d2 = x * x + y * y + z * z, r2 = fmaf(d2, u2, d2 * u2_lo);
+				const float3 d = p.sep(ld, q, P);
+				const float x = d.x, y = d.y, z = d.z, d2 = x * x + y * y + z * z, r2 = FIXED ? fmaf(d2, u2, d2 * u2_lo) : d2;
 				if(r2 < D.rc2) {
 					float e;
-					const float s = D.force(r2, pcut * (q.w ? D.half : 1.f), e);  // (per unit: scaled after the sum)
+					const float s = D.force(r2, pcut * (q.end() ? D.half : 1.f), e);  // (fixed point: per unit, scaled after the sum)
 					f.add(v3<float>{x * s, y * s, z * s});
 					if(ENERGY) {
 						KahanV<float>::kadd(acc.E, acc.Ec, e);
@@ -1333,8 +1358,8 @@ __global__ void __launch_bounds__(128, MINB) k_nonbonded_mixed(ForceArgs a, Spli
 					}
 				}
 			}
-			const v3<float> fu{f.s.x - f.c.x, f.s.y - f.c.y, f.s.z - f.c.z};
-			const v3<float> fs{fmaf(fu.x, unit, fu.x * unit_lo), fmaf(fu.y, unit, fu.y * unit_lo), fmaf(fu.z, unit, fu.z * unit_lo)};
+			v3<float> fs{f.s.x - f.c.x, f.s.y - f.c.y, f.s.z - f.c.z};
+			if(FIXED) fs = v3<float>{fmaf(fs.x, unit, fs.x * unit_lo), fmaf(fs.y, unit, fs.y * unit_lo), fmaf(fs.z, unit, fs.z * unit_lo)};
 			acc.F.add(fs);
 			acc.T.add(cross(v3<float>{back.x, back.y, back.z}, fs));
 		}
@@ -1342,7 +1367,7 @@ __global__ void __launch_bounds__(128, MINB) k_nonbonded_mixed(ForceArgs a, Spli
 		// pair inside its cutoff, ev_contact: a few in a thousand entries); the pairs found are
 		// evaluated refined after the window, and the others contribute nothing
 		const int nev = live ? min(a.ev_n[i], a.ev_cap) : 0;
-		const int4 pb = __ldg(a.site_base + i);
+		const int4 pb = FIXED ? __ldg(a.site_base + i) : make_int4(0, 0, 0, 0);
 		constexpr float m = 1.0001f;
 		const float iu2 = 1.f / u2;
 		const float t1 = float(EVc<1>::RC * EVc<1>::RC) * m * iu2, t2 = float(EVc<2>::RC * EVc<2>::RC) * m * iu2,
@@ -1358,8 +1383,17 @@ __global__ void __launch_bounds__(128, MINB) k_nonbonded_mixed(ForceArgs a, Spli
 			int n = 0;
 			for(int k = w0 + sub; k < wend; k += K, n++) {
 				const int j = a.ev_nb[(long long) k * N + i];
-				const int4 qk = __ldg(a.site_back + j), qb = __ldg(a.site_base + j);
-				if(sq(pb, qb) < t2 || sq(pk, qb) < t3 || sq(pb, qk) < t3 || sq(pk, qk) < t1) stiff |= 1ull << n;
+				if constexpr(FIXED) {
+					const int4 qk = __ldg(a.site_back + j), qb = __ldg(a.site_base + j);
+					if(sq(pb, qb) < t2 || sq(p.s, qb) < t3 || sq(pb, qk) < t3 || sq(p.s, qk) < t1) stiff |= 1ull << n;
+				}
+				else {
+					Nuc<float> ni, nj;
+					float4 h, l, qh, ql;
+					ld.full(i, ni, h, l);
+					ld.full(j, nj, qh, ql);
+					if(ev_contact(ni, nj, ld.sep(h, l, qh, ql, P).plain())) stiff |= 1ull << n;
+				}
 			}
 			while(stiff) {
 				const int nn = __ffsll((long long) stiff) - 1;
@@ -1895,8 +1929,10 @@ static void launch_split_t(const ForceArgs &a, Loader ld, cudaStream_t s) {
 			pair_blocks);
 	// the non-bonded kernel starts its Debye-Hueckel and excluded-volume work while the tail of
 	// the bonded and pair blocks runs; the external forces follow it the same way
-	auto nonbonded = [] {
-		if constexpr(sizeof(R) == 4) return &k_nonbonded_mixed<SPLIT, ENERGY, K, NBMINB, EDGE>;
+	auto nonbonded = [&] {
+		if constexpr(sizeof(R) == 4 && EDGE) return &k_nonbonded_mixed<SPLIT, ENERGY, K, NBMINB, EDGE>;
+		else if constexpr(sizeof(R) == 4)
+			return a.site_back ? &k_nonbonded_mixed<SPLIT, ENERGY, K, NBMINB> : &k_nonbonded_mixed<SPLIT, ENERGY, K, NBMINB, false, false>;
 		else return &k_nonbonded_split<R, Loader, SPLIT, ENERGY, K, EDGE>;
 	}();
 	launch_after(nonbonded, dim3(nonbonded_blocks(a.N, K)), dim3(tpb), 0, s, a, ld);

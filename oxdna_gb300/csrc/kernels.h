@@ -116,7 +116,8 @@ struct ForceArgs {
 	// (column-major: element k of nucleotide i at [k * N + i]) and the per-bond buffers
 	const float4 *fback;
 	const float4 *fa1lo, *fbacklo;            // remainders of fa1 / fback (null: the FP32 sites unrefined)
-	const int4 *site_back, *site_base;        // fixed-point backbone (w: strand end) and base sites (FP32 engines)
+	const int4 *site_back, *site_base;        // fixed-point backbone (w: strand end) and base sites (FP32 engines,
+	                                          // null with a box above FIXED_BOX_MAX)
 	const int *ev_nb, *ev_n, *pt_nb, *pt_n;
 	int ev_cap, pt_cap;                       // capacities (an overflowed list is read up to them)
 	void *bond_f, *bond_tp, *bond_tq;         // per bond owner p (q = n3[p]): f on q with w = energy, torques
@@ -154,6 +155,12 @@ struct ForceArgs {
 	int edge;
 	void *edge_acc;
 };
+
+// The largest box whose sites the FP32 engines keep in fixed point, in units of box / 2^32.  Against FP64, over
+// 24 systems in boxes of a range each: Debye-Hueckel energy 1.5e-7 to 1.65e-7 up to 2,048 (hi + lo positions
+// 2.2e-7), 2.1e-7 to 8,192, 3.2e-7 to 32,768 and 1.1e-6 beyond; forces 4.07e-7 either way up to 8,192, then 4.07e-7
+// and 4.16e-7.  From some 12,000 on, the sites' error also reaches the margin of the excluded-volume screen.
+constexpr double FIXED_BOX_MAX = 2048.0;
 
 // nucleotides whose owned pair-term entries are kept together (ForceArgs::own)
 constexpr int PAIR_GROUP = 32;
