@@ -1358,10 +1358,12 @@ __global__ void __launch_bounds__(128, MINB) k_nonbonded_mixed(ForceArgs a, Spli
 					}
 				}
 			}
-			v3<float> fs{f.s.x - f.c.x, f.s.y - f.c.y, f.s.z - f.c.z};
-			if(FIXED) fs = v3<float>{fmaf(fs.x, unit, fs.x * unit_lo), fmaf(fs.y, unit, fs.y * unit_lo), fmaf(fs.z, unit, fs.z * unit_lo)};
-			acc.F.add(fs);
-			acc.T.add(cross(v3<float>{back.x, back.y, back.z}, fs));
+			const v3<float> fs{f.s.x - f.c.x, f.s.y - f.c.y, f.s.z - f.c.z};
+			auto scaled = [&](const v3<float> &v) {
+				return FIXED ? v3<float>{fmaf(v.x, unit, v.x * unit_lo), fmaf(v.y, unit, v.y * unit_lo), fmaf(v.z, unit, v.z * unit_lo)} : v;
+			};
+			acc.F.add(scaled(fs));
+			acc.T.add(scaled(cross(v3<float>{back.x, back.y, back.z}, fs)));
 		}
 		// Excluded volume over its list: each window of 64 of the lane's entries is screened (a site
 		// pair inside its cutoff, ev_contact: a few in a thousand entries); the pairs found are
