@@ -50,16 +50,6 @@ inline cudaError_t launch_after(void (*kernel)(KArgs...), dim3 grid, dim3 block,
 // (the redraw probabilities SP_PT and SP_PR as draw_threshold gives them)
 enum { SP_T = 0, SP_SQRTT, SP_PT, SP_PR, SP_1MC, SP_A, SP_B, SP_INVN, SP_STRIDE = 8 };
 
-// A probability p as the number of 32-bit draws x with (x + 1) / 2^32 < p, in the bits of a double (one
-// of a table of doubles): the test of a draw is then one of integers, the same to the last draw.
-inline double draw_threshold(double p) {
-	const double c = std::ceil(p * 4294967296.0) - 1.0;
-	const unsigned long long n = c > 0.0 ? (unsigned long long) c : 0ull;
-	double bits;
-	std::memcpy(&bits, &n, sizeof bits);
-	return bits;
-}
-
 // Every engine handles a batch of independent systems packed one after the other (a plain run
 // is a batch of one): nucleotide i belongs to system sys[i], whose nucleotides are
 // sys_off[s] .. sys_off[s + 1] - 1.  The random streams are keyed by (system seed, step, index

@@ -317,6 +317,29 @@ OXGB_HD unsigned fixed_coord(float hi, float lo, float box_hi, float box_lo, flo
 OXGB_HD int fixed_site(unsigned c, float x) { return (int) (c + (unsigned) fixed_round(x)); }
 OXGB_HD int fixed_sep(int to, int from) { return (int) ((unsigned) to - (unsigned) from); }
 
+// ---------------------------------------------------------------- redraw probabilities
+
+// A probability p as the number of 32-bit draws x with (x + 1) / 2^32 < p, in the bits of a double (one
+// of a table of doubles): the test of a draw is then one of integers, the same to the last draw.
+inline double draw_threshold(double p) {
+	const double c = std::ceil(p * 4294967296.0) - 1.0;
+	const unsigned long long n = !(c > 0.0) ? 0ull : c < 4294967296.0 ? (unsigned long long) c : 4294967296ull;
+	double bits;
+	std::memcpy(&bits, &n, sizeof bits);
+	return bits;
+}
+
+// (x + 1) / 2^32 < p for a probability given as its threshold
+OXGB_HD bool drawn(unsigned x, double threshold) {
+#ifdef __CUDA_ARCH__
+	return (unsigned long long) x < (unsigned long long) __double_as_longlong(threshold);
+#else
+	unsigned long long n;
+	std::memcpy(&n, &threshold, sizeof n);
+	return x < n;
+#endif
+}
+
 // The rotation of the unit quaternion q = (x, y, z, w) by the angle dt |L| about the body-frame
 // angular momentum L (hd = dt / 2): q <- q (x) (sin(t/2) L^, cos(t/2)), t = dt |L|, written
 // as q + c with the small correction c = q (x) (delta, eps), delta = k L, eps = cos(t/2) - 1,

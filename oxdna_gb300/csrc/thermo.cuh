@@ -44,11 +44,6 @@ static __device__ __noinline__ double2 box_muller(unsigned ua, unsigned ub) {
 	return make_double2(r * c, r * s);
 }
 
-// u01(x) < p for a probability given as its threshold (draw_threshold): the same test on integers
-static __device__ __forceinline__ bool drawn(unsigned x, double threshold) {
-	return (unsigned long long) x < (unsigned long long) __double_as_longlong(threshold);
-}
-
 #define RNG_BROWNIAN 0x42524f57u
 #define RNG_BUSSI 0x42555353u
 
