@@ -375,15 +375,15 @@ int oxgb_md_info(oxgb_md *h, long long *n_rebuilds, long long *step, int *max_ne
 int oxgb_md_storage_order(oxgb_md *h, int *id);
 /* status bits raised by the kernels since the last call (and clears them): 0 = healthy */
 int oxgb_md_status(oxgb_md *h);
-/* the shape of the MD step's force kernels: nucleotides per pair-block warp queue, non-bonded
- * lanes per nucleotide, the register cap as resident blocks per SM, and (autotuned engines) the
+/* the shape of the MD step's force kernels: pair-block size (32: three groups of 32 nucleotides per
+ * block, 16: six, from 65,000 nucleotides on; one below, either way), non-bonded lanes per nucleotide, the register cap as resident blocks per SM, and (autotuned engines) the
  * measured launch time in microseconds (0 otherwise).  No counterpart in the reference. */
 int oxgb_md_force_shape(oxgb_md *h, int *pair_npw, int *nb_lanes, int *nb_min_blocks, double *launch_us);
 /* pins shape k (0 .. 5; 0 the default) of the MD step's force kernels, e.g. to repeat a tuned run
  * on another engine; the forces of the current state are recomputed with it.  No counterpart in
  * the reference. */
 int oxgb_md_set_force_shape(oxgb_md *h, int k);
-/* the shape table itself: shape k's nucleotides per pair-block warp queue, non-bonded lanes per
+/* the shape table itself: shape k's pair-block size, non-bonded lanes per
  * nucleotide and register cap (OXGB_E_INVALID past the last shape) */
 int oxgb_force_shape_table(int k, int *pair_npw, int *nb_lanes, int *nb_min_blocks);
 /* the lanes per nucleotide of the engine's list builds: OXGB_LIST_WARP, _THREAD or _GROUP4/8/16 */

@@ -1141,13 +1141,14 @@ static int compute_forces_now(oxgb_md *h) {
 
 // ---------------------------------------------------------------- autotuner
 //
-// The MD step's force kernels come in a few shapes (nucleotides per pair-block warp queue,
+// The MD step's force kernels come in a few shapes (pair-block size,
 // non-bonded lanes per nucleotide and register cap; force_shape_of).  With md.autotune the first
 // state uploaded picks one: every shape runs the step's force evaluation on that state (its own
 // lists and tables), timed with CUDA events on the engine's stream (median of 3 rounds of 10
 // launches after 2 warm-up launches), and the fastest is kept for the engine's life.  The choice
-// is cached per size class (precision, log2 of the nucleotide count, log2 of the mean system
-// size), so engines of the same class reuse it without timing.
+// is cached per size class (precision and form of the sites, log2 of the nucleotide count and the range
+// of sizes in which the shapes stand for the same kernels, log2 of the mean system size), so engines of the same
+// class reuse it without timing.  Shapes that stand for the same kernels are timed once.
 
 static std::mutex g_tune_mutex;
 struct TuneResult {
@@ -1155,7 +1156,7 @@ struct TuneResult {
 	double shape_us;
 	int list_kind;  // -1: not timed (the engine keeps its own choice)
 };
-static std::map<std::tuple<int, int, int>, TuneResult> g_tune_cache;
+static std::map<std::tuple<int, int, int, int>, TuneResult> g_tune_cache;
 
 static int ilog2(long long v) {
 	int k = 0;
@@ -1170,7 +1171,7 @@ static int read_status(oxgb_md *h);
 
 static int autotune_shape(oxgb_md *h) {
 	if(h->dbl || h->tuned) return OXGB_OK;
-	const auto key = std::make_tuple(h->md.precision, ilog2(h->N), ilog2(h->N / h->n_systems));
+	const auto key = std::make_tuple(2 * h->md.precision + (h->fixed_sites ? 1 : 0), ilog2(h->N), force_shape_range(h->N), ilog2(h->N / h->n_systems));
 	{
 		std::lock_guard<std::mutex> lock(g_tune_mutex);
 		auto it = g_tune_cache.find(key);
@@ -1188,6 +1189,7 @@ static int autotune_shape(oxgb_md *h) {
 	int best = 0;
 	double best_us = 1e30;
 	for(int k = 0; k < force_shape_count(); k++) {
+		if(!force_shape_distinct(k, h->N)) continue;
 		ForceArgs fa = force_args(h);
 		fa.shape = k;
 		for(int w = 0; w < 2; w++) CK(launch_forces_split(fa, false, false, false, h->stream));

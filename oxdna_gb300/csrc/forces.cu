@@ -1453,7 +1453,8 @@ int nonbonded_blocks(int N, int lanes) {
 }
 
 // The shapes of the MD step's force kernels (engine, mixed and float precision) the autotuner
-// chooses among: the pair blocks' size (32: three groups, 16: six, see launch_md_shape), lanes per nucleotide in the non-bonded
+// chooses among: the pair blocks' size (npw 32: three groups, 16: six, from PAIR_WIDE_N nucleotides on; below it one
+// either way, see launch_md_shape), lanes per nucleotide in the non-bonded
 // kernel and the resident blocks per SM its register cap asks for.  Shape 0 is the default, the
 // best of hand sweeps on the 40k and 250k workloads.
 struct ForceShapeDef {
@@ -1954,6 +1955,15 @@ constexpr int PAIR_WIDE_N = 65000;
 // 256 threads, us per step: 24 nucleotides 18.1, 16.7, 14.9, 1,000 duplex nucleotides 20.4, 17.0, 15.6; 128 and 256: 5,000:
 // 22.4, 19.3, 8,000: 22.8, 20.1, 12,000: 24.1, 23.4, 16,000: 25.2, 27.8; 10,000 strand nucleotides 17.4, 17.6.
 constexpr bool pair_small(int N) { return N / 32 + N / 128 <= 3 * 152; }
+// the three ranges of N in which a shape stands for different kernels, and whether shape k's differ there from
+// those of the shapes before it (below PAIR_WIDE_N the groups are one whatever npw)
+int force_shape_range(int N) { return pair_small(N) ? 0 : N < PAIR_WIDE_N ? 1 : 2; }
+bool force_shape_distinct(int k, int N) {
+	if(N >= PAIR_WIDE_N) return true;
+	for(int u = 0; u < k; u++)
+		if(FORCE_SHAPES[u].lanes == FORCE_SHAPES[k].lanes && FORCE_SHAPES[u].minb == FORCE_SHAPES[k].minb) return false;
+	return true;
+}
 template <int k>
 static void launch_md_shape(const ForceArgs &a, const SplitMixed &ld, cudaStream_t s) {
 	constexpr ForceShapeDef d = FORCE_SHAPES[k];

@@ -179,9 +179,14 @@ cudaError_t launch_forces_split(const ForceArgs &a, bool dbl, bool split, bool e
 // blocks of the split non-bonded kernel for N nucleotides at `lanes` lanes per nucleotide
 int nonbonded_blocks(int N, int lanes);
 // shapes of the MD step's force kernels (mixed / float engine, ForceArgs::shape): how many, and
-// shape k's nucleotides per pair-block warp queue, non-bonded lanes per nucleotide and register cap
+// shape k's pair-block size (npw 32 or 16: three or six groups of 32 nucleotides per block in large systems),
+// non-bonded lanes per nucleotide and register cap
 int force_shape_count();
 void force_shape_of(int k, int *npw, int *lanes, int *minb);
+// the range of sizes, of three, in which the shapes stand for the same kernels, and whether shape k's there are other
+// than those of the shapes before it
+int force_shape_range(int N);
+bool force_shape_distinct(int k, int N);
 
 // the blocks of a list build (all zero before the first one), each counter in a line of its own: who takes part
 // (roll, done, members; lists.cu), the members' barrier (count, gen), and the blocks that have left.  After a build
