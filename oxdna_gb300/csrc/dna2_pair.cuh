@@ -822,8 +822,8 @@ OXGB_HD bool dh_sites(const DNA2Table<R> &P, const v3<R> &rback, bool p_end, boo
 	if constexpr(sizeof(R) == 8) {
 		// one reciprocal square root instead of a square root and three divisions, each some ten operations
 		// of the FP64 pipe, which is what bounds the FP64 kernels
-		const R v = m_rsqrt(rb2), r = rb2 * v;
-		if(!(r < P.dh_rc)) return false;
+		const R v = m_rsqrt(rb2), r = rb2 * v;  // (coincident sites: not a number, and so is the energy)
+		if(r >= P.dh_rc) return false;
 		R s;
 		if(r < P.dh_rhigh) {
 			const R ex = P.dh_prefactor * m_exp(P.dh_minus_kappa * r) * cut * v;
