@@ -875,8 +875,8 @@ extern "C" int oxgb_md_create(int n_systems, const int *offsets, const double *b
 	h->sys_chunk0[n_systems] = h->n_chunks;
 	int tab_span = 1;
 	for(int b = 0; b < N; b += 128) tab_span = std::max(tab_span, sys[std::min(N, b + 128) - 1] - sys[b] + 1);
-	// the double engine takes at most 78 systems in 128 consecutive nucleotides
-	if(h->dbl && tab_span > 78) return bail(fail(OXGB_E_INVALID, "systems too small: one block would need the tables of " + std::to_string(tab_span) + " systems"));
+	// (the tables of more did not fit a block's shared memory, where they were once kept; still refused)
+	if(h->dbl && tab_span > 78) return bail(fail(OXGB_E_INVALID, "systems too small: the double engine takes at most 78 of them in 128 consecutive nucleotides, not " + std::to_string(tab_span)));
 	std::vector<unsigned long long> seeds(n_systems);
 	for(int k = 0; k < n_systems; k++) seeds[k] = h->md.seed + (unsigned long long) k;
 

@@ -607,6 +607,10 @@ OXGB_HD void pair_ev(const Nuc<R> &p, const Nuc<R> &q, const Sep<R> &sep, PairOu
 	}
 }
 
+// The pair terms written out for one pair, as far as pair_stack: the form with the fewest operations, which the FLOP
+// count of the roofline takes (flopcount.cpp).  The force kernels evaluate the same factors in stages, eight lanes
+// per term (pair_radial, pair_angles, pair_sums in forces.cu).
+//
 // The base-base vector of a pair and the cosines of its angles, shared by hydrogen bonding and
 // cross stacking (DNAInteraction.cpp:779-1021), with which of the two can be non-zero: each
 // needs its distance window and every angular factor inside its support (f4_may; else the term

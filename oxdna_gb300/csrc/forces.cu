@@ -220,12 +220,12 @@ cudaError_t launch_order_params(int mode, const float4 *poss, const float4 *quat
 //
 // A nucleotide has ~20-30 neighbours, only a few of them close enough for hydrogen bonding, cross or
 // coaxial stacking.  The split path
-//  * evaluates every bonded pair once, one thread per bond, for both nucleotides;
-//  * runs the non-bonded terms one thread per nucleotide, one loop per term over the term
-//    lists of the Verlet build (full rows for Debye-Hueckel, centre-close pairs for the
-//    excluded volume, base-close pairs for hydrogen bonding + cross stacking, stack-close
-//    pairs for coaxial stacking), so all lanes of a warp run the same term code;
-//  * gathers the bonded results in the non-bonded kernel's epilogue (fixed order, no atomics).
+//  * evaluates every bonded pair once, for both nucleotides, by two threads in different warps (bonded_block);
+//  * evaluates hydrogen bonding, cross and coaxial stacking once per pair of the pair-term lists, for both
+//    nucleotides, in stages with eight lanes per term (pair_block);
+//  * runs Debye-Hueckel and the excluded volume from both ends of a pair, K lanes per nucleotide over lists of
+//    their own (pairs whose sites can come into reach before the next build);
+//  * gathers the bonded and pair results in the non-bonded kernel's epilogue (fixed order, no atomics).
 
 namespace oxgb {
 

@@ -235,20 +235,8 @@ OXGB_HD void frame_mirror(const float qh[4], const float ql[4], float b1, float 
 	}
 }
 
-// The remainders of frame_mirror's a1 and backbone offset: a1 = a1_mirror + a1lo and back =
-// back_mirror + backlo to ~2^-46 (the mirrors are recomputed here, bit-identical)
-OXGB_HD void frame_remainders(const float qh[4], const float ql[4], float b1, float b2, float a1lo[3], float backlo[3]) {
-	F2 p1[3], p2[3], p3[3];
-	frame_pairs(qh, ql, p1, p2, p3);
-#pragma unroll
-	for(int k = 0; k < 3; k++) {
-		a1lo[k] = rem2(p1[k], round2(p1[k]));
-		const F2 bk = lin2_pair(b1, p1[k], b2, p2[k]);
-		backlo[k] = rem2(bk, round2(bk));
-	}
-}
-
-// frame_mirror and frame_remainders from one evaluation of the pairs
+// frame_mirror, and the remainders of its a1 and backbone offset: a1 = a1_mirror + a1lo and back = back_mirror +
+// backlo to ~2^-46
 OXGB_HD void frame_mirror_rem(const float qh[4], const float ql[4], float b1, float b2, float a1[3], float a3[3], float back[3],
 		float a1lo[3], float backlo[3]) {
 	F2 p1[3], p2[3], p3[3];

@@ -78,7 +78,8 @@ def md_settings(dt: float = 0.003, verlet_skin: float = 0.05, thermostat: str = 
 
 
 def force_shapes():
-    """the autotuner's shape table: (pair_npw, nb_lanes, nb_min_blocks) of shape 0, 1, ..."""
+    """the autotuner's shape table: (pair_npw, nb_lanes, nb_min_blocks) of shape 0, 1, ...; pair_npw stands for
+    the pair blocks' size, 32 for three groups of 32 nucleotides and 16 for six, from 65,000 nucleotides on"""
     out, k = [], 0
     a, b, c = C.c_int(), C.c_int(), C.c_int()
     while _abi.lib().oxgb_force_shape_table(k, C.byref(a), C.byref(b), C.byref(c)) == 0:
