@@ -189,11 +189,12 @@ int force_shape_range(int N);
 bool force_shape_distinct(int k, int N);
 
 // the blocks of a list build (all zero before the first one), each counter in a line of its own: who takes part
-// (roll, done, members; lists.cu), the members' barrier (count, gen), and the blocks that have left.  After a build
+// (roll, members; lists.cu), the members' barrier (count, gen), and the blocks that have left.  After a build
 // that gave up at a wait the roll stays closed: until the host has cleared this and the cell counts, later builds
 // return at once with OXGB_ERR_SYNC
 struct ListSync {
-	unsigned roll, pad0[31], done, members, pad1[30], count, gen, pad2[30], left, pad3[31];
+	unsigned long long roll, pad0[15];
+	unsigned members, pad1[31], count, gen, pad2[30], left, pad3[31];
 };
 constexpr int LIST_WAIT_POLLS = 4000000;  // some seconds
 constexpr int LIST_MAX_BLOCKS = 1024;   // (roll and left count to 16,383)

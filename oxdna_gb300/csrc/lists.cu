@@ -93,10 +93,16 @@ struct Member {
 	int id, n;
 };
 
-// ListSync::roll: closed | a build gave up | arrivals << 16 | items taken; left: blocks that gave up << 16 | blocks
-constexpr unsigned ROLL_CLOSED = 0x80000000u, ROLL_FAILED = 0x40000000u, ROLL_ONE = 0x10000u;
+// ListSync::roll: closed | a build gave up | arrivals << 32 | items taken << 16 | items done, in one word, so that
+// ending an item and asking for the next is one atomic (as two words, one waits for the other); left: blocks that
+// gave up << 16 | blocks
+typedef unsigned long long Roll;
+constexpr Roll ROLL_CLOSED = 1ull << 63, ROLL_FAILED = 1ull << 62, ROLL_ARRIVED = 1ull << 32, ROLL_TAKEN = 1ull << 16;
+constexpr unsigned LEFT_FAILED = 0x10000u;
 
-__device__ __forceinline__ int roll_arrivals(unsigned roll) { return (int) ((roll & (ROLL_FAILED - 1)) >> 16); }
+__device__ __forceinline__ unsigned roll_arrivals(Roll r) { return (unsigned) (r >> 32) & 0xffffu; }
+__device__ __forceinline__ unsigned roll_taken(Roll r) { return (unsigned) (r >> 16) & 0xffffu; }
+__device__ __forceinline__ unsigned roll_done(Roll r) { return (unsigned) r & 0xffffu; }
 
 // (thread 0) polls *at until it is not `from`; false if the wait ran out
 __device__ __forceinline__ bool poll(const ListArgs &a, const unsigned *at, unsigned from, unsigned &now) {
@@ -118,31 +124,28 @@ __device__ __forceinline__ bool first_phase(const ListArgs &a, volatile Member &
 		return true;
 	}
 	ListSync *y = a.sync;
-	__shared__ unsigned taken;
+	__shared__ Roll roll;
 	__shared__ int ok;
-	unsigned k = 0;
-	if(threadIdx.x == 0) k = atomicAdd(&y->roll, ROLL_ONE + 1);
+	Roll r = 0;
+	if(threadIdx.x == 0) r = atomicAdd(&y->roll, ROLL_ARRIVED + ROLL_TAKEN);
 	meanwhile();
 	if(threadIdx.x == 0) {
-		taken = k;
-		me.id = roll_arrivals(k);
+		roll = r;
+		me.id = (int) roll_arrivals(r);
 		me.n = 0;
 	}
 	__syncthreads();
-	k = taken;
-	if(k & ROLL_CLOSED) return !(k & ROLL_FAILED);
+	if(roll & ROLL_CLOSED) return !(roll & ROLL_FAILED);
 	unsigned closer = 0;  // (thread 0: the members, once this block has closed the roll)
-	for(k &= ROLL_ONE - 1; k < grid; k = taken & (ROLL_ONE - 1)) {
+	for(unsigned k = roll_taken(roll); k < grid; k = roll_taken(roll)) {
 		item((int) k);
-		__syncthreads();  // (everyone has read `taken`, too)
+		__syncthreads();  // (everyone has read `roll`, too)
 		if(threadIdx.x == 0) {
-			unsigned roll, done;
-			asm volatile("atom.add.relaxed.gpu.u32 %0, [%1], 1;" : "=r"(roll) : "l"(&y->roll) : "memory");
-			asm volatile("atom.add.acq_rel.gpu.u32 %0, [%1], 1;" : "=r"(done) : "l"(&y->done) : "memory");
-			taken = roll;
-			if(done == grid - 1) {
+			asm volatile("atom.add.acq_rel.gpu.u64 %0, [%1], %2;" : "=l"(r) : "l"(&y->roll), "l"(ROLL_TAKEN + 1) : "memory");
+			roll = r;
+			if(roll_done(r) == grid - 1) {
 				// (all have arrived, commonly; else nobody may any more)
-				closer = roll_arrivals(roll);
+				closer = roll_arrivals(r);
 				if(closer < grid) closer = roll_arrivals(atomicOr(&y->roll, ROLL_CLOSED));
 				asm volatile("st.release.gpu.u32 [%0], %1;" ::"l"(&y->members), "r"(closer) : "memory");
 			}
@@ -856,12 +859,12 @@ __global__ void __launch_bounds__(LIST_TPB, 1) k_list_build(ListArgs a, int n_ce
 		__threadfence();
 		last = 1;
 		if(gridDim.x > 1) {
-			const unsigned left = atomicAdd(&a.sync->left, whole ? 1u : ROLL_ONE + 1);
-			last = (left & (ROLL_ONE - 1)) == gridDim.x - 1;
+			const unsigned left = atomicAdd(&a.sync->left, whole ? 1u : LEFT_FAILED + 1);
+			last = (left & (LEFT_FAILED - 1)) == gridDim.x - 1;
 			if(last) {
-				if(!whole || left >= ROLL_ONE) last = 0;
+				if(!whole || left >= LEFT_FAILED) last = 0;
 				a.sync->roll = last ? 0 : ROLL_CLOSED | ROLL_FAILED;
-				a.sync->done = a.sync->members = a.sync->count = a.sync->left = 0;
+				a.sync->members = a.sync->count = a.sync->left = 0;
 			}
 		}
 	}
