@@ -62,8 +62,8 @@ WORKLOADS = {
 # dram__bytes_read.sum + dram__bytes_write.sum of k_bonded_pairs + k_nonbonded_mixed per force
 # launch (the MD step's variant, shape 0), from the one-kernel ncu --set full captures
 # summarised in profiles/k_*_{plain40k,large250k}.md (cold caches)
-FORCE_TRAFFIC = {"plain40k": 6.315264e6 + 2.304e3 + 15.066624e6 + 256.0,
-                 "large250k": 30.914048e6 + 9.216e3 + 43.348224e6 + 110.592e3}
+FORCE_TRAFFIC = {"plain40k": 6.315520e6 + 1.792e3 + 15.065600e6 + 0.0,
+                 "large250k": 30.916096e6 + 10.240e3 + 43.346944e6 + 73.984e3}
 
 
 def env_rank():

@@ -68,7 +68,7 @@ __device__ __forceinline__ bool rebuilt(const ListArgs &a, int s) { return !a.sy
 // cooperative launch, which starts all blocks or none, had every build wait for whatever else the GPU ran:
 // 40,000 nucleotides beside one-block kernels of 0.2 and 2 ms on another stream, 214 and 449 us per step
 // (alone 53), a list of 16,000 1,948 us (alone 35); without it 53 to 54, and 37.  So the blocks that run share the
-// work, which takes a build of the whole grid about 1 us more.  The first phase is
+// work, which takes a build of the whole grid 1 to 2 us more.  The first phase is
 // cut into as many items as the grid has blocks, each taken by whichever block asks for one; who asks before
 // the last item is done is a member of the build, and the later phases and their barriers are the members'
 // alone (their number changes no result).  A block that starts later finds the roll closed and leaves.  The
@@ -82,7 +82,7 @@ __device__ __forceinline__ bool rebuilt(const ListArgs &a, int s) { return !a.sy
 //
 // Measured, a rebuild / a step without one, before the one launch and now (us): 24 nucleotides 30 / 21.7 -> 11 / 14;
 // 40,000 duplex nucleotides 75 / 47.7 -> 62 / 38; 250,000 strand nucleotides 230 / 117.5 -> 172 / 107;
-// the plain list of 120,000 (no term lists) 97.3 -> 64.
+// the plain list of 120,000 (no term lists) 97.3 -> 64.7.
 constexpr int LIST_TPB = 1024;
 // shared memory of a block that fills a whole system's cells (system_cells): padded counts, nucleotides
 constexpr int LIST_LOCAL_SMEM = (LIST_LOCAL_CELLS + LIST_LOCAL_CELLS / 16 + 2 + LIST_LOCAL_N) * (int) sizeof(int);
